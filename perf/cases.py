@@ -254,3 +254,53 @@ def tolerance(case):
     if case["kind"] in ("gemv_f32", "gemm_f32", "conv_f32"):
         return {"rel": 2.5e-6}
     return {"rel": 3.6e-3} if case["kind"] == "conv_stage" else {"rel": 8e-4}
+
+
+def _matmul64(a, b_nk):
+    return torch.matmul(a.double(), b_nk.double().transpose(-1, -2))
+
+
+def _conv64(x, w, stride, pad):
+    """NHWC convolution in 64 bits, one matrix product per filter tap."""
+    x, w = x.double(), w.double()
+    n, h, wd, c = x.shape
+    ko, r, s, _ = w.shape
+    ho, wo = (h + 2 * pad - r) // stride + 1, (wd + 2 * pad - s) // stride + 1
+    xp = torch.zeros((n, h + 2 * pad, wd + 2 * pad, c), dtype=torch.float64, device=x.device)
+    xp[:, pad:pad + h, pad:pad + wd] = x
+    out = torch.zeros((n * ho * wo, ko), dtype=torch.float64, device=x.device)
+    for i in range(r):
+        for j in range(s):
+            tap = xp[:, i:i + (ho - 1) * stride + 1:stride, j:j + (wo - 1) * stride + 1:stride]
+            out.addmm_(tap.reshape(-1, c), w[:, i, j].t())
+    return out.view(n, ho, wo, ko)
+
+
+def exact(case, seed):
+    """What `run` returns on the inputs of (case, seed), in 64 bits.  A stage's layers read each other unrounded."""
+    state = prepare(case, seed)
+    kind = state["kind"]
+    if kind in ("gemv", "gemv_f32"):
+        return _matmul64(state["x"], state["w"])
+    if kind == "decode":
+        out = []
+        for l in state["launches"]:
+            a, b, _ = l._refs
+            out.append(_matmul64(b, a) if case["tokens"] <= 8 else _matmul64(a, b))
+        return out
+    if kind == "prefill":
+        return [_matmul64(x, w) for x, w in state["pairs"]]
+    if kind == "gemm":
+        return _matmul64(state["a"], state["b"])
+    if kind in ("bert", "resnet"):
+        return [_matmul64(a, b) if u["kind"] == "gemm" else _conv64(a, b, u["shape"][7], u["shape"][8])
+                for u, (a, b, _) in zip(state["sweep"].units, state["sweep"].tensors)]
+    if kind == "conv_stage":
+        x, out = state["x"], []
+        for l, (_, _, _, pad) in zip(state["launches"], _stage_layers(case)):
+            x = _conv64(x, l._refs[1], 1, pad)
+            out.append(x)
+        return out
+    if kind in ("conv", "conv_f32"):
+        return _conv64(state["x"], state["w"], state["stride"], state["pad"])
+    return torch.matmul(state["a"].double(), state["b"].double())
