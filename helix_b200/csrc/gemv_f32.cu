@@ -96,6 +96,131 @@ gemv_f32_kernel(const float* __restrict__ W, int64_t ldw, const float* __restric
   }
 }
 
+// Streaming kernel, the library's choice where K is not cut: one persistent CTA per SM with an equal share of the rows.
+// A warp owns RB rows at a time over the whole of K (the order of its sums is the one stated above), and every lane
+// streams its 16-byte chunks through a private FIFO of 12 slots in shared memory (cp.async; a lane reads only
+// what it copied, so there are no barriers): 96 KB per SM in flight however many registers the sums take.  The grid of
+// the kernel above is 512 CTAs for 8192 rows, i.e. four on some SMs and three on others.
+constexpr int kStream32Threads = 512;
+constexpr int kStream32Loads = 4;
+constexpr int kStream32Groups = 3;
+constexpr int kStream32RingBytes = kStream32Threads * kStream32Loads * kStream32Groups * 16;
+
+template <int MRHS, int RB>
+__global__ void __launch_bounds__(kStream32Threads, MRHS <= 2 ? 2 : 1)
+gemv_f32_stream_kernel(const float* __restrict__ W, int64_t ldw, const float* X, int64_t ldx, float* Y, int64_t ldy,
+                       int64_t ldy_inner, int rows, int K, int m, int kw) {
+  constexpr int U = kStream32Loads / RB;            // 128-element stretches of K per group
+  constexpr int kWarps = kStream32Threads / 32;
+  constexpr int kStep = U * 128;                    // elements of K per group
+  extern __shared__ __align__(16) unsigned char stream_smem[];
+  __shared__ float part[kWarps][RB * MRHS];
+  griddep_launch_dependents();
+  griddep_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r_begin = static_cast<int>(static_cast<int64_t>(rows) * blockIdx.x / gridDim.x);
+  const int r_end = static_cast<int>(static_cast<int64_t>(rows) * (blockIdx.x + 1) / gridDim.x);
+  const int blocks = (r_end - r_begin + RB - 1) / RB;
+  const uint32_t slot0 = smem_u32(stream_smem) + tid * 16;
+
+  // kw warps share a row block, taking its groups of K in turn (kw = 1: the order stated at the top of this file)
+  const int rw = kWarps / kw, kwi = warp % kw, rwi = warp / kw;
+  int pb = rwi, pk = kwi * kStep, pslot = 0;        // next group to issue: row block, first element
+  auto issue = [&]() {
+    if (pb < blocks && pk < K) {
+      const int row = r_begin + pb * RB;
+      const float* src = W + static_cast<int64_t>(row) * ldw + pk + lane * 4;
+#pragma unroll
+      for (int r = 0; r < RB; ++r)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const bool in = pk + u * 128 + lane * 4 < K && row + r < r_end;
+          cp_async_16_zfill(slot0 + (pslot * kStream32Loads + r * U + u) * kStream32Threads * 16,
+                            in ? src + r * ldw + u * 128 : W, in);
+        }
+      pk += kw * kStep;
+      if (pk >= K) { pk = kwi * kStep; pb += rw; }
+    }
+    cp_async_commit();
+    if (++pslot == kStream32Groups) pslot = 0;
+  };
+#pragma unroll
+  for (int i = 0; i < kStream32Groups; ++i) issue();
+
+  int cslot = 0;
+  for (int sb = 0; sb < blocks; sb += rw) {
+    const int b = sb + rwi;
+    const int r0 = r_begin + b * RB;
+    float acc[RB][MRHS];
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+#pragma unroll
+      for (int i = 0; i < MRHS; ++i) acc[r][i] = 0.0f;
+    for (int k0 = b < blocks ? kwi * kStep : K; k0 < K; k0 += kw * kStep) {
+      // X first: all loads of a group are independent (a right-hand side that does not exist reads the last one)
+      float4 xv[U][MRHS];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int k = min(k0 + u * 128 + lane * 4, K - 4);
+#pragma unroll
+        for (int i = 0; i < MRHS; ++i) xv[u][i] = *reinterpret_cast<const float4*>(X + min(i, m - 1) * ldx + k);
+      }
+      cp_async_wait<kStream32Groups - 1>();
+      float4 wv[RB][U];
+#pragma unroll
+      for (int r = 0; r < RB; ++r)
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(wv[r][u].x), "=f"(wv[r][u].y), "=f"(wv[r][u].z), "=f"(wv[r][u].w)
+                       : "r"(slot0 + (cslot * kStream32Loads + r * U + u) * kStream32Threads * 16)
+                       : "memory");
+      issue();
+      if (++cslot == kStream32Groups) cslot = 0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (k0 + u * 128 + lane * 4 < K) {
+#pragma unroll
+          for (int i = 0; i < MRHS; ++i)
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+              acc[r][i] = fmaf(wv[r][u].x, xv[u][i].x, acc[r][i]);
+              acc[r][i] = fmaf(wv[r][u].y, xv[u][i].y, acc[r][i]);
+              acc[r][i] = fmaf(wv[r][u].z, xv[u][i].z, acc[r][i]);
+              acc[r][i] = fmaf(wv[r][u].w, xv[u][i].w, acc[r][i]);
+            }
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r)
+#pragma unroll
+      for (int i = 0; i < MRHS; ++i) {
+        float v = acc[r][i];
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        if (kw > 1) {
+          if (lane == 0) part[warp][r * MRHS + i] = v;
+        } else if (lane == 0 && r0 + r < r_end && i < m) {
+          Y[i * ldy + static_cast<int64_t>(r0 + r) * ldy_inner] = v;
+        }
+      }
+    if (kw > 1) {                                   // the shares of K in the order of the warps
+      __syncthreads();
+      for (int o = tid; o < rw * RB * MRHS; o += kStream32Threads) {
+        const int grp = o / (RB * MRHS), e = o - grp * (RB * MRHS), r = e / MRHS, i = e - r * MRHS;
+        const int row = r_begin + (sb + grp) * RB + r;
+        if (row < r_end && i < m) {
+          float sum = 0.0f;
+          for (int q = 0; q < kw; ++q) sum += part[grp * kw + q][e];
+          Y[i * ldy + static_cast<int64_t>(row) * ldy_inner] = sum;
+        }
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // Sums the split-K partials in slice order (deterministic).
 __global__ void gemv_f32_splitk_reduce_kernel(const float* __restrict__ partial, float* __restrict__ Y, int64_t ldy,
                                               int64_t ldy_inner, int rows, int m, int split_k) {
@@ -142,6 +267,37 @@ static int launch_gemv32(const float* W, int64_t ldw, const float* X, int64_t ld
   return cudaGetLastError() == cudaSuccess ? HELIX_OK : HELIX_ERR_CUDA;
 }
 
+template <int MRHS, int RB>
+static int launch_stream32(const float* W, int64_t ldw, const float* X, int64_t ldx, float* Y, int64_t ldy,
+                           int64_t ldy_inner, int rows, int K, int m, int kw, int sm_count, cudaStream_t stream,
+                           int64_t* launches) {
+  auto kern = gemv_f32_stream_kernel<MRHS, RB>;
+  static thread_local int attr_dev = -1;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (attr_dev != dev) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kStream32RingBytes) != cudaSuccess)
+      return HELIX_ERR_CUDA;
+    // one CTA of these per SM: what its FIFOs leave of the shared memory is L1 for X, which every row block reads again
+    if (MRHS > 2 && cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 50) != cudaSuccess)
+      return HELIX_ERR_CUDA;
+    attr_dev = dev;
+  }
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(std::min(sm_count, rows));
+  lc.blockDim = dim3(kStream32Threads);
+  lc.dynamicSmemBytes = kStream32RingBytes;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  if (cudaLaunchKernelEx(&lc, kern, W, ldw, X, ldx, Y, ldy, ldy_inner, rows, K, m, kw) != cudaSuccess) return HELIX_ERR_CUDA;
+  ++*launches;
+  return HELIX_OK;
+}
+
 int gemv_f32_launch(const helix_cfg_t* cfg, const float* W, int64_t ldw, const float* X, int64_t ldx, float* Y,
                     int64_t ldy, int64_t ldy_inner, int rows, int K, int m, void* ws, size_t ws_bytes, int sm_count,
                     cudaStream_t stream, int64_t* launches) {
@@ -160,6 +316,26 @@ int gemv_f32_launch(const helix_cfg_t* cfg, const float* W, int64_t ldw, const f
   if (need > 0 && (!ws || ws_bytes < need)) {
     if (own && cfg->split_k > 1) return HELIX_ERR_WORKSPACE;
     split_k = 1;
+  }
+  // short rows of several right-hand sides stay with the kernel above (10000 x 304, m = 2: 5.3 us against 6.7)
+  if (!own && (m == 1 || K >= 512) && (split_k == 1 || (rows >= sm_count && K <= 32768))) {
+    // rows per warp: as many as share one read of X while the warps of an SM still have a block each; where the library
+    // would have cut K (few rows), the warps of a CTA share a row block's K instead
+    const int per_sm = (rows + sm_count - 1) / sm_count;
+#define HELIX_STREAM32(MR, RB, KW) \
+  return launch_stream32<MR, RB>(W, ldw, X, ldx, Y, ldy, ldy_inner, rows, K, m, KW, sm_count, stream, launches)
+    if (split_k > 1) {
+      if (m == 1) HELIX_STREAM32(1, 2, 8);
+      if (m == 2) HELIX_STREAM32(2, 2, 8);
+      if (m <= 4) HELIX_STREAM32(4, 4, 16);
+      HELIX_STREAM32(8, 4, 16);
+    }
+    if (m == 1) { if (per_sm > 32) HELIX_STREAM32(1, 2, 1); HELIX_STREAM32(1, 1, 1); }
+    if (m == 2) { if (per_sm > 32) HELIX_STREAM32(2, 2, 1); HELIX_STREAM32(2, 1, 1); }
+    if (m <= 4) { if (per_sm > 32) HELIX_STREAM32(4, 4, 1); HELIX_STREAM32(4, 2, 1); }
+    if (per_sm > 32) HELIX_STREAM32(8, 4, 1);
+    HELIX_STREAM32(8, 2, 1);
+#undef HELIX_STREAM32
   }
   float* part = static_cast<float*>(ws);
   // tile_n = rows per warp (1 or 2), load_group = 16-byte loads in flight per row and thread (2, 4 or 8)

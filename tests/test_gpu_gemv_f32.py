@@ -68,3 +68,19 @@ def test_gemv_f32_rejects_unaligned_k():
     with pytest.raises(Exception) as e:
         ops.gemv_f32(w, x)
     assert "-2" in str(e.value)
+
+
+@pytest.mark.parametrize("rows,K,m", [(149, 132, 1), (4737, 516, 2), (4800, 520, 3), (9000, 1028, 8), (1185, 2052, 6)])
+def test_streaming_gemv_f32_keeps_the_stated_order_at_its_edges(oracle, rows, K, m):
+    w, x = _data(rows, K, m, rows)
+    got = ops.gemv_f32(torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda()).cpu().numpy()
+    assert np.array_equal(got, oracle.gemv_f32_lane_tree(w, x))
+
+
+@pytest.mark.parametrize("rows,K,m", [(149, 8196, 1), (700, 3000, 2), (300, 2052, 4), (180, 16384, 7)])
+def test_streaming_gemv_f32_shares_k_among_warps_deterministically(rows, K, m):
+    w, x = _data(rows, K, m, K)
+    wd, xd = torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda()
+    a, b = ops.gemv_f32(wd, xd), ops.gemv_f32(wd, xd)
+    assert torch.equal(a, b)
+    util.assert_f32_close(a.cpu().numpy(), x.astype(np.float64) @ w.astype(np.float64).T, f"fp32 GEMV {rows}x{K} m={m}")
