@@ -102,6 +102,7 @@ int dispatch(const helix_launch_t* l, void* status_dev, cudaStream_t stream) {
     if (l->cfg.max_ctas > 0) s = std::max(2, std::min(s, l->cfg.max_ctas));
     return s;
   };
+  const int gemv_order = (l->flags & HELIX_LAUNCH_INDEPENDENT) ? 2 : (l->flags & HELIX_LAUNCH_STATIC_A) ? 1 : 0;
   switch (l->op) {
     case HELIX_OP_GEMM_F16:
       if ((rc = current_device(&info, true)) != HELIX_OK) return rc;
@@ -113,22 +114,15 @@ int dispatch(const helix_launch_t* l, void* status_dev, cudaStream_t stream) {
     case HELIX_OP_GEMV_F16:
       if ((rc = current_device(&info, false)) != HELIX_OK) return rc;
       // Three or more right-hand sides: the SIMT kernel becomes issue bound (measured 11.7 us at
-      // m = 4 and 22 us at m = 8 on 4096 x 4096) while the tcgen05 kernel streams the same weights
-      // in 6.4 us with X as a 128-row A box of which only m rows are fetched.  Taken only for the
-      // library's own configuration, the plain output layout and TMA-compatible operands.
-      if (!cfg && l->M >= 3 && l->M <= 8 && info.cc_major == 10 && l->N >= 1024 && l->K >= 512 &&
-          (l->ldc_inner == 0 || l->ldc_inner == 1) && (l->K % 8) == 0 &&
-          ((l->lda == 0 ? l->K : l->lda) % 8) == 0 && ((l->ldb == 0 ? l->K : l->ldb) % 8) == 0 &&
-          (reinterpret_cast<uintptr_t>(l->a) & 15) == 0 && (reinterpret_cast<uintptr_t>(l->b) & 15) == 0) {
-        rc = helix::gemm_f16_launch(nullptr, l->b, l->ldb, l->a, l->lda, l->c, l->ldc == 0 ? l->N : l->ldc, l->M,
-                                    l->N, l->K, 1, 0, 0, 0, nullptr, 0, static_cast<int*>(status_dev),
-                                    sms_of(info), (l->flags & HELIX_LAUNCH_INDEPENDENT) != 0, stream, &n);
+      // m = 4 and 22 us at m = 8 on 4096 x 4096); the streaming kernel contracts on the matrix units.
+      if (!cfg && l->M >= 3 && l->M <= 8) {
+        rc = helix::gemv_f16_stream_launch(l->a, l->lda, l->b, l->ldb, l->c, l->ldc, l->ldc_inner, l->N, l->K, l->M,
+                                           sms_of(info), gemv_order, stream, &n);
         break;
       }
       rc = helix::gemv_f16_launch(cfg, l->a, l->lda, l->b, l->ldb, l->c, l->ldc, l->ldc_inner, l->N, l->K, l->M,
                                   l->ws, l->ws_bytes, sms_of(info),
-                                  (l->flags & HELIX_LAUNCH_INDEPENDENT) ? 2 : (l->flags & HELIX_LAUNCH_STATIC_A) ? 1 : 0,
-                                  stream, &n);
+                                  gemv_order, stream, &n);
       break;
     case HELIX_OP_CONV_F16: {
       if ((rc = current_device(&info, true)) != HELIX_OK) return rc;

@@ -1571,6 +1571,8 @@ int gemm_f16_launch(const helix_cfg_t* cfg_in, const void* A, int64_t lda, const
   if (cfg_in && cfg_in->tile_m != 0) {
     cfg = *cfg_in;
   } else {
+    if (batch == 1 && gemv_f16_stream_covers(B, ldb, A, lda, N, K, M))
+      return gemv_f16_stream_launch(B, ldb, A, lda, C, ldc, 1, N, K, M, sm_count, independent ? 2 : 0, stream, launches);
     gemm_f16_default_config(M, N, K, batch, sm_count, false, &cfg);
     // the automatic choice degrades to the workspace-free schedule when no scratch was passed
     if (!ws || ws_bytes < gemm_f16_workspace_bytes(&cfg, M, N, K, batch, sm_count)) {

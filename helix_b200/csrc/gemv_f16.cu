@@ -10,6 +10,7 @@
 // Mapping: one warp owns RPW consecutive rows; lane l reads the 16-byte chunk l of each
 // 512-byte row segment, UNROLL segments in flight per row, so a thread keeps RPW*UNROLL
 // independent 128-bit streaming loads outstanding.  Lanes are reduced with a shuffle tree.
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -126,6 +127,337 @@ gemv_f16_kernel(const __half* __restrict__ W, int64_t ldw, const __half* __restr
   if (!waited) griddep_wait();
 }
 
+// ---------------------------------------------------------------------------------------------
+// Streaming kernels: one persistent CTA per SM, an equal share of the rows each.
+//
+// What bounds a GEMV is HBM, and what keeps it from HBM's rate is not the arithmetic but the shape of the grid
+// and the bursts of the loads: with a warp per two rows, 4096 rows are 256 CTAs on 148 SMs (two on some, one
+// on others), and a warp that has issued its batch of loads computes before it issues the next.  Here the
+// rows are cut into sm_count contiguous ranges that differ by at most one row, the 16 warps of a CTA split K (KW of
+// them) and, where K is short, the row blocks (16 / KW groups), and every lane streams its 16-byte chunks through a
+// private FIFO of 12 slots in shared memory (cp.async): a slot is refilled as soon as it has been read, so
+// 96 KB per SM are in flight all the time, no barrier is needed (a lane reads only what it copied itself) and
+// two CTAs fit an SM, so the next launch on the stream can fill its FIFOs while this one drains.
+// Chains of ordered launches on distinct buffers, us before -> after (static weights): 4096 x 4096, m = 1: 9.3 -> 8.2
+// (8.7 -> 7.0), m = 2: 13.6 -> 9.8; 12288 x 4096: 20.6 -> 18.5 (20.6 -> 17.8); 4096 x 11008: 20.1 -> 17.0; m = 4 and 8,
+// 4096 x 4096: 19.5 -> 9.6 and 9.8, 8192 x 8192: 37.5 -> 28.  What is left above the HBM time of the weights is some
+// 2.5 us per launch: the predecessor's completion, the first loads' latency, the last rows' sums.
+constexpr int kStreamThreads = 512;
+constexpr int kStreamWarps = kStreamThreads / 32;
+constexpr int kStreamLoads = 4;      // 16-byte loads of one group
+constexpr int kStreamGroups = 3;     // groups in flight
+constexpr int kStreamRingBytes = kStreamThreads * kStreamLoads * kStreamGroups * 16;
+
+// Rows [begin, end) of this CTA.
+__device__ __forceinline__ void stream_rows(int rows, int& begin, int& end) {
+  begin = static_cast<int>(static_cast<int64_t>(rows) * blockIdx.x / gridDim.x);
+  end = static_cast<int>(static_cast<int64_t>(rows) * (blockIdx.x + 1) / gridDim.x);
+}
+
+__device__ __forceinline__ uint4 lds_16(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gsrc) : "memory");
+}
+
+// One or two right-hand sides, fp32 fused multiply-adds.  A warp takes 256-element chunks of K (16 bytes a
+// lane) of four rows at a time.
+template <int MRHS>
+__global__ void __launch_bounds__(kStreamThreads, 2)
+gemv_f16_stream_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, int64_t ldx, __half* Y,
+                       int64_t ldy, int64_t ldy_inner, int rows, int K, int kw, int order_mode) {
+  constexpr int kBlockRows = kStreamLoads;          // rows per block of a warp
+  constexpr int kSuperRows = kStreamWarps * kBlockRows;
+  extern __shared__ __align__(16) unsigned char stream_smem[];
+  float* part = reinterpret_cast<float*>(stream_smem + kStreamRingBytes);   // [2][kw][MRHS][kSuperRows]
+  griddep_launch_dependents();
+  if (order_mode == 0) griddep_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rw = kStreamWarps / kw;                 // row groups
+  const int kwi = warp % kw, rwi = warp / kw;
+  int r_begin, r_end;
+  stream_rows(rows, r_begin, r_end);
+  const int blocks = (r_end - r_begin + kBlockRows - 1) / kBlockRows;
+  const uint32_t slot0 = smem_u32(stream_smem) + tid * 16;
+
+  // the group that is issued next: row block pb, elements pk ... pk + 7 of this lane
+  const int k_first = kwi * 256 + lane * 8;
+  const int k_step = kw * 256;
+  const int k_limit = (K + 255) / 256 * 256;        // the lanes of a warp leave the chunk loop together
+  int pb = rwi, pk = k_first, pslot = 0;
+  auto issue = [&]() {
+    if (pb < blocks && pk < k_limit) {
+      const int row = r_begin + pb * kBlockRows;
+      const __half* src = W + static_cast<int64_t>(row) * ldw + pk;
+      const bool k_in = pk < K;
+#pragma unroll
+      for (int u = 0; u < kStreamLoads; ++u) {
+        const bool in = k_in && row + u < r_end;
+        cp_async_16_zfill(slot0 + (pslot * kStreamLoads + u) * kStreamThreads * 16, in ? src + u * ldw : W, in);
+      }
+      pk += k_step;
+      if (pk >= k_limit) { pk = k_first; pb += rw; }
+    }
+    cp_async_commit();
+    if (++pslot == kStreamGroups) pslot = 0;
+  };
+#pragma unroll
+  for (int i = 0; i < kStreamGroups; ++i) issue();
+  if (order_mode == 1) griddep_wait();
+
+  int cslot = 0, buf = 0;
+  for (int sb = 0; sb < blocks; sb += kStreamWarps, buf ^= 1) {      // one superblock of up to 64 rows
+    float* p = part + buf * kw * MRHS * kSuperRows;
+    for (int b = sb + rwi; b < min(blocks, sb + kStreamWarps); b += rw) {
+      float acc[kBlockRows][MRHS];
+#pragma unroll
+      for (int r = 0; r < kBlockRows; ++r)
+#pragma unroll
+        for (int i = 0; i < MRHS; ++i) acc[r][i] = 0.0f;
+      for (int kc = kwi * 256; kc < k_limit; kc += k_step) {
+        const int k = kc + lane * 8;
+        uint4 xv[MRHS];
+#pragma unroll
+        for (int i = 0; i < MRHS; ++i)
+          xv[i] = k < K ? *reinterpret_cast<const uint4*>(X + i * ldx + k) : make_uint4(0u, 0u, 0u, 0u);
+        cp_async_wait<kStreamGroups - 1>();
+        uint4 wv[kBlockRows];
+#pragma unroll
+        for (int u = 0; u < kBlockRows; ++u) wv[u] = lds_16(slot0 + (cslot * kStreamLoads + u) * kStreamThreads * 16);
+        issue();
+        if (++cslot == kStreamGroups) cslot = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float2 xf[MRHS];
+#pragma unroll
+          for (int i = 0; i < MRHS; ++i) xf[i] = __half22float2(reinterpret_cast<const __half2*>(&xv[i])[j]);
+#pragma unroll
+          for (int r = 0; r < kBlockRows; ++r) {
+            const float2 wf = __half22float2(reinterpret_cast<const __half2*>(&wv[r])[j]);
+#pragma unroll
+            for (int i = 0; i < MRHS; ++i) {
+              acc[r][i] = fmaf(wf.x, xf[i].x, acc[r][i]);
+              acc[r][i] = fmaf(wf.y, xf[i].y, acc[r][i]);
+            }
+          }
+        }
+      }
+      // four sums over 32 lanes: halve the number of values with the first two exchanges
+#pragma unroll
+      for (int i = 0; i < MRHS; ++i) {
+        const bool hi = lane & 16, mid = lane & 8;
+        float v0 = hi ? acc[2][i] : acc[0][i], v1 = hi ? acc[3][i] : acc[1][i];
+        v0 += __shfl_xor_sync(0xffffffffu, hi ? acc[0][i] : acc[2][i], 16);
+        v1 += __shfl_xor_sync(0xffffffffu, hi ? acc[1][i] : acc[3][i], 16);
+        float v = mid ? v1 : v0;
+        v += __shfl_xor_sync(0xffffffffu, mid ? v0 : v1, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        if ((lane & 7) == 0) p[(kwi * MRHS + i) * kSuperRows + (b - sb) * kBlockRows + (lane >> 3)] = v;
+      }
+    }
+    __syncthreads();
+    // the K slices of every row in slice order; the other buffer takes the next superblock's partial sums
+    const int row0 = r_begin + sb * kBlockRows;
+    if (tid < kSuperRows * MRHS) {
+      const int i = tid / kSuperRows, r = tid - i * kSuperRows;
+      if (row0 + r < r_end) {
+        float s = 0.0f;
+        for (int q = 0; q < kw; ++q) s += p[(q * MRHS + i) * kSuperRows + r];
+        Y[i * ldy + static_cast<int64_t>(row0 + r) * ldy_inner] = __float2half_rn(s);
+      }
+    }
+  }
+  if (order_mode == 2) griddep_wait();
+}
+
+__device__ __forceinline__ void mma_f16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                                uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Three to 8 * NT right-hand sides: the same stream, contracted by warp-level matrix instructions (16 x 8 x 16, fp32
+// accumulation).  The rate they need is small (8 multiply-adds per weight against some 23 bytes of weights per
+// SM and clock); what they save is the issue slots of NT * 8 scalar multiply-adds per weight, and against a
+// 128-row tcgen05 tile they save the quantisation of the rows: a CTA's rows are cut into equal blocks of at most 32,
+// and absent rows cost no traffic.  The fragments need no shuffle: lane (g, t) of a fragment takes the 8
+// consecutive elements at k + 8 t of row g as the K positions 2t, 2t + 1, 2t + 8, 2t + 9 of two instructions, for the
+// weights and for X alike, so every product still meets its partner.  X does not fit the L1 that two resident CTAs
+// leave, so its fragments come from L2 and are fetched one group ahead, which takes registers: 8 warps of up
+// to 128, each with a FIFO of 24 slots (the same 96 KB).
+constexpr int kMmaThreads = 256;
+constexpr int kMmaWarps = kMmaThreads / 32;
+constexpr int kMmaSlots = 24;
+
+template <int NT>
+__global__ void __launch_bounds__(kMmaThreads, 2)
+gemv_f16_mma_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, int64_t ldx, __half* Y, int64_t ldy,
+                    int64_t ldy_inner, int rows, int K, int m, int kw, int order_mode) {
+  constexpr int kMaxRows = 32;                      // rows per block of a warp: two 16-row fragments
+  constexpr int kTok = NT * 8;
+  constexpr int J = 2;                              // 32-element pieces of K per group
+  constexpr int kGroups = kMmaSlots / (4 * J);
+  extern __shared__ __align__(16) unsigned char stream_smem[];
+  float* part = reinterpret_cast<float*>(stream_smem + kMmaThreads * kMmaSlots * 16);   // [warp][kTok][16 rows]
+  griddep_launch_dependents();
+  if (order_mode == 0) griddep_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int rw = kMmaWarps / kw;
+  const int kwi = warp % kw, rwi = warp / kw;
+  int r_begin, r_end;
+  stream_rows(rows, r_begin, r_end);
+  const int n = r_end - r_begin;
+  // equal blocks of at most 32 rows, and where K leaves several row groups at least 16 rows for each
+  const int blocks = max((n + kMaxRows - 1) / kMaxRows, min(rw, (n + 15) / 16));
+  const int height = blocks ? (n + blocks - 1) / blocks : 0;
+  // the kw warps take groups of K in turn: together they read contiguous stretches of every row
+  const int k_begin = kwi * 32 * J, k_step = kw * 32 * J;
+  const uint32_t slot0 = smem_u32(stream_smem) + tid * 16;
+  const uint32_t slot_last = slot0 + (kGroups - 1) * 8 * kMmaThreads * 16;
+
+  // Rows beyond the block read its last row again and right-hand sides beyond m the last one (the same lines; nothing is
+  // written for them), so that only the end of a K that is no multiple of 64 needs predicates.
+  int pb = rwi, pk = k_begin;
+  uint32_t pslot = slot0;
+  const __half* src[4];
+  auto block_rows = [&]() {
+    const int row = pb * height, last = min(height, n - row) - 1;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      src[u] = W + static_cast<int64_t>(r_begin + row + max(0, min(u * 8 + g, last))) * ldw + k_begin + t * 8;
+  };
+  block_rows();
+  auto issue = [&]() {
+    if (pb < blocks && pk < K) {
+      if (pk + 64 <= K) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u * 8 < height) {
+            cp_async_16(pslot + (u * 2) * kMmaThreads * 16, src[u]);
+            cp_async_16(pslot + (u * 2 + 1) * kMmaThreads * 16, src[u] + 32);
+          }
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const bool in = pk + j * 32 + t * 8 < K;
+            cp_async_16_zfill(pslot + (u * 2 + j) * kMmaThreads * 16, in ? src[u] + j * 32 : W, in);
+          }
+      }
+      pk += k_step;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) src[u] += k_step;
+      if (pk >= K) {
+        pk = k_begin;
+        pb += rw;
+        if (pb < blocks) block_rows();
+      }
+    }
+    cp_async_commit();
+    pslot = pslot == slot_last ? slot0 : pslot + 8 * kMmaThreads * 16;
+  };
+#pragma unroll
+  for (int i = 0; i < kGroups; ++i) issue();
+  if (order_mode == 1) griddep_wait();
+
+  const __half* xrow[NT];                           // this lane's right-hand side of each group of eight
+#pragma unroll
+  for (int q = 0; q < NT; ++q) xrow[q] = X + min(q * 8 + g, m - 1) * ldx + t * 8;
+  auto load_x = [&](int k, uint4 (&x)[J][NT]) {
+    if (k + 64 <= K) {
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int q = 0; q < NT; ++q) x[j][q] = *reinterpret_cast<const uint4*>(xrow[q] + k + j * 32);
+    } else {
+#pragma unroll
+      for (int j = 0; j < J; ++j)
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+          x[j][q] = k + j * 32 + t * 8 < K ? *reinterpret_cast<const uint4*>(xrow[q] + k + j * 32)
+                                           : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+  uint32_t cslot = slot0;
+  for (int sb = 0; sb < blocks; sb += rw) {         // one block per row group
+    const int b = sb + rwi;
+    float acc[2][NT][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int q = 0; q < NT; ++q)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[h][q][e] = 0.0f;
+    if (b < blocks) {
+      uint4 xn[J][NT];
+      load_x(k_begin, xn);
+      for (int k = k_begin; k < K; k += k_step) {
+        uint4 xv[J][NT];
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+          for (int q = 0; q < NT; ++q) xv[j][q] = xn[j][q];
+        load_x(k + k_step, xn);
+        cp_async_wait<kGroups - 1>();
+        uint4 wv[4][J];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int j = 0; j < J; ++j) wv[u][j] = lds_16(cslot + (u * J + j) * kMmaThreads * 16);
+        issue();
+        cslot = cslot == slot_last ? slot0 : cslot + 8 * kMmaThreads * 16;
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+              const uint4 w0 = wv[2 * h][j], w1 = wv[2 * h + 1][j];
+              mma_f16_16x8x16(acc[h][q], w0.x, w1.x, w0.y, w1.y, xv[j][q].x, xv[j][q].y);
+              mma_f16_16x8x16(acc[h][q], w0.z, w1.z, w0.w, w1.w, xv[j][q].z, xv[j][q].w);
+            }
+      }
+    }
+    // 16 rows of every row group at a time: partial sums to shared memory, slices added in slice order
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h * 16 < height) {
+        __syncthreads();                            // the previous sums have been read
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            part[(warp * kTok + q * 8 + t * 2 + (e & 1)) * 16 + g + (e >> 1) * 8] = acc[h][q][e];
+        __syncthreads();
+        for (int o = tid; o < rw * kTok * 16; o += kMmaThreads) {
+          const int r16 = o & 15, tok = (o >> 4) % kTok, grp = (o >> 4) / kTok;
+          const int r = h * 16 + r16, row = (sb + grp) * height + r;
+          if (tok < m && r < height && sb + grp < blocks && row < n) {
+            float s = 0.0f;
+            for (int q = 0; q < kw; ++q) s += part[((grp * kw + q) * kTok + tok) * 16 + r16];
+            Y[tok * ldy + static_cast<int64_t>(r_begin + row) * ldy_inner] = __float2half_rn(s);
+          }
+        }
+      }
+    }
+  }
+  if (order_mode == 2) griddep_wait();
+}
+
 // Sums the split-K partials in slice order (deterministic) and rounds once.
 __global__ void gemv_splitk_reduce_kernel(const float* __restrict__ partial, __half* __restrict__ Y, int64_t ldy,
                                           int64_t ldy_inner, int rows, int m, int split_k) {
@@ -218,6 +550,77 @@ static int launch_gemv_variant(int rpw, int unroll, const __half* W, int64_t ldw
   return HELIX_ERR_UNSUPPORTED;
 }
 
+// Warps that split K: a power of two with at least `unit` elements of K for each.
+static int stream_k_warps(int K, int unit, int warps) {
+  int kw = warps;
+  while (kw > 1 && (int64_t)(kw / 2) * unit >= K) kw /= 2;
+  return kw;
+}
+
+template <typename... Params, typename... Args>
+static int launch_stream(void (*kern)(Params...), int& attr_dev, int grid, int threads, int smem, cudaStream_t stream,
+                         int64_t* launches, Args... args) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (attr_dev != dev) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return HELIX_ERR_CUDA;
+    attr_dev = dev;
+  }
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(threads);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  if (cudaLaunchKernelEx(&lc, kern, args...) != cudaSuccess) return HELIX_ERR_CUDA;
+  ++*launches;
+  return HELIX_OK;
+}
+
+int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y, int64_t ldy,
+                           int64_t ldy_inner, int rows, int K, int m, int sm_count, int order_mode,
+                           cudaStream_t stream, int64_t* launches) {
+  if (!W || !X || !Y || rows <= 0 || K <= 0 || m <= 0 || m > 16) return HELIX_ERR_INVALID;
+  if (ldw == 0) ldw = K;
+  if (ldx == 0) ldx = K;
+  if (ldy == 0) ldy = rows;
+  if (ldy_inner == 0) ldy_inner = 1;
+  if ((K & 7) || (ldw & 7) || (ldx & 7) || (reinterpret_cast<uintptr_t>(W) & 15) ||
+      (reinterpret_cast<uintptr_t>(X) & 15))
+    return HELIX_ERR_ALIGN;
+  const __half* w = static_cast<const __half*>(W);
+  const __half* x = static_cast<const __half*>(X);
+  __half* y = static_cast<__half*>(Y);
+  const int grid = std::min(sm_count, rows);
+  static thread_local int attr_dev[4] = {-1, -1, -1, -1};   // device the kernel's shared-memory size was last raised on
+  if (m <= 2) {
+    const int kw = stream_k_warps(K, 256, kStreamWarps);
+    const int smem = kStreamRingBytes + 2 * kStreamWarps * m * kStreamWarps * kStreamLoads * 4;
+    if (m == 1)
+      return launch_stream(gemv_f16_stream_kernel<1>, attr_dev[0], grid, kStreamThreads, smem, stream, launches, w, ldw, x, ldx, y, ldy,
+                           ldy_inner, rows, K, kw, order_mode);
+    return launch_stream(gemv_f16_stream_kernel<2>, attr_dev[1], grid, kStreamThreads, smem, stream, launches, w, ldw, x, ldx, y, ldy,
+                         ldy_inner, rows, K, kw, order_mode);
+  }
+  const int kw = stream_k_warps(K, 64, kMmaWarps);
+  const int smem = kMmaThreads * kMmaSlots * 16 + kMmaWarps * (m <= 8 ? 8 : 16) * 16 * 4;
+  if (m <= 8)
+    return launch_stream(gemv_f16_mma_kernel<1>, attr_dev[2], grid, kMmaThreads, smem, stream, launches, w, ldw, x, ldx, y,
+                         ldy, ldy_inner, rows, K, m, kw, order_mode);
+  return launch_stream(gemv_f16_mma_kernel<2>, attr_dev[3], grid, kMmaThreads, smem, stream, launches, w, ldw, x, ldx, y, ldy,
+                       ldy_inner, rows, K, m, kw, order_mode);
+}
+
+bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m) {
+  return m >= 1 && m <= 16 && rows >= 1024 && K >= 512 && (K & 7) == 0 && ((ldw ? ldw : K) & 7) == 0 &&
+         ((ldx ? ldx : K) & 7) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
+         (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+}
+
 int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y,
                     int64_t ldy, int64_t ldy_inner, int rows, int K, int m, void* ws, size_t ws_bytes,
                     int sm_count, int order_mode, cudaStream_t stream, int64_t* launches) {
@@ -237,6 +640,13 @@ int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const vo
                                                               : gemv_f16_default_split(rows, K, sm_count);
   if (split_k > 1 && (K + split_k - 1) / split_k < 256) split_k = 1;
   const size_t need = gemv_f16_workspace_bytes(rows, m, split_k);
+  // The streaming kernel needs no partial sums in memory and cuts K among the warps of a CTA, so it also takes row counts
+  // for which the kernel above would split K over CTAs (700 x 12000: 11.9 -> 6.7 us, ordered launches).  Below 2 M
+  // elements a lone launch is all latency and the plain grid is shorter (256 x 256: 1.4 against 1.9 us); with K beyond
+  // 32768 and few rows the split keeps more SMs equally busy.
+  if (!(cfg && cfg->tile_m != 0) && m <= 2 && (int64_t)rows * K >= (1 << 21) &&
+      (split_k == 1 || (rows >= sm_count && K <= 32768)))
+    return gemv_f16_stream_launch(W, ldw, X, ldx, Y, ldy, ldy_inner, rows, K, m, sm_count, order_mode, stream, launches);
   if (need > 0 && (!ws || ws_bytes < need)) {
     if (cfg && cfg->tile_m != 0 && cfg->split_k > 1) return HELIX_ERR_WORKSPACE;
     split_k = 1;  // automatic choice falls back to the workspace-free variant

@@ -14,6 +14,13 @@ int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const vo
                     int64_t ldy, int64_t ldy_inner, int rows, int K, int m, void* ws, size_t ws_bytes,
                     int sm_count, int order_mode, cudaStream_t stream, int64_t* launches);
 
+// Streaming kernels for up to 16 right-hand sides (no scratch); order_mode as above.
+int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y, int64_t ldy,
+                           int64_t ldy_inner, int rows, int K, int m, int sm_count, int order_mode,
+                           cudaStream_t stream, int64_t* launches);
+// Skinny products the streaming kernels take from the tcgen05 tiles: 16-byte-aligned operands, enough rows for the SMs.
+bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m);
+
 // Variant with the split-K partials in an array that is part of the library image.
 size_t gemv_f16_static_capacity_floats();
 int gemv_f16_static_launch(const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y, int64_t ldy,

@@ -98,11 +98,20 @@ def default_config(launch):
 
 def kernel_name(launch):
     """Name of the main kernel `launch` resolves to, as a profiler lists it."""
-    c = launch.cfg if launch.cfg.tile_n or launch.cfg.tile_m else default_config(launch)
+    own = launch.cfg.tile_n or launch.cfg.tile_m
+    c = launch.cfg if own else default_config(launch)
+    # the library's own choice streams (the rules of gemv_f16_launch, gemv_f32_launch and gemv_f16_stream_covers)
+    streams = not own and (c.split_k <= 1 or (launch.N >= device_info().sm_count and launch.K <= 32768))
     if launch.op == _lib.OP_GEMV_F16:
-        return "gemv_f16_kernel"
+        if not own and launch.M >= 3:
+            return "gemv_f16_mma_kernel<1>"
+        return "gemv_f16_stream_kernel<%d>" % launch.M if streams and launch.N * launch.K >= 1 << 21 else "gemv_f16_kernel"
     if launch.op == _lib.OP_GEMV_F32:
-        return "gemv_f32_kernel"
+        return "gemv_f32_stream_kernel" if streams and (launch.M == 1 or launch.K >= 512) else "gemv_f32_kernel"
+    if launch.op == OP_GEMM_F16 and not own and launch.batch <= 1 and launch.M <= 16 and launch.N >= 1024 and launch.K >= 512:
+        if launch.M <= 2:
+            return "gemv_f16_stream_kernel<%d>" % launch.M
+        return "gemv_f16_mma_kernel<%d>" % (1 if launch.M <= 8 else 2)
     if launch.op == _lib.OP_GEMM_F32:
         return "sgemm_f32_kernel<%d,%d>" % (c.tile_m, c.tile_n)
     if c.cta_group == 2:

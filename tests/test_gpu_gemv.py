@@ -89,3 +89,40 @@ def test_gemv_launch_ordering_flags_do_not_change_results(oracle, flag):
         assert torch.equal(o, ref)
     _, ref32 = oracle.hgemm_naive(x, w)
     util.assert_f16_close(ref.cpu().numpy(), ref32, "gemv flags")
+
+
+@pytest.mark.parametrize("rows,K,m", [(149, 16392, 1), (2048, 1032, 2), (1185, 2056, 1), (9473, 296, 2), (5, 72, 3),
+                                      (4885, 520, 8), (300, 4104, 5), (148, 64, 4), (2100, 504, 7)])
+def test_streaming_gemv_at_the_edges_of_its_row_and_k_blocks(oracle, rows, K, m):
+    """One row more than SMs, K that leaves part of a chunk, a stretch or a warp's share, blocks of fewer rows than a
+    fragment; every right-hand-side count class; plain, static and independent launches bit-identical."""
+    w, x = datagen.c2_gemv(rows, K, m, seed=rows + K)
+    got = _run(w, x)
+    _, ref32 = oracle.hgemm_naive(x, w)
+    util.assert_f16_close(got, ref32, f"streaming gemv {rows}x{K} m={m}")
+    assert np.array_equal(_run(w, x, transposed=True), got)
+    wd, xd = torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda()
+    for flag in (1, 2):
+        out = torch.full((m, rows), float("nan"), dtype=torch.float16, device="cuda")
+        l = ops.launch_gemv_f16(wd, xd, out)
+        l.flags = flag
+        ops.run(l)
+        assert np.array_equal(out.cpu().numpy(), got)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 512), (2, 1025, 520), (3, 1191, 1000), (9, 1024, 520), (16, 5003, 536)])
+def test_skinny_gemm_through_the_streaming_kernel(oracle, M, N, K):
+    """Up to 16 rows of A: strided operands and output, odd N, a K that is no multiple of 64; unaligned rows keep failing."""
+    w, x = datagen.c2_gemv(N, K, M, seed=M + N)
+    a = torch.full((M, K + 8), float("nan"), dtype=torch.float16, device="cuda")
+    b = torch.full((N, K + 16), float("nan"), dtype=torch.float16, device="cuda")
+    out = torch.full((M, N + 3), 7.0, dtype=torch.float16, device="cuda")
+    a[:, :K], b[:, :K] = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    ops.run(ops.launch_gemm_f16(a[:, :K], b[:, :K], out[:, :N]))
+    torch.cuda.synchronize()
+    _, ref32 = oracle.hgemm_naive(x, w)
+    util.assert_f16_close(out[:, :N].cpu().numpy(), ref32, f"skinny gemm {M}x{N}x{K}")
+    assert torch.all(out[:, N:] == 7.0)
+    with pytest.raises(Exception) as e:
+        ops.run(ops.launch_gemm_f16(a[:, 1:K - 7], b[:, :K - 8], out[:, :N]))
+    assert "-2" in str(e.value)
