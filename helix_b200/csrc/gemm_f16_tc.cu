@@ -471,14 +471,14 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 fast_divmod(kb, p.fd_cblocks, tap, cb);
                 fast_divmod(tap, p.fd_s, fr, fs);
                 if (p.swap) {
-                  if (load_a) tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, kb * kBK, w.m_blk * kBM, 0);
+                  if (load_a) tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK, tap, w.m_blk * kBM);
                   if (load_b) tma_load_im2col_4d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK,
                                                  pix_w, pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
                 } else {
                   if (load_a) tma_load_im2col_4d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK,
                                                  pix_w, pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
-                  if (load_b) tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, kb * kBK,
-                                          w.n_blk * BN, w.b);
+                  if (load_b) tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK, tap,
+                                          w.n_blk * BN);
                 }
               } else {
                 if (load_a) tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, kb * kBK, w.m_blk * kBM, w.b);
@@ -486,19 +486,19 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                                         w.n_blk * BN, w.b);
               }
             } else if (p.im2col) {
-              // K is ordered (r, s, c): slab kb is filter tap kb / cblocks, channels 64 * (kb % cblocks)
+              // K is ordered (r, s, c): slab kb is filter tap kb / cblocks, channels from 64 * (kb % cblocks); channels
+              // beyond C arrive as zeros on both sides (weights through a map of channel, tap, output channel)
               int tap, cb, fr, fs;
               fast_divmod(kb, p.fd_cblocks, tap, cb);
               fast_divmod(tap, p.fd_s, fr, fs);
               if (p.swap) {   // weights on the 128-row axis, BN pixels per im2col box on the other
-                tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, kb * kBK, w.m_blk * kBM, 0);
+                tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK, tap, w.m_blk * kBM);
                 tma_load_im2col_4d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK, pix_w,
                                    pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
               } else {
                 tma_load_im2col_4d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK, pix_w,
                                    pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
-                tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, kb * kBK, w.n_blk * BN,
-                            w.b);
+                tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK, tap, w.n_blk * BN);
               }
             } else {
               tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, kb * kBK, w.m_blk * kBM, w.b);
@@ -975,32 +975,32 @@ static EncodeTiledFn get_encode_fn() {
 struct TmapKey {
   const void* base;
   int64_t K, rows, batch, ld, bs;
-  int box_rows;
+  int box_rows, box_batch;
   bool operator==(const TmapKey& o) const {
     return base == o.base && K == o.K && rows == o.rows && batch == o.batch && ld == o.ld && bs == o.bs &&
-           box_rows == o.box_rows;
+           box_rows == o.box_rows && box_batch == o.box_batch;
   }
 };
 struct TmapKeyHash {
   size_t operator()(const TmapKey& k) const {
     size_t h = reinterpret_cast<size_t>(k.base);
     auto mix = [&h](int64_t v) { h ^= (size_t)v + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2); };
-    mix(k.K); mix(k.rows); mix(k.batch); mix(k.ld); mix(k.bs); mix(k.box_rows);
+    mix(k.K); mix(k.rows); mix(k.batch); mix(k.ld); mix(k.bs); mix(k.box_rows); mix(k.box_batch);
     return h;
   }
 };
 
 // K-major fp16 matrix [batch][rows][K] with leading dimension ld and batch stride bs (elements);
-// box = 64 halves x box_rows x 1, 128-byte swizzle, out-of-bounds elements read as zero.
+// box = 64 halves x box_rows x box_batch, 128-byte swizzle, out-of-bounds elements read as zero.
 static int make_tmap(CUtensorMap* map, const void* base, int64_t K, int64_t rows, int64_t batch, int64_t ld, int64_t bs,
-                     int box_rows) {
+                     int box_rows, int box_batch = 1) {
   EncodeTiledFn fn = get_encode_fn();
   if (!fn) return HELIX_ERR_CUDA;
   if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld & 7) || (batch > 1 && (bs & 7))) return HELIX_ERR_ALIGN;
   if (batch <= 1) bs = rows * ld;
   static std::mutex mu;
   static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> cache;
-  const TmapKey key{base, K, rows, batch, ld, bs, box_rows};
+  const TmapKey key{base, K, rows, batch, ld, bs, box_rows, box_batch};
   {
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
@@ -1011,7 +1011,7 @@ static int make_tmap(CUtensorMap* map, const void* base, int64_t K, int64_t rows
   }
   cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)std::max<int64_t>(batch, 1)};
   cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)bs * 2};
-  cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, 1};
+  cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, (cuuint32_t)box_batch};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1041,12 +1041,19 @@ static EncodeIm2colFn get_encode_im2col_fn() {
   return fn;
 }
 
-// The im2col path needs whole 64-channel blocks per filter tap (one 128-byte swizzled row per
-// pixel), window parameters inside the tensor map's field widths, and an activation tensor of
-// at least 128 KiB (smaller ones stay on the gathering kernel, as do all other geometries).
+// The im2col path reads 64-channel blocks of one filter tap (one 128-byte swizzled row per pixel; the last block of a
+// C that is no multiple of 64 is filled with zeros, on the weights' side too), and needs window parameters inside the
+// tensor map's field widths and an activation tensor of at least 128 KiB (smaller ones stay on the gathering kernel, as
+// do all other geometries).  Filled channels cost a slab as much as real ones, and rows of pixels that do not start on
+// 64-byte boundaries arrive more slowly, so the map is used up to 4/3 of the real channels where C is a multiple of 32,
+// and from 96 channels on up to 6/5 otherwise; measured against gathering (us): 3 x 3, C = 96, 28 x 28 x 16: 9.8 / 12.3;
+// C = 328, stride 2: 20.4 / 22.5; C = 504: 23.9 / 28.4; but C = 56: 10.6 / 10.0, C = 200: 22.9 / 21.2,
+// C = 88: 15.8 / 11.7, C = 40, 5 x 5: 28.5 / 13.5.
 static bool conv_im2col_eligible(const ConvGeom& g) {
   const int64_t bytes = (int64_t)g.NB * g.H * g.W * g.C * 2;
-  return (g.C % kBK) == 0 && g.stride >= 1 && g.stride <= 8 && g.pad <= 127 && g.R <= 128 && g.S <= 128 &&
+  const int filled = (g.C + kBK - 1) / kBK * kBK;
+  const bool worth = g.C % 32 == 0 ? filled * 3 <= g.C * 4 : filled * 5 <= g.C * 6 && g.C >= 96;
+  return (g.C % 8) == 0 && worth && g.stride >= 1 && g.stride <= 8 && g.pad <= 127 && g.R <= 128 && g.S <= 128 &&
          g.pad - (g.R - 1) >= -128 && g.pad - (g.S - 1) >= -128 && bytes >= 131072 && g.C <= 65535 &&
          get_encode_im2col_fn() != nullptr;
 }
@@ -1096,6 +1103,14 @@ static int make_tmap_im2col(CUtensorMap* map, const void* x, const ConvGeom& g, 
   cache.emplace(key, *map);
   return HELIX_OK;
 }
+
+// Weights w[KO][R][S][C] as a map of (channel, tap, output channel): one box is 64 channels of one tap for `rows` output
+// channels, laid out as the K-major tile the MMAs read.
+static int make_tmap_filter(CUtensorMap* map, const void* w, const ConvGeom& g, int rows) {
+  const int taps = g.R * g.S;
+  return make_tmap(map, w, g.C, taps, g.KO, g.C, (int64_t)taps * g.C, 1, rows);
+}
+static int im2col_k(const ConvGeom& g) { return g.R * g.S * ((g.C + kBK - 1) / kBK * kBK); }
 
 static const int kTileNs[] = {256, 128, 64, 32, 16};
 constexpr int kNumTileNs = sizeof(kTileNs) / sizeof(kTileNs[0]);
@@ -1306,7 +1321,7 @@ void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) 
   if (g.R == 1 && g.S == 1 && g.stride == 1 && g.pad == 0)
     default_config_impl(M, g.KO, K, 1, sm_count, false, true, out);
   else if (conv_im2col_eligible(g)) {
-    default_config_impl(M, g.KO, K, 1, sm_count, false, false, out);
+    default_config_impl(M, g.KO, im2col_k(g), 1, sm_count, false, false, out);
     // A 128 x N x 16 step costs max(N / 2 cycles of pipe time, (128 + N) / 4 cycles of operand fetch from shared
     // memory): the wide tile does twice the work of a 128-wide one in 1.5x the fetch time, so 65..128 output channels
     // are better spent as the 128 rows with 256 pixels per step: measured 17.1 -> 13.9 us on 3x3, 128 -> 128
@@ -1334,6 +1349,12 @@ void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) 
     out->conv_gather = 4;
   }
   out->op = HELIX_OP_CONV_F16;
+}
+
+// The reduction length of the implicit GEMM as the kernel walks it (whole 64-channel blocks on the im2col path).
+int64_t conv_f16_gemm_k(const ConvGeom& g) {
+  const bool as_gemm = g.R == 1 && g.S == 1 && g.stride == 1 && g.pad == 0;
+  return !as_gemm && conv_im2col_eligible(g) ? (int64_t)im2col_k(g) : (int64_t)g.R * g.S * g.C;
 }
 
 // Stream-K decomposition of `tiles` tiles over `grid` CTAs.
@@ -1524,7 +1545,7 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   p.fd_num_kb = make_fastdiv(p.num_kb);
   p.fd_howo = make_fastdiv((conv || p.im2col) ? p.g.Ho * p.g.Wo : 1);
   p.fd_wo = make_fastdiv((conv || p.im2col) ? p.g.Wo : 1);
-  p.fd_cblocks = make_fastdiv(p.im2col ? p.g.C / kBK : 1);
+  p.fd_cblocks = make_fastdiv(p.im2col ? (p.g.C + kBK - 1) / kBK : 1);
   p.fd_s = make_fastdiv(p.im2col ? p.g.S : 1);
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
@@ -1652,7 +1673,7 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     cfg = *cfg_in;
   } else {
     conv_f16_default_config(g, sm_count, &cfg);
-    if (!ws || ws_bytes < gemm_f16_workspace_bytes(&cfg, M, N, K, 1, sm_count)) {
+    if (!ws || ws_bytes < gemm_f16_workspace_bytes(&cfg, M, N, (int)conv_f16_gemm_k(g), 1, sm_count)) {
       cfg.stream_k = 0;
       cfg.split_k = 1;
     }
@@ -1666,14 +1687,14 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     GemmParams ps{};
     ps.PM = N;
     ps.PN = M;
-    ps.K = K;
+    ps.K = im2col_k(g);
     ps.batch = 1;
     ps.status = status_dev;
     ps.g = g;
     ps.im2col = 1;
     CUtensorMap tw, tx;
     int rcs;
-    if ((rcs = make_tmap(&tw, w, K, N, 1, K, 0, kBM)) != HELIX_OK) return rcs;
+    if ((rcs = make_tmap_filter(&tw, w, g, kBM)) != HELIX_OK) return rcs;
     if ((rcs = make_tmap_im2col(&tx, x, g, cfg.tile_n)) != HELIX_OK) return rcs;
     return launch_common(cfg, false, tw, tx, ps, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
   }
@@ -1687,14 +1708,16 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
   p.g = g;
   CUtensorMap ta, tb;
   int rc;
-  if ((rc = make_tmap(&tb, w, K, N, 1, K, 0, cfg.tile_n)) != HELIX_OK) return rc;
   if (im2col) {
     // Same kernel as a GEMM: the one producer thread asks the im2col map for 128 pixels x 64
     // channels of one filter tap per K slab.
     if ((rc = make_tmap_im2col(&ta, x, g, kBM)) != HELIX_OK) return rc;
+    if ((rc = make_tmap_filter(&tb, w, g, cfg.tile_n)) != HELIX_OK) return rc;
+    p.K = im2col_k(g);
     p.im2col = 1;
     return launch_common(cfg, false, ta, tb, p, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
   }
+  if ((rc = make_tmap(&tb, w, K, N, 1, K, 0, cfg.tile_n)) != HELIX_OK) return rc;
   return launch_common(cfg, true, tb, tb, p, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
 }
 

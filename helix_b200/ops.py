@@ -125,9 +125,17 @@ def kernel_name(launch):
         if rows_geom and c.conv_gather == 4:    # explicit, or the library's default for this geometry
             return "conv_f16_rows_kernel"
         as_gemm = r == 1 and s == 1 and stride == 1 and pad == 0
-        im2col = ch % 64 == 0 and n * h * w * ch * 2 >= 131072 and stride <= 8 and not c.conv_gather
+        im2col = conv_reads_tensor_map(n, h, w, ch, stride) and not c.conv_gather
         gathers = not as_gemm and not im2col
     return "gemm_f16_tc_kernel<%d,%d>" % (c.tile_n, 1 if gathers else 0)
+
+
+def conv_reads_tensor_map(n, h, w, ch, stride):
+    """True where the implicit GEMM fetches its input through the im2col tensor map (conv_im2col_eligible in
+    csrc/gemm_f16_tc.cu): the channels a 64-channel block is filled up with must be few."""
+    filled = (ch + 63) // 64 * 64
+    few = filled * 3 <= ch * 4 if ch % 32 == 0 else filled * 5 <= ch * 6 and ch >= 96
+    return ch % 8 == 0 and few and n * h * w * ch * 2 >= 131072 and stride <= 8
 
 
 def make_cfg(op, tile_m=128, tile_n=128, tile_k=64, stages=0, cta_group=1, split_k=1, swap_ab=0, raster=8,

@@ -352,3 +352,28 @@ def test_conv_f32_workspace_contract():
     l1 = ops.launch_conv2d_f32(torch.rand((1, 6, 6, 8), device="cuda"), torch.rand((4, 1, 1, 8), device="cuda"),
                                torch.empty((1, 6, 6, 4), device="cuda"), 1, 0)
     assert load().helix_workspace_bytes(ctypes.byref(l1)) == 256  # 1x1: only the transposed weights (8 x 4 floats)
+
+
+@pytest.mark.parametrize("geom", [
+    (3, 96, 26, 26, 136, 5, 5, 1, 2),     # half a block beyond one, pixels on 64-byte boundaries
+    (2, 160, 21, 23, 64, 3, 3, 2, 1),     # two blocks and a half, stride 2
+    (4, 120, 19, 19, 40, 3, 3, 1, 1),     # 56 of 64 channels in the last block, 240-byte pixels
+    (2, 184, 20, 20, 96, 1, 1, 2, 0),     # one tap
+    (21, 112, 28, 28, 72, 3, 3, 1, 1),    # enough pixels for the operand-swapped tile
+])
+def test_conv_im2col_map_fills_the_last_channel_block(oracle, geom):
+    B, C, H, W, OC, kh, kw, stride, pad = geom
+    assert C % 64 != 0 and ops.conv_reads_tensor_map(B, H, W, C, stride)
+    x, w = datagen.c4_conv(*geom, seed=31)
+    got = _run(x, w, stride, pad)
+    n = min(B, 3)                          # the oracle is slow: first images
+    _, y32 = oracle.conv2d_nhwc_f16(np.ascontiguousarray(x[:n]), w, stride, pad)
+    util.assert_f16_close(got[:n], y32, f"conv {geom}")
+    # the gathering producer sums the same products in slabs of other limits: the last image as well
+    gather = _run(x, w, stride, pad, ops.make_cfg(OP_CONV_F16, tile_m=128, tile_n=128, tile_k=64, conv_gather=1))
+    util.assert_f16_close(got[-1], gather[-1].astype(np.float32), f"conv {geom} against gathering")
+    # a channel that does not exist must not meet an infinite weight of the next tap
+    w[:, -1, -1, 0] = np.inf
+    x[:] = 1.0
+    y = _run(x, w, stride, pad)
+    assert not np.isnan(y[:, :-2, :-2]).any()        # (beyond, the tap lies in the padding: 0 x inf)
