@@ -1,4 +1,4 @@
-// True-fp32 NHWC convolution = column matrix + FFMA GEMM.
+// True-fp32 NHWC convolution: implicit GEMM on the ring kernel, or column matrix + FFMA GEMM.
 //
 // The reference's fp32 convolution is an explicit im2col (src_template/Ampere_FP32/im2col.cu:37-97,
 // NCHW) followed by its SIMT GEMM on M = B*Ho*Wo, N = OC, K = IC*kH*kW
@@ -8,8 +8,11 @@
 // y[M][KO] = col x wt with its usual guarantee (every output one fmaf chain over ascending k).  A
 // 1x1, stride-1, unpadded convolution uses x itself as the column matrix.  Both matrices live in the
 // caller's workspace.
-#include "common.cuh"
-#include "kernels.h"
+//
+// Filters of up to 32 taps on images of less than 2^31 elements form the column matrix only in shared memory: the ring
+// kernel's loader gathers the windows and transposes the filters (same order of k, the same bits), which saves the
+// write and the reads of a matrix R * S times the input's size and two launches.
+#include "sgemm_f32_ring.cuh"
 
 namespace helix {
 
@@ -81,6 +84,42 @@ size_t conv_f32_workspace_bytes(const ConvGeom& g) {
   return col + align256((size_t)K * g.KO * sizeof(float));
 }
 
+template <typename T>
+static int launch_implicit(const RingParams& p, bool as_gemm, cudaStream_t stream) {
+  // 16-byte chunks of four channels where every pixel starts on 16 bytes (not on the widest tile, see launch_any of the GEMM)
+  const bool x16 = (p.Cin & 3) == 0 && (reinterpret_cast<uintptr_t>(p.A) & 15) == 0;
+  if constexpr (T::BM * T::BN <= 8192)
+    if (x16) return as_gemm ? launch_ring<T, kRows16, kRows4>(p, stream) : launch_ring<T, kWindow16, kRows4>(p, stream);
+  return as_gemm ? launch_ring<T, kRows4, kRows4>(p, stream) : launch_ring<T, kWindow4, kRows4>(p, stream);
+}
+
+// HELIX_ERR_UNSUPPORTED where the ring kernel does not cover the call (a tile it has no loader for).
+static int conv_f32_implicit(const helix_cfg_t* cfg, const float* x, const float* w, float* y, const ConvGeom& g, int M,
+                             int K, bool as_gemm, int sm_count, cudaStream_t stream) {
+  if (K >= (1 << 23)) return HELIX_ERR_UNSUPPORTED;
+  helix_cfg_t c{};
+  if (cfg && cfg->tile_m != 0) c = *cfg;
+  else sgemm_f32_default_config(M, g.KO, sm_count, &c);
+  if (c.stages < 3) return HELIX_ERR_UNSUPPORTED;
+  RingParams p{};
+  p.A = x; p.B = w; p.C = y;
+  p.lda = g.C; p.ldb = K; p.ldc = g.KO;
+  p.M = M; p.N = g.KO; p.K = K;
+  p.vec_c = (g.KO & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+  p.H = g.H; p.W = g.W; p.Cin = g.C; p.S = g.S; p.R = g.R; p.stride = g.stride; p.pad = g.pad;
+  p.fd_c = make_fastdiv(g.C);
+  p.fd_s = make_fastdiv(g.S);
+  p.fd_wo = make_fastdiv(g.Wo);
+  p.fd_ho = make_fastdiv(g.Ho);
+  const int bm = c.tile_m, bn = c.tile_n, bk = c.tile_k ? c.tile_k : 16;
+  if (bm == 128 && bn == 128 && bk == 16) return launch_implicit<RingTile128x128>(p, as_gemm, stream);
+  if (bm == 128 && bn == 64 && bk == 16) return launch_implicit<RingTile128x64>(p, as_gemm, stream);
+  if (bm == 64 && bn == 64 && bk == 16) return launch_implicit<RingTile64x64>(p, as_gemm, stream);
+  if (bm == 32 && bn == 64 && bk == 16) return launch_implicit<RingTile32x64>(p, as_gemm, stream);
+  if (bm == 32 && bn == 32 && bk == 32) return launch_implicit<RingTile32x32>(p, as_gemm, stream);
+  return HELIX_ERR_UNSUPPORTED;
+}
+
 int conv_f32_launch(const helix_cfg_t* cfg, const float* x, const float* w, float* y, const ConvGeom& g, void* ws,
                     size_t ws_bytes, int sm_count, cudaStream_t stream, int64_t* launches) {
   if (!x || !w || !y || g.NB <= 0 || g.H <= 0 || g.W <= 0 || g.C <= 0 || g.KO <= 0 || g.R <= 0 || g.S <= 0 ||
@@ -93,6 +132,11 @@ int conv_f32_launch(const helix_cfg_t* cfg, const float* x, const float* w, floa
   if (!ws || ws_bytes < need) return HELIX_ERR_WORKSPACE;
   if (reinterpret_cast<uintptr_t>(ws) & 255) return HELIX_ERR_ALIGN;
   const bool as_gemm = conv_f32_is_gemm(g);
+  if (as_gemm || (g.R * g.S <= 32 && (int64_t)g.NB * g.H * g.W * g.C < 0x7fffffff)) {
+    const int rc = conv_f32_implicit(cfg, x, w, y, g, M, K, as_gemm, sm_count, stream);
+    if (rc == HELIX_OK) ++*launches;
+    if (rc != HELIX_ERR_UNSUPPORTED) return rc;
+  }
   float* col = static_cast<float*>(ws);
   float* wt = reinterpret_cast<float*>(static_cast<char*>(ws) + (as_gemm ? 0 : align256((size_t)M * K * sizeof(float))));
   {

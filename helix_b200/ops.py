@@ -113,7 +113,7 @@ def kernel_name(launch):
             return "gemv_f16_stream_kernel<%d>" % launch.M
         return "gemv_f16_mma_kernel<%d>" % (1 if launch.M <= 8 else 2)
     if launch.op == _lib.OP_GEMM_F32:
-        return "sgemm_f32_kernel<%d,%d>" % (c.tile_m, c.tile_n)
+        return "%s<%d,%d>" % ("sgemm_f32_ring_kernel" if c.stages >= 3 else "sgemm_f32_kernel", c.tile_m, c.tile_n)
     if c.cta_group == 2:
         return "gemm_f16_tc2_kernel<%d>" % c.tile_n
     gathers = False

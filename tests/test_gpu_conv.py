@@ -377,3 +377,23 @@ def test_conv_im2col_map_fills_the_last_channel_block(oracle, geom):
     x[:] = 1.0
     y = _run(x, w, stride, pad)
     assert not np.isnan(y[:, :-2, :-2]).any()        # (beyond, the tap lies in the padding: 0 x inf)
+
+
+@pytest.mark.parametrize("cfg_idx", [None, 0, 2, 10, 11, 12])
+@pytest.mark.parametrize("geom", [
+    (2, 5, 9, 11, 33, 3, 3, 1, 1),         # channels not a multiple of 4: 4-byte copies
+    (3, 12, 7, 7, 30, 5, 5, 2, 2),         # 25 taps, windows that leave the image on both sides
+    (1, 8, 6, 40, 20, 1, 32, 1, 0),        # 32 taps in one row
+    (1, 4, 12, 12, 17, 6, 6, 1, 3),        # 36 taps: through the column matrix
+    (2, 20, 13, 13, 70, 1, 1, 1, 0),       # a plain GEMM over the pixels
+])
+def test_conv_f32_implicit_tiles_keep_the_fmaf_chain(oracle, geom, cfg_idx):
+    from helix_b200._lib import OP_CONV_F32
+    B, C, H, W, OC, kh, kw, stride, pad = geom
+    rng = np.random.default_rng(sum(geom))
+    x = rng.uniform(-1, 1, (B, H, W, C)).astype(np.float32)
+    w = (rng.standard_normal((OC, kh, kw, C)) * (2.0 / (C * kh * kw)) ** 0.5).astype(np.float32)
+    cfg = None if cfg_idx is None else ops.configs(OP_CONV_F32)[cfg_idx]
+    y = ops.conv2d_f32_nhwc(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), stride, pad, cfg=cfg)
+    want = oracle.conv2d_nhwc_f32(x, w, stride, pad, fma=True)
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32)), geom

@@ -86,3 +86,26 @@ def test_sgemm_golden_vectors_from_reference_loop():
         util.assert_f32_close(got, g[n + "_c"], n)
     assert np.all(_run(g["s_one_a"], g["s_one_b"]) == 1000.0)
     assert np.array_equal(_run(g["s_id_a"], g["s_id_b"]), g["s_id_a"])
+
+
+@pytest.mark.parametrize("trans_a", [False, True])
+@pytest.mark.parametrize("cfg_idx", [0, 2, 10, 11, 12])
+@pytest.mark.parametrize("shape", [(33, 65, 4), (129, 131, 67), (31, 36, 40), (64, 64, 33), (200, 68, 100)])
+def test_sgemm_ring_tiles_take_any_alignment_and_stay_the_fmaf_chain(oracle, shape, cfg_idx, trans_a):
+    """The tiles the library chooses from: aligned operands (16-byte copies), unaligned ones (4-byte copies), K that ends
+    inside a slab, inside a 16-byte chunk, and before the ring is full."""
+    M, N, K = shape
+    a, b = datagen.c1_fp32_gemm(M, N, K, seed=50 + cfg_idx)
+    cfg = ops.configs(OP_GEMM_F32)[cfg_idx]
+    assert cfg.stages >= 3
+    got = _run(np.ascontiguousarray(a.T) if trans_a else a, b, trans_a, cfg)
+    want = oracle.sgemm_naive(a, b, fma=True)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+    # the same matrices behind rows of 16-byte-aligned and of odd lengths
+    for pad in (4 - (N % 4), 5):
+        big = torch.full((K, N + pad), float("nan"), device="cuda")
+        big[:, :N] = torch.from_numpy(b).cuda()
+        ad = torch.from_numpy(np.ascontiguousarray(a.T) if trans_a else a).cuda()
+        out = torch.empty((M, N), device="cuda")
+        ops.run(ops.launch_gemm_f32(ad, big[:, :N], out, trans_a, cfg))
+        assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32)), pad
