@@ -615,8 +615,11 @@ int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ld
                        ldy_inner, rows, K, m, kw, order_mode);
 }
 
+// Nine to sixteen right-hand sides read twice the X per weight, from L2 and once per block of rows; with more than some 100 MB
+// of weights the stream-K tcgen05 tiles are ahead (16 x 16000 x 5120: 37.8 us here, 36.3 there; 16 x 12288 x 4096: 24.9 and
+// 26.0; 16 x 4096 x 4096: 10.6 and 15.0).
 bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m) {
-  return m >= 1 && m <= 16 && rows >= 1024 && K >= 512 && (K & 7) == 0 && ((ldw ? ldw : K) & 7) == 0 &&
+  return m >= 1 && m <= 16 && (m <= 8 || (int64_t)rows * K <= 52 << 20) && rows >= 1024 && K >= 512 && (K & 7) == 0 && ((ldw ? ldw : K) & 7) == 0 &&
          ((ldx ? ldx : K) & 7) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
          (reinterpret_cast<uintptr_t>(X) & 15) == 0;
 }
