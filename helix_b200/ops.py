@@ -24,16 +24,19 @@ def _require_cuda(*tensors):
             raise ValueError("helix_b200 operators take CUDA tensors only (there is no CPU path)")
 
 
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream(dev=None):
+    """Handle of torch's current stream.  torch.cuda.current_stream() builds a Stream object to hold it (3.4 us, as much as
+    the launch itself); the raw getter returns the integer."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if dev is None else dev)
 
 
 def status_word(device=None):
     """Per-device int32 the kernels write HELIX_ERR_TIMEOUT into when a bounded wait runs out."""
-    dev = torch.cuda.current_device() if device is None else torch.device(device).index
-    if dev not in _status_words:
-        _status_words[dev] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{dev}")
-    return _status_words[dev]
+    dev = device if isinstance(device, int) else torch.cuda.current_device() if device is None else torch.device(device).index
+    word = _status_words.get(dev)
+    if word is None:
+        word = _status_words[dev] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{dev}")
+    return word
 
 
 def check_status(device=None):
@@ -108,7 +111,8 @@ def kernel_name(launch):
         return "gemv_f16_stream_kernel<%d>" % launch.M if streams and launch.N * launch.K >= 1 << 21 else "gemv_f16_kernel"
     if launch.op == _lib.OP_GEMV_F32:
         return "gemv_f32_stream_kernel" if streams and (launch.M == 1 or launch.K >= 512) else "gemv_f32_kernel"
-    if launch.op == OP_GEMM_F16 and not own and launch.batch <= 1 and launch.M <= 16 and launch.N >= 1024 and launch.K >= 512:
+    if (launch.op == OP_GEMM_F16 and not own and launch.batch <= 1 and launch.N >= 1024 and launch.K >= 512 and
+            (launch.M <= 8 or launch.M <= 16 and launch.N * launch.K <= 52 << 20)):
         if launch.M <= 2:
             return "gemv_f16_stream_kernel<%d>" % launch.M
         return "gemv_f16_mma_kernel<%d>" % (1 if launch.M <= 8 else 2)
@@ -236,7 +240,7 @@ def launch_gemv_f32(w, x, out, cfg=None, ws=None, out_transposed=False):
 
 def gemv_f32(w, x, out=None, cfg=None):
     if out is None:
-        out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float32, device=w.device)
+        out = w.new_empty((x.shape[0], w.shape[0]))
     run(launch_gemv_f32(w, x, out, cfg))
     return out
 
@@ -314,7 +318,7 @@ def conv2d_f32_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
     KO, R, S, _ = w.shape
     Ho, Wo = conv_out_hw(H, W, R, S, stride, pad)
     if out is None:
-        out = torch.empty((N, Ho, Wo, KO), dtype=torch.float32, device=x.device)
+        out = x.new_empty((N, Ho, Wo, KO))
     run(launch_conv2d_f32(x, w, out, stride, pad, cfg))
     return out
 
@@ -342,22 +346,24 @@ def launch_gemm_f32(a, b, out, trans_a=False, cfg=None):
 
 def run(launch):
     """Queue a prepared launch on torch's current stream."""
-    check(_lib.load().helix_launch(ctypes.byref(launch), ctypes.c_void_p(status_word().data_ptr()), _stream()),
-          "helix_launch")
+    dev = torch.cuda.current_device()
+    rc = _lib.load().helix_launch(ctypes.byref(launch), status_word(dev).data_ptr(), _stream(dev))
+    if rc != 0:
+        check(rc, "helix_launch")
 
 
 # ----------------------------------------------------------------------------- eager operators
 def gemm_f16(a, b_nk, out=None, cfg=None):
     shape = (*a.shape[:-1], b_nk.shape[-2])
     if out is None:
-        out = torch.empty(shape, dtype=torch.float16, device=a.device)
+        out = a.new_empty(shape)
     run(launch_gemm_f16(a, b_nk, out, cfg))
     return out
 
 
 def gemv_f16(w, x, out=None, cfg=None):
     if out is None:
-        out = torch.empty((x.shape[0], w.shape[0]), dtype=torch.float16, device=w.device)
+        out = w.new_empty((x.shape[0], w.shape[0]))
     run(launch_gemv_f16(w, x, out, cfg))
     return out
 
@@ -365,7 +371,7 @@ def gemv_f16(w, x, out=None, cfg=None):
 def conv2d_f16_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
     if out is None:
         Ho, Wo = conv_out_hw(x.shape[1], x.shape[2], w.shape[1], w.shape[2], stride, pad)
-        out = torch.empty((x.shape[0], Ho, Wo, w.shape[0]), dtype=torch.float16, device=x.device)
+        out = x.new_empty((x.shape[0], Ho, Wo, w.shape[0]))
     run(launch_conv2d_f16(x, w, out, stride, pad, cfg))
     return out
 
@@ -373,7 +379,7 @@ def conv2d_f16_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
 def gemm_f32(a, b, trans_a=False, out=None, cfg=None):
     M = a.shape[1] if trans_a else a.shape[0]
     if out is None:
-        out = torch.empty((M, b.shape[1]), dtype=torch.float32, device=a.device)
+        out = a.new_empty((M, b.shape[1]))
     run(launch_gemm_f32(a, b, out, trans_a, cfg))
     return out
 
