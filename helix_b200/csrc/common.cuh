@@ -307,6 +307,49 @@ __device__ __forceinline__ void tma_store_wait_read_1() { asm volatile("cp.async
 // until they have completed altogether
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// ---------------------------------------------------------------- epilogue staging
+// A warp's 32 rows (lane = row) x 64 accumulator columns, rounded once to fp16, into a 128-byte-swizzled box of 32 x 128
+// bytes in shared memory (the layout a TMA store with SWIZZLE_128B reads).
+__device__ __forceinline__ void stage_rows_f16(uint32_t row_base, const uint32_t (&lo)[32], const uint32_t (&hi)[32],
+                                               int lane) {
+#pragma unroll
+  for (int ch = 0; ch < 8; ++ch) {
+    const uint32_t* src = ch < 4 ? &lo[ch * 8] : &hi[(ch - 4) * 8];
+    __half2 h0 = __floats2half2_rn(__uint_as_float(src[0]), __uint_as_float(src[1]));
+    __half2 h1 = __floats2half2_rn(__uint_as_float(src[2]), __uint_as_float(src[3]));
+    __half2 h2 = __floats2half2_rn(__uint_as_float(src[4]), __uint_as_float(src[5]));
+    __half2 h3 = __floats2half2_rn(__uint_as_float(src[6]), __uint_as_float(src[7]));
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((ch ^ (lane & 7)) << 4)),
+                 "r"(*reinterpret_cast<uint32_t*>(&h0)), "r"(*reinterpret_cast<uint32_t*>(&h1)),
+                 "r"(*reinterpret_cast<uint32_t*>(&h2)), "r"(*reinterpret_cast<uint32_t*>(&h3))
+                 : "memory");
+  }
+}
+// Such a box to rows of C that TMA cannot store (a leading dimension or base that is no multiple of 16 bytes): row by row
+// with the lanes along the columns, 4 bytes each, shifted by one element where a row starts on an odd one.  (A lane per row
+// writes 2 bytes to 32 different lines per instruction: 2595 x 1685 x 200 took 50.8 us instead of 19.)  dst: row 0, column
+// 0 of the block; `rows` and `cols` of it exist.
+__device__ __forceinline__ void drain_box_any(uint32_t box, __half* dst, int64_t ldc, int rows, int cols) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  auto element = [&](int r, int e) {
+    uint16_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(box + r * 128 + (((e >> 3) ^ (r & 7)) << 4) + (e & 7) * 2) : "memory");
+    return v;
+  };
+#pragma unroll 4
+  for (int r = 0; r < rows; ++r) {
+    __half* d = dst + r * ldc;
+    const int odd = static_cast<int>(reinterpret_cast<uintptr_t>(d) >> 1) & 1;
+    const int e = 2 * lane + odd;
+    const uint16_t v0 = element(r, e), v1 = element(r, (e + 1) & 63);
+    if (e + 1 < cols) *reinterpret_cast<uint32_t*>(d + e) = static_cast<uint32_t>(v0) | static_cast<uint32_t>(v1) << 16;
+    else if (e < cols) *reinterpret_cast<uint16_t*>(d + e) = v0;
+    if (odd && lane == 0) *reinterpret_cast<uint16_t*>(d) = element(r, 0);
+  }
+  __syncwarp();   // the box is free again
+}
+
 // ---------------------------------------------------------------- named barriers (sub-CTA groups)
 // All `nthreads` threads of the group (whole warps) must call these the same number of times.
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {

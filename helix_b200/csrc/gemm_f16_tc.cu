@@ -96,7 +96,8 @@ struct GemmParams {
   // convolution only
   const __half* x;
   ConvGeom g;
-  int im2col;      // A tiles come from an im2col tensor map over x (C a multiple of 64): no gather warps
+  int im2col;      // A tiles come from an im2col tensor map over x: no gather warps
+  int wtaps;       // the weights' map is (channel, tap, output channel): the last channel block of a tap is filled
   // optional per-CTA timeline (null = off): kTraceWords 64-bit words per CTA, see trace_mark
   unsigned long long* trace;
   // reciprocals of the divisors the tile decoders use
@@ -306,7 +307,9 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
       }
 }
 
-template <int BN, bool CONV>
+// ANY: rows of C that a TMA store cannot write.  A variant of its own: as a branch beside the TMA store it made chains of
+// short launches 2 % slower.
+template <int BN, bool CONV, bool ANY>
 __global__ void __launch_bounds__(CONV ? kConvThreads : kGemmThreads, 1)
 gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
@@ -471,14 +474,15 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 fast_divmod(kb, p.fd_cblocks, tap, cb);
                 fast_divmod(tap, p.fd_s, fr, fs);
                 if (p.swap) {
-                  if (load_a) tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK, tap, w.m_blk * kBM);
+                  if (load_a) tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, p.wtaps ? cb * kBK : kb * kBK,
+                            p.wtaps ? tap : w.m_blk * kBM, p.wtaps ? w.m_blk * kBM : 0);
                   if (load_b) tma_load_im2col_4d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK,
                                                  pix_w, pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
                 } else {
                   if (load_a) tma_load_im2col_4d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK,
                                                  pix_w, pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
-                  if (load_b) tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK, tap,
-                                          w.n_blk * BN);
+                  if (load_b) tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, p.wtaps ? cb * kBK : kb * kBK,
+                                          p.wtaps ? tap : w.n_blk * BN, p.wtaps ? w.n_blk * BN : 0);
                 }
               } else {
                 if (load_a) tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, kb * kBK, w.m_blk * kBM, w.b);
@@ -492,13 +496,15 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
               fast_divmod(kb, p.fd_cblocks, tap, cb);
               fast_divmod(tap, p.fd_s, fr, fs);
               if (p.swap) {   // weights on the 128-row axis, BN pixels per im2col box on the other
-                tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK, tap, w.m_blk * kBM);
+                tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, p.wtaps ? cb * kBK : kb * kBK,
+                            p.wtaps ? tap : w.m_blk * kBM, p.wtaps ? w.m_blk * kBM : 0);
                 tma_load_im2col_4d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK, pix_w,
                                    pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
               } else {
                 tma_load_im2col_4d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, cb * kBK, pix_w,
                                    pix_h, pix_n, (uint16_t)fs, (uint16_t)fr);
-                tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK, tap, w.n_blk * BN);
+                tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, p.wtaps ? cb * kBK : kb * kBK,
+                            p.wtaps ? tap : w.n_blk * BN, p.wtaps ? w.n_blk * BN : 0);
               }
             } else {
               tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, kb * kBK, w.m_blk * kBM, w.b);
@@ -630,22 +636,10 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         const int col0 = w.n_blk * BN + c0;
         if (col0 >= p.PN) return;   // warp-uniform: padding columns only
         uint8_t* stage_box = stage_boxes + box * (32 * 128);
-        const uint32_t row_base = smem_u32(stage_box) + lane * 128;
         box ^= 1;
         if (lane == 0) tma_store_wait_read_1();   // the store issued two boxes ago has left this buffer
         __syncwarp();
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          const uint32_t* src = ch < 4 ? &lo[ch * 8] : &hi[(ch - 4) * 8];
-          __half2 h0 = __floats2half2_rn(__uint_as_float(src[0]), __uint_as_float(src[1]));
-          __half2 h1 = __floats2half2_rn(__uint_as_float(src[2]), __uint_as_float(src[3]));
-          __half2 h2 = __floats2half2_rn(__uint_as_float(src[4]), __uint_as_float(src[5]));
-          __half2 h3 = __floats2half2_rn(__uint_as_float(src[6]), __uint_as_float(src[7]));
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((ch ^ (lane & 7)) << 4)),
-                       "r"(*reinterpret_cast<uint32_t*>(&h0)), "r"(*reinterpret_cast<uint32_t*>(&h1)),
-                       "r"(*reinterpret_cast<uint32_t*>(&h2)), "r"(*reinterpret_cast<uint32_t*>(&h3))
-                       : "memory");
-        }
+        stage_rows_f16(smem_u32(stage_box) + lane * 128, lo, hi, lane);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
@@ -653,7 +647,30 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           tma_store_commit();
         }
       };
+      // the same columns where TMA cannot store the rows of C
+      auto emit_any = [&](const uint32_t (&lo)[32], const uint32_t (&hi)[32], int c0) {
+        const int col0 = w.n_blk * BN + c0, row0 = w.m_blk * kBM + quarter * 32;
+        if (col0 >= p.PN) return;
+        stage_rows_f16(smem_u32(stage_boxes) + lane * 128, lo, hi, lane);
+        drain_box_any(smem_u32(stage_boxes), p.C + (int64_t)w.b * p.stride_c + (int64_t)row0 * p.ldc + col0, p.ldc,
+                      min(32, p.PM - row0), min(64, p.PN - col0));
+      };
       if constexpr (BN >= 64) {
+        if (ANY && w.mode == kOutDirect) {
+#pragma unroll 1
+          for (int c0 = 0; c0 < BN; c0 += 64) {
+            uint32_t lo[32], hi[32];
+            tmem_ld_32x32b_x32(taddr + c0, lo);
+            tmem_ld_32x32b_x32(taddr + c0 + 32, hi);
+            tmem_ld_wait();
+            emit_any(lo, hi, c0);
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+          if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+          continue;
+        }
         if (p.tma_store && w.mode == kOutDirect) {
           // Fast path: 64 columns at a time go TMEM -> registers -> fp16 -> this warp's swizzled
           // 32 x 128-byte staging box -> one TMA store (full 128-byte lines, edges clipped by the
@@ -842,13 +859,14 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             };
             bool done = false;
             if constexpr (BN >= 64) {
-              if (p.tma_store) {
+              if (ANY || p.tma_store) {
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 64) {
                   uint32_t lo[32], hi[32];
                   sum_chunk(lo, c0);
                   sum_chunk(hi, c0 + 32);
-                  emit(lo, hi, c0);
+                  if constexpr (ANY) emit_any(lo, hi, c0);
+                  else emit(lo, hi, c0);
                 }
                 done = true;
               }
@@ -1104,10 +1122,12 @@ static int make_tmap_im2col(CUtensorMap* map, const void* x, const ConvGeom& g, 
   return HELIX_OK;
 }
 
-// Weights w[KO][R][S][C] as a map of (channel, tap, output channel): one box is 64 channels of one tap for `rows` output
-// channels, laid out as the K-major tile the MMAs read.
+// Weights w[KO][R][S][C]: a box is 64 channels of one tap for `rows` output channels, laid out as the K-major tile the MMAs
+// read.  With whole 64-channel blocks that is the plain matrix [KO][R * S * C]; otherwise a map of (channel, tap, output
+// channel), whose boxes do not run into the next tap.
 static int make_tmap_filter(CUtensorMap* map, const void* w, const ConvGeom& g, int rows) {
   const int taps = g.R * g.S;
+  if (g.C % kBK == 0) return make_tmap(map, w, (int64_t)taps * g.C, g.KO, 1, (int64_t)taps * g.C, 0, rows);
   return make_tmap(map, w, g.C, taps, g.KO, g.C, (int64_t)taps * g.C, 1, rows);
 }
 static int im2col_k(const ConvGeom& g) { return g.R * g.S * ((g.C + kBK - 1) / kBK * kBK); }
@@ -1333,8 +1353,8 @@ void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) 
       out->stream_k = 0;
       out->split_k = 1;
       out->tile_n = 256;
-      out->stages = max_stages(256, false);
     }
+    out->stages = max_stages(out->tile_n, false);
   } else
     default_config_impl(M, g.KO, K, 1, sm_count, true, false, out);
   // 64 -> 64 channels, 3 x 3 where the row-pair kernel's tile fits: that kernel (no tile to choose)
@@ -1408,11 +1428,11 @@ unsigned long long* gemm_f16_trace_for_grid(int grid) {
   return (g_trace_buf && g_trace_bytes >= (size_t)grid * kTraceWords * 8) ? g_trace_buf : nullptr;
 }
 
-template <int BN, bool CONV>
+template <int BN, bool CONV, bool ANY>
 static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
                                   const GemmParams& p, int grid, size_t smem, cudaStream_t stream) {
   constexpr int threads = CONV ? kConvThreads : kGemmThreads;
-  auto kern = gemm_f16_tc_kernel<BN, CONV>;
+  auto kern = gemm_f16_tc_kernel<BN, CONV, ANY>;
   // the opt-in shared-memory size is sticky per function and device: raise it only when needed
   static std::mutex mu;
   static size_t granted[64] = {0};
@@ -1549,11 +1569,13 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   p.fd_s = make_fastdiv(p.im2col ? p.g.S : 1);
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
+  const bool any = !p.swap && !p.tma_store;
   cudaError_t e = cudaErrorInvalidValue;
 #define HELIX_BN_CASE(BNV)                                                                 \
   case BNV:                                                                                \
-    e = conv ? launch_variant<BNV, true>(ta, tb, tc, p, grid, smem, stream)                \
-             : launch_variant<BNV, false>(ta, tb, tc, p, grid, smem, stream);              \
+    e = conv  ? launch_variant<BNV, true, false>(ta, tb, tc, p, grid, smem, stream)        \
+        : any ? launch_variant<BNV, false, (BNV >= 64)>(ta, tb, tc, p, grid, smem, stream) \
+              : launch_variant<BNV, false, false>(ta, tb, tc, p, grid, smem, stream);      \
     break;
   switch (bn) {
     HELIX_BN_CASE(256)
@@ -1692,6 +1714,7 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     ps.status = status_dev;
     ps.g = g;
     ps.im2col = 1;
+    ps.wtaps = g.C % kBK != 0;
     CUtensorMap tw, tx;
     int rcs;
     if ((rcs = make_tmap_filter(&tw, w, g, kBM)) != HELIX_OK) return rcs;
@@ -1715,6 +1738,7 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     if ((rc = make_tmap_filter(&tb, w, g, cfg.tile_n)) != HELIX_OK) return rc;
     p.K = im2col_k(g);
     p.im2col = 1;
+    p.wtaps = g.C % kBK != 0;
     return launch_common(cfg, false, ta, tb, p, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
   }
   if ((rc = make_tmap(&tb, w, K, N, 1, K, 0, cfg.tile_n)) != HELIX_OK) return rc;

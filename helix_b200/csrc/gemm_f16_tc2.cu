@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -269,7 +270,8 @@ __device__ __forceinline__ void pair_dual_issue_loop(const Gemm2Params& p, const
   if (nslab > 0 && ((nslab - 1) & 1) != ME) named_bar_sync(kTokBarrier2 + ((nslab - 1) & 1), 64);
 }
 
-template <int BN>
+// ANY: rows of C that a TMA store cannot write (see the one-CTA kernel)
+template <int BN, bool ANY>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_c, const Gemm2Params p) {
@@ -463,7 +465,6 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // ------------------------------------------------------------------ epilogue (each CTA: its 128 rows)
     const int quarter = warp & 3;
     bool ok = true;
-    const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) && ((p.stride_c & 7) == 0);
     int box = 0;   // staging box in use; alternates over the whole run of the warp, across tiles
     Item2 it;
     for (int idx = 0; ok && get_item2(p, pair, num_pairs, idx, it); ++idx) {
@@ -477,7 +478,6 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (quarter == 0 && lane == 0) trace2_tile(p, idx, 4);
       const int cta_row0 = w.m_blk * 2 * kBM + (int)rank * kBM;
       const int row0 = cta_row0 + quarter * 32;
-      const int row = row0 + lane;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       if (it.slot >= 0) {
         // part of a tile's K range: the fp32 accumulator (padding included) goes to this pair's slot of
@@ -502,6 +502,26 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (quarter == 0 && lane == 0) trace2_tile(p, idx, 5);
         continue;
       }
+      if constexpr (ANY) {   // 64 columns of a warp's 32 rows at a time
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN; c0 += 64) {
+          const int col0 = w.n_blk * BN + c0;
+          if (col0 >= p.PN) break;
+          uint32_t lo[32], hi[32];
+          tmem_ld_32x32b_x32(taddr + c0, lo);
+          tmem_ld_32x32b_x32(taddr + c0 + 32, hi);
+          tmem_ld_wait();
+          const uint32_t warp_box = smem_u32(sC) + quarter * (32 * 128);
+          stage_rows_f16(warp_box + lane * 128, lo, hi, lane);
+          drain_box_any(warp_box, p.C + (int64_t)w.b * p.stride_c + (int64_t)row0 * p.ldc + col0, p.ldc,
+                        min(32, p.PM - row0), min(64, p.PN - col0));
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
+        if (quarter == 0 && lane == 0) trace2_tile(p, idx, 5);
+        continue;
+      }
       uint32_t ra[32], rb[32], na[32], nb[32];
       // 64 columns at a time: the four warps put their 32 rows each into one 128-row staging box
       // and one thread sends the box with a single TMA store (issuing a tensor copy holds its
@@ -510,52 +530,17 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       auto emit = [&](const uint32_t (&lo)[32], const uint32_t (&hi)[32], int c0) {
         const int col0 = w.n_blk * BN + c0;
         if (col0 >= p.PN || cta_row0 >= p.PM) return;   // uniform over the four warps: nothing but padding
-        if (p.tma_store) {
-          uint8_t* stage_box = sC + box * (128 * 128);
-          const uint32_t row_base = smem_u32(stage_box) + (quarter * 32 + lane) * 128;
-          box ^= 1;
-          if (quarter == 0 && lane == 0) tma_store_wait_read_1();   // the store issued two boxes ago has left this buffer
-          named_bar_sync(kEpiBarrier, 128);
-#pragma unroll
-          for (int ch = 0; ch < 8; ++ch) {
-            const uint32_t* src = ch < 4 ? &lo[ch * 8] : &hi[(ch - 4) * 8];
-            __half2 h0 = __floats2half2_rn(__uint_as_float(src[0]), __uint_as_float(src[1]));
-            __half2 h1 = __floats2half2_rn(__uint_as_float(src[2]), __uint_as_float(src[3]));
-            __half2 h2 = __floats2half2_rn(__uint_as_float(src[4]), __uint_as_float(src[5]));
-            __half2 h3 = __floats2half2_rn(__uint_as_float(src[6]), __uint_as_float(src[7]));
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((ch ^ (lane & 7)) << 4)),
-                         "r"(*reinterpret_cast<uint32_t*>(&h0)), "r"(*reinterpret_cast<uint32_t*>(&h1)),
-                         "r"(*reinterpret_cast<uint32_t*>(&h2)), "r"(*reinterpret_cast<uint32_t*>(&h3))
-                         : "memory");
-          }
-          fence_proxy_async_smem();
-          named_bar_sync(kEpiBarrier, 128);
-          if (quarter == 0 && lane == 0) {
-            tma_store_3d(&tmap_c, stage_box, col0, cta_row0, w.b);
-            tma_store_commit();
-          }
-        } else if (row < p.PM) {
-          __half* dst = p.C + (int64_t)w.b * p.stride_c + (int64_t)row * p.ldc + col0;
-#pragma unroll
-          for (int jj = 0; jj < 64; jj += 8) {
-            const uint32_t* src = jj < 32 ? &lo[jj] : &hi[jj - 32];
-            if (vec_ok && col0 + jj + 8 <= p.PN) {
-              uint4 v;
-              __half2 h0 = __floats2half2_rn(__uint_as_float(src[0]), __uint_as_float(src[1]));
-              __half2 h1 = __floats2half2_rn(__uint_as_float(src[2]), __uint_as_float(src[3]));
-              __half2 h2 = __floats2half2_rn(__uint_as_float(src[4]), __uint_as_float(src[5]));
-              __half2 h3 = __floats2half2_rn(__uint_as_float(src[6]), __uint_as_float(src[7]));
-              v.x = *reinterpret_cast<uint32_t*>(&h0);
-              v.y = *reinterpret_cast<uint32_t*>(&h1);
-              v.z = *reinterpret_cast<uint32_t*>(&h2);
-              v.w = *reinterpret_cast<uint32_t*>(&h3);
-              *reinterpret_cast<uint4*>(dst + jj) = v;
-            } else {
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (col0 + jj + q < p.PN) dst[jj + q] = __float2half_rn(__uint_as_float(src[q]));
-            }
-          }
+        uint8_t* stage_box = sC + box * (128 * 128);
+        const uint32_t row_base = smem_u32(stage_box) + (quarter * 32 + lane) * 128;
+        box ^= 1;
+        if (quarter == 0 && lane == 0) tma_store_wait_read_1();   // the store issued two boxes ago has left this buffer
+        named_bar_sync(kEpiBarrier, 128);
+        stage_rows_f16(row_base, lo, hi, lane);
+        fence_proxy_async_smem();
+        named_bar_sync(kEpiBarrier, 128);
+        if (quarter == 0 && lane == 0) {
+          tma_store_3d(&tmap_c, stage_box, col0, cta_row0, w.b);
+          tma_store_commit();
         }
       };
       tmem_ld_32x32b_x32(taddr, ra);
@@ -677,10 +662,10 @@ int make_map(CUtensorMap* map, const void* base, int64_t inner, int64_t rows, in
   return r == CUDA_SUCCESS ? HELIX_OK : HELIX_ERR_CUDA;
 }
 
-template <int BN>
+template <int BN, bool ANY>
 cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Gemm2Params& p,
                         int grid, size_t smem, cudaStream_t stream) {
-  auto kern = gemm_f16_tc2_kernel<BN>;
+  auto kern = gemm_f16_tc2_kernel<BN, ANY>;
   static std::mutex mu;
   static size_t granted[64] = {0};
   int dev = 0;
@@ -801,9 +786,13 @@ int gemm_f16_pair_launch(const helix_cfg_t& cfg, const void* A, int64_t lda, con
       make_map(&tc, C, N, M, batch, ldc, sc, kBM) == HELIX_OK)
     p.tma_store = 1;
   const size_t smem = 1024 + (size_t)p.stages * (kATileBytes + (bn / 2) * kBK * 2) + kStagingBytes + 256;
-  const cudaError_t e = bn == 256   ? launch_pair<256>(ta, tb, tc, p, 2 * pairs, smem, stream)
-                        : bn == 192 ? launch_pair<192>(ta, tb, tc, p, 2 * pairs, smem, stream)
-                                    : launch_pair<128>(ta, tb, tc, p, 2 * pairs, smem, stream);
+  auto launch = [&](auto any) {
+    constexpr bool kAny = decltype(any)::value;
+    return bn == 256   ? launch_pair<256, kAny>(ta, tb, tc, p, 2 * pairs, smem, stream)
+           : bn == 192 ? launch_pair<192, kAny>(ta, tb, tc, p, 2 * pairs, smem, stream)
+                       : launch_pair<128, kAny>(ta, tb, tc, p, 2 * pairs, smem, stream);
+  };
+  const cudaError_t e = p.tma_store ? launch(std::false_type{}) : launch(std::true_type{});
   if (e != cudaSuccess) return HELIX_ERR_CUDA;
   ++*launches;
   if (fixup) {

@@ -397,3 +397,26 @@ def test_two_issuing_warps_give_the_same_bits(shape, bn):
     ops.check_status()
     assert torch.equal(pair_one, pair_two)
     assert float((pair_two.float() - ref).norm() / ref.norm()) < 2e-3
+
+
+@pytest.mark.parametrize("case", [(300, 131, 72, 64, 1, 1), (257, 333, 136, 128, 1, 1), (129, 201, 200, 128, 1, 1),
+                                  (200, 515, 264, 256, 1, 1), (130, 67, 1024, 64, 3, 1), (300, 389, 512, 256, 1, 2),
+                                  (513, 203, 512, 128, 1, 2)])
+def test_rows_of_any_alignment_leave_through_the_staging_box(oracle, case):
+    """Output rows that a TMA store cannot write: odd leading dimensions (every second row starts on an odd element), a base
+    that is 2-byte aligned only, rows and columns that end inside a box; nothing is written beside them."""
+    M, N, K, bn, split, group = case
+    a, b = datagen.c3_gemm(M, N, K, seed=M)
+    cfg = ops.make_cfg(OP_GEMM_F16, tile_m=128, tile_n=bn, tile_k=64, split_k=split, cta_group=group)
+    _, ref32 = oracle.hgemm_naive(a, b)
+    ad, bd = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+    for ld, off in ((N, 0), (N + 1 + N % 2, 1), (N + N % 2, 3), (N + 8 - N % 8, 2)):
+        buf = torch.full((M * ld + off + 64,), 9.0, dtype=torch.float16, device="cuda")
+        out = torch.as_strided(buf, (M, N), (ld, 1), off)
+        ops.run(ops.launch_gemm_f16(ad, bd, out, cfg))
+        torch.cuda.synchronize()
+        util.assert_f16_close(out.cpu().numpy(), ref32, f"{case} ld={ld} offset={off}")
+        rest = torch.ones_like(buf, dtype=torch.bool)
+        torch.as_strided(rest, (M, N), (ld, 1), off).fill_(False)
+        assert torch.all(buf[rest] == 9.0)
+    ops.check_status()
