@@ -1174,11 +1174,18 @@ static int max_stages(int bn, bool conv) {
 static double slab_us(int bn) {
   switch (bn) {
     case 256: return 0.43;
+    case 192: return 0.375;
     case 128: return 0.34;
     case 64: return 0.33;
     case 32: return 0.33;
     default: return 0.33;
   }
+}
+
+constexpr int kWholeMachineSms = 100;
+static int64_t plain_rounds(int pm, int pn, int bn, int batch, int sm_count) {
+  const int64_t tiles = (int64_t)((pm + kBM - 1) / kBM) * ((pn + bn - 1) / bn) * batch;
+  return (tiles + sm_count - 1) / sm_count;
 }
 
 // Built-in choice when the caller brings no profiled dictionary (the profiled cost model of
@@ -1305,6 +1312,20 @@ static void default_config_impl(int M, int N, int K, int batch, int sm_count, bo
       }
     }
   }
+  // 192-wide tiles are there for tile counts that quantise badly at 128 and 256 when a launch has the machine to itself
+  // (256 -> 1024 channels, 1 x 1, 14 x 14 x 32: 8.6 -> 7.8 us); in concurrent chains on a share of the SMs rounds matter little.
+  const bool whole_machine = sm_count >= kWholeMachineSms;
+  bool medium = false;
+  if (!conv && !swap && whole_machine && pn > 128) {
+    const double dp = (double)plain_rounds(pm, pn, 192, batch, sm_count) * num_kb * slab_us(192) + 4.0;
+    if (dp < best) {
+      best = dp;
+      medium = true;
+      out->tile_n = 192;
+      out->stream_k = 0;
+      out->split_k = 1;
+    }
+  }
   out->stages = max_stages(out->tile_n, conv);
   // CTA pairs on a 256 x 256 tile: half the B bytes per CTA and a 6-deep ring; measured about
   // 0.41 us per 64-deep slab of a pair tile, i.e. twice the work of a 128 x 256 slab in less time.
@@ -1317,8 +1338,9 @@ static void default_config_impl(int M, int N, int K, int batch, int sm_count, bo
       const int bn = widths[i];
       const int64_t pair_tiles = (int64_t)((M + 2 * kBM - 1) / (2 * kBM)) * ((N + bn - 1) / bn) * batch;
       const double t2 = (double)((pair_tiles + pairs - 1) / pairs) * num_kb * slab[i] + 4.0;
-      if (t2 < best) {
+      if (t2 < (medium ? best - 0.2 : best)) {   // a pair launch has the longer set-up (512 -> 2048, 7 x 7 x 32: 8.4 against 7.8 us)
         best = t2;
+        medium = false;
         out->cta_group = 2;
         out->tile_n = bn;
         out->stream_k = 0;
@@ -1353,6 +1375,18 @@ void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) 
       out->stream_k = 0;
       out->split_k = 1;
       out->tile_n = 256;
+    }
+    // 192 pixels per step where that takes fewer or shorter rounds of a machine the launch has to itself (us: 3x3,
+    // 240 -> 240, 20 x 20 x 32: 21.2 -> 19.3; 5x5, 96 -> 256, 26 x 26 x 20: 26.1 -> 22.9), if the slabs of K are many enough:
+    // 128 -> 128, 28 x 28 x 32, gains 1.3 us in a chain of cold launches but loses 1 us between a stage's 1x1 layers
+    if (sm_count >= kWholeMachineSms && g.KO > 64 && out->split_k <= 1 && !out->stream_k) {
+      const int64_t now = plain_rounds(out->swap_ab ? g.KO : M, out->swap_ab ? M : g.KO, out->tile_n, 1, sm_count);
+      const int64_t then = plain_rounds(g.KO, M, 192, 1, sm_count);
+      const int num_kb = im2col_k(g) / kBK;
+      if (then * num_kb * slab_us(192) + 1.4 < now * num_kb * slab_us(out->tile_n)) {
+        out->swap_ab = 1;
+        out->tile_n = 192;
+      }
     }
     out->stages = max_stages(out->tile_n, false);
   } else
@@ -1472,6 +1506,7 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
                          GemmParams& p, void* C, int64_t ldc, int64_t sc, void* ws, size_t ws_bytes, int sm_count,
                          bool independent, cudaStream_t stream, int64_t* launches) {
   const int bn = cfg.tile_n;
+  if (bn == 192 && (cfg.stream_k || cfg.split_k > 1)) return HELIX_ERR_UNSUPPORTED;   // whole tiles only
   p.tiles_m = (p.PM + kBM - 1) / kBM;
   p.tiles_n = (p.PN + bn - 1) / bn;
   p.num_kb = (p.K + kBK - 1) / kBK;
@@ -1579,6 +1614,7 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
     break;
   switch (bn) {
     HELIX_BN_CASE(256)
+    HELIX_BN_CASE(192)
     HELIX_BN_CASE(128)
     HELIX_BN_CASE(64)
     HELIX_BN_CASE(32)

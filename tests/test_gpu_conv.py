@@ -397,3 +397,13 @@ def test_conv_f32_implicit_tiles_keep_the_fmaf_chain(oracle, geom, cfg_idx):
     y = ops.conv2d_f32_nhwc(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), stride, pad, cfg=cfg)
     want = oracle.conv2d_nhwc_f32(x, w, stride, pad, fma=True)
     assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32)), geom
+
+
+@pytest.mark.parametrize("geom", [(2, 64, 30, 30, 96, 3, 3, 1, 1), (3, 96, 17, 19, 200, 5, 5, 1, 2), (4, 128, 23, 23, 130, 3, 3, 2, 1)])
+def test_conv_192_pixel_tiles(oracle, geom):
+    """Output channels on the 128-row axis, 192 pixels per im2col box; pixel counts that end inside a box and inside 64 columns."""
+    B, C, H, W, OC, kh, kw, stride, pad = geom
+    x, w = datagen.c4_conv(*geom, seed=41)
+    got = _run(x, w, stride, pad, ops.make_cfg(OP_CONV_F16, tile_m=128, tile_n=192, tile_k=64, swap_ab=1))
+    _, y32 = oracle.conv2d_nhwc_f16(x, w, stride, pad)
+    util.assert_f16_close(got, y32, f"conv {geom}")

@@ -399,7 +399,29 @@ def test_two_issuing_warps_give_the_same_bits(shape, bn):
     assert float((pair_two.float() - ref).norm() / ref.norm()) < 2e-3
 
 
-@pytest.mark.parametrize("case", [(300, 131, 72, 64, 1, 1), (257, 333, 136, 128, 1, 1), (129, 201, 200, 128, 1, 1),
+@pytest.mark.parametrize("swap", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(128, 192, 64), (200, 392, 264), (130, 191, 72), (256, 576, 512)])
+def test_192_wide_tiles(oracle, M, N, K, swap):
+    """Edges of the 192-wide tile on either operand order; K cut into slices is not built for it."""
+    a, b = datagen.c3_gemm(M, N, K, seed=M + N)
+    got = _run(a, b, _cfg(192, swap=swap))
+    _, ref32 = oracle.hgemm_naive(a, b)
+    util.assert_f16_close(got, ref32, f"192-wide {M}x{N}x{K} swap={swap}")
+    with pytest.raises(Exception) as e:
+        _run(a, b, _cfg(192, split_k=2, swap=swap))
+    assert "-6" in str(e.value)
+
+
+def test_192_wide_tiles_are_chosen_for_a_whole_machine_only():
+    def tile(M, N, K, ctas=0):
+        l = ops.Launch()
+        l.op, l.M, l.N, l.K, l.batch = OP_GEMM_F16, M, N, K, 1
+        l.cfg.max_ctas = ctas
+        return ops.default_config(l).tile_n
+    assert tile(6272, 1024, 256) == 192 and tile(6272, 1024, 256, 38) != 192
+
+
+@pytest.mark.parametrize("case", [(300, 131, 72, 64, 1, 1), (257, 333, 136, 128, 1, 1), (129, 201, 200, 192, 1, 1),
                                   (200, 515, 264, 256, 1, 1), (130, 67, 1024, 64, 3, 1), (300, 389, 512, 256, 1, 2),
                                   (513, 203, 512, 128, 1, 2)])
 def test_rows_of_any_alignment_leave_through_the_staging_box(oracle, case):
