@@ -797,7 +797,7 @@ int gemm_f16_pair_launch(const helix_cfg_t& cfg, const void* A, int64_t lda, con
   ++*launches;
   if (fixup) {
     const dim3 fgrid((2 * kBM * (bn >> 2) + 255) / 256, p.sk_tiles);
-    gemm2_streamk_fixup_kernel<<<fgrid, 256, 0, stream>>>(p, bn, pairs);
+    gemm2_streamk_fixup_kernel<<<fgrid, 256, 0, stream>>>(p, bn, pairs);   // many blocks: a plain launch
     if (cudaGetLastError() != cudaSuccess) return HELIX_ERR_CUDA;
     ++*launches;
   }

@@ -461,11 +461,13 @@ gemv_f16_mma_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, 
 // Sums the split-K partials in slice order (deterministic) and rounds once.
 __global__ void gemv_splitk_reduce_kernel(const float* __restrict__ partial, __half* __restrict__ Y, int64_t ldy,
                                           int64_t ldy_inner, int rows, int m, int split_k) {
+  griddep_launch_dependents();
+  griddep_wait();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * m) return;
   const int i = idx / rows, r = idx - i * rows;
   float s = 0.0f;
-  for (int ks = 0; ks < split_k; ++ks) s += partial[((int64_t)ks * m + i) * rows + r];
+  for (int ks = 0; ks < split_k; ++ks) s += __ldcg(&partial[((int64_t)ks * m + i) * rows + r]);
   Y[(int64_t)i * ldy + (int64_t)r * ldy_inner] = __float2half_rn(s);
 }
 
@@ -524,7 +526,9 @@ static int launch_gemv(const __half* W, int64_t ldw, const __half* X, int64_t ld
   ++*launches;
   if (split_k > 1) {
     const int n = rows * m;
-    gemv_splitk_reduce_kernel<<<(n + 255) / 256, 256, 0, stream>>>(partial, Y, ldy, ldy_inner, rows, m, split_k);
+    if (launch_overlapped(gemv_splitk_reduce_kernel, dim3((n + 255) / 256), dim3(256), 0, stream, partial, Y, ldy, ldy_inner,
+                          rows, m, split_k) != cudaSuccess)
+      return HELIX_ERR_CUDA;
     ++*launches;
   }
   return cudaGetLastError() == cudaSuccess ? HELIX_OK : HELIX_ERR_CUDA;
@@ -566,17 +570,7 @@ static int launch_stream(void (*kern)(Params...), int& attr_dev, int grid, int t
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return HELIX_ERR_CUDA;
     attr_dev = dev;
   }
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(grid);
-  lc.blockDim = dim3(threads);
-  lc.dynamicSmemBytes = smem;
-  lc.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  if (cudaLaunchKernelEx(&lc, kern, args...) != cudaSuccess) return HELIX_ERR_CUDA;
+  if (launch_overlapped(kern, dim3(grid), dim3(threads), smem, stream, args...) != cudaSuccess) return HELIX_ERR_CUDA;
   ++*launches;
   return HELIX_OK;
 }

@@ -283,17 +283,9 @@ static int launch_stream32(const float* W, int64_t ldw, const float* X, int64_t 
       return HELIX_ERR_CUDA;
     attr_dev = dev;
   }
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(std::min(sm_count, rows));
-  lc.blockDim = dim3(kStream32Threads);
-  lc.dynamicSmemBytes = kStream32RingBytes;
-  lc.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = attr;
-  lc.numAttrs = 1;
-  if (cudaLaunchKernelEx(&lc, kern, W, ldw, X, ldx, Y, ldy, ldy_inner, rows, K, m, kw) != cudaSuccess) return HELIX_ERR_CUDA;
+  if (launch_overlapped(kern, dim3(std::min(sm_count, rows)), dim3(kStream32Threads), kStream32RingBytes, stream, W, ldw, X, ldx,
+                        Y, ldy, ldy_inner, rows, K, m, kw) != cudaSuccess)
+    return HELIX_ERR_CUDA;
   ++*launches;
   return HELIX_OK;
 }

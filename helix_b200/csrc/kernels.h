@@ -7,6 +7,23 @@
 
 namespace helix {
 
+// Launch that may be scheduled while its predecessor on the stream drains; the kernel orders itself with griddep_wait().
+template <typename... Params, typename... Args>
+inline cudaError_t launch_overlapped(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                     Args... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid;
+  lc.blockDim = block;
+  lc.dynamicSmemBytes = smem;
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, kern, static_cast<Params>(args)...);
+}
+
 // ---- gemv_f16.cu
 size_t gemv_f16_workspace_bytes(int rows, int m, int split_k);
 int gemv_f16_default_split(int rows, int K, int sm_count);
