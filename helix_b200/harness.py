@@ -408,7 +408,7 @@ def gemm_f32_result(prof_dict, M, N, K):
 
 
 def time_conv_f32(batch, IC, H, W, OC, kH, kW, stride, pad, cfg=None, iters=10):
-    """Seconds of one true-fp32 NHWC convolution: weight transpose + column matrix + FFMA GEMM."""
+    """Seconds of one true-fp32 NHWC convolution as the library runs it."""
     x = torch.rand((batch, H, W, IC), device="cuda") * 2 - 1
     w = torch.randn((OC, kH, kW, IC), device="cuda") * math.sqrt(2.0 / (IC * kH * kW))
     Ho, Wo = ops.conv_out_hw(H, W, kH, kW, stride, pad)
@@ -419,9 +419,8 @@ def time_conv_f32(batch, IC, H, W, OC, kH, kW, stride, pad, cfg=None, iters=10):
 
 
 def conv_f32_result(prof_dict, batch, IC, H, W, OC, kH, kW, stride, pad):
-    """(cost_ms, tflops) of one fp32 convolution the reference's way: explicit column matrix, then the GEMM on
-    M = B*Ho*Wo, N = OC, K = IC*kH*kW with the configuration the cost model picks for that shape
-    (Ampere_FP32_conv.py:101-113); the time covers all three kernels."""
+    """(cost_ms, tflops) of one fp32 convolution as the GEMM on M = B*Ho*Wo, N = OC, K = IC*kH*kW with the configuration
+    the cost model picks for that shape (Ampere_FP32_conv.py:101-113); the time covers every kernel the call launches."""
     require_gpu()
     Ho, Wo = ops.conv_out_hw(H, W, kH, kW, stride, pad)
     M, N, K = batch * Ho * Wo, OC, IC * kH * kW

@@ -295,7 +295,7 @@ def launch_conv2d_f16(x, w, out, stride, pad, cfg=None, ws=None):
 
 
 def launch_conv2d_f32(x, w, out, stride, pad, cfg=None, ws=None):
-    """x[N,H,W,C], w[KO,R,S,C] -> out[N,Ho,Wo,KO], true fp32 (column matrix + FFMA GEMM in the workspace)."""
+    """x[N,H,W,C], w[KO,R,S,C] -> out[N,Ho,Wo,KO], true fp32 (FFMA GEMM over the windows, see conv_f32.cu)."""
     _require_cuda(x, w, out)
     assert x.dtype == w.dtype == out.dtype == torch.float32
     assert x.is_contiguous() and w.is_contiguous() and out.is_contiguous()

@@ -48,7 +48,7 @@ typedef enum helix_op {
   HELIX_OP_GEMV_F16 = 1, /* memory-bound SIMT GEMV for 1..8 right-hand sides              */
   HELIX_OP_CONV_F16 = 2, /* implicit-GEMM NHWC convolution on the same tensor-core path   */
   HELIX_OP_GEMM_F32 = 3, /* SIMT FFMA GEMM, true fp32                                     */
-  HELIX_OP_CONV_F32 = 4, /* true-fp32 NHWC convolution: column matrix + the FFMA GEMM      */
+  HELIX_OP_CONV_F32 = 4, /* true-fp32 NHWC convolution: the FFMA GEMM over its windows      */
   HELIX_OP_GEMV_F32 = 5  /* true-fp32 memory-bound GEMV for 1..8 right-hand sides          */
 } helix_op_t;
 
@@ -213,20 +213,22 @@ int helix_gemm_f32(const helix_cfg_t* cfg, const float* A, int64_t lda, int tran
  * Y[i*ldy + r*ldy_inner].  K and the leading dimensions are multiples of 4 floats, bases 16-byte aligned.
  * Each output is the shuffle-tree sum (xor 16, 8, 4, 2, 1) of 32 lane chains, lane l adding the elements
  * 4l..4l+3 of every 128-element stretch of K in ascending order: a fixed order, so results repeat bit for
- * bit.  cfg: tile_n = rows per warp (1, 2), load_group = loads in flight (2, 4, 8), split_k; NULL = library
- * choice.  Stands in for the reference's fp32 GEMV template, which none of its scripts builds
+ * bit.  Where rows are few and K is long and the library chooses, warps (or, with split_k > 1, launches' slices)
+ * share the stretches of K and their sums are added in order, again the same one every time.  cfg: tile_n = rows per
+ * warp (1, 2), load_group = loads in flight (2, 4, 8), split_k; NULL = library choice.  Stands in for the reference's fp32 GEMV template, which none of its scripts builds
  * (src_template/Ampere_FP32/gemv_template_fp32.cu:153-218). */
 int helix_gemv_f32(const helix_cfg_t* cfg, const float* W, int64_t ldw, const float* X, int64_t ldx, float* Y,
                    int64_t ldy, int64_t ldy_inner, int rows, int K, int m, void* ws, size_t ws_bytes,
                    void* status_dev, void* stream);
 
-/* y[N,Ho,Wo,KO] = conv2d(x[N,H,W,C], w[KO,R,S,C]) in true fp32, zero padding: a column matrix
- * col[N*Ho*Wo][R*S*C] and the transposed weights are written into the caller's workspace
- * (helix_workspace_bytes; 256-byte aligned), then the FFMA GEMM of helix_gemm_f32 runs on them, so
- * every output is one fmaf chain over (r, s, c) ascending.  Replaces the im2col executable plus
+/* y[N,Ho,Wo,KO] = conv2d(x[N,H,W,C], w[KO,R,S,C]) in true fp32, zero padding; every output is one fmaf
+ * chain over (r, s, c) ascending.  Filters of up to 32 taps are one launch whose loader gathers the windows; for the others
+ * (and for cfg tiles without such a loader) a column matrix col[N*Ho*Wo][R*S*C] and the transposed weights are written
+ * into the caller's workspace and the FFMA GEMM of helix_gemm_f32 runs on them.  The workspace (helix_workspace_bytes;
+ * 256-byte aligned) is asked for in either case.  Replaces the im2col executable plus
  * sgemm executable pair of get_Ampere_FP32_conv_Helix_result
  * (scripts/Ampere_FP32/Ampere_FP32_conv.py:101-113, src_template/Ampere_FP32/im2col.cu:37-97).
- * A 1x1, stride-1, unpadded convolution needs no column matrix.  cfg: a HELIX_OP_GEMM_F32
+ * A 1x1, stride-1, unpadded convolution has no column matrix.  cfg: a HELIX_OP_GEMM_F32
  * configuration or NULL. */
 int helix_conv2d_f32_nhwc(const helix_cfg_t* cfg, const float* x, const float* w, float* y,
                           int N, int H, int W, int C, int KO, int R, int S, int stride, int pad,
