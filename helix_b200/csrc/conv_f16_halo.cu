@@ -110,7 +110,7 @@ __device__ __forceinline__ int issuer_first_tap(int first, int nissue, int issue
 __global__ void __launch_bounds__(kThreads, 1)
 conv_f16_win_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                     const WinParams p) {
-  griddep_launch_dependents();
+  if (p.independent) griddep_launch_dependents();   // else after the wait (common.cuh)
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -167,7 +167,10 @@ conv_f16_win_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  if (!p.independent) griddep_wait();
+  if (!p.independent) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
   if (threadIdx.x == 0) wtrace(p, 2);
 
   if (warp == 0) {

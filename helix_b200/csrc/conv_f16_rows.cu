@@ -63,7 +63,7 @@ struct RowsParams {
 __global__ void __launch_bounds__(kThreads, 1)
 conv_f16_rows_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                      const __grid_constant__ CUtensorMap tmap_y, const RowsParams p) {
-  griddep_launch_dependents();
+  if (p.independent) griddep_launch_dependents();   // else after the wait (common.cuh)
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -106,7 +106,10 @@ conv_f16_rows_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  if (!p.independent) griddep_wait();
+  if (!p.independent) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------------ weights once, then one window per item

@@ -116,7 +116,7 @@ __device__ __forceinline__ void tr(const StemParams& p, int word, unsigned long 
 template <int NACC>
 __global__ void __launch_bounds__(kThreads, 2)
 conv_f16_stem_kernel(const __grid_constant__ CUtensorMap tmap_y, const StemParams p) {
-  griddep_launch_dependents();
+  if (p.independent) griddep_launch_dependents();   // else after the wait (common.cuh)
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -169,7 +169,10 @@ conv_f16_stem_kernel(const __grid_constant__ CUtensorMap tmap_y, const StemParam
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
-  if (!p.independent) griddep_wait();
+  if (!p.independent) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
 
   if (warp != 0) {
     // weights -> [K chunk j = r * 4 + jj][KO / 8][8 rows x 16 bytes]; chunk jj of filter row r holds window

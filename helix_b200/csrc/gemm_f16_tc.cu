@@ -319,9 +319,9 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   constexpr int kTmemCols = L::tmem_cols();
   constexpr uint32_t kIdesc = umma_idesc_f16(kBM, BN);
 
-  // The next kernel on the stream may be scheduled as soon as every CTA of this one has started:
-  // its CTAs then fill SMs as ours retire instead of waiting for the whole grid to drain.
-  griddep_launch_dependents();
+  // The next kernel on the stream may be scheduled once every CTA of this one has got here (an ordered launch: past
+  // its wait): its CTAs then fill SMs as ours retire instead of waiting for the whole grid to drain.
+  if (p.independent) griddep_launch_dependents();
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -388,7 +388,10 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   // Everything above touched only this CTA's shared memory and TMEM, so it may overlap the tail of
   // the preceding kernel.  From here on global memory is read and written: unless the caller
   // declared the launch independent of its predecessor, wait for that kernel to complete.
-  if (!p.independent) griddep_wait();
+  if (!p.independent) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
   if (threadIdx.x == 0 && p.trace != nullptr) p.trace[(size_t)cta * kTraceWords + 2] = (unsigned long long)clock64();
 
   // the MMA-issuing role: warp kMmaWarp, and with dual issue also warp 3, which then issues no loads
@@ -932,8 +935,8 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 // of 128-wide tiles that costs more than it saves (128 x 4096 x 4096: 18.7 -> 23.0; 106 x 2304 x 6920: +4 us).
 __global__ void gemm_streamk_fixup_kernel(const GemmParams p, int bn, int grid, bool overlap) {
   if (overlap) {
-    griddep_launch_dependents();
     griddep_wait();
+    griddep_launch_dependents();
   }
   const int j = blockIdx.y;  // dealt-out tile index
   const int u_lo = j * p.num_kb, u_hi = (j + 1) * p.num_kb;
@@ -1664,7 +1667,7 @@ int gemm_f16_launch(const helix_cfg_t* cfg_in, const void* A, int64_t lda, const
     cfg = *cfg_in;
   } else {
     if (batch == 1 && gemv_f16_stream_covers(B, ldb, A, lda, N, K, M))
-      return gemv_f16_stream_launch(B, ldb, A, lda, C, ldc, 1, N, K, M, sm_count, independent ? 2 : 0, stream, launches);
+      return gemv_f16_stream_launch(B, ldb, A, lda, C, ldc, 1, N, K, M, sm_count, independent ? 2 | kHoldNext : 0, stream, launches);
     gemm_f16_default_config(M, N, K, batch, sm_count, false, &cfg);
     // the automatic choice degrades to the workspace-free schedule when no scratch was passed
     if (!ws || ws_bytes < gemm_f16_workspace_bytes(&cfg, M, N, K, batch, sm_count)) {

@@ -280,7 +280,7 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   constexpr int kTmemCols = 2 * BN <= 256 ? 256 : 512;
   constexpr uint32_t kIdesc = umma_idesc_f16(2 * kBM, BN);
 
-  griddep_launch_dependents();
+  if (p.independent) griddep_launch_dependents();   // else after the wait (common.cuh)
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -328,7 +328,10 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  if (!p.independent) griddep_wait();
+  if (!p.independent) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
   if (threadIdx.x == 0) trace2(p, 2);
 
   if (warp == 0 || warp >= 6) {

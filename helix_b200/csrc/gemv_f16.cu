@@ -32,10 +32,11 @@ gemv_f16_kernel(const __half* __restrict__ W, int64_t ldw, const __half* __restr
   //   2  nothing is shared with it: no wait before the work.
   // In modes 1 and 2 every thread that has not waited yet does so just before it exits, after its last
   // store: this kernel then cannot complete before its predecessor has, so a later kernel that waits
-  // for this one is still ordered after everything queued earlier.
-  griddep_launch_dependents();
+  // for this one is still ordered after everything queued earlier.  The next kernel may start after the wait in mode
+  // 0, at once in modes 1 and 2 (common.cuh).
   bool waited = order_mode == 0;
   if (order_mode == 0) griddep_wait();
+  griddep_launch_dependents();
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int warps_per_block = blockDim.x >> 5;
@@ -147,6 +148,9 @@ constexpr int kStreamWarps = kStreamThreads / 32;
 constexpr int kStreamLoads = 4;      // 16-byte loads of one group
 constexpr int kStreamGroups = 3;     // groups in flight
 constexpr int kStreamRingBytes = kStreamThreads * kStreamLoads * kStreamGroups * 16;
+// order_mode 0, 1 and 2 as above; with kHoldNext the next kernel is held back until after the wait of modes 1 and 2 (used
+// where these kernels stand for launches with a workspace, which are ordered whatever their flags: what was queued before
+// them is complete when a flagged successor starts)
 
 // Rows [begin, end) of this CTA.
 __device__ __forceinline__ void stream_rows(int rows, int& begin, int& end) {
@@ -177,8 +181,8 @@ gemv_f16_stream_kernel(const __half* __restrict__ W, int64_t ldw, const __half* 
   constexpr int kSuperRows = kStreamWarps * kBlockRows;
   extern __shared__ __align__(16) unsigned char stream_smem[];
   float* part = reinterpret_cast<float*>(stream_smem + kStreamRingBytes);   // [2][kw][MRHS][kSuperRows]
-  griddep_launch_dependents();
   if (order_mode == 0) griddep_wait();
+  if (!(order_mode & kHoldNext)) griddep_launch_dependents();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rw = kStreamWarps / kw;                 // row groups
   const int kwi = warp % kw, rwi = warp / kw;
@@ -210,7 +214,10 @@ gemv_f16_stream_kernel(const __half* __restrict__ W, int64_t ldw, const __half* 
   };
 #pragma unroll
   for (int i = 0; i < kStreamGroups; ++i) issue();
-  if (order_mode == 1) griddep_wait();
+  if (order_mode & 1) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
 
   int cslot = 0, buf = 0;
   for (int sb = 0; sb < blocks; sb += kStreamWarps, buf ^= 1) {      // one superblock of up to 64 rows
@@ -276,7 +283,7 @@ gemv_f16_stream_kernel(const __half* __restrict__ W, int64_t ldw, const __half* 
       }
     }
   }
-  if (order_mode == 2) griddep_wait();
+  if (order_mode & 2) griddep_wait();
 }
 
 __device__ __forceinline__ void mma_f16_16x8x16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -311,8 +318,8 @@ gemv_f16_mma_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, 
   constexpr int kGroups = kMmaSlots / (4 * J);
   extern __shared__ __align__(16) unsigned char stream_smem[];
   float* part = reinterpret_cast<float*>(stream_smem + kMmaThreads * kMmaSlots * 16);   // [warp][kTok][16 rows]
-  griddep_launch_dependents();
   if (order_mode == 0) griddep_wait();
+  if (!(order_mode & kHoldNext)) griddep_launch_dependents();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   const int rw = kMmaWarps / kw;
@@ -372,7 +379,10 @@ gemv_f16_mma_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, 
   };
 #pragma unroll
   for (int i = 0; i < kGroups; ++i) issue();
-  if (order_mode == 1) griddep_wait();
+  if (order_mode & 1) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
 
   const __half* xrow[NT];                           // this lane's right-hand side of each group of eight
 #pragma unroll
@@ -455,14 +465,14 @@ gemv_f16_mma_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, 
       }
     }
   }
-  if (order_mode == 2) griddep_wait();
+  if (order_mode & 2) griddep_wait();
 }
 
 // Sums the split-K partials in slice order (deterministic) and rounds once.
 __global__ void gemv_splitk_reduce_kernel(const float* __restrict__ partial, __half* __restrict__ Y, int64_t ldy,
                                           int64_t ldy_inner, int rows, int m, int split_k) {
-  griddep_launch_dependents();
   griddep_wait();
+  griddep_launch_dependents();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * m) return;
   const int i = idx / rows, r = idx - i * rows;
@@ -642,8 +652,10 @@ int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const vo
   // elements a lone launch is all latency and the plain grid is shorter (256 x 256: 1.4 against 1.9 us); with K beyond
   // 32768 and few rows the split keeps more SMs equally busy.
   if (!(cfg && cfg->tile_m != 0) && m <= 2 && (int64_t)rows * K >= (1 << 21) &&
-      (split_k == 1 || (rows >= sm_count && K <= 32768)))
-    return gemv_f16_stream_launch(W, ldw, X, ldx, Y, ldy, ldy_inner, rows, K, m, sm_count, order_mode, stream, launches);
+      (split_k == 1 || (rows >= sm_count && K <= 32768))) {
+    const int order = split_k > 1 && order_mode != 0 ? order_mode | kHoldNext : order_mode;
+    return gemv_f16_stream_launch(W, ldw, X, ldx, Y, ldy, ldy_inner, rows, K, m, sm_count, order, stream, launches);
+  }
   if (need > 0 && (!ws || ws_bytes < need)) {
     if (cfg && cfg->tile_m != 0 && cfg->split_k > 1) return HELIX_ERR_WORKSPACE;
     split_k = 1;  // automatic choice falls back to the workspace-free variant

@@ -115,8 +115,8 @@ gemv_f32_stream_kernel(const float* __restrict__ W, int64_t ldw, const float* X,
   constexpr int kStep = U * 128;                    // elements of K per group
   extern __shared__ __align__(16) unsigned char stream_smem[];
   __shared__ float part[kWarps][RB * MRHS];
-  griddep_launch_dependents();
   griddep_wait();
+  griddep_launch_dependents();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r_begin = static_cast<int>(static_cast<int64_t>(rows) * blockIdx.x / gridDim.x);
   const int r_end = static_cast<int>(static_cast<int64_t>(rows) * (blockIdx.x + 1) / gridDim.x);

@@ -31,7 +31,8 @@ int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const vo
                     int64_t ldy, int64_t ldy_inner, int rows, int K, int m, void* ws, size_t ws_bytes,
                     int sm_count, int order_mode, cudaStream_t stream, int64_t* launches);
 
-// Streaming kernels for up to 16 right-hand sides (no scratch); order_mode as above.
+// Streaming kernels for up to 16 right-hand sides (no scratch); order_mode as above, or with kHoldNext added to 1 or 2.
+constexpr int kHoldNext = 4;
 int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y, int64_t ldy,
                            int64_t ldy_inner, int rows, int K, int m, int sm_count, int order_mode,
                            cudaStream_t stream, int64_t* launches);

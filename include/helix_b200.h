@@ -134,16 +134,20 @@ typedef struct helix_launch {
   uint32_t flags;        /* HELIX_LAUNCH_* bits                                 */
 } helix_launch_t;
 
-/* The caller asserts that nothing this launch reads or writes is written by the kernel queued just
- * before it on the same stream (independent shapes of a sweep).  The kernel then does not wait for
- * that kernel to finish before it loads operands, so consecutive launches overlap at their edges.
- * Without the flag only the set-up phase overlaps.  Ignored for launches that use a workspace.
+/* The caller asserts that this launch shares nothing that either of them writes with the launch queued just
+ * before it on the same stream (independent shapes of a sweep); where that one carries a flag too,
+ * also with the one before it, and so on up to and including the nearest launch without a flag (a kernel of another
+ * library is one).  The kernel then does not wait for them to finish before it loads operands, so
+ * consecutive launches overlap at their edges.  What was queued before that nearest launch is
+ * complete when this one starts.  Without the flag only the set-up phase overlaps.  Ignored for launches that use a
+ * workspace, which count as launches without a flag.
  * A flagged kernel still waits for its predecessor before it exits, so it never completes first: a
  * later launch that is ordered after the flagged one is ordered after everything queued before it. */
 #define HELIX_LAUNCH_INDEPENDENT 1u
-/* GEMV: the caller asserts that operand `a` (the matrix W: weights) is not written by the kernel
- * queued just before this launch, while X may be.  The kernel issues its first batch of W loads,
- * then waits for that kernel, then reads X: launch latency and ramp-up hide behind its tail. */
+/* GEMV: the caller asserts that operand `a` (the matrix W: weights) is not written by the launch queued just
+ * before this one nor, where that one carries a flag, by those before it up to and including the nearest launch without
+ * one, while X may be.  The kernel issues its first batch of W loads, then waits for the launch before it, then reads X:
+ * launch latency and ramp-up hide behind its tail. */
 #define HELIX_LAUNCH_STATIC_A 2u
 
 /* Library version (major*100 + minor). */
