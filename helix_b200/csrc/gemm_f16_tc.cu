@@ -1375,6 +1375,10 @@ void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) 
     default_config_impl(M, g.KO, K, 1, sm_count, false, true, out);
   else if (conv_im2col_eligible(g)) {
     default_config_impl(M, g.KO, im2col_k(g), 1, sm_count, false, false, out);
+    // Few pixels: a GEMM would put them on the tile's wide axis and cut K, but a swapped tile reads its pixels in whole
+    // boxes of 32 and more and is not built for a cut K.  The plain tiles cut K as well.
+    if (out->swap_ab && (out->stream_k || out->split_k > 1 || out->tile_n < 32))
+      default_config_impl(M, g.KO, im2col_k(g), 1, sm_count, true, false, out);
     // A 128 x N x 16 step costs max(N / 2 cycles of pipe time, (128 + N) / 4 cycles of operand fetch from shared
     // memory): the wide tile does twice the work of a 128-wide one in 1.5x the fetch time, so 65..128 output channels
     // are better spent as the 128 rows with 256 pixels per step: measured 17.1 -> 13.9 us on 3x3, 128 -> 128

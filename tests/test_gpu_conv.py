@@ -407,3 +407,28 @@ def test_conv_192_pixel_tiles(oracle, geom):
     got = _run(x, w, stride, pad, ops.make_cfg(OP_CONV_F16, tile_m=128, tile_n=192, tile_k=64, swap_ab=1))
     _, y32 = oracle.conv2d_nhwc_f16(x, w, stride, pad)
     util.assert_f16_close(got, y32, f"conv {geom}")
+
+
+@pytest.mark.parametrize("geom", [
+    (1, 480, 14, 14, 512, 3, 3, 2, 1),     # 49 pixels, filled channel block
+    (1, 512, 14, 14, 512, 3, 3, 2, 1),     # the same, whole blocks
+    (1, 1056, 8, 8, 1024, 1, 1, 2, 0),     # 16 pixels, many output channels: a GEMM would deal out slabs of K
+    (1, 1088, 8, 8, 136, 1, 1, 2, 0),      # 16 pixels: a tile narrower than the pixel boxes
+    (2, 608, 8, 8, 256, 3, 3, 2, 1),       # 32 pixels
+    (1, 1000, 9, 9, 1024, 5, 5, 1, 0),     # 25 pixels, long K
+])
+def test_conv_of_few_pixels_over_the_im2col_map(oracle, geom):
+    B, C, H, W, OC, kh, kw, stride, pad = geom
+    assert ops.conv_reads_tensor_map(B, H, W, C, stride)
+    x, w = datagen.c4_conv(*geom, seed=43)
+    _, y32 = oracle.conv2d_nhwc_f16(x, w, stride, pad)
+    util.assert_f16_close(_run(x, w, stride, pad), y32, f"conv {geom}")
+    out = torch.full(y32.shape, float("nan"), dtype=torch.float16, device="cuda")
+    l = ops.launch_conv2d_f16(torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda(), out, stride, pad)
+    l.ws, l.ws_bytes = None, 0             # the choice without scratch
+    ops.run(l)
+    torch.cuda.synchronize()
+    # One accumulator per output: up to 25000 products are K / 16 rounded steps of a sum of size 1, i.e. an error of
+    # sqrt(K / 16) * 2^-23 = 5e-6 and four times that at the largest of 25600 outputs, which for an output of 1e-3 is more than
+    # the element bound of 1e-2 (1e-5).  The norm bound holds whatever K.
+    assert util.rel_fro(out.cpu().numpy(), y32) <= util.F16_FRO_TOL
