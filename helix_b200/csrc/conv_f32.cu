@@ -103,6 +103,7 @@ static int conv_f32_implicit(const helix_cfg_t* cfg, const float* x, const float
   if (c.stages < 3) return HELIX_ERR_UNSUPPORTED;
   RingParams p{};
   p.A = x; p.B = w; p.C = y;
+  p.none = x;                  // the filters always go by 4 bytes
   p.lda = g.C; p.ldb = K; p.ldc = g.KO;
   p.M = M; p.N = g.KO; p.K = K;
   p.vec_c = (g.KO & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;

@@ -313,6 +313,7 @@ int sgemm_f32_launch(const helix_cfg_t* cfg, const float* A, int64_t lda, int tr
     p.vec_c = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
     const bool a16 = (lda & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
     const bool b16 = (ldb & 3) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
+    p.none = b16 ? B : A;      // columns of B go by 16 bytes with b16, rows and columns of A only where B's do too
     int rc = HELIX_ERR_UNSUPPORTED;
     if (bm == 128 && bn == 128 && bk == 16) rc = launch_any<RingTile128x128>(p, ta, a16, b16, stream);
     else if (bm == 128 && bn == 64 && bk == 16) rc = launch_any<RingTile128x64>(p, ta, a16, b16, stream);

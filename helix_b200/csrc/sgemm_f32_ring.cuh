@@ -32,6 +32,9 @@ struct RingParams {
   const float* B;
   float* C;
   int64_t lda, ldb, ldc;
+  // Source of copies of nothing (an absent row, column or k): these too need a source aligned to their size.  A or B, one
+  // that starts on 16 bytes where a loader copies 16.
+  const float* none;
   int M, N, K, tiles_n;
   int vec_c;                         // rows of C may be written 16 bytes at a time
   // kWindow4, kWindow16: A is x[N][H][W][C]
@@ -98,7 +101,7 @@ struct RingLoader<kRows4, ROWS, BK, NT, PITCH> {
 #pragma unroll
         for (int o = 0; o < BK / 8; ++o) {
           const bool in = k0 + o * 8 + kk < p.K;
-          ring_cp4(dst + stage_off + (o * 8 * PITCH + i * kPassRows) * 4, in ? run + off[i] + o * 8 : p.A, in ? 4 : 0);
+          ring_cp4(dst + stage_off + (o * 8 * PITCH + i * kPassRows) * 4, in ? run + off[i] + o * 8 : p.none, in ? 4 : 0);
         }
     }
     run += BK;
@@ -129,7 +132,7 @@ struct RingLoader<kCols16, ROWS, BK, NT, PITCH> {
 #pragma unroll
       for (int i = 0; i < kPasses; ++i) {
         const int b = k0 + kr + i * kPassK < p.K ? bytes : 0;
-        ring_cp16(dst + stage_off + i * kPassK * PITCH * 4, b ? run + i * kPassK * ld : p.A, b);
+        ring_cp16(dst + stage_off + i * kPassK * PITCH * 4, b ? run + i * kPassK * ld : p.none, b);
       }
     }
     if (bytes) run += BK * ld;
@@ -157,7 +160,7 @@ struct RingLoader<kCols4, ROWS, BK, NT, PITCH> {
 #pragma unroll
     for (int i = 0; i < kPasses; ++i) {
       const bool ok = in && k0 + kr + i * kPassK < p.K;
-      ring_cp4(dst + stage_off + i * kPassK * PITCH * 4, ok ? run + i * kPassK * ld : p.A, ok ? 4 : 0);
+      ring_cp4(dst + stage_off + i * kPassK * PITCH * 4, ok ? run + i * kPassK * ld : p.none, ok ? 4 : 0);
     }
     run += BK * ld;
   }
@@ -241,7 +244,7 @@ struct RingLoader<kRows16, ROWS, BK, NT, PITCH> {
       const int bytes = max(0, min(4, p.K - (k0 + kk))) * 4;
 #pragma unroll
       for (int i = 0; i < kPasses; ++i)
-        ring_cp16(dst + stage_off + i * kPassRows * BK * 4, bytes ? run + off[i] : p.A, bytes);
+        ring_cp16(dst + stage_off + i * kPassRows * BK * 4, bytes ? run + off[i] : p.none, bytes);
     }
     run += BK;
   }

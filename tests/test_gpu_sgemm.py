@@ -109,3 +109,21 @@ def test_sgemm_ring_tiles_take_any_alignment_and_stay_the_fmaf_chain(oracle, sha
         out = torch.empty((M, N), device="cuda")
         ops.run(ops.launch_gemm_f32(ad, big[:, :N], out, trans_a, cfg))
         assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32)), pad
+
+
+@pytest.mark.parametrize("cfg_idx", [None, 0, 1, 2, 3, 4, 10, 11, 12])
+@pytest.mark.parametrize("M,N,K,lda,ldb", [(70, 36, 21, 24, 36), (33, 130, 50, 53, 132), (129, 67, 7, 8, 68)])
+def test_sgemm_ring_with_a_base_of_its_own_alignment(oracle, M, N, K, lda, ldb, cfg_idx):
+    """A starts 4 bytes behind a 16-byte boundary while B's rows start on one: columns and k that do not exist are copies of
+    nothing whose source must be aligned all the same."""
+    a, b = datagen.c1_fp32_gemm(M, N, K, seed=M)
+    ad = torch.as_strided(torch.full((M * lda + 4,), float("nan"), device="cuda"), (M, K), (lda, 1), 1)
+    bd = torch.full((K, ldb), float("nan"), device="cuda")
+    ad.copy_(torch.from_numpy(a))
+    bd[:, :N] = torch.from_numpy(b).cuda()
+    assert ad.data_ptr() % 16 == 4 and bd.data_ptr() % 16 == 0
+    out = torch.empty((M, N), device="cuda")
+    cfg = None if cfg_idx is None else ops.configs(OP_GEMM_F32)[cfg_idx]
+    ops.run(ops.launch_gemm_f32(ad, bd[:, :N], out, cfg=cfg))
+    want = oracle.sgemm_naive(a, b, fma=True)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
