@@ -67,6 +67,15 @@ __device__ __forceinline__ void ring_cp16(uint32_t dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
+// Row r of the tile at r0, relative to r0.  Rows that do not exist are read from the tile before: their results are not
+// stored.  Not from the last row, but in the only tile: every column tile reading that up to 31 times at once is a hot spot of
+// the L2 (130 x 3000 x 60 took 7.2 us, now 3.9; 140 x 2140 x 60: 6.9, now 3.6).
+template <int ROWS>
+__device__ __forceinline__ int ring_row(int r0, int r, int rows) {
+  const int absent = r0 > 0 ? r - ROWS : rows - 1;
+  return r0 + r < rows ? r : absent;
+}
+
 // ROWS rows of the operand from r0 on; slabs are asked for in order, one issue() per slab.
 template <int SRC, int ROWS, int BK, int NT, int PITCH>
 struct RingLoader;
@@ -84,8 +93,7 @@ struct RingLoader<kRows4, ROWS, BK, NT, PITCH> {
     kk = threadIdx.x % 8;
     run = p + r0 * ld + kk;
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i)      // rows that do not exist repeat the last one: their results are not stored
-      off[i] = static_cast<int>((min(r0 + r + i * kPassRows, rows - 1) - r0) * ld);
+    for (int i = 0; i < kPasses; ++i) off[i] = static_cast<int>(ring_row<ROWS>(r0, r + i * kPassRows, rows) * ld);
     dst = smem + (kk * PITCH + r) * 4;
   }
   __device__ __forceinline__ void issue(const RingParams& p, int k0, uint32_t stage_off) {
@@ -168,7 +176,7 @@ struct RingLoader<kCols4, ROWS, BK, NT, PITCH> {
 
 // A row of the column matrix: output pixel m, k ordered (r, s, c).  A thread keeps, per row, the offset of the window's
 // origin and one bit per filter tap that says whether the tap lies inside the image (R * S <= 32).
-__device__ __forceinline__ void ring_window(const RingParams& p, int m, int& off, uint32_t& taps) {
+__device__ __forceinline__ void ring_window(const RingParams& p, int m, int rows, int& off, uint32_t& taps) {
   int t, wo, n, ho;
   fast_divmod(m, p.fd_wo, t, wo);
   fast_divmod(t, p.fd_ho, n, ho);
@@ -177,6 +185,7 @@ __device__ __forceinline__ void ring_window(const RingParams& p, int m, int& off
   const int s_lo = max(0, -w), s_hi = min(p.S, p.W - w);
   const uint32_t cols = s_hi > s_lo ? static_cast<uint32_t>((1ull << s_hi) - (1ull << s_lo)) : 0u;
   taps = 0;
+  if (m >= rows) return;                   // a pixel that does not exist
   for (int q = max(0, -h); q < min(p.R, p.H - h); ++q) taps |= cols << (q * p.S);
 }
 template <int ROWS, int BK, int NT, int PITCH>
@@ -191,7 +200,7 @@ struct RingLoader<kWindow4, ROWS, BK, NT, PITCH> {
     const int r = threadIdx.x / 8;
     kk = threadIdx.x % 8;
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i) ring_window(p, min(r0 + r + i * kPassRows, rows - 1), off[i], taps[i]);
+    for (int i = 0; i < kPasses; ++i) ring_window(p, r0 + r + i * kPassRows, rows, off[i], taps[i]);
     dst = smem + (kk * PITCH + r) * 4;
   }
   __device__ __forceinline__ void issue(const RingParams& p, int k0, uint32_t stage_off) {
@@ -232,8 +241,7 @@ struct RingLoader<kRows16, ROWS, BK, NT, PITCH> {
     kk = ch * 4;
     run = p + r0 * ld + kk;
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i)
-      off[i] = static_cast<int>((min(r0 + r + i * kPassRows, rows - 1) - r0) * ld);
+    for (int i = 0; i < kPasses; ++i) off[i] = static_cast<int>(ring_row<ROWS>(r0, r + i * kPassRows, rows) * ld);
     dst = smem + (r * BK + (ch ^ ring_swizzle<BK>(r)) * 4) * 4;
   }
   __device__ __forceinline__ void issue(const RingParams& p, int k0, uint32_t stage_off) {
@@ -262,7 +270,7 @@ struct RingLoader<kWindow16, ROWS, BK, NT, PITCH> {     // channels a multiple o
     const int r = threadIdx.x / kChunks, ch = threadIdx.x % kChunks;
     kk = ch * 4;
 #pragma unroll
-    for (int i = 0; i < kPasses; ++i) ring_window(p, min(r0 + r + i * kPassRows, rows - 1), off[i], taps[i]);
+    for (int i = 0; i < kPasses; ++i) ring_window(p, r0 + r + i * kPassRows, rows, off[i], taps[i]);
     dst = smem + (r * BK + (ch ^ ring_swizzle<BK>(r)) * 4) * 4;
   }
   __device__ __forceinline__ void issue(const RingParams& p, int k0, uint32_t stage_off) {

@@ -127,3 +127,19 @@ def test_sgemm_ring_with_a_base_of_its_own_alignment(oracle, M, N, K, lda, ldb, 
     ops.run(ops.launch_gemm_f32(ad, bd[:, :N], out, cfg=cfg))
     want = oracle.sgemm_naive(a, b, fma=True)
     assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("cfg_idx", [None, 0, 2, 10, 11, 12])
+@pytest.mark.parametrize("M,N,K", [(130, 132, 60), (145, 96, 12), (33, 68, 16), (257, 40, 32)])
+def test_sgemm_tiles_that_end_inside_the_rows(oracle, M, N, K, cfg_idx):
+    """Tiles that end one or two rows into A, a K of less than a slab, of whole slabs and with a tail: nothing behind A's last
+    row is read or written, and the result stays the fmaf chain."""
+    a, b = datagen.c1_fp32_gemm(M, N, K, seed=M + K)
+    store = torch.full(((M + 128) * K,), float("nan"), device="cuda")
+    store[:M * K] = torch.from_numpy(a).cuda().flatten()
+    out = torch.full((M + 4, N), -3.0, device="cuda")
+    cfg = None if cfg_idx is None else ops.configs(OP_GEMM_F32)[cfg_idx]
+    ops.run(ops.launch_gemm_f32(store[:M * K].view(M, K), torch.from_numpy(b).cuda(), out[:M], cfg=cfg))
+    got = out.cpu().numpy()
+    want = oracle.sgemm_naive(a, b, fma=True)
+    assert np.array_equal(got[:M].view(np.uint32), want.view(np.uint32)) and np.all(got[M:] == -3.0)
