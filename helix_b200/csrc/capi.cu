@@ -265,13 +265,14 @@ int helix_default_config(const helix_launch_t* l, helix_cfg_t* out) {
       out->split_k = helix::gemv_f32_default_split(l->N, l->K, sms);
       return HELIX_OK;
     case HELIX_OP_GEMM_F32:
-      helix::sgemm_f32_default_config(l->M, l->N, sms, out);
+      helix::sgemm_f32_default_config(l->M, l->N, l->K, sms, out);
       return HELIX_OK;
     case HELIX_OP_CONV_F32: {
       const helix::ConvGeom g = conv_geom(l->conv);
       const int64_t M = (int64_t)g.NB * g.Ho * g.Wo;
       if (M <= 0 || M > 0x7fffffff || g.KO <= 0) return HELIX_ERR_INVALID;
-      helix::sgemm_f32_default_config((int)M, g.KO, sms, out);
+      const int64_t K = std::min<int64_t>((int64_t)g.R * g.S * g.C, 0x7fffffff);
+      helix::sgemm_f32_default_config((int)M, g.KO, (int)K, sms, out);
       out->op = HELIX_OP_CONV_F32;
       return HELIX_OK;
     }

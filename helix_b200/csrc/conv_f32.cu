@@ -99,7 +99,7 @@ static int conv_f32_implicit(const helix_cfg_t* cfg, const float* x, const float
   if (K >= (1 << 23)) return HELIX_ERR_UNSUPPORTED;
   helix_cfg_t c{};
   if (cfg && cfg->tile_m != 0) c = *cfg;
-  else sgemm_f32_default_config(M, g.KO, sm_count, &c);
+  else sgemm_f32_default_config(M, g.KO, K, sm_count, &c);
   if (c.stages < 3) return HELIX_ERR_UNSUPPORTED;
   RingParams p{};
   p.A = x; p.B = w; p.C = y;

@@ -56,7 +56,7 @@ int gemv_f32_launch(const helix_cfg_t* cfg, const float* W, int64_t ldw, const f
 // ---- sgemm_f32.cu
 int sgemm_f32_num_configs();
 void sgemm_f32_get_config(int idx, helix_cfg_t* out);
-void sgemm_f32_default_config(int M, int N, int sm_count, helix_cfg_t* out);
+void sgemm_f32_default_config(int M, int N, int K, int sm_count, helix_cfg_t* out);
 int sgemm_f32_launch(const helix_cfg_t* cfg, const float* A, int64_t lda, int trans_a, const float* B, int64_t ldb,
                      float* C, int64_t ldc, int M, int N, int K, int sm_count, cudaStream_t stream,
                      int64_t* launches);
