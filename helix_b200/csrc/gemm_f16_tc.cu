@@ -1521,7 +1521,8 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
                          GemmParams& p, void* C, int64_t ldc, int64_t sc, void* ws, size_t ws_bytes, int sm_count,
                          bool independent, cudaStream_t stream, int64_t* launches) {
   const int bn = cfg.tile_n;
-  if (bn == 192 && (cfg.stream_k || cfg.split_k > 1)) return HELIX_ERR_UNSUPPORTED;   // whole tiles only
+  // 192 wide: whole tiles of the tensor-map kernel only
+  if (bn == 192 && (conv || cfg.stream_k || cfg.split_k > 1)) return HELIX_ERR_UNSUPPORTED;
   p.tiles_m = (p.PM + kBM - 1) / kBM;
   p.tiles_n = (p.PN + bn - 1) / bn;
   p.num_kb = (p.K + kBK - 1) / kBK;
@@ -1629,7 +1630,10 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
     break;
   switch (bn) {
     HELIX_BN_CASE(256)
-    HELIX_BN_CASE(192)
+    case 192:
+      e = any ? launch_variant<192, false, true>(ta, tb, tc, p, grid, smem, stream)
+              : launch_variant<192, false, false>(ta, tb, tc, p, grid, smem, stream);
+      break;
     HELIX_BN_CASE(128)
     HELIX_BN_CASE(64)
     HELIX_BN_CASE(32)

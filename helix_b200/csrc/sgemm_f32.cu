@@ -306,6 +306,7 @@ int sgemm_f32_launch(const helix_cfg_t* cfg, const float* A, int64_t lda, int tr
     stages = def.stages;
   }
   const bool ta = trans_a != 0;
+  if (bm == 32 && bn == 32 && !(stages >= 3 && bk == 32)) return HELIX_ERR_UNSUPPORTED;   // a ring tile only
   // the ring kernel addresses the rows of a tile with 32-bit offsets
   if (stages >= 3 && lda < (1 << 23) && ldb < (1 << 23)) {
     RingParams p{};

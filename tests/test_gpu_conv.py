@@ -432,3 +432,11 @@ def test_conv_of_few_pixels_over_the_im2col_map(oracle, geom):
     # sqrt(K / 16) * 2^-23 = 5e-6 and four times that at the largest of 25600 outputs, which for an output of 1e-3 is more than
     # the element bound of 1e-2 (1e-5).  The norm bound holds whatever K.
     assert util.rel_fro(out.cpu().numpy(), y32) <= util.F16_FRO_TOL
+
+
+def test_gathering_convolution_has_no_192_wide_tile():
+    x = torch.zeros((1, 9, 9, 16), dtype=torch.float16, device="cuda")
+    w = torch.zeros((24, 3, 3, 16), dtype=torch.float16, device="cuda")
+    with pytest.raises(Exception) as e:
+        ops.conv2d_f16_nhwc(x, w, 1, 1, cfg=ops.make_cfg(OP_CONV_F16, tile_m=128, tile_n=192, tile_k=64))
+    assert "-6" in str(e.value)

@@ -143,3 +143,12 @@ def test_sgemm_tiles_that_end_inside_the_rows(oracle, M, N, K, cfg_idx):
     got = out.cpu().numpy()
     want = oracle.sgemm_naive(a, b, fma=True)
     assert np.array_equal(got[:M].view(np.uint32), want.view(np.uint32)) and np.all(got[M:] == -3.0)
+
+
+@pytest.mark.parametrize("tile", [(32, 32, 16, 2), (32, 32, 16, 4), (32, 32, 32, 2), (32, 32, 8, 3)])
+@pytest.mark.parametrize("n", [64, 66])
+def test_sgemm_refuses_a_32x32_tile_that_is_not_the_rings(tile, n):
+    cfg = ops.make_cfg(OP_GEMM_F32, tile_m=tile[0], tile_n=tile[1], tile_k=tile[2], stages=tile[3])
+    with pytest.raises(Exception) as e:
+        ops.gemm_f32(torch.zeros((64, 64), device="cuda"), torch.zeros((64, n), device="cuda"), cfg=cfg)
+    assert "-6" in str(e.value)
