@@ -113,13 +113,6 @@ int dispatch(const helix_launch_t* l, void* status_dev, cudaStream_t stream) {
       break;
     case HELIX_OP_GEMV_F16:
       if ((rc = current_device(&info, false)) != HELIX_OK) return rc;
-      // Three or more right-hand sides: the SIMT kernel becomes issue bound (measured 11.7 us at
-      // m = 4 and 22 us at m = 8 on 4096 x 4096); the streaming kernel contracts on the matrix units.
-      if (!cfg && l->M >= 3 && l->M <= 8) {
-        rc = helix::gemv_f16_stream_launch(l->a, l->lda, l->b, l->ldb, l->c, l->ldc, l->ldc_inner, l->N, l->K, l->M,
-                                           sms_of(info), gemv_order, stream, &n);
-        break;
-      }
       rc = helix::gemv_f16_launch(cfg, l->a, l->lda, l->b, l->ldb, l->c, l->ldc, l->ldc_inner, l->N, l->K, l->M,
                                   l->ws, l->ws_bytes, sms_of(info),
                                   gemv_order, stream, &n);

@@ -1,4 +1,5 @@
-// Memory-bound fp16 GEMV for 1..8 right-hand sides (non tensor core).
+// Memory-bound fp16 GEMV for 1..8 right-hand sides, and products of up to 16 rows: a plain kernel (explicit configurations, split
+// K, small problems), and streaming kernels, with scalar multiply-adds up to two right-hand sides and mma.sync beyond.
 //
 //   Y[i, r] = sum_k W[r, k] * X[i, k]        W: rows x K (row-major, the HBM stream)
 //                                              X: m x K, m <= 8 (stays in L1/L2)
@@ -7,7 +8,7 @@
 // (gemv_splitK.cu:153-221); unlike those it accumulates in fp32, takes any row count and any
 // K that is a multiple of 8, and reduces split-K partials deterministically.
 //
-// Mapping: one warp owns RPW consecutive rows; lane l reads the 16-byte chunk l of each
+// Mapping of the plain kernel: one warp owns RPW consecutive rows; lane l reads the 16-byte chunk l of each
 // 512-byte row segment, UNROLL segments in flight per row, so a thread keeps RPW*UNROLL
 // independent 128-bit streaming loads outstanding.  Lanes are reduced with a shuffle tree.
 #include <algorithm>
@@ -303,7 +304,8 @@ __device__ __forceinline__ void mma_f16_16x8x16(float (&d)[4], uint32_t a0, uint
 // consecutive elements at k + 8 t of row g as the K positions 2t, 2t + 1, 2t + 8, 2t + 9 of two instructions, for the
 // weights and for X alike, so every product still meets its partner.  X does not fit the L1 that two resident CTAs
 // leave, so its fragments come from L2 and are fetched one group ahead, which takes registers: 8 warps of up
-// to 128, each with a FIFO of 24 slots (the same 96 KB).
+// to 128, each with a FIFO of 24 slots (the same 96 KB where a block has 32 rows; a CTA of fewer keeps 3 KB per row in flight,
+// which is why few rows over a long K go elsewhere).
 constexpr int kMmaThreads = 256;
 constexpr int kMmaWarps = kMmaThreads / 32;
 constexpr int kMmaSlots = 24;
@@ -564,7 +566,7 @@ static int launch_gemv_variant(int rpw, int unroll, const __half* W, int64_t ldw
   return HELIX_ERR_UNSUPPORTED;
 }
 
-// Warps that split K: a power of two with at least `unit` elements of K for each.
+// Warps that split K: the smallest power of two whose shares of whole `unit`s cover K.
 static int stream_k_warps(int K, int unit, int warps) {
   int kw = warps;
   while (kw > 1 && (int64_t)(kw / 2) * unit >= K) kw /= 2;
@@ -619,6 +621,30 @@ int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ld
                        ldy_inner, rows, K, m, kw, order_mode);
 }
 
+// Which GEMVs without a configuration of their own the streaming kernels run (whatever their flags, which change no bits).
+// `split`: what gemv_f16_default_split says, `scratch`: there is room for its partial sums.  us, ordered, kernel above /
+// streaming:
+static bool gemv_f16_streams(int rows, int K, int m, int split, bool scratch, int sm_count) {
+  const int64_t work = (int64_t)rows * K;
+  if (m <= 2) {
+    // Below 2 M elements a lone launch is all latency and the plain grid is shorter (256 x 256: 1.4 / 1.9).
+    if (work < 1 << 21) return false;
+    // Streaming needs no partial sums in memory and cuts K among the warps of a CTA, so it also takes row counts for which
+    // the kernel above would split K over CTAs (700 x 12000: 11.9 / 6.7); with K beyond 32768 and few rows the split keeps
+    // more SMs equally busy.
+    if (split > 1) return rows >= sm_count && K <= 32768;
+    // Many short rows: every 64 of them end in a barrier and a sum over the warps.  m = 1: 4096 x 768 3.3 / 3.5, 5000 x 1536
+    // 5.4 / 5.7, 8192 x 1024 4.8 / 5.6, 12000 x 3072 14.8 / 15.7; 4096 x 1280 4.7 / 4.7, 6000 x 2048 6.9 / 7.1 (with static
+    // weights 5.7 / 5.5), 8192 x 4096 13.6 / 13.2.
+    return m == 2 || rows < 4096 || K > 3072 || (rows < 8192 && K > 1536) || (rows < 5000 && K > 768);
+  }
+  // The matrix kernel's chain over K takes about K / 1000 us whatever m, the split kernel's m times K / split: m = 3,
+  // 64 x 65536 15.3 / 66, 512 x 8192 9.2 / 10.9 (split 4), 700 x 8192 14.9 / 11.0 (split 2); m = 8, 64 x 65536 36 / 74 (split
+  // 16), 148 x 16384 19.1 / 20.4, 296 x 16384 34.9 / 20.6 (split 4).
+  if (scratch) return split < m || (split == m && rows < 64);
+  return !(m == 3 && K <= 256 && rows <= 512);         // 256 x 256: 1.9 / 2.2
+}
+
 // Nine to sixteen right-hand sides read twice the X per weight, from L2 and once per block of rows; with more than some 100 MB
 // of weights the stream-K tcgen05 tiles are ahead (16 x 16000 x 5120: 37.8 us here, 36.3 there; 16 x 12288 x 4096: 24.9 and
 // 26.0; 16 x 4096 x 4096: 10.6 and 15.0).
@@ -647,13 +673,9 @@ int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const vo
                                                               : gemv_f16_default_split(rows, K, sm_count);
   if (split_k > 1 && (K + split_k - 1) / split_k < 256) split_k = 1;
   const size_t need = gemv_f16_workspace_bytes(rows, m, split_k);
-  // The streaming kernel needs no partial sums in memory and cuts K among the warps of a CTA, so it also takes row counts
-  // for which the kernel above would split K over CTAs (700 x 12000: 11.9 -> 6.7 us, ordered launches).  Below 2 M
-  // elements a lone launch is all latency and the plain grid is shorter (256 x 256: 1.4 against 1.9 us); with K beyond
-  // 32768 and few rows the split keeps more SMs equally busy.
-  if (!(cfg && cfg->tile_m != 0) && m <= 2 && (int64_t)rows * K >= (1 << 21) &&
-      (split_k == 1 || (rows >= sm_count && K <= 32768))) {
-    const int order = split_k > 1 && order_mode != 0 ? order_mode | kHoldNext : order_mode;
+  const bool scratch = need > 0 && ws && ws_bytes >= need;
+  if (!(cfg && cfg->tile_m != 0) && gemv_f16_streams(rows, K, m, split_k, scratch, sm_count)) {
+    const int order = scratch && order_mode != 0 ? order_mode | kHoldNext : order_mode;
     return gemv_f16_stream_launch(W, ldw, X, ldx, Y, ldy, ldy_inner, rows, K, m, sm_count, order, stream, launches);
   }
   if (need > 0 && (!ws || ws_bytes < need)) {

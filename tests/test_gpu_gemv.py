@@ -126,3 +126,39 @@ def test_skinny_gemm_through_the_streaming_kernel(oracle, M, N, K):
     with pytest.raises(Exception) as e:
         ops.run(ops.launch_gemm_f16(a[:, 1:K - 7], b[:, :K - 8], out[:, :N]))
     assert "-2" in str(e.value)
+
+
+@pytest.mark.parametrize("rows,K,m,launches", [(64, 65536, 3, 2), (64, 16384, 8, 2), (148, 32768, 4, 2), (512, 8192, 3, 2),
+                                               (700, 8192, 3, 1), (296, 16384, 8, 1), (40, 4096, 4, 1)])
+def test_few_long_rows_are_cut_over_ctas_where_that_is_faster(oracle, rows, K, m, launches):
+    """Three and more right-hand sides: split over CTAs (a kernel and the sum of its slices) or shared by the warps of one."""
+    w, x = datagen.c2_gemv(rows, K, m, seed=rows + m)
+    wd, xd = torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda()
+    out = torch.empty((m, rows), dtype=torch.float16, device="cuda")
+    l = ops.launch_gemv_f16(wd, xd, out)
+    before = ops.launch_count()
+    ops.run(l)
+    assert ops.launch_count() - before == launches
+    _, ref32 = oracle.hgemm_naive(x, w)
+    util.assert_f16_close(out.cpu().numpy(), ref32, f"gemv {rows}x{K} m={m}")
+    l.ws, l.ws_bytes = None, 0             # without room for partial sums: one launch
+    out.zero_()
+    ops.run(l)
+    assert ops.launch_count() - before == launches + 1
+    util.assert_f16_close(out.cpu().numpy(), ref32, f"gemv {rows}x{K} m={m} without scratch")
+
+
+@pytest.mark.parametrize("rows,K,m", [(8192, 3072, 1), (8192, 3080, 1), (4096, 2048, 1), (6000, 1536, 1), (256, 256, 3),
+                                      (512, 2048, 4), (777, 2048, 8), (2048, 1024, 4), (4096, 4104, 8), (4104, 4096, 3)])
+@pytest.mark.parametrize("flag", [0, 1, 2])
+def test_gemv_on_both_sides_of_its_kernel_choice(oracle, rows, K, m, flag):
+    w, x = datagen.c2_gemv(rows, K, m, seed=rows + K + m)
+    wd, xd = torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda()
+    _, ref32 = oracle.hgemm_naive(x, w)
+    for transposed in (False, True):
+        out = torch.full((rows, m) if transposed else (m, rows), float("nan"), dtype=torch.float16, device="cuda")
+        l = ops.launch_gemv_f16(wd, xd, out, out_transposed=transposed)
+        l.flags = flag
+        ops.run(l)
+        got = out.cpu().numpy()
+        util.assert_f16_close(got.T if transposed else got, ref32, f"gemv {rows}x{K} m={m} flag={flag}")
