@@ -1674,11 +1674,14 @@ int gemm_f16_launch(const helix_cfg_t* cfg_in, const void* A, int64_t lda, const
   if (cfg_in && cfg_in->tile_m != 0) {
     cfg = *cfg_in;
   } else {
-    if (batch == 1 && gemv_f16_stream_covers(B, ldb, A, lda, N, K, M))
-      return gemv_f16_stream_launch(B, ldb, A, lda, C, ldc, 1, N, K, M, sm_count, independent ? 2 | kHoldNext : 0, stream, launches);
     gemm_f16_default_config(M, N, K, batch, sm_count, false, &cfg);
+    const size_t need = gemm_f16_workspace_bytes(&cfg, M, N, K, batch, sm_count);
+    const bool scratch = need > 0 && ws && ws_bytes >= need;
+    if (batch == 1 && gemv_f16_stream_covers(B, ldb, A, lda, N, K, M, sm_count, scratch))
+      return gemv_f16_stream_launch(B, ldb, A, lda, C, ldc, 1, N, K, M, sm_count,
+                                    !independent ? 0 : scratch ? 2 | kHoldNext : 2, stream, launches);
     // the automatic choice degrades to the workspace-free schedule when no scratch was passed
-    if (!ws || ws_bytes < gemm_f16_workspace_bytes(&cfg, M, N, K, batch, sm_count)) {
+    if (!ws || ws_bytes < need) {
       cfg.stream_k = 0;
       cfg.split_k = 1;
     }

@@ -645,13 +645,25 @@ static bool gemv_f16_streams(int rows, int K, int m, int split, bool scratch, in
   return !(m == 3 && K <= 256 && rows <= 512);         // 256 x 256: 1.9 / 2.2
 }
 
-// Nine to sixteen right-hand sides read twice the X per weight, from L2 and once per block of rows; with more than some 100 MB
-// of weights the stream-K tcgen05 tiles are ahead (16 x 16000 x 5120: 37.8 us here, 36.3 there; 16 x 12288 x 4096: 24.9 and
-// 26.0; 16 x 4096 x 4096: 10.6 and 15.0).
-bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m) {
-  return m >= 1 && m <= 16 && (m <= 8 || (int64_t)rows * K <= 52 << 20) && rows >= 1024 && K >= 512 && (K & 7) == 0 && ((ldw ? ldw : K) & 7) == 0 &&
-         ((ldx ? ldx : K) & 7) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
-         (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+// Skinny products: the streaming kernels against the stream-K tcgen05 tiles (or, without scratch, plain tiles, which lose
+// everywhere).  A launch of the matrix kernel lasts as long as one CTA's chain over K for each of its blocks of up to 32 rows, so
+// it loses where rows are few and K is long, and where the last block is half empty; nine to sixteen right-hand sides read
+// twice the X per weight and lose to the tiles from some 100 MB of weights on.  us, tiles / streaming:
+// m = 8: 1024 x 10240 14.6 / 14.3, 1024 x 14336 15.5 / 18.9, 3000 x 20480 29.0 / 31.6, 4096 x 14336 28.0 / 25.2, 6000 x 14336 36.4 / 42.6;
+// m = 16: 1024 x 8192 14.4 / 13.1, 2048 x 10240 16.4 / 17.5, 4096 x 14336 28.1 / 27.5, 14592 x 1536 16.4 / 16.1, 16000 x 2048
+// 18.8 / 19.6, 32000 x 512 13.7 / 15.0.
+bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m, int sm_count,
+                            bool scratch) {
+  if (m < 1 || m > 16 || rows < 1024 || K < 512 || (K & 7) || ((ldw ? ldw : K) & 7) || ((ldx ? ldx : K) & 7) ||
+      (reinterpret_cast<uintptr_t>(W) & 15) || (reinterpret_cast<uintptr_t>(X) & 15))
+    return false;
+  if (m <= 2 || !scratch) return true;
+  const int64_t work = (int64_t)rows * K;
+  if (m > 8 && (work > 52 << 20 || rows > 24576 || (rows > 13312 && work > 24 << 20))) return false;
+  const int per_sm = (rows + sm_count - 1) / sm_count, blocks = (per_sm + 31) / 32;
+  if (per_sm < 24) return K <= (m <= 8 ? 10240 : 8192);
+  if (blocks > 1 && per_sm < blocks * 24) return m <= 8 && K <= 12288;
+  return K <= 16384;
 }
 
 int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y,

@@ -37,7 +37,9 @@ int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ld
                            int64_t ldy_inner, int rows, int K, int m, int sm_count, int order_mode,
                            cudaStream_t stream, int64_t* launches);
 // Skinny products the streaming kernels take from the tcgen05 tiles: 16-byte-aligned operands, enough rows for the SMs.
-bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m);
+// `scratch`: the tiles could cut K (stream-K).
+bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m, int sm_count,
+                            bool scratch);
 
 // Variant with the split-K partials in an array that is part of the library image.
 size_t gemv_f16_static_capacity_floats();

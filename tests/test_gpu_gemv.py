@@ -162,3 +162,22 @@ def test_gemv_on_both_sides_of_its_kernel_choice(oracle, rows, K, m, flag):
         ops.run(l)
         got = out.cpu().numpy()
         util.assert_f16_close(got.T if transposed else got, ref32, f"gemv {rows}x{K} m={m} flag={flag}")
+
+
+@pytest.mark.parametrize("M,N,K,launches", [(8, 1024, 10240, 1), (8, 1024, 10248, 2), (16, 2048, 8192, 1), (9, 2048, 8200, 2),
+                                            (3, 3552, 10248, 1), (16, 24584, 512, 2), (2, 1024, 32768, 1)])
+def test_skinny_gemm_leaves_long_k_of_few_rows_to_the_tiles(oracle, M, N, K, launches):
+    w, x = datagen.c2_gemv(N, K, M, seed=M + K)
+    a, b = torch.from_numpy(x).cuda(), torch.from_numpy(w).cuda()
+    out = torch.empty((M, N), dtype=torch.float16, device="cuda")
+    l = ops.launch_gemm_f16(a, b, out)
+    before = ops.launch_count()
+    ops.run(l)
+    assert ops.launch_count() - before == launches
+    _, ref32 = oracle.hgemm_fast(x, w)
+    util.assert_f16_close(out.cpu().numpy(), ref32, f"skinny {M}x{N}x{K}")
+    l.ws, l.ws_bytes = None, 0
+    out.zero_()
+    ops.run(l)
+    assert ops.launch_count() - before == launches + 1
+    util.assert_f16_close(out.cpu().numpy(), ref32, f"skinny {M}x{N}x{K} without scratch")
