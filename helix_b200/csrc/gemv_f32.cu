@@ -290,6 +290,30 @@ static int launch_stream32(const float* W, int64_t ldw, const float* X, int64_t 
   return HELIX_OK;
 }
 
+// Which GEMVs without a configuration of their own the streaming kernel runs.  us, the kernel above / streaming:
+static bool gemv_f32_streams(int rows, int K, int m, int split, int sm_count) {
+  const int per_sm = (rows + sm_count - 1) / sm_count;
+  if (m > 1 && K < 512) return false;                  // 10000 x 304, m = 2: 5.3 / 6.7
+  if (split > 1) {
+    if (rows < sm_count || K > 32768) return false;
+    // cut only because K is very long: sharing it among warps pays with few rows, or where m makes the kernel above issue bound
+    // (16384 long: m = 1, 3000 rows 44.6 / 40.6, 6000 66 / 72; m = 2, 1300 26.1 / 25.1, 2048 29.1 / 33.8; m = 3, 2048 43.8 / 42.0,
+    // 3000 51 / 62; m = 5, 3000 70 / 62)
+    return m >= 4 || per_sm <= (m == 1 ? 32 : m == 2 ? 10 : 16);
+  }
+  // Short rows: a warp takes whole rows, so its few loads per row leave its FIFO empty between rows (m = 1: 3000 x 256 2.8 / 2.9,
+  // 6000 x 768 5.9 / 6.3, 6000 x 1500 10.1 / 9.5; m = 2: 4096 x 768 4.9 / 5.7; m = 5: 3000 x 768 6.2 / 6.5)
+  if (m == 1) return per_sm <= 16 || (K >= 512 && per_sm <= 32) || K >= 1024;
+  if (per_sm > 16 && K < 1024 && (m == 2 || m >= 5)) return false;
+  if (per_sm <= 32) return true;
+  // Several rows per warp: two of them do not earn the second right-hand side's reads back (m = 2: 4800 x 8192 35 / 50, 8192 x 8192
+  // 45 / 51) but in the middle of the range (12000 x 2048 21.4 / 19.5); blocks of four must fill the CTA's 16 warps (m = 3:
+  // 4800 x 4096, 9 blocks, 23.5 / 26.8; 8192 x 4096, 14 blocks, 38.3 / 30.3; 12000 x 4096, 21 blocks, 44.1 / 45.4).
+  if (m == 2) return per_sm > 64 && K >= 1024 && K <= 4096;
+  const int blocks = (per_sm + 3) / 4, turns = (blocks + 15) / 16;
+  return blocks * 5 >= turns * 64;
+}
+
 int gemv_f32_launch(const helix_cfg_t* cfg, const float* W, int64_t ldw, const float* X, int64_t ldx, float* Y,
                     int64_t ldy, int64_t ldy_inner, int rows, int K, int m, void* ws, size_t ws_bytes, int sm_count,
                     cudaStream_t stream, int64_t* launches) {
@@ -309,8 +333,7 @@ int gemv_f32_launch(const helix_cfg_t* cfg, const float* W, int64_t ldw, const f
     if (own && cfg->split_k > 1) return HELIX_ERR_WORKSPACE;
     split_k = 1;
   }
-  // short rows of several right-hand sides stay with the kernel above (10000 x 304, m = 2: 5.3 us against 6.7)
-  if (!own && (m == 1 || K >= 512) && (split_k == 1 || (rows >= sm_count && K <= 32768))) {
+  if (!own && gemv_f32_streams(rows, K, m, split_k, sm_count)) {
     // rows per warp: as many as share one read of X while the warps of an SM still have a block each; where the library
     // would have cut K (few rows), the warps of a CTA share a row block's K instead
     const int per_sm = (rows + sm_count - 1) / sm_count;

@@ -84,3 +84,11 @@ def test_streaming_gemv_f32_shares_k_among_warps_deterministically(rows, K, m):
     a, b = ops.gemv_f32(wd, xd), ops.gemv_f32(wd, xd)
     assert torch.equal(a, b)
     util.assert_f32_close(a.cpu().numpy(), x.astype(np.float64) @ w.astype(np.float64).T, f"fp32 GEMV {rows}x{K} m={m}")
+
+
+@pytest.mark.parametrize("rows,K,m", [(4737, 1024, 2), (4737, 1020, 1), (2500, 508, 1), (2500, 764, 2), (4800, 1028, 3),
+                                      (6000, 516, 5), (9600, 1024, 2), (12000, 516, 4), (7200, 600, 8)])
+def test_gemv_f32_keeps_the_stated_order_on_both_sides_of_its_kernel_choice(oracle, rows, K, m):
+    w, x = _data(rows, K, m, rows + m)
+    got = ops.gemv_f32(torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda()).cpu().numpy()
+    assert np.array_equal(got, oracle.gemv_f32_lane_tree(w, x))
