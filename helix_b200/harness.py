@@ -378,7 +378,7 @@ def conv_f16_result(prof_dict, batch, IC, H, W, OC, kH, kW, stride, pad):
     if ops.conv_has_fixed_kernel(batch, C, H, W, OC, kH, kW, stride, pad):   # nothing for the cost model to pick
         cost_ms = time_conv_f16(batch, IC, H, W, OC, kH, kW, stride, pad) * 1e3
         return cost_ms, 2.0 * M * N * K / 1e9 / cost_ms
-    im2col = ops.conv_reads_tensor_map(batch, H, W, C, stride)
+    im2col = ops.conv_reads_tensor_map(batch, H, W, C, stride, OC, kH, kW, pad)
     # the convolution harness times one buffer set with ordered launches: a lone launch
     real_bytes = 2.0 * (batch * H * W * C + OC * kH * kW * C + M * N)        # x, w and y once each
     key = costmodel.cost_model(prof_dict, M, N, (K + 7) // 8 * 8, 1,

@@ -129,16 +129,21 @@ def kernel_name(launch):
         if rows_geom and c.conv_gather == 4:    # explicit, or the library's default for this geometry
             return "conv_f16_rows_kernel"
         as_gemm = r == 1 and s == 1 and stride == 1 and pad == 0
-        im2col = conv_reads_tensor_map(n, h, w, ch, stride) and not c.conv_gather
+        im2col = conv_reads_tensor_map(n, h, w, ch, stride, ko, r, s, pad) and not c.conv_gather
         gathers = not as_gemm and not im2col
     return "gemm_f16_tc_kernel<%d,%d>" % (c.tile_n, 1 if gathers else 0)
 
 
-def conv_reads_tensor_map(n, h, w, ch, stride):
+def conv_reads_tensor_map(n, h, w, ch, stride, ko=0, r=1, s=1, pad=0):
     """True where the implicit GEMM fetches its input through the im2col tensor map (conv_im2col_eligible in
-    csrc/gemm_f16_tc.cu): the channels a 64-channel block is filled up with must be few."""
+    csrc/gemm_f16_tc.cu): the channels a 64-channel block is filled up with must be few and, where ch is no multiple of 16,
+    the layer small (`ko` output channels of an r x s filter)."""
     filled = (ch + 63) // 64 * 64
     few = filled * 3 <= ch * 4 if ch % 32 == 0 else filled * 5 <= ch * 6 and ch >= 96
+    if ch % 16 != 0:
+        ho, wo = conv_out_hw(h, w, r, s, stride, pad)
+        macs = n * ho * wo * ko * r * s * ch
+        few = few and (macs <= 4e9 or filled * 16 <= ch * 17 and macs <= 3e10)
     return ch % 8 == 0 and few and n * h * w * ch * 2 >= 131072 and stride <= 8
 
 

@@ -440,3 +440,20 @@ def test_gathering_convolution_has_no_192_wide_tile():
     with pytest.raises(Exception) as e:
         ops.conv2d_f16_nhwc(x, w, 1, 1, cfg=ops.make_cfg(OP_CONV_F16, tile_m=128, tile_n=192, tile_k=64))
     assert "-6" in str(e.value)
+
+
+@pytest.mark.parametrize("geom", [
+    (8, 168, 26, 26, 424, 5, 5, 1, 2),     # pixels off 32-byte sectors, large: gathers
+    (2, 168, 26, 26, 200, 5, 5, 1, 2),     # the same, small: through the map
+    (12, 312, 20, 20, 320, 3, 3, 1, 1),    # large, next to nothing filled: through the map
+])
+def test_conv_on_both_sides_of_its_operand_choice(oracle, geom):
+    B, C, H, W, OC, kh, kw, stride, pad = geom
+    mapped = ops.conv_reads_tensor_map(B, H, W, C, stride, OC, kh, kw, pad)
+    assert mapped == (geom[0] != 8)
+    x, w = datagen.c4_conv(*geom, seed=47)
+    got = _run(x, w, stride, pad)
+    _, y32 = oracle.conv2d_nhwc_f16(x[:1], w, stride, pad)
+    util.assert_f16_close(got[:1], y32, f"conv {geom}")
+    gather = _run(x, w, stride, pad, ops.make_cfg(OP_CONV_F16, tile_m=128, tile_n=128, tile_k=64, conv_gather=1))
+    util.assert_f16_close(got, gather.astype(np.float32), f"conv {geom} against gathering")

@@ -73,6 +73,14 @@ def test_sgemm_cost_model():
     assert small[0] * small[1] < 128 * 128                       # few tiles: smaller tiles fill more SMs
 
 
+def test_the_map_rule_for_channels_off_32_byte_sectors_counts_the_layer():
+    from helix_b200.ops import conv_reads_tensor_map as reads
+    assert reads(8, 26, 26, 168, 1) and reads(2, 26, 26, 168, 1, 200, 5, 5, 2)
+    assert not reads(8, 26, 26, 168, 1, 424, 5, 5, 2)
+    assert reads(12, 20, 20, 312, 1, 320, 3, 3, 1) and not reads(60, 40, 40, 312, 1, 320, 3, 3, 1)
+    assert reads(60, 40, 40, 176, 1, 768, 3, 3, 1) and reads(60, 40, 40, 96, 1, 768, 3, 3, 1)
+
+
 def test_workloads_match_the_published_totals():
     units = workloads.model_level_sweep()
     assert len(units) == 125 and sum(u["kind"] == "conv" for u in units) == 53
