@@ -28,7 +28,7 @@ import math
 
 TILE_M = 128
 TILE_K = 64
-GEMM_TILE_NS = (256, 128, 64, 32, 16)
+GEMM_TILE_NS = (256, 128, 64, 32, 16)      # the 192-wide one-CTA tile is a choice of the library's own rules only
 GEMV_VARIANTS = ((2, 4), (1, 4), (1, 8), (2, 2))   # (rows per warp, 16-byte loads in flight per row)
 GEMV_SPLITS = (1, 2, 4, 8)
 DEFAULT_SMS = 148
@@ -37,10 +37,11 @@ SPLIT_MODES = (2, 3, 4)     # mode values that mean split-K over that many slice
 
 # FP32 SIMT tiles: (BM, BN, BK, TM, TN, stages), the analogue of the reference's
 # (BM, BN, BK, TM, TN, WARP_ROW_THREAD, COPY_A, COPY_B) keys (build_Ampere_FP32.py:37-63)
-SGEMM_TILES = ((128, 128, 16, 8, 8, 4), (128, 128, 32, 8, 8, 3), (128, 64, 16, 8, 4, 4), (128, 64, 32, 8, 4, 3),
-               (64, 128, 16, 4, 8, 4),
+SGEMM_TILES = ((128, 128, 16, 8, 8, 4), (128, 128, 32, 8, 8, 3), (128, 64, 16, 8, 8, 4), (128, 64, 32, 8, 8, 3),
+               (64, 128, 16, 8, 8, 4),
                (128, 128, 16, 8, 8, 2), (128, 64, 16, 8, 4, 2), (64, 128, 16, 4, 8, 2), (64, 64, 16, 4, 4, 2),
-               (32, 64, 16, 4, 4, 2))
+               (32, 64, 16, 4, 4, 2),
+               (64, 64, 16, 4, 8, 4), (32, 64, 16, 4, 4, 6), (32, 32, 32, 2, 4, 4))
 
 
 def is_valid_config(tile_n, swap_ab, mode, stages):

@@ -381,7 +381,9 @@ def conv_f16_result(prof_dict, batch, IC, H, W, OC, kH, kW, stride, pad):
     im2col = ops.conv_reads_tensor_map(batch, H, W, C, stride, OC, kH, kW, pad)
     # the convolution harness times one buffer set with ordered launches: a lone launch
     real_bytes = 2.0 * (batch * H * W * C + OC * kH * kW * C + M * N)        # x, w and y once each
-    key = costmodel.cost_model(prof_dict, M, N, (K + 7) // 8 * 8, 1,
+    # through the map the kernel walks whole 64-channel blocks of every tap
+    Kw = kH * kW * (-(-C // 64) * 64) if im2col and not as_gemm else (K + 7) // 8 * 8
+    key = costmodel.cost_model(prof_dict, M, N, Kw, 1,
                                conv=False if as_gemm else ("im2col" if im2col else True), operand_bytes=real_bytes)
     if key is None or key[0] == 0:
         key = (costmodel.max_stages(128), 128, 128, 1, 0, 0)

@@ -73,12 +73,32 @@ def test_sgemm_cost_model():
     assert small[0] * small[1] < 128 * 128                       # few tiles: smaller tiles fill more SMs
 
 
+def test_sgemm_search_space_is_the_librarys():
+    from helix_b200 import ops
+    from helix_b200._lib import OP_GEMM_F32
+    assert tuple((c.tile_m, c.tile_n, c.tile_k, c.thread_m, c.thread_n, c.stages)
+                 for c in ops.configs(OP_GEMM_F32)) == costmodel.SGEMM_TILES
+
+
 def test_the_map_rule_for_channels_off_32_byte_sectors_counts_the_layer():
     from helix_b200.ops import conv_reads_tensor_map as reads
     assert reads(8, 26, 26, 168, 1) and reads(2, 26, 26, 168, 1, 200, 5, 5, 2)
     assert not reads(8, 26, 26, 168, 1, 424, 5, 5, 2)
     assert reads(12, 20, 20, 312, 1, 320, 3, 3, 1) and not reads(60, 40, 40, 312, 1, 320, 3, 3, 1)
     assert reads(60, 40, 40, 176, 1, 768, 3, 3, 1) and reads(60, 40, 40, 96, 1, 768, 3, 3, 1)
+
+
+def test_the_cost_model_of_a_convolution_sees_the_blocks_its_kernel_walks(monkeypatch):
+    from helix_b200 import harness
+    seen = []
+    monkeypatch.setattr(harness, "require_gpu", lambda: None)
+    monkeypatch.setattr(harness, "time_conv_f16", lambda *a, **k: 1e-5)
+    monkeypatch.setattr(harness.costmodel, "cost_model", lambda d, M, N, K, *a, **k: seen.append(K))
+    harness.conv_f16_result({}, 20, 96, 26, 26, 256, 5, 5, 1, 2)      # 96 channels: two blocks of 64 per tap
+    harness.conv_f16_result({}, 20, 64, 26, 26, 256, 5, 5, 1, 2)
+    harness.conv_f16_result({}, 20, 96, 26, 26, 256, 1, 1, 1, 0)      # a plain GEMM over the pixels
+    harness.conv_f16_result({}, 20, 40, 26, 26, 256, 3, 3, 1, 1)      # gathered: no filling
+    assert seen == [25 * 128, 25 * 64, 96, 9 * 40]
 
 
 def test_workloads_match_the_published_totals():
