@@ -642,13 +642,15 @@ static bool gemv_f16_streams(int rows, int K, int m, int split, bool scratch, in
     if (split > 1) return rows >= sm_count && K <= 32768;
     // Many short rows: every 64 of them end in a barrier and a sum over the warps.  m = 1: 4096 x 768 3.3 / 3.5, 5000 x 1536
     // 5.4 / 5.7, 8192 x 1024 4.8 / 5.6, 12000 x 3072 14.8 / 15.7; 4096 x 1280 4.7 / 4.7, 6000 x 2048 6.9 / 7.1 (with static
-    // weights 5.7 / 5.5), 8192 x 4096 13.6 / 13.2.
-    return m == 2 || rows < 4096 || K > 3072 || (rows < 8192 && K > 1536) || (rows < 5000 && K > 768);
+    // weights 5.7 / 5.5), 8192 x 4096 13.6 / 13.2; 12000 x 256 with static weights 3.1 / 2.5, otherwise 3.6 / 3.7.
+    return m == 2 || rows < 4096 || K > 3072 || (rows < 8192 && K > 1536) || (rows < 5000 && K > 768) ||
+           (rows >= 10000 && K < 512);
   }
   // The matrix kernel's chain over K takes about K / 1000 us whatever m, the split kernel's m times K / split: m = 3,
   // 64 x 65536 15.3 / 66, 512 x 8192 9.2 / 10.9 (split 4), 700 x 8192 14.9 / 11.0 (split 2); m = 8, 64 x 65536 36 / 74 (split
-  // 16), 148 x 16384 19.1 / 20.4, 296 x 16384 34.9 / 20.6 (split 4).
-  if (scratch) return split < m || (split == m && rows < 64);
+  // 16), 148 x 16384 19.1 / 20.4, 296 x 16384 34.9 / 20.6 (split 4).  From 1024 rows on the slices are more warps than fit
+  // (m = 4, 2048 x 65536: 135 / 80).
+  if (scratch && rows < 1024) return split < m || (split == m && rows < 64);
   return !(m == 3 && K <= 256 && rows <= 512);         // 256 x 256: 1.9 / 2.2
 }
 
@@ -656,7 +658,8 @@ static bool gemv_f16_streams(int rows, int K, int m, int split, bool scratch, in
 // everywhere).  A launch of the matrix kernel lasts as long as one CTA's chain over K for each of its blocks of up to 32 rows, so
 // it loses where rows are few and K is long, and where the last block is half empty; nine to sixteen right-hand sides read
 // twice the X per weight and lose to the tiles from some 100 MB of weights on.  us, tiles / streaming:
-// m = 8: 1024 x 10240 14.6 / 14.3, 1024 x 14336 15.5 / 18.9, 3000 x 20480 29.0 / 31.6, 4096 x 14336 28.0 / 25.2, 6000 x 14336 36.4 / 42.6;
+// m = 3: 2048 x 12288 17.8 / 16.0, 1024 x 14336 15.4 / 17.1, 3000 x 24576 35.9 / 33.0, 4096 x 32768 52.0 / 52.0; m = 8: 1024 x 10240
+// 14.6 / 14.3, 1024 x 14336 15.5 / 18.9, 3000 x 20480 29.0 / 31.6, 4096 x 14336 28.0 / 25.2, 6000 x 14336 36.4 / 42.6;
 // m = 16: 1024 x 8192 14.4 / 13.1, 2048 x 10240 16.4 / 17.5, 4096 x 14336 28.1 / 27.5, 14592 x 1536 16.4 / 16.1, 16000 x 2048
 // 18.8 / 19.6, 32000 x 512 13.7 / 15.0.
 bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m, int sm_count,
@@ -668,9 +671,9 @@ bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t l
   const int64_t work = (int64_t)rows * K;
   if (m > 8 && (work > 52 << 20 || rows > 24576 || (rows > 13312 && work > 24 << 20))) return false;
   const int per_sm = (rows + sm_count - 1) / sm_count, blocks = (per_sm + 31) / 32;
-  if (per_sm < 24) return K <= (m <= 8 ? 10240 : 8192);
+  if (per_sm < 24) return K <= (m > 8 ? 8192 : m > 4 ? 10240 : per_sm < 16 ? 12288 : 20480);
   if (blocks > 1 && per_sm < blocks * 24) return m <= 8 && K <= 12288;
-  return K <= 16384;
+  return K <= (m > 8 ? 16384 : 24576);
 }
 
 int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y,
