@@ -304,14 +304,15 @@ static bool gemv_f32_streams(int rows, int K, int m, int split, int sm_count) {
   // Short rows: a warp takes whole rows, so its few loads per row leave its FIFO empty between rows (m = 1: 3000 x 256 2.8 / 2.9,
   // 6000 x 768 5.9 / 6.3, 6000 x 1500 10.1 / 9.5; m = 2: 4096 x 768 4.9 / 5.7; m = 5: 3000 x 768 6.2 / 6.5)
   if (m == 1) return per_sm <= 16 || (K >= 512 && per_sm <= 32) || K >= 1024;
-  if (per_sm > 16 && K < 1024 && (m == 2 || m >= 5)) return false;
-  if (per_sm <= 32) return true;
+  if (per_sm <= 32) return K >= 1024 || per_sm <= 16 || m == 3 || m == 4 || m == 8;
   // Several rows per warp: two of them do not earn the second right-hand side's reads back (m = 2: 4800 x 8192 35 / 50, 8192 x 8192
-  // 45 / 51) but in the middle of the range (12000 x 2048 21.4 / 19.5); blocks of four must fill the CTA's 16 warps (m = 3:
-  // 4800 x 4096, 9 blocks, 23.5 / 26.8; 8192 x 4096, 14 blocks, 38.3 / 30.3; 12000 x 4096, 21 blocks, 44.1 / 45.4).
+  // 45 / 51) but in the middle of the range (12000 x 2048 21.4 / 19.5); blocks of four should fill the CTA's 16 warps (m = 3:
+  // 4800 x 4096, 9 blocks, 23.5 / 26.8; 8192 x 4096, 14 blocks, 38.3 / 30.3; 12000 x 4096, 21 blocks, 44.1 / 45.4), unless the kernel
+  // above, whose cost follows m, spends more on a full set of right-hand sides (m = 4: 6000 x 2048 17.2 / 15.8, 6000 x 512 6.0 / 6.2;
+  // m = 8: 6000 x 4096 36.6 / 33.4, 4800 x 1024 10.4 / 11.2).
   if (m == 2) return per_sm > 64 && K >= 1024 && K <= 4096;
   const int blocks = (per_sm + 3) / 4, turns = (blocks + 15) / 16;
-  return blocks * 5 >= turns * 64;
+  return blocks * 5 >= turns * 64 || (m == 4 && K >= 1024) || (m >= 7 && K >= 2048);
 }
 
 int gemv_f32_launch(const helix_cfg_t* cfg, const float* W, int64_t ldw, const float* X, int64_t ldx, float* Y,
