@@ -1080,15 +1080,15 @@ static EncodeIm2colFn get_encode_im2col_fn() {
 // C = 88: 15.8 / 11.7, C = 40, 5 x 5: 28.5 / 13.5.  Where every second pixel starts off a 32-byte sector (C = 8 mod 16) that
 // is true of small layers only: from some 4 G multiply-adds on gathering hides its latency (3 x 3, 5 x 5, map / gathering, G in
 // brackets: C = 168 [1.7] 16.6 / 17.5, [4.6] 33.8 / 30.6, [12] 57 / 48; C = 216 [26] 97 / 88, [39] 149 / 111; C = 280 [15] 75 / 66; C = 328
-// [22] 73 / 67), and to 30 G with next to nothing filled (C = 616 [6] 29 / 33, 680 [22] 79 / 89, 312 [19] 71 / 71; but 728 [43] 124 / 105,
-// 440 [215] 600 / 557); C = 8 k with even k keeps its gain at any size (176, 304, 336, 432, 496, 560, 688: 0.57 ... 0.89).
+// [22] 73 / 67), and to 30 G with a tenth filled at most (C = 408 [7] 32 / 36, 472 [16] 79 / 92, 680 [22] 79 / 89, 312 [19] 71 / 71; but 232 [16]
+// 71 / 64, 728 [43] 124 / 105, 440 [215] 600 / 557); C = 8 k with even k keeps its gain at any size (176, 304, 336, 432, 496, 560, 688: 0.57 ... 0.89).
 static bool conv_im2col_eligible(const ConvGeom& g) {
   const int64_t bytes = (int64_t)g.NB * g.H * g.W * g.C * 2;
   const int filled = (g.C + kBK - 1) / kBK * kBK;
   bool worth = g.C % 32 == 0 ? filled * 3 <= g.C * 4 : filled * 5 <= g.C * 6 && g.C >= 96;
   if (g.C % 16 != 0) {
     const double macs = (double)g.NB * g.Ho * g.Wo * g.KO * g.R * g.S * g.C;
-    worth = worth && (macs <= 4e9 || (filled * 16 <= g.C * 17 && macs <= 3e10));
+    worth = worth && (macs <= 4e9 || (filled * 10 <= g.C * 11 && macs <= 3e10));
   }
   return (g.C % 8) == 0 && worth && g.stride >= 1 && g.stride <= 8 && g.pad <= 127 && g.R <= 128 && g.S <= 128 &&
          g.pad - (g.R - 1) >= -128 && g.pad - (g.S - 1) >= -128 && bytes >= 131072 && g.C <= 65535 &&

@@ -143,7 +143,7 @@ def conv_reads_tensor_map(n, h, w, ch, stride, ko=0, r=1, s=1, pad=0):
     if ch % 16 != 0:
         ho, wo = conv_out_hw(h, w, r, s, stride, pad)
         macs = n * ho * wo * ko * r * s * ch
-        few = few and (macs <= 4e9 or filled * 16 <= ch * 17 and macs <= 3e10)
+        few = few and (macs <= 4e9 or filled * 10 <= ch * 11 and macs <= 3e10)
     return ch % 8 == 0 and few and n * h * w * ch * 2 >= 131072 and stride <= 8
 
 
