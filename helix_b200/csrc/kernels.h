@@ -73,7 +73,7 @@ void gemm_f16_get_config(int idx, helix_cfg_t* out);
 void gemm_f16_default_config(int M, int N, int K, int batch, int sm_count, bool conv, helix_cfg_t* out);
 void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out);
 int64_t conv_f16_gemm_k(const ConvGeom& g);
-// ---- conv_f32.cu (column matrix + FFMA GEMM)
+// ---- conv_f32.cu (FFMA GEMM over the windows, gathered by its loader or through a column matrix)
 size_t conv_f32_workspace_bytes(const ConvGeom& g);
 int conv_f32_launch(const helix_cfg_t* cfg, const float* x, const float* w, float* y, const ConvGeom& g, void* ws,
                     size_t ws_bytes, int sm_count, cudaStream_t stream, int64_t* launches);

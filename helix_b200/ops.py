@@ -100,22 +100,17 @@ def default_config(launch):
 
 
 def kernel_name(launch):
-    """Name of the main kernel `launch` resolves to, as a profiler lists it."""
+    """Name of the main kernel `launch` resolves to (its first template arguments).  GEMVs and products of up to 16 rows without
+    a configuration are one family each, whose kernel the library picks by sizes (gemv_f16_streams, gemv_f16_stream_covers and
+    gemv_f32_streams in csrc/)."""
     own = launch.cfg.tile_n or launch.cfg.tile_m
     c = launch.cfg if own else default_config(launch)
-    # the library's own choice streams (the rules of gemv_f16_launch, gemv_f32_launch and gemv_f16_stream_covers)
-    streams = not own and (c.split_k <= 1 or (launch.N >= device_info().sm_count and launch.K <= 32768))
     if launch.op == _lib.OP_GEMV_F16:
-        if not own and launch.M >= 3:
-            return "gemv_f16_mma_kernel<1>"
-        return "gemv_f16_stream_kernel<%d>" % launch.M if streams and launch.N * launch.K >= 1 << 21 else "gemv_f16_kernel"
+        return "gemv_f16_kernel" if own else "gemv_f16"
     if launch.op == _lib.OP_GEMV_F32:
-        return "gemv_f32_stream_kernel" if streams and (launch.M == 1 or launch.K >= 512) else "gemv_f32_kernel"
-    if (launch.op == OP_GEMM_F16 and not own and launch.batch <= 1 and launch.N >= 1024 and launch.K >= 512 and
-            (launch.M <= 8 or launch.M <= 16 and launch.N * launch.K <= 52 << 20)):
-        if launch.M <= 2:
-            return "gemv_f16_stream_kernel<%d>" % launch.M
-        return "gemv_f16_mma_kernel<%d>" % (1 if launch.M <= 8 else 2)
+        return "gemv_f32_kernel" if own else "gemv_f32"
+    if launch.op == OP_GEMM_F16 and not own and launch.batch <= 1 and launch.M <= 16 and launch.N >= 1024 and launch.K >= 512:
+        return "gemm_f16_skinny"
     if launch.op == _lib.OP_GEMM_F32:
         return "%s<%d,%d>" % ("sgemm_f32_ring_kernel" if c.stages >= 3 else "sgemm_f32_kernel", c.tile_m, c.tile_n)
     if c.cta_group == 2:

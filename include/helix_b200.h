@@ -91,7 +91,7 @@ typedef struct helix_cfg {
                     remaining tiles dealt evenly to all CTAs or CTA pairs (needs a workspace);
                     overrides split_k                                                    */
   int conv_gather; /* CONV_F16: 0 = activations arrive through an im2col tensor map wherever the
-                      geometry allows it (C a multiple of 64, tensor of 128 KiB or more), else
+                      geometry allows it (C a multiple of 64 or not far below one, tensor of 128 KiB or more), else
                       through gathering producer warps; 1 = always gather (cp.async);
                       3 = window-resident kernel (stride 1, C a multiple of 64, W + 2*pad <= 256);
                       4 = row-pair kernel (3 x 3, stride 1, pad 1, 64 -> 64 channels, W <= 62: pixels on
@@ -167,10 +167,13 @@ int helix_get_config(int op, int idx, helix_cfg_t* out);
 
 /* The configuration the library would pick for `launch` when launch->cfg is zeroed: the built-in
  * analytic stand-in for cost_model() (scripts/Ampere_FP16/Ampere_FP16_gemm.py:420-430), used when
- * no profiled dictionary is at hand. */
+ * no profiled dictionary is at hand.  For GEMVs and fp16 products of up to 16 rows it is that of the kernels which
+ * configurations select; a zeroed cfg may also run one of the streaming kernels, which none names. */
 int helix_default_config(const helix_launch_t* launch, helix_cfg_t* out);
 
-/* Bytes of workspace a launch needs (0 when none). */
+/* Bytes of workspace a launch needs (0 when none).  Decided by sizes: a kernel that the pointers' alignment
+ * or the geometry then selects may leave it unread (streaming GEMVs and skinny products, fp32
+ * convolutions without a column matrix). */
 size_t helix_workspace_bytes(const helix_launch_t* launch);
 
 /* Queue one launch.  Generic form of the four typed entry points below. */
