@@ -287,6 +287,20 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
       : "r"(taddr)
       : "memory");
 }
+// 16 lanes x 64 columns as fragments of 8 x 8: in r[4 i ... 4 i + 3] thread t of the warp receives columns 8 i + 2 (t % 4) and
+// the next one of row t / 4 (r[4 i], r[4 i + 1]) and of row t / 4 + 8.
+__device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---------------------------------------------------------------- TMA store (shared -> global)
@@ -324,6 +338,23 @@ __device__ __forceinline__ void stage_rows_f16(uint32_t row_base, const uint32_t
                  "r"(*reinterpret_cast<uint32_t*>(&h2)), "r"(*reinterpret_cast<uint32_t*>(&h3))
                  : "memory");
   }
+}
+// The transposed box: 64 accumulator columns become 64 rows of 128 bytes, `chunk` ... chunk + 3 of whose eight 16-byte
+// chunks are this warp's 32 rows (lo: rows 0 ... 15, hi: 16 ... 31, as tmem_ld_16x256b_x8 delivers them).  A transposing
+// stmatrix writes 8 rows x 4 chunks without a bank conflict.
+__device__ __forceinline__ void stage_columns_f16(uint32_t box, const uint32_t (&lo)[32], const uint32_t (&hi)[32], int chunk,
+                                                  int lane) {
+  auto pack = [](uint32_t a, uint32_t b) {
+    const __half2 h = __floats2half2_rn(__uint_as_float(a), __uint_as_float(b));
+    return *reinterpret_cast<const uint32_t*>(&h);
+  };
+  const uint32_t dst = box + (lane & 7) * 128 + (((chunk + (lane >> 3)) ^ (lane & 7)) << 4);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(dst + i * 1024),
+                 "r"(pack(lo[4 * i], lo[4 * i + 1])), "r"(pack(lo[4 * i + 2], lo[4 * i + 3])),
+                 "r"(pack(hi[4 * i], hi[4 * i + 1])), "r"(pack(hi[4 * i + 2], hi[4 * i + 3]))
+                 : "memory");
 }
 // Such a box to rows of C that TMA cannot store (a leading dimension or base that is no multiple of 16 bytes): row by row
 // with the lanes along the columns, 4 bytes each, shifted by one element where a row starts on an odd one.  (A lane per row

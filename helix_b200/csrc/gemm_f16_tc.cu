@@ -56,6 +56,7 @@ constexpr int kStoreStagingBytes = 4 * 2 * 32 * 128;              // two 32-row 
 constexpr int kEpiBarrier = 1;                                    // named barrier of the 128 epilogue threads
 constexpr int kFwdBarrier = 2;   // named barriers 2..9: arrival of one group of ring stages, forwarded to the MMA warp
 constexpr int kTokBarrier = 10;  // named barriers 10, 11: issue order of two MMA warps that alternate K slabs
+constexpr int kBoxBarrier = 12;  // named barriers 12, 13: two epilogue warps that share a transposed staging box
 
 enum OutMode { kOutDirect = 0, kOutSplitSlice = 1, kOutStreamSlot = 2 };
 
@@ -542,7 +543,6 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       const int pw = threadIdx.x >> 5;       // producer warp 0..7
       const int j = lane & 7;                // 16-byte chunk of the 128-byte slab
       const int sub = lane >> 3;             // row within a pass, 0..3
-      const int HoWo = p.g.Ho * p.g.Wo;
       const int chunks = p.K >> 3;
       int stage = 0;
       uint32_t phase = 0;
@@ -673,6 +673,57 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           if (lane == 0) mbar_arrive(&tmem_empty[acc]);
           if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
           continue;
+        }
+        if constexpr (!CONV && !ANY) {
+        if (p.tma_store && p.swap && w.mode == kOutDirect) {
+          // Swapped operands: TMEM lanes index the contiguous axis of C (for a convolution the output channels of a
+          // pixel), so 64 columns at a time are transposed on their way to shared memory; two warps fill one box of 64 rows
+          // x 64 channels, and one TMA store sends it.  (2-byte stores of a lane per channel, which this replaces, took 10500 cycles
+          // per 128 x 256 tile between the dependent layers of a CNN stage.)
+          const int side = quarter >> 1, row_first = w.m_blk * kBM + side * 64;
+          uint8_t* const boxes = sC + (size_t)side * (2 * 64 * 128);
+          auto emit_columns = [&](const uint32_t (&lo)[32], const uint32_t (&hi)[32], int c0) {
+            const int col0 = w.n_blk * BN + c0;
+            if (col0 >= p.PN || row_first >= p.PM) return;   // uniform over the two warps
+            uint8_t* stage_box = boxes + box * (64 * 128);
+            box ^= 1;
+            if ((quarter & 1) == 0 && lane == 0) tma_store_wait_read_1();   // the store issued two boxes ago has left this buffer
+            named_bar_sync(kBoxBarrier + side, 64);
+            stage_columns_f16(smem_u32(stage_box), lo, hi, (quarter & 1) * 4, lane);
+            fence_proxy_async_smem();
+            named_bar_sync(kBoxBarrier + side, 64);
+            if ((quarter & 1) == 0 && lane == 0) {
+              tma_store_3d(&tmap_c, stage_box, row_first, col0, w.b);
+              tma_store_commit();
+            }
+          };
+          const uint32_t upper = 16u << 16;   // lanes 16 ... 31 of the quarter
+          uint32_t ra[32], rb[32], na[32], nb[32];
+          tmem_ld_16x256b_x8(taddr, ra);
+          tmem_ld_16x256b_x8(taddr + upper, rb);
+#pragma unroll
+          for (int c0 = 0; c0 < BN; c0 += 128) {
+            tmem_ld_wait();
+            if (c0 + 64 < BN) {
+              tmem_ld_16x256b_x8(taddr + c0 + 64, na);
+              tmem_ld_16x256b_x8(taddr + upper + c0 + 64, nb);
+            }
+            emit_columns(ra, rb, c0);
+            if (c0 + 64 < BN) {
+              tmem_ld_wait();
+              if (c0 + 128 < BN) {
+                tmem_ld_16x256b_x8(taddr + c0 + 128, ra);
+                tmem_ld_16x256b_x8(taddr + upper + c0 + 128, rb);
+              }
+              emit_columns(na, nb, c0 + 64);
+            }
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+          if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+          continue;
+        }
         }
         if (p.tma_store && w.mode == kOutDirect) {
           // Fast path: 64 columns at a time go TMEM -> registers -> fp16 -> this warp's swizzled
@@ -1609,11 +1660,12 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   }
   const size_t smem = 1024 + (size_t)p.stages * (kATileBytes + bn * kBK * 2) + kStoreStagingBytes + 256 +
                       (conv ? kConvTableEntries * 4 : 0);
-  // whole tiles of a row-major, 16-byte-aligned C leave through a TMA store
+  // whole tiles of a row-major, 16-byte-aligned C leave through a TMA store, swapped ones transposed (not the M = 64 ones)
   CUtensorMap tc = tb;
   p.tma_store = 0;
-  if (!p.swap && bn >= 64 && (ldc & 7) == 0 && (sc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
-      make_tmap(&tc, C, p.PN, p.PM, p.batch, ldc, sc, 32) == HELIX_OK)
+  if (bn >= 64 && (ldc & 7) == 0 && (sc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
+      !(p.swap && (p.m64 || p.split_k > 1)) &&
+      (p.swap ? make_tmap(&tc, C, p.PM, p.PN, p.batch, ldc, sc, 64) : make_tmap(&tc, C, p.PN, p.PM, p.batch, ldc, sc, 32)) == HELIX_OK)
     p.tma_store = 1;
   // a launch that shares its workspace with its neighbours on the stream is never independent of them
   p.independent = (independent && !fixup && !reduce) ? 1 : 0;
