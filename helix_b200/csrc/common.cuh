@@ -413,6 +413,15 @@ __device__ __forceinline__ bool named_bar_and(int id, int nthreads, bool pred) {
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Reads a kernel's parameters once: their lines are cold in every launch, and a role that meets them one after the other
+// behind griddep_wait() pays for each (2300 cycles from the wait to the first load in the GEMM kernel).
+template <typename P>
+__device__ __forceinline__ void touch_params(const P& p) {
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(&p);
+#pragma unroll
+  for (unsigned i = 0; i < sizeof(P) / 4; i += 8) asm volatile("" ::"r"(w[i]));
+}
+
 // ---------------------------------------------------------------- misc loads
 __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {
   uint4 v;

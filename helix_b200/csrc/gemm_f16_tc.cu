@@ -346,6 +346,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const int lane = threadIdx.x & 31;
   const int cta = blockIdx.x;
   const int grid = gridDim.x;
+  if (warp > kMmaWarp) touch_params(p);   // warps with nothing to set up
 
   if (threadIdx.x == 0) {
     if (p.trace != nullptr) {
@@ -386,14 +387,9 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  // Everything above touched only this CTA's shared memory and TMEM, so it may overlap the tail of
-  // the preceding kernel.  From here on global memory is read and written: unless the caller
-  // declared the launch independent of its predecessor, wait for that kernel to complete.
-  if (!p.independent) {
-    griddep_wait();
-    griddep_launch_dependents();
-  }
-  if (threadIdx.x == 0 && p.trace != nullptr) p.trace[(size_t)cta * kTraceWords + 2] = (unsigned long long)clock64();
+  // Everything above touched only this CTA's shared memory and TMEM, so it may overlap the tail of the preceding kernel.
+  // Unless the caller declared the launch independent of its predecessor, the roles that read or write global memory wait
+  // for that kernel to complete: the producers when their first load is ready to be issued, the epilogue warps first thing.
 
   // the MMA-issuing role: warp kMmaWarp, and with dual issue also warp 3, which then issues no loads
   const bool second_issuer = !CONV && p.dual && warp == 3;
@@ -459,6 +455,10 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             pix_w = wo * p.g.stride - p.g.pad;
           }
           const int nkb = w.kb1 - w.kb0;
+          if (idx == 0 && !p.independent) {
+            griddep_wait();
+            if (pwarp == 0) griddep_launch_dependents();
+          }
           if (pwarp == 0) trace_mark(p, idx, 0);
           for (; my_n < n_start + nkb; my_n += p.load_warps) {
             const int kb = w.kb0 + (my_n - n_start);
@@ -553,6 +553,10 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         const int row = pw * 16 + it * 4 + sub;
         dst_off[it] = row * 128 + ((j ^ (row & 7)) << 4);
       }
+      if (!p.independent) {
+        griddep_wait();
+        griddep_launch_dependents();
+      }
       WorkItem w;
       for (int idx = 0; ok && get_item(p, cta, grid, idx, w); ++idx) {
         int64_t base_off[kConvRowsPerThread];  // element offset of the (possibly padded) window origin
@@ -613,6 +617,8 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter + 32)
+    if (!p.independent) griddep_wait();
+    if (quarter == 0 && lane == 0 && p.trace != nullptr) p.trace[(size_t)cta * kTraceWords + 2] = (unsigned long long)clock64();
     bool ok = true;
     const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
                         ((p.stride_c & 7) == 0);

@@ -301,6 +301,7 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
+  if (warp >= 2 && warp < 6) touch_params(p);   // warps with nothing to set up
 
   if (threadIdx.x == 0) {
     if (p.trace != nullptr) {
@@ -328,11 +329,8 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  if (!p.independent) {
-    griddep_wait();
-    griddep_launch_dependents();
-  }
-  if (threadIdx.x == 0) trace2(p, 2);
+  // Nothing so far has touched global memory: the roles that do wait for the predecessor, when their first load is ready to
+  // be issued, or first thing (epilogue).
 
   if (warp == 0 || warp >= 6) {
     // ------------------------------------------------------------------ TMA producers (each CTA)
@@ -374,6 +372,10 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       for (int tidx = 0; ok && get_item2(p, pair, num_pairs, tidx, it); ++tidx) {
         const Tile2 w = decode_tile2(p, it.tile);
         const int nkb = it.kb1 - it.kb0;
+        if (tidx == 0 && !p.independent) {
+          griddep_wait();
+          if (issuer == 0) griddep_launch_dependents();
+        }
         if (issuer == 0) trace2_tile(p, tidx, 0);
         for (; my_n < n_start + nkb; my_n += p.load_warps) {
           const int kb = it.kb0 + (my_n - n_start);
@@ -467,6 +469,8 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   } else {
     // ------------------------------------------------------------------ epilogue (each CTA: its 128 rows)
     const int quarter = warp & 3;
+    if (!p.independent) griddep_wait();
+    if (quarter == 0 && lane == 0) trace2(p, 2);
     bool ok = true;
     int box = 0;   // staging box in use; alternates over the whole run of the warp, across tiles
     Item2 it;
