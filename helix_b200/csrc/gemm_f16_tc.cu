@@ -308,13 +308,16 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
       }
 }
 
-// ANY: rows of C that a TMA store cannot write.  A variant of its own: as a branch beside the TMA store it made chains of
-// short launches 2 % slower.
-template <int BN, bool CONV, bool ANY>
+// How whole tiles leave: by TMA stores of 32 rows (or directly, where neither that nor the others apply), rows of C that a TMA
+// store cannot write, swapped tiles by transposed TMA stores.  Variants of their own: as branches beside the TMA store
+// the others made chains of short launches 2 % slower.
+enum TileOut { kOutRows = 0, kOutAny = 1, kOutColumns = 2 };
+template <int BN, bool CONV, int OUT>
 __global__ void __launch_bounds__(CONV ? kConvThreads : kGemmThreads, 1)
 gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
   using L = SmemLayout<BN>;
+  constexpr bool ANY = OUT == kOutAny;
   constexpr int kProducerWarps = CONV ? kConvProducerWarps : kGemmProducerWarps;
   constexpr int kMmaWarp = kProducerWarps;
   constexpr int kTmemCols = L::tmem_cols();
@@ -680,8 +683,8 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
           continue;
         }
-        if constexpr (!CONV && !ANY) {
-        if (p.tma_store && p.swap && w.mode == kOutDirect) {
+        if constexpr (OUT == kOutColumns) {
+        if (w.mode == kOutDirect) {
           // Swapped operands: TMEM lanes index the contiguous axis of C (for a convolution the output channels of a
           // pixel), so 64 columns at a time are transposed on their way to shared memory; two warps fill one box of 64 rows
           // x 64 channels, and one TMA store sends it.  (2-byte stores of a lane per channel, which this replaces, took 10500 cycles
@@ -731,7 +734,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           continue;
         }
         }
-        if (p.tma_store && w.mode == kOutDirect) {
+        if (OUT == kOutRows && p.tma_store && w.mode == kOutDirect) {
           // Fast path: 64 columns at a time go TMEM -> registers -> fp16 -> this warp's swizzled
           // 32 x 128-byte staging box -> one TMA store (full 128-byte lines, edges clipped by the
           // tensor map).  The TMEM load of the next 64 columns is in flight while the current ones
@@ -766,7 +769,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         }
       }
       if constexpr (BN >= 32) {
-        if (p.swap && w.mode == kOutDirect) {
+        if (OUT == kOutRows && p.swap && w.mode == kOutDirect) {
           // Swapped operands: TMEM lanes index the contiguous axis of C (C[col][row]: for a convolution the
           // output channels of one pixel).  A warp holds 32 consecutive rows of every tile column, so one
           // 2-byte store per lane writes 64 contiguous bytes of one C row: no transposition through shared
@@ -919,7 +922,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             };
             bool done = false;
             if constexpr (BN >= 64) {
-              if (ANY || p.tma_store) {
+              if (ANY || (OUT == kOutRows && p.tma_store)) {
 #pragma unroll 1
                 for (int c0 = 0; c0 < BN; c0 += 64) {
                   uint32_t lo[32], hi[32];
@@ -1542,11 +1545,11 @@ unsigned long long* gemm_f16_trace_for_grid(int grid) {
   return (g_trace_buf && g_trace_bytes >= (size_t)grid * kTraceWords * 8) ? g_trace_buf : nullptr;
 }
 
-template <int BN, bool CONV, bool ANY>
+template <int BN, bool CONV, int OUT>
 static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
                                   const GemmParams& p, int grid, size_t smem, cudaStream_t stream) {
   constexpr int threads = CONV ? kConvThreads : kGemmThreads;
-  auto kern = gemm_f16_tc_kernel<BN, CONV, ANY>;
+  auto kern = gemm_f16_tc_kernel<BN, CONV, OUT>;
   // the opt-in shared-memory size is sticky per function and device: raise it only when needed
   static std::mutex mu;
   static size_t granted[64] = {0};
@@ -1686,19 +1689,21 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   p.fd_s = make_fastdiv(p.im2col ? p.g.S : 1);
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
-  const bool any = !p.swap && !p.tma_store;
+  const bool any = !p.swap && !p.tma_store, columns = p.swap && p.tma_store;
   cudaError_t e = cudaErrorInvalidValue;
-#define HELIX_BN_CASE(BNV)                                                                 \
-  case BNV:                                                                                \
-    e = conv  ? launch_variant<BNV, true, false>(ta, tb, tc, p, grid, smem, stream)        \
-        : any ? launch_variant<BNV, false, (BNV >= 64)>(ta, tb, tc, p, grid, smem, stream) \
-              : launch_variant<BNV, false, false>(ta, tb, tc, p, grid, smem, stream);      \
+#define HELIX_BN_CASE(BNV)                                                                                        \
+  case BNV:                                                                                                       \
+    e = conv      ? launch_variant<BNV, true, kOutRows>(ta, tb, tc, p, grid, smem, stream)                        \
+        : any     ? launch_variant<BNV, false, BNV >= 64 ? kOutAny : kOutRows>(ta, tb, tc, p, grid, smem, stream) \
+        : columns ? launch_variant<BNV, false, BNV >= 64 ? kOutColumns : kOutRows>(ta, tb, tc, p, grid, smem, stream) \
+                  : launch_variant<BNV, false, kOutRows>(ta, tb, tc, p, grid, smem, stream);                      \
     break;
   switch (bn) {
     HELIX_BN_CASE(256)
     case 192:
-      e = any ? launch_variant<192, false, true>(ta, tb, tc, p, grid, smem, stream)
-              : launch_variant<192, false, false>(ta, tb, tc, p, grid, smem, stream);
+      e = any       ? launch_variant<192, false, kOutAny>(ta, tb, tc, p, grid, smem, stream)
+          : columns ? launch_variant<192, false, kOutColumns>(ta, tb, tc, p, grid, smem, stream)
+                    : launch_variant<192, false, kOutRows>(ta, tb, tc, p, grid, smem, stream);
       break;
     HELIX_BN_CASE(128)
     HELIX_BN_CASE(64)
