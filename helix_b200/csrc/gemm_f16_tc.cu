@@ -1272,7 +1272,7 @@ static int64_t plain_rounds(int pm, int pn, int bn, int batch, int sm_count) {
 // tile width minimising waves x slabs x slab time wins; stream-K is used when whole-tile
 // scheduling would leave a large part of the machine idle.
 static void default_config_impl(int M, int N, int K, int batch, int sm_count, bool conv, bool allow_pair,
-                                helix_cfg_t* out) {
+                                helix_cfg_t* out, bool tma_c = true) {
   *out = helix_cfg_t{};
   out->op = conv ? HELIX_OP_CONV_F16 : HELIX_OP_GEMM_F16;
   out->tile_m = kBM;
@@ -1405,6 +1405,23 @@ static void default_config_impl(int M, int N, int K, int batch, int sm_count, bo
       out->split_k = 1;
     }
   }
+  // Swapped tiles, M along the wide axis: where N fills its 128-row blocks, 192 or 256 of the other axis per tile often take
+  // fewer rounds than 128 (512 -> 128 channels, 1 x 1, 28 x 28 x 32: 196 tiles of 128 x 128 in two rounds, 131 of 192 x 128 in one).
+  // Only for a C that the transposed TMA store can write.
+  if (tma_c && !conv && !swap && whole_machine && N % 8 == 0 && N > kBM / 2 && M > kBM) {
+    const int wide[3] = {256, 192, 128};
+    for (int i = 0; i < 3; ++i) {
+      const double dp = (double)plain_rounds(N, M, wide[i], batch, sm_count) * num_kb * slab_us(wide[i]) + 4.0;
+      if (dp < best - 0.4) {
+        best = dp;
+        medium = false;
+        out->swap_ab = 1;
+        out->tile_n = wide[i];
+        out->stream_k = 0;
+        out->split_k = 1;
+      }
+    }
+  }
   out->stages = max_stages(out->tile_n, conv);
   // CTA pairs on a 256 x 256 tile: half the B bytes per CTA and a 6-deep ring; measured about
   // 0.41 us per 64-deep slab of a pair tile, i.e. twice the work of a 128 x 256 slab in less time.
@@ -1421,6 +1438,7 @@ static void default_config_impl(int M, int N, int K, int batch, int sm_count, bo
         best = t2;
         medium = false;
         out->cta_group = 2;
+        out->swap_ab = 0;
         out->tile_n = bn;
         out->stream_k = 0;
         out->split_k = 1;
@@ -1745,7 +1763,8 @@ int gemm_f16_launch(const helix_cfg_t* cfg_in, const void* A, int64_t lda, const
   if (cfg_in && cfg_in->tile_m != 0) {
     cfg = *cfg_in;
   } else {
-    gemm_f16_default_config(M, N, K, batch, sm_count, false, &cfg);
+    const bool tma_c = (ldc & 7) == 0 && (sc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    default_config_impl(M, N, K, batch, sm_count, false, true, &cfg, tma_c);
     const size_t need = gemm_f16_workspace_bytes(&cfg, M, N, K, batch, sm_count);
     const bool scratch = need > 0 && ws && ws_bytes >= need;
     if (batch == 1 && gemv_f16_stream_covers(B, ldb, A, lda, N, K, M, sm_count, scratch))

@@ -53,3 +53,25 @@ def test_convolution_pixels_on_the_wide_axis(bn, geom):
     ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), f.double().permute(0, 3, 1, 2), stride=stride,
                                      padding=pad).permute(0, 2, 3, 1)
     assert float((got.double() - ref).norm() / ref.norm()) < 2.0 ** -11
+
+
+@pytest.mark.parametrize("m,n,k,swapped", [(25088, 128, 512, 1), (25000, 136, 264, 0), (6468, 1024, 256, 1), (12544, 128, 512, 0),
+                                           (3291, 5648, 232, 1)])
+def test_library_choice_of_swapped_tiles(m, n, k, swapped):
+    """Both sides of the choice, and the same shapes with a C that only plain stores can write."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(m)
+    a = torch.empty((m, k), dtype=torch.float16, device="cuda").normal_(0, 1, generator=gen)
+    b = torch.empty((n, k), dtype=torch.float16, device="cuda").normal_(0, 0.1, generator=gen)
+    ref = torch.matmul(a.float(), b.float().t())
+    for pad in (0, 3):
+        c = torch.full((m, n + pad), 7.0, dtype=torch.float16, device="cuda")
+        l = ops.launch_gemm_f16(a, b, c[:, :n])
+        if ops.device_info().sm_count == 148:
+            assert ops.default_config(l).swap_ab == swapped
+        ops.run(l)
+        torch.cuda.synchronize()
+        ops.check_status()
+        assert bool((c[:, n:] == 7.0).all())
+        # one rounding to half, and fp32 sums of k products on both sides
+        assert float((c[:, :n].float() - ref).norm() / ref.norm()) < 2.0 ** -11
