@@ -13,6 +13,7 @@
 // independent 128-bit streaming loads outstanding.  Lanes are reduced with a shuffle tree.
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -470,6 +471,207 @@ gemv_f16_mma_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, 
   if (order_mode & 2) griddep_wait();
 }
 
+// The same product where the stream is long (gemv_f16_deep): X does not fit the SM, so it goes through the same per-lane FIFO
+// as the weights (NT of a group's 2 F + NT slots per 32 elements of K), and its trips to L2 are as deeply pipelined as the
+// weights' trips to HBM.  It is read once per block, so blocks are as high as pays (16 F rows); a group is J pieces of 32
+// elements, one CTA has the SM's shared memory to itself.  Ordered chains on distinct buffers, us above / here: m = 8,
+// 4096 x 4096 9.9 / 9.3, 12288 x 4096 22.6 / 20.9, 8192 x 8192 28.3 / 26.0, 1024 x 8192 12.2 / 8.0, 900 x 12000 16.4 / 10.0; m = 16,
+// 12288 x 4096 25.1 / 23.0, 11008 x 4096 23.9 / 21.6, 4096 x 11008 22.7 / 20.6.  On small problems its longer set-up shows:
+// 1000 x 3000, m = 8, 4.9 / 5.5; 600 x 600 3.1 / 3.5.
+constexpr int kMmaSlotBytes = kMmaThreads * 16;
+
+template <int NT, int F, int J, int CTAS>
+struct DeepStream {
+  static constexpr int kTok = NT * 8;
+  static constexpr int kSumFrags = CTAS > 1 ? 1 : F < 3 ? F : 3;      // 16-row fragments summed at a time
+  static constexpr int kSumPitch = 16 * kSumFrags + 4;        // floats per right-hand side: lanes of a quad 8 banks apart
+  static constexpr int kPartBytes = kMmaWarps * kTok * kSumPitch * 4;
+  static constexpr int kSlots = (2 * F + NT) * J;             // 16-byte slots of a lane per 32 J elements of K
+  static constexpr int kFit = ((CTAS == 1 ? 226 : 112) * 1024 - kPartBytes) / (kMmaSlotBytes * kSlots);
+  static constexpr int kGroups = kFit < 8 ? kFit : 8;         // groups in flight
+  static constexpr int kSmem = kGroups * kSlots * kMmaSlotBytes + kPartBytes;
+  static_assert(kGroups >= 2, "a group is read while others are in flight");
+};
+
+template <int NT, int F, int J, int CTAS>
+__global__ void __launch_bounds__(kMmaThreads, CTAS)
+gemv_f16_deep_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X, int64_t ldx, __half* Y, int64_t ldy,
+                    int64_t ldy_inner, int rows, int K, int m, int kw, int order_mode) {
+  using S = DeepStream<NT, F, J, CTAS>;
+  constexpr int kMaxRows = 16 * F, kTok = S::kTok, kGroups = S::kGroups, kSlots = S::kSlots;
+  constexpr int kXSlot = 2 * F * J;                 // X follows the weights in a group
+  extern __shared__ __align__(16) unsigned char stream_smem[];
+  float* part = reinterpret_cast<float*>(stream_smem + kGroups * kSlots * kMmaSlotBytes);   // [warp][kTok][kSumPitch]
+  if (order_mode == 0) griddep_wait();
+  if (!(order_mode & kHoldNext)) griddep_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int rw = kMmaWarps / kw;
+  const int kwi = warp % kw, rwi = warp / kw;
+  int r_begin, r_end;
+  stream_rows(rows, r_begin, r_end);
+  const int n = r_end - r_begin;
+  // equal blocks of at most 16 F rows, and where K leaves several row groups at least 16 rows for each
+  const int blocks = max((n + kMaxRows - 1) / kMaxRows, min(rw, (n + 15) / 16));
+  const int height = blocks ? (n + blocks - 1) / blocks : 0;
+  // the kw warps take 32 J elements of K in turn: together they read contiguous stretches of every row
+  const int k_begin = kwi * 32 * J, k_step = kw * 32 * J;
+  const uint32_t slot0 = smem_u32(stream_smem) + tid * 16;
+  const uint32_t slot_last = slot0 + (kGroups - 1) * kSlots * kMmaSlotBytes;
+  auto next_group = [&](uint32_t s) { return s == slot_last ? slot0 : s + kSlots * kMmaSlotBytes; };
+
+  // Rows beyond the block and right-hand sides beyond m are not copied: their slots hold whatever was there, which reaches
+  // only rows and columns of the product that are not stored.
+  int pb = rwi, pk = k_begin;
+  uint32_t pslot = slot0;
+  const __half* src[2 * F];
+  uint32_t live = 0;                                // bit u: row u * 8 + g exists
+  auto block_rows = [&]() {
+    const int row = pb * height, here = min(height, n - row);
+    live = 0;
+#pragma unroll
+    for (int u = 0; u < 2 * F; ++u) {
+      if (u * 8 + g < here) live |= 1u << u;
+      src[u] = W + static_cast<int64_t>(r_begin + row + u * 8 + g) * ldw + k_begin + t * 8;
+    }
+  };
+  block_rows();
+  auto issue_w = [&]() {
+    if (pb < blocks && pk < K) {
+      if (pk + 32 * J <= K) {
+#pragma unroll
+        for (int u = 0; u < 2 * F; ++u)
+          if (live >> u & 1)
+#pragma unroll
+            for (int j = 0; j < J; ++j) cp_async_16(pslot + (u * J + j) * kMmaSlotBytes, src[u] + j * 32);
+      } else {
+#pragma unroll
+        for (int u = 0; u < 2 * F; ++u)
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            const bool in = (live >> u & 1) && pk + j * 32 + t * 8 < K;
+            cp_async_16_zfill(pslot + (u * J + j) * kMmaSlotBytes, in ? src[u] + j * 32 : W, in);
+          }
+      }
+      pk += k_step;
+#pragma unroll
+      for (int u = 0; u < 2 * F; ++u) src[u] += k_step;
+      if (pk >= K) {
+        pk = k_begin;
+        pb += rw;
+        if (pb < blocks) block_rows();
+      }
+    }
+    pslot = next_group(pslot);
+  };
+  int xb = rwi, xk = k_begin;
+  uint32_t xslot = slot0 + kXSlot * kMmaSlotBytes;
+  const uint32_t xslot_last = slot_last + kXSlot * kMmaSlotBytes;
+  const __half* const xrow = X + g * ldx + t * 8;   // this lane's right-hand sides: g, g + 8, ...
+  auto issue_x = [&]() {
+    if (xb < blocks && xk < K) {
+#pragma unroll
+      for (int q = 0; q < NT; ++q)
+        if (q * 8 + g < m)
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            const bool in = xk + j * 32 + t * 8 < K;
+            cp_async_16_zfill(xslot + (q * J + j) * kMmaSlotBytes, in ? xrow + q * 8 * ldx + xk + j * 32 : X, in);
+          }
+      xk += k_step;
+      if (xk >= K) {
+        xk = k_begin;
+        xb += rw;
+      }
+    }
+    xslot = xslot == xslot_last ? slot0 + kXSlot * kMmaSlotBytes : xslot + kSlots * kMmaSlotBytes;
+  };
+  // The first groups' weights and, after the wait of mode 1, their X are commit groups of their own; from then on a group is
+  // one.  Whatever precedes X's group i is complete when at most kGroups - 1 later ones are pending, so one count serves all.
+#pragma unroll
+  for (int i = 0; i < kGroups; ++i) {
+    issue_w();
+    cp_async_commit();
+  }
+  if (order_mode & 1) {
+    griddep_wait();
+    griddep_launch_dependents();
+  }
+#pragma unroll
+  for (int i = 0; i < kGroups; ++i) {
+    issue_x();
+    cp_async_commit();
+  }
+
+  uint32_t cslot = slot0;
+  for (int sb = 0; sb < blocks; sb += rw) {         // one block per row group
+    const int b = sb + rwi;
+    float acc[F][NT][4];
+#pragma unroll
+    for (int h = 0; h < F; ++h)
+#pragma unroll
+      for (int q = 0; q < NT; ++q)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[h][q][e] = 0.0f;
+    if (b < blocks) {
+      for (int k = k_begin; k < K; k += k_step) {
+        cp_async_wait<kGroups - 1>();
+        uint4 xv[NT][J], wv[2 * F][J];
+#pragma unroll
+        for (int q = 0; q < NT; ++q)
+#pragma unroll
+          for (int j = 0; j < J; ++j) xv[q][j] = lds_16(cslot + (kXSlot + q * J + j) * kMmaSlotBytes);
+#pragma unroll
+        for (int u = 0; u < 2 * F; ++u)
+          if ((u & ~1) * 8 < height)
+#pragma unroll
+            for (int j = 0; j < J; ++j) wv[u][j] = lds_16(cslot + (u * J + j) * kMmaSlotBytes);
+        issue_w();
+        issue_x();
+        cp_async_commit();
+        cslot = next_group(cslot);
+#pragma unroll
+        for (int h = 0; h < F; ++h)
+          if (h * 16 < height)
+#pragma unroll
+            for (int j = 0; j < J; ++j)
+#pragma unroll
+              for (int q = 0; q < NT; ++q) {
+                const uint4 w0 = wv[2 * h][j], w1 = wv[2 * h + 1][j];
+                mma_f16_16x8x16(acc[h][q], w0.x, w1.x, w0.y, w1.y, xv[q][j].x, xv[q][j].y);
+                mma_f16_16x8x16(acc[h][q], w0.z, w1.z, w0.w, w1.w, xv[q][j].z, xv[q][j].w);
+              }
+      }
+    }
+    // some fragments of every row group at a time: partial sums to shared memory, slices added in slice order
+#pragma unroll
+    for (int h0 = 0; h0 < F; h0 += S::kSumFrags) {
+      if (h0 * 16 < height) {
+        __syncthreads();                            // the previous sums have been read
+#pragma unroll
+        for (int h = h0; h < F && h < h0 + S::kSumFrags; ++h)
+#pragma unroll
+          for (int q = 0; q < NT; ++q)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              part[(warp * kTok + q * 8 + t * 2 + (e & 1)) * S::kSumPitch + (h - h0) * 16 + g + (e >> 1) * 8] = acc[h][q][e];
+        __syncthreads();
+        constexpr int kSumRows = 16 * S::kSumFrags;
+        for (int o = tid; o < rw * kTok * kSumRows; o += kMmaThreads) {
+          const int rr = o % kSumRows, tok = (o / kSumRows) % kTok, grp = (o / kSumRows) / kTok;
+          const int r = h0 * 16 + rr, row = (sb + grp) * height + r;
+          if (tok < m && r < height && sb + grp < blocks && row < n) {
+            float s = 0.0f;
+            for (int q = 0; q < kw; ++q) s += part[((grp * kw + q) * kTok + tok) * S::kSumPitch + rr];
+            Y[tok * ldy + static_cast<int64_t>(r_begin + row) * ldy_inner] = __float2half_rn(s);
+          }
+        }
+      }
+    }
+  }
+  if (order_mode & 2) griddep_wait();
+}
+
 // Sums the split-K partials in slice order (deterministic) and rounds once.
 __global__ void gemv_splitk_reduce_kernel(const float* __restrict__ partial, __half* __restrict__ Y, int64_t ldy,
                                           int64_t ldy_inner, int rows, int m, int split_k) {
@@ -587,6 +789,11 @@ static int launch_stream(void (*kern)(Params...), int& attr_dev, int grid, int t
   return HELIX_OK;
 }
 
+// Streams that are worth the deep kernel's set-up: some 8 MB where K is long, 20 MB otherwise (us, above / deep: 1184 x 4096, m = 8,
+// 7.3 / 6.7; 700 x 8192 12.0 / 9.8; 300 x 4096 5.2 / 5.4; 3582 x 3048, m = 6, 7.3 / 7.2; 1852 x 3288, m = 4, 7.0 / 7.4; 22912 x 792, m = 3,
+// 11.6 / 14.4).
+static bool gemv_f16_deep(int rows, int K) { return K >= 1024 && (int64_t)rows * K > (K >= 4096 ? 4 << 20 : 10 << 20); }
+
 int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y, int64_t ldy,
                            int64_t ldy_inner, int rows, int K, int m, int sm_count, int order_mode,
                            cudaStream_t stream, int64_t* launches) {
@@ -619,13 +826,37 @@ int gemv_f16_stream_launch(const void* W, int64_t ldw, const void* X, int64_t ld
     return launch_stream(gemv_f16_stream_kernel<2>, attr_dev[1], grid, kStreamThreads, smem, stream, launches, w, ldw, x, ldx, y, ldy,
                          ldy_inner, rows, K, kw, order_mode);
   }
-  const int kw = stream_k_warps(K, 64, kMmaWarps);
-  const int smem = kMmaThreads * kMmaSlots * 16 + kMmaWarps * (m <= 8 ? 8 : 16) * 16 * 4;
-  if (m <= 8)
-    return launch_stream(gemv_f16_mma_kernel<1>, attr_dev[2], grid, kMmaThreads, smem, stream, launches, w, ldw, x, ldx, y,
-                         ldy, ldy_inner, rows, K, m, kw, order_mode);
-  return launch_stream(gemv_f16_mma_kernel<2>, attr_dev[3], grid, kMmaThreads, smem, stream, launches, w, ldw, x, ldx, y, ldy,
-                       ldy_inner, rows, K, m, kw, order_mode);
+  if (!gemv_f16_deep(rows, K)) {
+    const int kw = stream_k_warps(K, 64, kMmaWarps);
+    const int smem = kMmaThreads * kMmaSlots * 16 + kMmaWarps * (m <= 8 ? 8 : 16) * 16 * 4;
+    if (m <= 8)
+      return launch_stream(gemv_f16_mma_kernel<1>, attr_dev[2], grid, kMmaThreads, smem, stream, launches, w, ldw, x, ldx, y, ldy,
+                           ldy_inner, rows, K, m, kw, order_mode);
+    return launch_stream(gemv_f16_mma_kernel<2>, attr_dev[3], grid, kMmaThreads, smem, stream, launches, w, ldw, x, ldx, y, ldy,
+                         ldy_inner, rows, K, m, kw, order_mode);
+  }
+  auto deep = [&](auto nt, auto f, auto j, auto ctas) {
+    constexpr int NT = decltype(nt)::value, F = decltype(f)::value, J = decltype(j)::value, CTAS = decltype(ctas)::value;
+    const int kw = stream_k_warps(K, 32 * J, kMmaWarps);
+    static thread_local int deep_dev = -1;
+    return launch_stream(gemv_f16_deep_kernel<NT, F, J, CTAS>, deep_dev, grid, kMmaThreads, DeepStream<NT, F, J, CTAS>::kSmem, stream,
+                         launches, w, ldw, x, ldx, y, ldy, ldy_inner, rows, K, m, kw, order_mode);
+  };
+  const std::integral_constant<int, 1> one{};
+  const std::integral_constant<int, 2> two{};
+  const std::integral_constant<int, 4> four{};
+  // J sets the order of a row's sums, so it follows from the sizes alone (us at J = 2 / 4: 1024 x 8192, m = 8, 8.7 / 8.0, 4096 x
+  // 4096 9.3 / 9.3; 1200 x 16384, m = 16, 17.7 / 15.2).  F and the CTAs to an SM do not: blocks of 64 rows where they replace two of
+  // 32 that would be half empty, or where X is twice as long (5120 x 5120, m = 8, F = 2 / 4: 13.9 / 12.9; 12288 x 4096, m = 16, 23.7 /
+  // 23.0); independent launches share SMs (8656 x 1280, m = 3: 5.8 alone on an SM, 4.6 two to one).
+  const bool share = order_mode == 2;
+  const int per_cta = (rows + grid - 1) / grid;
+  if (rows < 2400) {
+    if (m > 8) return deep(two, two, four, one);
+    return share ? deep(one, one, four, two) : deep(one, two, four, one);
+  }
+  if (m > 8) return share ? deep(two, two, two, two) : per_cta > 32 ? deep(two, four, two, one) : deep(two, two, two, one);
+  return share ? deep(one, two, two, two) : per_cta > 32 && per_cta <= 48 ? deep(one, four, two, one) : deep(one, two, two, one);
 }
 
 // Which GEMVs without a configuration of their own the streaming kernels run (whatever their flags, which change no bits).
@@ -646,22 +877,24 @@ static bool gemv_f16_streams(int rows, int K, int m, int split, bool scratch, in
     return m == 2 || rows < 4096 || K > 3072 || (rows < 8192 && K > 1536) || (rows < 5000 && K > 768) ||
            (rows >= 10000 && K < 512);
   }
-  // The matrix kernel's chain over K takes about K / 1000 us whatever m, the split kernel's m times K / split: m = 3,
-  // 64 x 65536 15.3 / 66, 512 x 8192 9.2 / 10.9 (split 4), 700 x 8192 14.9 / 11.0 (split 2); m = 8, 64 x 65536 36 / 74 (split
-  // 16), 148 x 16384 19.1 / 20.4, 296 x 16384 34.9 / 20.6 (split 4).  From 1024 rows on the slices are more warps than fit
-  // (m = 4, 2048 x 65536: 135 / 80).
-  if (scratch && rows < 1024) return split < m || (split == m && rows < 64);
+  // A CTA's chain over K takes some time per 1000 elements whatever m, the split kernel's m times K / split.  Split / streaming, the
+  // kernel for small streams: m = 3, 64 x 65536 15.3 / 66; m = 8, 64 x 65536 36 / 74 (split 16); from 1024 rows on the slices are more
+  // warps than fit.  The deep one, 0.6 us per 1000: m = 3, 111 x 60672 15.2 / 34.4, 120 x 40280 11.8 / 24.2, 644 x 52288 88 / 31; m = 4, 186 x
+  // 22344 14.0 / 19.0, 248 x 39640 23.4 / 24.8; m = 5, 142 x 42960 19.9 / 25.6, 374 x 16584 22.1 / 14.1; m = 8, 296 x 16384 20.5 / 16.0.
+  if (scratch && rows < 1024) {
+    if (!gemv_f16_deep(rows, K)) return split < m || (split == m && rows < 64);
+    return rows >= 256 || K < (m <= 4 ? 16384 : 40000);
+  }
   return !(m == 3 && K <= 256 && rows <= 512);         // 256 x 256: 1.9 / 2.2
 }
 
 // Skinny products: the streaming kernels against the stream-K tcgen05 tiles (or, without scratch, plain tiles, which lose
-// everywhere).  A launch of the matrix kernel lasts as long as one CTA's chain over K for each of its blocks of up to 32 rows, so
-// it loses where rows are few and K is long, and where the last block is half empty; nine to sixteen right-hand sides read
-// twice the X per weight and lose to the tiles from some 100 MB of weights on.  us, tiles / streaming:
-// m = 3: 2048 x 12288 17.8 / 16.0, 1024 x 14336 15.4 / 17.1, 3000 x 24576 35.9 / 33.0, 4096 x 32768 52.0 / 52.0; m = 8: 1024 x 10240
-// 14.6 / 14.3, 1024 x 14336 15.5 / 18.9, 3000 x 20480 29.0 / 31.6, 4096 x 14336 28.0 / 25.2, 6000 x 14336 36.4 / 42.6;
-// m = 16: 1024 x 8192 14.4 / 13.1, 2048 x 10240 16.4 / 17.5, 4096 x 14336 28.1 / 27.5, 14592 x 1536 16.4 / 16.1, 16000 x 2048
-// 18.8 / 19.6, 32000 x 512 13.7 / 15.0.
+// everywhere).  us, tiles / streaming.  Up to eight rows streaming wins at every size where rows of W start on 32 bytes (m = 3, 1827 x 14336
+// 17.2 / 12.8, 12496 x 16384 71 / 69; m = 8, 1024 x 14336 14.4 / 11.2, 8737 x 27904 83 / 81); where they do not, a copy of 64 bytes
+// touches a third sector and large ones lose (16512 x 10072 62 / 69, 22016 x 11512 86 / 100, but 9216 x 872 9.7 / 7.1).
+// Nine to sixteen rows bring twice the X: m = 16, 1283 x 19968 17.4 / 19.0, 1200 x 16384 16.0 / 15.2; m = 12, 2525 x 17584 23.1 / 24.9,
+// 2330 x 15968 20.6 / 19.4, 4992 x 16128 34.2 / 32.3; m = 16, 5760 x 1024 9.5 / 7.6, 16384 x 6144 41.0 / 40.5, 24576 x 4096 41.0 / 42.0, 18944 x 4096
+// 30.6 / 33.2, 19000 x 4096 34.2 / 31.9; m = 12, 21329 x 768 12.6 / 13.3; 2816 x 8792 (rows on 16 bytes) 16.8 / 18.1.
 bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t ldx, int rows, int K, int m, int sm_count,
                             bool scratch) {
   if (m < 1 || m > 16 || rows < 1024 || K < 512 || (K & 7) || ((ldw ? ldw : K) & 7) || ((ldx ? ldx : K) & 7) ||
@@ -669,11 +902,10 @@ bool gemv_f16_stream_covers(const void* W, int64_t ldw, const void* X, int64_t l
     return false;
   if (m <= 2 || !scratch) return true;
   const int64_t work = (int64_t)rows * K;
-  if (m > 8 && (work > 52 << 20 || rows > 24576 || (rows > 13312 && work > 24 << 20))) return false;
-  const int per_sm = (rows + sm_count - 1) / sm_count, blocks = (per_sm + 31) / 32;
-  if (per_sm < 24) return K <= (m > 8 ? 8192 : m > 4 ? 10240 : per_sm < 16 ? 12288 : 20480);
-  if (blocks > 1 && per_sm < blocks * 24) return m <= 8 && K <= 12288;
-  return K <= (m > 8 ? 16384 : 24576);
+  const bool on_sectors = ((ldw ? ldw : K) & 15) == 0 && (reinterpret_cast<uintptr_t>(W) & 31) == 0;
+  if (!on_sectors && (work > (m > 8 ? 12 << 20 : 64 << 20) || (rows < 24 * sm_count && K > (m > 8 ? 8192 : 10240)))) return false;
+  if (m <= 8) return K <= 32768;
+  return rows <= 20480 && (rows <= 18000 || K >= 1024) && (rows > 4096 || K <= 16384);
 }
 
 int gemv_f16_launch(const helix_cfg_t* cfg, const void* W, int64_t ldw, const void* X, int64_t ldx, void* Y,
