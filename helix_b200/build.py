@@ -11,6 +11,7 @@ import hashlib
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
@@ -21,6 +22,30 @@ SOURCES = ["capi.cu", "gemv_f16.cu", "sgemm_f32.cu", "gemm_f16_tc.cu", "gemm_f16
 HEADERS = ["common.cuh", "conv_common.cuh", "sgemm_f32_ring.cuh", "kernels.h", os.path.join("..", "..", "include", "helix_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
+
+
+EAGER_SRC = os.path.join(CSRC, "eager_call.cpp")
+EAGER_PATH = os.path.join(PKG_DIR, "_eager_call.so")
+
+
+def _build_eager():
+    """The Python module of the eager operators: host code against torch's C++ headers."""
+    import torch
+    home = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"] +
+           ["-I" + d for d in (os.path.join(home, "include"), os.path.join(home, "include", "torch", "csrc", "api", "include"),
+                               os.path.join(cuda, "include"), sysconfig.get_paths()["include"])] +
+           [EAGER_SRC, "-o", EAGER_PATH, "-L" + os.path.join(home, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+    stamp = os.path.join(OBJ_DIR, "eager_call.sha")
+    dig = _digest([EAGER_SRC, os.path.join(CSRC, HEADERS[-1])], " ".join(cmd) + torch.__version__)
+    if os.path.exists(EAGER_PATH) and os.path.exists(stamp) and open(stamp).read() == dig:
+        return
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for eager_call.cpp:\n{res.stdout}\n{res.stderr}")
+    with open(stamp, "w") as f:
+        f.write(dig)
 
 
 def _digest(paths, extra=""):
@@ -66,6 +91,7 @@ def build(verbose=False, force=False):
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    _build_eager()
     return LIB_PATH
 
 

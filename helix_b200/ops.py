@@ -16,6 +16,24 @@ from ._lib import Cfg, DevInfo, Launch, OP_CONV_F16, OP_GEMM_F16, OP_GEMM_F32, O
 
 _status_words = {}
 _workspaces = {}
+_eager = None
+
+
+def _native():
+    """The native form of the eager operators (csrc/eager_call.cpp): a call it does not cover returns None and goes through
+    the Python implementation below."""
+    global _eager
+    if _eager is None:
+        lib = _lib.load()
+        try:
+            from . import _eager_call
+        except ImportError as e:
+            raise ImportError("helix_b200/_eager_call is missing: build it with `python -m helix_b200.build`.") from e
+        _eager_call.connect(ctypes.cast(lib.helix_launch, ctypes.c_void_p).value,
+                            ctypes.cast(lib.helix_workspace_bytes, ctypes.c_void_p).value,
+                            _status_words, status_word, workspace, check)
+        _eager = _eager_call
+    return _eager
 
 
 def _require_cuda(*tensors):
@@ -239,6 +257,8 @@ def launch_gemv_f32(w, x, out, cfg=None, ws=None, out_transposed=False):
 
 
 def gemv_f32(w, x, out=None, cfg=None):
+    if cfg is None and (y := _native().gemv_f32(w, x, out)) is not None:
+        return y
     if out is None:
         out = w.new_empty((x.shape[0], w.shape[0]))
     run(launch_gemv_f32(w, x, out, cfg))
@@ -314,6 +334,8 @@ def launch_conv2d_f32(x, w, out, stride, pad, cfg=None, ws=None):
 
 
 def conv2d_f32_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
+    if cfg is None and (y := _native().conv2d_f32(x, w, stride, pad, out)) is not None:
+        return y
     N, H, W, _ = x.shape
     KO, R, S, _ = w.shape
     Ho, Wo = conv_out_hw(H, W, R, S, stride, pad)
@@ -346,14 +368,13 @@ def launch_gemm_f32(a, b, out, trans_a=False, cfg=None):
 
 def run(launch):
     """Queue a prepared launch on torch's current stream."""
-    dev = torch.cuda.current_device()
-    rc = _lib.load().helix_launch(ctypes.byref(launch), status_word(dev).data_ptr(), _stream(dev))
-    if rc != 0:
-        check(rc, "helix_launch")
+    _native().run(launch)
 
 
 # ----------------------------------------------------------------------------- eager operators
 def gemm_f16(a, b_nk, out=None, cfg=None):
+    if cfg is None and (y := _native().gemm_f16(a, b_nk, out)) is not None:
+        return y
     shape = (*a.shape[:-1], b_nk.shape[-2])
     if out is None:
         out = a.new_empty(shape)
@@ -362,6 +383,8 @@ def gemm_f16(a, b_nk, out=None, cfg=None):
 
 
 def gemv_f16(w, x, out=None, cfg=None):
+    if cfg is None and (y := _native().gemv_f16(w, x, out)) is not None:
+        return y
     if out is None:
         out = w.new_empty((x.shape[0], w.shape[0]))
     run(launch_gemv_f16(w, x, out, cfg))
@@ -369,6 +392,8 @@ def gemv_f16(w, x, out=None, cfg=None):
 
 
 def conv2d_f16_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
+    if cfg is None and (y := _native().conv2d_f16(x, w, stride, pad, out)) is not None:
+        return y
     if out is None:
         Ho, Wo = conv_out_hw(x.shape[1], x.shape[2], w.shape[1], w.shape[2], stride, pad)
         out = x.new_empty((x.shape[0], Ho, Wo, w.shape[0]))
@@ -377,6 +402,8 @@ def conv2d_f16_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
 
 
 def gemm_f32(a, b, trans_a=False, out=None, cfg=None):
+    if cfg is None and (y := _native().gemm_f32(a, b, trans_a, out)) is not None:
+        return y
     M = a.shape[1] if trans_a else a.shape[0]
     if out is None:
         out = a.new_empty((M, b.shape[1]))
