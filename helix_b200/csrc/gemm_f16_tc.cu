@@ -110,13 +110,15 @@ struct GemmParams {
 // kTraceTiles work items six clock64 stamps: producer first / last request, MMA issue start / end,
 // epilogue start / end.
 
+template <bool LEAN>
 __device__ __forceinline__ void trace_slab(const GemmParams& p, int which, int n) {
-  if (p.trace != nullptr && n < kTraceSlabs)
+  if (!LEAN && p.trace != nullptr && n < kTraceSlabs)
     p.trace[(size_t)blockIdx.x * kTraceWords + 8 + 6 * kTraceTiles + which * kTraceSlabs + n] =
         (unsigned long long)clock64();
 }
+template <bool LEAN>
 __device__ __forceinline__ void trace_mark(const GemmParams& p, int idx, int slot) {
-  if (p.trace != nullptr && idx < kTraceTiles)
+  if (!LEAN && p.trace != nullptr && idx < kTraceTiles)
     p.trace[(size_t)blockIdx.x * kTraceWords + 8 + idx * 6 + slot] = (unsigned long long)clock64();
 }
 
@@ -145,7 +147,18 @@ __device__ __forceinline__ void decode_tile(const GemmParams& p, int t, WorkItem
 }
 
 // The idx-th work item of CTA `cta`; every role of the CTA walks the same sequence.
+template <bool LEAN>
 __device__ __forceinline__ bool get_item(const GemmParams& p, int cta, int grid, int idx, WorkItem& w) {
+  if constexpr (LEAN) {
+    w.tile = cta + idx * grid;
+    if (w.tile >= p.total_items) return false;
+    decode_tile(p, w.tile, w);
+    w.kb0 = 0;
+    w.kb1 = p.num_kb;
+    w.mode = kOutDirect;
+    w.aux = 0;
+    return true;
+  }
   if (!p.stream_k) {
     int t = cta + idx * grid;
     if (t >= p.total_items) return false;
@@ -202,12 +215,12 @@ struct SmemLayout {
 // uniform registers instead of being moved there per operand from one lane's registers.  DUAL: two warps run this loop
 // and issue alternate slabs (ME = 0 / 1).  Both are compile-time constants of each copy of the loop so that
 // everything it computes stays warp-uniform for the compiler.
-template <int BN, bool CONV, bool DUAL, int ME>
+template <int BN, bool CONV, bool DUAL, int ME, bool LEAN>
 __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int cta, const int grid, const int lane,
                                                const int stages, uint8_t* sA, uint8_t* sB, uint64_t* full_bar,
                                                uint64_t* empty_bar, uint64_t* tmem_full, uint64_t* tmem_empty,
                                                volatile int* abort_flag, const uint32_t tmem_base) {
-  const uint32_t kIdesc = p.m64 ? umma_idesc_f16(64, BN) : umma_idesc_f16(kBM, BN);
+  const uint32_t kIdesc = !LEAN && p.m64 ? umma_idesc_f16(64, BN) : umma_idesc_f16(kBM, BN);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -215,7 +228,7 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
       int gpos = 0, gidx = 0;   // position of the next slab inside its group of stages, and the group
       // with timeline capture on: where the issuing warp's cycles go, summed over its slabs (barrier wait, fence +
       // descriptors, the four MMAs, commit, everything between one slab's commit and the next slab's wait)
-      const bool tr = p.trace != nullptr && ME == 0;
+      const bool tr = !LEAN && p.trace != nullptr && ME == 0;
       unsigned int c_wait = 0, c_desc = 0, c_mma = 0, c_commit = 0, c_rest = 0, c_slabs = 0;
       long long t_prev = 0;
       WorkItem w;
@@ -223,13 +236,13 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
       // named barrier shared with warp 0; the sequence is then walked to its end even after a failed wait
       // (ok = false: nothing is issued any more, only the rendezvous are kept).
       constexpr bool kForward = !CONV;
-      for (int idx = 0; (kForward || ok) && get_item(p, cta, grid, idx, w); ++idx) {
+      for (int idx = 0; (kForward || ok) && get_item<LEAN>(p, cta, grid, idx, w); ++idx) {
         const int acc = idx & 1;
         const uint32_t acc_phase = (idx >> 1) & 1;
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status));
         if (!ok && !kForward) break;
         tc_fence_after_sync();
-        if (lane == 0 && ME == 0) trace_mark(p, idx, 2);
+        if (lane == 0 && ME == 0) trace_mark<LEAN>(p, idx, 2);
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
           // One wait per group of stages: reading shared memory (the barrier) costs the issuing warp some 200
@@ -260,7 +273,7 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
           const bool mine = !DUAL || (n & 1) == ME;
           long long t2 = 0, t3 = 0;
           if (mine) {
-          if (lane == 0) trace_slab(p, 1, n);
+          if (lane == 0) trace_slab<LEAN>(p, 1, n);
           const uint64_t da = umma_desc_sw128(smem_u32(sA + (size_t)stage * kATileBytes));
           const uint64_t db = umma_desc_sw128(smem_u32(sB + (size_t)stage * SmemLayout<BN>::kBTileBytes));
           if (DUAL && n > 0) {   // everything but the MMAs themselves is done before the token is awaited
@@ -268,7 +281,7 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
             tc_fence_after_sync();
           }
           t2 = tr ? clock64() : 0;
-          if (ok && !(p.probe & 1)) {
+          if (ok && (LEAN || !(p.probe & 1))) {
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k) {
               // advancing 16 halves = 32 bytes along K inside the swizzle atom: +2 in the address field
@@ -294,7 +307,7 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
           }
         }
         if (ok) umma_commit_elect(&tmem_full[acc]);      // dual: both warps, each for its own MMAs (count 2)
-        if (lane == 0 && ME == 0) trace_mark(p, idx, 3);
+        if (lane == 0 && ME == 0) trace_mark<LEAN>(p, idx, 3);
       }
       // the token of the last slab is met by the warp that did not issue it, so that no arrival is left over
       if (DUAL && nslab > 0 && ((nslab - 1) & 1) != ME) named_bar_sync(kTokBarrier + ((nslab - 1) & 1), 64);
@@ -311,13 +324,17 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
 // How whole tiles leave: by TMA stores of 32 rows (or directly, where neither that nor the others apply), rows of C that a TMA
 // store cannot write, swapped tiles by transposed TMA stores.  Variants of their own: as branches beside the TMA store
 // the others made chains of short launches 2 % slower.
+// LEAN: whole tiles only, one issuing warp, no probes and no timeline -- what most launches are.  The code that is left out
+// is not run by them, but a launch of a few us starts with a cold instruction cache and pays for what lies in between.
 enum TileOut { kOutRows = 0, kOutAny = 1, kOutColumns = 2 };
-template <int BN, bool CONV, int OUT>
+template <int BN, bool CONV, int OUT, bool LEAN>
 __global__ void __launch_bounds__(CONV ? kConvThreads : kGemmThreads, 1)
 gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
   using L = SmemLayout<BN>;
   constexpr bool ANY = OUT == kOutAny;
+  const bool dual = !CONV && !LEAN && p.dual;
+  const bool swap = LEAN ? OUT == kOutColumns : p.swap != 0;
   constexpr int kProducerWarps = CONV ? kConvProducerWarps : kGemmProducerWarps;
   constexpr int kMmaWarp = kProducerWarps;
   constexpr int kTmemCols = L::tmem_cols();
@@ -352,7 +369,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   if (warp > kMmaWarp) touch_params(p);   // warps with nothing to set up
 
   if (threadIdx.x == 0) {
-    if (p.trace != nullptr) {
+    if (!LEAN && p.trace != nullptr) {
       p.trace[(size_t)cta * kTraceWords + 0] = global_timer_ns();
       p.trace[(size_t)cta * kTraceWords + 1] = (unsigned long long)clock64();
     }
@@ -363,7 +380,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
-      mbar_init(&tmem_full[a], p.dual ? 2 : 1);
+      mbar_init(&tmem_full[a], dual ? 2 : 1);
       mbar_init(&tmem_empty[a], 4);
     }
     *abort_flag = 0;
@@ -395,16 +412,16 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   // for that kernel to complete: the producers when their first load is ready to be issued, the epilogue warps first thing.
 
   // the MMA-issuing role: warp kMmaWarp, and with dual issue also warp 3, which then issues no loads
-  const bool second_issuer = !CONV && p.dual && warp == 3;
+  const bool second_issuer = dual && warp == 3;
   if (warp == kMmaWarp) {
-    if (!CONV && p.dual)
-      mma_issue_loop<BN, CONV, true, 0>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+    if (dual)
+      mma_issue_loop<BN, CONV, !LEAN, 0, LEAN>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                         abort_flag, tmem_base);
     else
-      mma_issue_loop<BN, CONV, false, 0>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+      mma_issue_loop<BN, CONV, false, 0, LEAN>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                          abort_flag, tmem_base);
   } else if (second_issuer) {
-    mma_issue_loop<BN, CONV, !CONV, 1>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+    mma_issue_loop<BN, CONV, !CONV && !LEAN, 1, LEAN>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                        abort_flag, tmem_base);
   } else if (warp < kProducerWarps) {
     // ------------------------------------------------------------------ producers
@@ -427,11 +444,11 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         int stage = 0, gpos = 0, gidx = 0;
         uint32_t phase = 0;
         WorkItem w;
-        for (int idx = 0; get_item(p, cta, grid, idx, w); ++idx) {
+        for (int idx = 0; get_item<LEAN>(p, cta, grid, idx, w); ++idx) {
           for (int kb = w.kb0; kb < w.kb1; ++kb) {
             if (gpos == 0) {
               if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[gidx], phase, abort_flag, p.status));
-              named_bar_sync(kFwdBarrier + gidx, p.dual ? 96 : 64);
+              named_bar_sync(kFwdBarrier + gidx, dual ? 96 : 64);
             }
             if (++gpos == p.group) { gpos = 0; ++gidx; }
             if (++stage == stages) { stage = 0; phase ^= 1; gidx = 0; }
@@ -446,13 +463,13 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         int stage = pwarp;    // load_warps <= stages, so no wrap yet
         uint32_t phase = 0;
         WorkItem w;
-        for (int idx = 0; ok && get_item(p, cta, grid, idx, w); ++idx) {
+        for (int idx = 0; ok && get_item<LEAN>(p, cta, grid, idx, w); ++idx) {
           // convolution through the im2col map: base pixel of the tile's first output pixel
           int pix_w = 0, pix_h = 0, pix_n = 0;
           if (p.im2col) {
             int rem, ho, wo;
             // pixels run along the 128-row axis, or along the BN axis when the operands are swapped
-            fast_divmod(p.swap ? w.n_blk * BN : w.m_blk * kBM, p.fd_howo, pix_n, rem);
+            fast_divmod(swap ? w.n_blk * BN : w.m_blk * kBM, p.fd_howo, pix_n, rem);
             fast_divmod(rem, p.fd_wo, ho, wo);
             pix_h = ho * p.g.stride - p.g.pad;
             pix_w = wo * p.g.stride - p.g.pad;
@@ -462,19 +479,19 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             griddep_wait();
             if (pwarp == 0) griddep_launch_dependents();
           }
-          if (pwarp == 0) trace_mark(p, idx, 0);
+          if (pwarp == 0) trace_mark<LEAN>(p, idx, 0);
           for (; my_n < n_start + nkb; my_n += p.load_warps) {
             const int kb = w.kb0 + (my_n - n_start);
             ok = mbar_wait(&empty_bar[stage >> p.eshift], phase ^ 1, abort_flag, p.status);
             if (!ok) break;
-            trace_slab(p, 0, my_n);
+            trace_slab<LEAN>(p, 0, my_n);
             uint64_t* const fb = &full_bar[fast_div(stage, p.fd_grp)];
-            const bool load_a = !(p.probe & 2), load_b = !(p.probe & 4);
+            const bool load_a = LEAN || !(p.probe & 2), load_b = LEAN || !(p.probe & 4);
             if (load_a || load_b)
               mbar_arrive_expect_tx(fb, (load_a ? kATileBytes : 0) + (load_b ? L::kBTileBytes : 0));
             else
               mbar_arrive(fb);
-            if (p.probe & 6) {
+            if (!LEAN && (p.probe & 6)) {
               // probe runs: the same requests minus the operand(s) left out; results are meaningless
               if (p.im2col) {
                 int tap, cb, fr, fs;
@@ -502,7 +519,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
               int tap, cb, fr, fs;
               fast_divmod(kb, p.fd_cblocks, tap, cb);
               fast_divmod(tap, p.fd_s, fr, fs);
-              if (p.swap) {   // weights on the 128-row axis, BN pixels per im2col box on the other
+              if (swap) {   // weights on the 128-row axis, BN pixels per im2col box on the other
                 tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, p.wtaps ? cb * kBK : kb * kBK,
                             p.wtaps ? tap : w.m_blk * kBM, p.wtaps ? w.m_blk * kBM : 0);
                 tma_load_im2col_4d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, cb * kBK, pix_w,
@@ -522,7 +539,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             if (stage >= stages) { stage -= stages; phase ^= 1; }
           }
           n_start += nkb;
-          if (pwarp == 0) trace_mark(p, idx, 1);
+          if (pwarp == 0) trace_mark<LEAN>(p, idx, 1);
         }
         // The last group of the CTA's slab sequence may be short: its missing slabs are made up by plain
         // arrivals, each ordered after the release of its ring stage like a real slab.
@@ -561,7 +578,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         griddep_launch_dependents();
       }
       WorkItem w;
-      for (int idx = 0; ok && get_item(p, cta, grid, idx, w); ++idx) {
+      for (int idx = 0; ok && get_item<LEAN>(p, cta, grid, idx, w); ++idx) {
         int64_t base_off[kConvRowsPerThread];  // element offset of the (possibly padded) window origin
         uint32_t in_r[kConvRowsPerThread];     // bit r: filter row r of the window falls inside the image
         uint32_t in_s[kConvRowsPerThread];     // bit s: filter column s does
@@ -589,7 +606,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
           if (!ok) break;
           if (threadIdx.x == 0) {
-            if (kb == w.kb0) trace_mark(p, idx, 0);
+            if (kb == w.kb0) trace_mark<LEAN>(p, idx, 0);
             mbar_arrive_expect_tx(&full_bar[stage], L::kBTileBytes);
             tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, &full_bar[stage], kb * kBK, w.n_blk * BN, 0);
           }
@@ -613,7 +630,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           cp_async_mbar_arrive_noinc(&full_bar[stage]);
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
-        if (threadIdx.x == 0) trace_mark(p, idx, 1);
+        if (threadIdx.x == 0) trace_mark<LEAN>(p, idx, 1);
       }
       cp_async_wait<0>();  // nothing of this thread's is in flight when the CTA tears down
     }
@@ -621,24 +638,24 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter + 32)
     if (!p.independent) griddep_wait();
-    if (quarter == 0 && lane == 0 && p.trace != nullptr) p.trace[(size_t)cta * kTraceWords + 2] = (unsigned long long)clock64();
+    if (!LEAN && quarter == 0 && lane == 0 && p.trace != nullptr) p.trace[(size_t)cta * kTraceWords + 2] = (unsigned long long)clock64();
     bool ok = true;
     const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
                         ((p.stride_c & 7) == 0);
     WorkItem w;
     int box = 0;   // staging box in use; alternates over the whole run of the warp, across tiles
-    for (int idx = 0; ok && get_item(p, cta, grid, idx, w); ++idx) {
+    for (int idx = 0; ok && get_item<LEAN>(p, cta, grid, idx, w); ++idx) {
       const int acc = idx & 1;
       const uint32_t acc_phase = (idx >> 1) & 1;
       ok = mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.status);
       ok = named_bar_and(kEpiBarrier, 128, ok);   // the four warps go on, or give up, together
       if (!ok) break;
       tc_fence_after_sync();
-      if (quarter == 0 && lane == 0) trace_mark(p, idx, 4);
+      if (quarter == 0 && lane == 0) trace_mark<LEAN>(p, idx, 4);
       const int trow = quarter * 32 + lane;      // row inside the tile
       // index on the 128-row (A side) axis; an M = 64 accumulator keeps row r in lane (r / 16) * 32 + r % 16, i.e. the
       // lower 16 lanes of each warp's quarter hold rows 16 * quarter ... (measured layout), the upper 16 nothing
-      const int row = p.m64 ? (lane < 16 ? quarter * 16 + lane : p.PM) : w.m_blk * kBM + trow;
+      const int row = !LEAN && p.m64 ? (lane < 16 ? quarter * 16 + lane : p.PM) : w.m_blk * kBM + trow;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
       // 64 columns of this warp's 32 rows, rounded once to fp16, through the warp's swizzled 32 x 128-byte
       // staging box and one TMA store (full 128-byte lines, edges clipped by the tensor map); two boxes per
@@ -680,11 +697,11 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-          if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+          if (quarter == 0 && lane == 0) trace_mark<LEAN>(p, idx, 5);
           continue;
         }
         if constexpr (OUT == kOutColumns) {
-        if (w.mode == kOutDirect) {
+        if (LEAN || w.mode == kOutDirect) {
           // Swapped operands: TMEM lanes index the contiguous axis of C (for a convolution the output channels of a
           // pixel), so 64 columns at a time are transposed on their way to shared memory; two warps fill one box of 64 rows
           // x 64 channels, and one TMA store sends it.  (2-byte stores of a lane per channel, which this replaces, took 10500 cycles
@@ -730,11 +747,11 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-          if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+          if (quarter == 0 && lane == 0) trace_mark<LEAN>(p, idx, 5);
           continue;
         }
         }
-        if (OUT == kOutRows && p.tma_store && w.mode == kOutDirect) {
+        if (OUT == kOutRows && (LEAN || (p.tma_store && w.mode == kOutDirect))) {
           // Fast path: 64 columns at a time go TMEM -> registers -> fp16 -> this warp's swizzled
           // 32 x 128-byte staging box -> one TMA store (full 128-byte lines, edges clipped by the
           // tensor map).  The TMEM load of the next 64 columns is in flight while the current ones
@@ -764,7 +781,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-          if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+          if (quarter == 0 && lane == 0) trace_mark<LEAN>(p, idx, 5);
           continue;
         }
       }
@@ -806,7 +823,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-          if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+          if (quarter == 0 && lane == 0) trace_mark<LEAN>(p, idx, 5);
           continue;
         }
       }
@@ -946,7 +963,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           // the flag is rewritten for the next item only after every thread has read it
           named_bar_sync(kEpiBarrier, 128);
         }
-        if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+        if (quarter == 0 && lane == 0) trace_mark<LEAN>(p, idx, 5);
         continue;
       }
 #pragma unroll 1
@@ -961,7 +978,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-      if (quarter == 0 && lane == 0) trace_mark(p, idx, 5);
+      if (quarter == 0 && lane == 0) trace_mark<LEAN>(p, idx, 5);
     }
     // the staging boxes must have been read before the CTA's shared memory goes away; the writes
     // themselves complete with the grid
@@ -975,7 +992,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   // store: the kernel then cannot complete before everything queued ahead of it has, so completion
   // order along the stream stays transitive for whatever is queued next.
   if (p.independent) griddep_wait();
-  if (threadIdx.x == 0 && p.trace != nullptr) {
+  if (threadIdx.x == 0 && !LEAN && p.trace != nullptr) {
     p.trace[(size_t)cta * kTraceWords + 3] = (unsigned long long)clock64();
     p.trace[(size_t)cta * kTraceWords + 4] = global_timer_ns();
   }
@@ -1563,11 +1580,11 @@ unsigned long long* gemm_f16_trace_for_grid(int grid) {
   return (g_trace_buf && g_trace_bytes >= (size_t)grid * kTraceWords * 8) ? g_trace_buf : nullptr;
 }
 
-template <int BN, bool CONV, int OUT>
+template <int BN, bool CONV, int OUT, bool LEAN>
 static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
                                   const GemmParams& p, int grid, size_t smem, cudaStream_t stream) {
   constexpr int threads = CONV ? kConvThreads : kGemmThreads;
-  auto kern = gemm_f16_tc_kernel<BN, CONV, OUT>;
+  auto kern = gemm_f16_tc_kernel<BN, CONV, OUT, LEAN>;
   // the opt-in shared-memory size is sticky per function and device: raise it only when needed
   static std::mutex mu;
   static size_t granted[64] = {0};
@@ -1708,29 +1725,33 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
   const bool any = !p.swap && !p.tma_store, columns = p.swap && p.tma_store;
+  const bool lean = !conv && bn >= 64 && p.tma_store && !p.stream_k && p.split_k <= 1 && !p.dual && p.probe == 0 && !p.trace;
   cudaError_t e = cudaErrorInvalidValue;
-#define HELIX_BN_CASE(BNV)                                                                                        \
-  case BNV:                                                                                                       \
-    e = conv      ? launch_variant<BNV, true, kOutRows>(ta, tb, tc, p, grid, smem, stream)                        \
-        : any     ? launch_variant<BNV, false, BNV >= 64 ? kOutAny : kOutRows>(ta, tb, tc, p, grid, smem, stream) \
-        : columns ? launch_variant<BNV, false, BNV >= 64 ? kOutColumns : kOutRows>(ta, tb, tc, p, grid, smem, stream) \
-                  : launch_variant<BNV, false, kOutRows>(ta, tb, tc, p, grid, smem, stream);                      \
-    break;
+  auto go = [&](auto width, auto gather, auto out, auto slim) {
+    return launch_variant<decltype(width)::value, decltype(gather)::value, decltype(out)::value, decltype(slim)::value>(
+        ta, tb, tc, p, grid, smem, stream);
+  };
+  const std::true_type yes{};
+  const std::false_type no{};
+  const std::integral_constant<int, kOutRows> as_rows{};
+  const std::integral_constant<int, kOutAny> as_any{};
+  const std::integral_constant<int, kOutColumns> as_columns{};
+  auto wide = [&](auto width) {   // tiles of 64 and more columns
+    if (any) return go(width, no, as_any, no);
+    if (columns) return lean ? go(width, no, as_columns, yes) : go(width, no, as_columns, no);
+    return lean ? go(width, no, as_rows, yes) : go(width, no, as_rows, no);
+  };
+#define HELIX_BN(V) std::integral_constant<int, V>{}
   switch (bn) {
-    HELIX_BN_CASE(256)
-    case 192:
-      e = any       ? launch_variant<192, false, kOutAny>(ta, tb, tc, p, grid, smem, stream)
-          : columns ? launch_variant<192, false, kOutColumns>(ta, tb, tc, p, grid, smem, stream)
-                    : launch_variant<192, false, kOutRows>(ta, tb, tc, p, grid, smem, stream);
-      break;
-    HELIX_BN_CASE(128)
-    HELIX_BN_CASE(64)
-    HELIX_BN_CASE(32)
-    HELIX_BN_CASE(16)
-    default:
-      return HELIX_ERR_UNSUPPORTED;
+    case 256: e = conv ? go(HELIX_BN(256), yes, as_rows, no) : wide(HELIX_BN(256)); break;
+    case 192: e = wide(HELIX_BN(192)); break;
+    case 128: e = conv ? go(HELIX_BN(128), yes, as_rows, no) : wide(HELIX_BN(128)); break;
+    case 64: e = conv ? go(HELIX_BN(64), yes, as_rows, no) : wide(HELIX_BN(64)); break;
+    case 32: e = conv ? go(HELIX_BN(32), yes, as_rows, no) : go(HELIX_BN(32), no, as_rows, no); break;
+    case 16: e = conv ? go(HELIX_BN(16), yes, as_rows, no) : go(HELIX_BN(16), no, as_rows, no); break;
+    default: return HELIX_ERR_UNSUPPORTED;
   }
-#undef HELIX_BN_CASE
+#undef HELIX_BN
   if (e != cudaSuccess) return HELIX_ERR_CUDA;
   ++*launches;
   if (fixup) {

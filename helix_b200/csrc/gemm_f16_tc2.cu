@@ -68,14 +68,18 @@ struct Item2 {
   int slot;   // < 0: the whole K range, result goes straight to C
 };
 
+// LEAN (all of these): whole tiles only, two issuing warps, no probes and no timeline (see the one-CTA kernel)
+template <bool LEAN>
 __device__ __forceinline__ void trace2(const Gemm2Params& p, int word) {
-  if (p.trace != nullptr) p.trace[(size_t)blockIdx.x * kTraceWords + word] = (unsigned long long)clock64();
+  if (!LEAN && p.trace != nullptr) p.trace[(size_t)blockIdx.x * kTraceWords + word] = (unsigned long long)clock64();
 }
+template <bool LEAN>
 __device__ __forceinline__ void trace2_tile(const Gemm2Params& p, int idx, int slot) {
-  if (idx < kTraceTiles) trace2(p, 8 + idx * 6 + slot);
+  if (idx < kTraceTiles) trace2<LEAN>(p, 8 + idx * 6 + slot);
 }
+template <bool LEAN>
 __device__ __forceinline__ void trace2_slab(const Gemm2Params& p, int which, int n) {
-  if (n < kTraceSlabs) trace2(p, 8 + 6 * kTraceTiles + which * kTraceSlabs + n);
+  if (n < kTraceSlabs) trace2<LEAN>(p, 8 + 6 * kTraceTiles + which * kTraceSlabs + n);
 }
 
 struct Tile2 {
@@ -96,13 +100,14 @@ __device__ __forceinline__ Tile2 decode_tile2(const Gemm2Params& p, int t) {
 }
 
 // The idx-th work item of a pair; every role of both CTAs walks the same sequence.
+template <bool LEAN>
 __device__ __forceinline__ bool get_item2(const Gemm2Params& p, int pair, int num_pairs, int idx, Item2& it) {
-  if (!p.stream_k || idx < p.dp_rounds) {
+  if (LEAN || !p.stream_k || idx < p.dp_rounds) {
     it.tile = pair + idx * num_pairs;
     it.kb0 = 0;
     it.kb1 = p.num_kb;
     it.slot = -1;
-    return p.stream_k || it.tile < p.total_tiles;
+    return (!LEAN && p.stream_k) || it.tile < p.total_tiles;
   }
   const int s = idx - p.dp_rounds;   // first / second tile the pair's slab range touches
   if (s > 1) return false;
@@ -220,7 +225,7 @@ __device__ __forceinline__ void umma_commit_pair_elect(uint64_t* bar) {
 // a token: the owner of slab n - 1 arrives at a named barrier after issuing, fenced, and the owner of slab n meets
 // it there before issuing, so the accumulation order -- every bit of the result -- is that of one issuer.  Both
 // warps walk the whole sequence whatever happens (after a failed wait nothing is issued, the rendezvous are kept).
-template <int BN, int ME>
+template <int BN, int ME, bool LEAN>
 __device__ __forceinline__ void pair_dual_issue_loop(const Gemm2Params& p, const int pair, const int num_pairs,
                                                      const int lane, const int stages, uint8_t* sA, uint8_t* sB,
                                                      uint64_t* full_bar, uint64_t* empty_bar, uint64_t* tmem_full,
@@ -233,18 +238,18 @@ __device__ __forceinline__ void pair_dual_issue_loop(const Gemm2Params& p, const
   bool ok = true;
   int nslab = 0;
   Item2 it;
-  for (int idx = 0; get_item2(p, pair, num_pairs, idx, it); ++idx) {
+  for (int idx = 0; get_item2<LEAN>(p, pair, num_pairs, idx, it); ++idx) {
     const int acc = idx & 1;
     const uint32_t acc_phase = (idx >> 1) & 1;
     if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status));
     tc_fence_after_sync();
-    if (lane == 0 && ME == 0) trace2_tile(p, idx, 2);
+    if (lane == 0 && ME == 0) trace2_tile<LEAN>(p, idx, 2);
     const uint32_t d_tmem = tmem_base + acc * BN;
     for (int kb = it.kb0; kb < it.kb1; ++kb) {
       const int n = nslab++;
       if ((n & 1) == ME) {
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[stage], phase, abort_flag, p.status));
-        if (lane == 0) trace2_slab(p, 1, n);
+        if (lane == 0) trace2_slab<LEAN>(p, 1, n);
         tc_fence_after_sync();
         const uint64_t da = umma_desc_sw128(smem_u32(sA + (size_t)stage * kATileBytes));
         const uint64_t db = umma_desc_sw128(smem_u32(sB + (size_t)stage * kBHalfBytes));
@@ -252,7 +257,7 @@ __device__ __forceinline__ void pair_dual_issue_loop(const Gemm2Params& p, const
           named_bar_sync(kTokBarrier2 + ((n - 1) & 1), 64);
           tc_fence_after_sync();
         }
-        if (ok && !(p.probe & 1)) {
+        if (ok && (LEAN || !(p.probe & 1))) {
 #pragma unroll
           for (int k = 0; k < kBK / 16; ++k)
             umma_f16_ss_pair_elect(d_tmem, da + 2 * k, db + 2 * k, kIdesc, (kb > it.kb0) || (k > 0));
@@ -264,14 +269,14 @@ __device__ __forceinline__ void pair_dual_issue_loop(const Gemm2Params& p, const
       if (++stage == stages) { stage = 0; phase ^= 1; }
     }
     if (ok) umma_commit_pair_elect(&tmem_full[acc]);   // both warps, each for its own MMAs (barrier count 2)
-    if (lane == 0 && ME == 0) trace2_tile(p, idx, 3);
+    if (lane == 0 && ME == 0) trace2_tile<LEAN>(p, idx, 3);
   }
   // the token of the last slab is met by the warp that did not issue it, so that no arrival is left over
   if (nslab > 0 && ((nslab - 1) & 1) != ME) named_bar_sync(kTokBarrier2 + ((nslab - 1) & 1), 64);
 }
 
 // ANY: rows of C that a TMA store cannot write (see the one-CTA kernel)
-template <int BN, bool ANY>
+template <int BN, bool ANY, bool LEAN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_c, const Gemm2Params p) {
@@ -280,6 +285,8 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   constexpr int kTmemCols = 2 * BN <= 256 ? 256 : 512;
   constexpr uint32_t kIdesc = umma_idesc_f16(2 * kBM, BN);
 
+  const bool dual = LEAN || p.dual;
+  const int load_warps = LEAN ? 2 : p.load_warps, group = LEAN ? 1 : p.group;
   if (p.independent) griddep_launch_dependents();   // else after the wait (common.cuh)
 
   extern __shared__ uint8_t smem_raw[];
@@ -304,16 +311,16 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (warp >= 2 && warp < 6) touch_params(p);   // warps with nothing to set up
 
   if (threadIdx.x == 0) {
-    if (p.trace != nullptr) {
+    if (!LEAN && p.trace != nullptr) {
       p.trace[(size_t)blockIdx.x * kTraceWords + 0] = global_timer_ns();
-      trace2(p, 1);
+      trace2<LEAN>(p, 1);
     }
     for (int s = 0; s < stages; ++s) {
-      if (s * p.group < stages) mbar_init(&full_bar[s], p.group);
+      if (s * group < stages) mbar_init(&full_bar[s], group);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
-      mbar_init(&tmem_full[a], p.dual ? 2 : 1);
+      mbar_init(&tmem_full[a], dual ? 2 : 1);
       mbar_init(&tmem_empty[a], 8);
     }
     *abort_flag = 0;
@@ -342,48 +349,48 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // and meets it at a named barrier per group of stages: a shared-memory read by the MMA warp itself would queue
     // behind the MMAs it has just issued.  Both warps walk the same sequence of groups to its end whatever
     // happens (after a failed wait only the rendezvous are kept), in lockstep per group.
-    if (p.dual) {
+    if (dual) {
       if (warp == 7 && rank == 0)   // second MMA-issuing warp (it issues no loads: load_warps <= 2)
-        pair_dual_issue_loop<BN, 1>(p, pair, num_pairs, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+        pair_dual_issue_loop<BN, 1, LEAN>(p, pair, num_pairs, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                     abort_flag, tmem_base);
-    } else if (warp == 7 && rank == 0 && p.load_warps < kPairProducerWarps) {
+    } else if (warp == 7 && rank == 0 && load_warps < kPairProducerWarps) {
       bool ok = true;
       int stage = 0, gpos = 0, gidx = 0;
       uint32_t phase = 0;
       Item2 it;
-      for (int idx = 0; get_item2(p, pair, num_pairs, idx, it); ++idx) {
+      for (int idx = 0; get_item2<LEAN>(p, pair, num_pairs, idx, it); ++idx) {
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
           if (gpos == 0) {
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[gidx], phase, abort_flag, p.status));
             named_bar_sync(kFwdBarrier2 + gidx, 64);
           }
-          if (++gpos == p.group) { gpos = 0; ++gidx; }
+          if (++gpos == group) { gpos = 0; ++gidx; }
           if (++stage == stages) { stage = 0; phase ^= 1; gidx = 0; }
         }
       }
     }
-    if (lane == 0 && issuer < p.load_warps) {
+    if (lane == 0 && issuer < load_warps) {
       bool ok = true;
       int n_start = 0;
       int my_n = issuer;     // next slab this issuer requests; stage and use parity follow it
       int stage = issuer;    // load_warps <= stages
       uint32_t phase = 0;
       Item2 it;
-      for (int tidx = 0; ok && get_item2(p, pair, num_pairs, tidx, it); ++tidx) {
+      for (int tidx = 0; ok && get_item2<LEAN>(p, pair, num_pairs, tidx, it); ++tidx) {
         const Tile2 w = decode_tile2(p, it.tile);
         const int nkb = it.kb1 - it.kb0;
         if (tidx == 0 && !p.independent) {
           griddep_wait();
           if (issuer == 0) griddep_launch_dependents();
         }
-        if (issuer == 0) trace2_tile(p, tidx, 0);
-        for (; my_n < n_start + nkb; my_n += p.load_warps) {
+        if (issuer == 0) trace2_tile<LEAN>(p, tidx, 0);
+        for (; my_n < n_start + nkb; my_n += load_warps) {
           const int kb = it.kb0 + (my_n - n_start);
           ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status);
           if (!ok) break;
-          trace2_slab(p, 0, my_n);
-          const bool load_a = !(p.probe & 2), load_b = !(p.probe & 4);
-          uint64_t* const fb = &full_bar[fast_div(stage, p.fd_grp)];
+          trace2_slab<LEAN>(p, 0, my_n);
+          const bool load_a = LEAN || !(p.probe & 2), load_b = LEAN || !(p.probe & 4);
+          uint64_t* const fb = &full_bar[LEAN ? stage : fast_div(stage, p.fd_grp)];
           if (rank == 0) {
             if (load_a || load_b)
               mbar_arrive_expect_tx(fb, 2 * ((load_a ? kATileBytes : 0) + (load_b ? kBHalfBytes : 0)));
@@ -397,20 +404,20 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (load_b)
             tma_load_3d_pair(sB + (size_t)stage * kBHalfBytes, &tmap_b, full_leader, kb * kBK,
                              w.n_blk * BN + (int)rank * (BN / 2), w.b);
-          stage += p.load_warps;
+          stage += load_warps;
           if (stage >= stages) { stage -= stages; phase ^= 1; }
         }
         n_start += nkb;
-        if (issuer == 0) trace2_tile(p, tidx, 1);
+        if (issuer == 0) trace2_tile<LEAN>(p, tidx, 1);
       }
       // a short last group of the pair's slab sequence is completed by plain arrivals (even CTA: the
       // barriers live there), each ordered after the release of its ring stage like a real slab
-      const int n_pad = (n_start + p.group - 1) / p.group * p.group;
-      for (; ok && my_n < n_pad; my_n += p.load_warps) {
+      const int n_pad = (n_start + group - 1) / group * group;
+      for (; ok && my_n < n_pad; my_n += load_warps) {
         ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status);
         if (!ok) break;
         if (rank == 0) mbar_arrive(&full_bar[fast_div(stage, p.fd_grp)]);
-        stage += p.load_warps;
+        stage += load_warps;
         if (stage >= stages) { stage -= stages; phase ^= 1; }
       }
     }
@@ -419,24 +426,24 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // The whole warp walks the loop convergently (warp-uniform state, waits end in a vote) and one elected lane
     // issues.  With a watcher warp (forward) the arrival of a group of stages comes through a named barrier and the
     // sequence is walked to its end even after a failed wait (ok = false: only the rendezvous are kept).
-    if (rank == 0 && p.dual) {
-      pair_dual_issue_loop<BN, 0>(p, pair, num_pairs, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+    if (rank == 0 && dual) {
+      pair_dual_issue_loop<BN, 0, LEAN>(p, pair, num_pairs, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                   abort_flag, tmem_base);
     } else if (rank == 0) {
-      const bool forward = p.load_warps < kPairProducerWarps;
+      const bool forward = load_warps < kPairProducerWarps;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       int nslab = 0;
       int gpos = 0, gidx = 0;   // position of the next slab inside its group of stages, and the group
       Item2 it;
-      for (int idx = 0; (forward || ok) && get_item2(p, pair, num_pairs, idx, it); ++idx) {
+      for (int idx = 0; (forward || ok) && get_item2<LEAN>(p, pair, num_pairs, idx, it); ++idx) {
         const int acc = idx & 1;
         const uint32_t acc_phase = (idx >> 1) & 1;
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status));
         if (!ok && !forward) break;
         tc_fence_after_sync();
-        if (lane == 0) trace2_tile(p, idx, 2);
+        if (lane == 0) trace2_tile<LEAN>(p, idx, 2);
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
           // one rendezvous (or wait) per group of stages; the stages are still released one by one
@@ -448,8 +455,8 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               if (!ok) break;
             }
           }
-          if (++gpos == p.group) { gpos = 0; ++gidx; }
-          if (lane == 0) trace2_slab(p, 1, nslab);
+          if (++gpos == group) { gpos = 0; ++gidx; }
+          if (lane == 0) trace2_slab<LEAN>(p, 1, nslab);
           ++nslab;
           tc_fence_after_sync();
           const uint64_t da = umma_desc_sw128(smem_u32(sA + (size_t)stage * kATileBytes));
@@ -463,18 +470,18 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           if (++stage == stages) { stage = 0; phase ^= 1; gidx = 0; }
         }
         if (ok) umma_commit_pair_elect(&tmem_full[acc]);
-        if (lane == 0) trace2_tile(p, idx, 3);
+        if (lane == 0) trace2_tile<LEAN>(p, idx, 3);
       }
     }
   } else {
     // ------------------------------------------------------------------ epilogue (each CTA: its 128 rows)
     const int quarter = warp & 3;
     if (!p.independent) griddep_wait();
-    if (quarter == 0 && lane == 0) trace2(p, 2);
+    if (quarter == 0 && lane == 0) trace2<LEAN>(p, 2);
     bool ok = true;
     int box = 0;   // staging box in use; alternates over the whole run of the warp, across tiles
     Item2 it;
-    for (int idx = 0; ok && get_item2(p, pair, num_pairs, idx, it); ++idx) {
+    for (int idx = 0; ok && get_item2<LEAN>(p, pair, num_pairs, idx, it); ++idx) {
       const Tile2 w = decode_tile2(p, it.tile);
       const int acc = idx & 1;
       const uint32_t acc_phase = (idx >> 1) & 1;
@@ -482,11 +489,11 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       ok = named_bar_and(kEpiBarrier, 128, ok);   // the four warps go on, or give up, together
       if (!ok) break;
       tc_fence_after_sync();
-      if (quarter == 0 && lane == 0) trace2_tile(p, idx, 4);
+      if (quarter == 0 && lane == 0) trace2_tile<LEAN>(p, idx, 4);
       const int cta_row0 = w.m_blk * 2 * kBM + (int)rank * kBM;
       const int row0 = cta_row0 + quarter * 32;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
-      if (it.slot >= 0) {
+      if (!LEAN && it.slot >= 0) {
         // part of a tile's K range: the fp32 accumulator (padding included) goes to this pair's slot of
         // 256 x BN floats, stored lane-major (the four floats (row, 4j..4j+3) of a warp's 32 rows side by side),
         // so that every store of a warp covers 512 contiguous bytes
@@ -506,7 +513,7 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
-        if (quarter == 0 && lane == 0) trace2_tile(p, idx, 5);
+        if (quarter == 0 && lane == 0) trace2_tile<LEAN>(p, idx, 5);
         continue;
       }
       if constexpr (ANY) {   // 64 columns of a warp's 32 rows at a time
@@ -526,7 +533,7 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
-        if (quarter == 0 && lane == 0) trace2_tile(p, idx, 5);
+        if (quarter == 0 && lane == 0) trace2_tile<LEAN>(p, idx, 5);
         continue;
       }
       uint32_t ra[32], rb[32], na[32], nb[32];
@@ -572,7 +579,7 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&tmem_empty[acc]), 0));
-      if (quarter == 0 && lane == 0) trace2_tile(p, idx, 5);
+      if (quarter == 0 && lane == 0) trace2_tile<LEAN>(p, idx, 5);
     }
     // the staging boxes must have been read before the CTA's shared memory goes away; the writes
     // themselves complete with the grid
@@ -587,8 +594,8 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   // store: the kernel then cannot complete before everything queued ahead of it has, so completion
   // order along the stream stays transitive for whatever is queued next.
   if (p.independent) griddep_wait();
-  if (threadIdx.x == 0 && p.trace != nullptr) {
-    trace2(p, 3);
+  if (threadIdx.x == 0 && !LEAN && p.trace != nullptr) {
+    trace2<LEAN>(p, 3);
     p.trace[(size_t)blockIdx.x * kTraceWords + 4] = global_timer_ns();
   }
   if (warp == 1) {
@@ -669,10 +676,10 @@ int make_map(CUtensorMap* map, const void* base, int64_t inner, int64_t rows, in
   return r == CUDA_SUCCESS ? HELIX_OK : HELIX_ERR_CUDA;
 }
 
-template <int BN, bool ANY>
+template <int BN, bool ANY, bool LEAN>
 cudaError_t launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Gemm2Params& p,
                         int grid, size_t smem, cudaStream_t stream) {
-  auto kern = gemm_f16_tc2_kernel<BN, ANY>;
+  auto kern = gemm_f16_tc2_kernel<BN, ANY, LEAN>;
   static std::mutex mu;
   static size_t granted[64] = {0};
   int dev = 0;
@@ -793,13 +800,16 @@ int gemm_f16_pair_launch(const helix_cfg_t& cfg, const void* A, int64_t lda, con
       make_map(&tc, C, N, M, batch, ldc, sc, kBM) == HELIX_OK)
     p.tma_store = 1;
   const size_t smem = 1024 + (size_t)p.stages * (kATileBytes + (bn / 2) * kBK * 2) + kStagingBytes + 256;
-  auto launch = [&](auto any) {
-    constexpr bool kAny = decltype(any)::value;
-    return bn == 256   ? launch_pair<256, kAny>(ta, tb, tc, p, 2 * pairs, smem, stream)
-           : bn == 192 ? launch_pair<192, kAny>(ta, tb, tc, p, 2 * pairs, smem, stream)
-                       : launch_pair<128, kAny>(ta, tb, tc, p, 2 * pairs, smem, stream);
+  auto launch = [&](auto any, auto slim) {
+    constexpr bool kAny = decltype(any)::value, kLean = decltype(slim)::value;
+    return bn == 256   ? launch_pair<256, kAny, kLean>(ta, tb, tc, p, 2 * pairs, smem, stream)
+           : bn == 192 ? launch_pair<192, kAny, kLean>(ta, tb, tc, p, 2 * pairs, smem, stream)
+                       : launch_pair<128, kAny, kLean>(ta, tb, tc, p, 2 * pairs, smem, stream);
   };
-  const cudaError_t e = p.tma_store ? launch(std::false_type{}) : launch(std::true_type{});
+  const bool lean = p.tma_store && !p.stream_k && p.dual && p.load_warps == 2 && p.probe == 0 && !p.trace;
+  const cudaError_t e = lean          ? launch(std::false_type{}, std::true_type{})
+                        : p.tma_store ? launch(std::false_type{}, std::false_type{})
+                                      : launch(std::true_type{}, std::false_type{});
   if (e != cudaSuccess) return HELIX_ERR_CUDA;
   ++*launches;
   if (fixup) {
