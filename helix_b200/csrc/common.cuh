@@ -99,16 +99,18 @@ __device__ __forceinline__ bool mbar_try_wait_parked(uint64_t* bar, uint32_t par
 // this CTA already gave up.  While the phase is incomplete the thread is parked by the hardware (a
 // try_wait with a suspend-time hint) instead of polling: a polling warp competes with the MMA-issuing
 // warp for its scheduler and for the shared-memory pipe (measured 3-7 % on narrow-tile kernels).
+// One rolled loop: there are dozens of waits in a kernel, and code that a launch of a few us fetches for nothing costs it time.
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                 int* status_dev, unsigned long long limit_ns) {
-  for (int i = 0; i < 16; ++i)
+  unsigned long long t0 = 0;
+#pragma unroll 1
+  for (int i = 0;; ++i) {
     if (mbar_try_wait_parked(bar, parity, 20000u)) return true;
-  const unsigned long long t0 = global_timer_ns();
-  while (true) {
-    for (int i = 0; i < 8; ++i)
-      if (mbar_try_wait_parked(bar, parity, 20000u)) return true;
+    if ((i & 7) != 7) continue;
     if (*abort_flag) return false;
-    if (global_timer_ns() - t0 > limit_ns) {
+    const unsigned long long now = global_timer_ns();
+    if (t0 == 0) t0 = now;
+    if (now - t0 > limit_ns) {
       *abort_flag = 1;
       if (status_dev) atomicExch(status_dev, (int)HELIX_ERR_TIMEOUT);
       return false;

@@ -786,7 +786,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         }
       }
       if constexpr (BN >= 32) {
-        if (OUT == kOutRows && p.swap && w.mode == kOutDirect) {
+        if (OUT == kOutRows && swap && w.mode == kOutDirect) {
           // Swapped operands: TMEM lanes index the contiguous axis of C (C[col][row]: for a convolution the
           // output channels of one pixel).  A warp holds 32 consecutive rows of every tile column, so one
           // 2-byte store per lane writes 64 contiguous bytes of one C row: no transposition through shared
@@ -833,7 +833,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       auto store_direct = [&](const uint32_t (&r)[kChunk], int c0) {
         const int col0 = w.n_blk * BN + c0;  // index on the BN (B side) axis
         if (col0 >= p.PN || row >= p.PM) return;
-        if (p.swap) {
+        if (swap) {
           // rows index N of C, columns index M: C[m, n] with m = col, n = row
           __half* dst = p.C + (int64_t)w.b * p.stride_c + row;
 #pragma unroll
@@ -1725,7 +1725,8 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
   const bool any = !p.swap && !p.tma_store, columns = p.swap && p.tma_store;
-  const bool lean = !conv && bn >= 64 && p.tma_store && !p.stream_k && p.split_k <= 1 && !p.dual && p.probe == 0 && !p.trace;
+  // (narrow tiles are stored directly, and swapped ones among them keep the general variant)
+  const bool lean = (bn >= 64 ? p.tma_store : !p.swap) && !p.stream_k && p.split_k <= 1 && !p.dual && p.probe == 0 && !p.trace;
   cudaError_t e = cudaErrorInvalidValue;
   auto go = [&](auto width, auto gather, auto out, auto slim) {
     return launch_variant<decltype(width)::value, decltype(gather)::value, decltype(out)::value, decltype(slim)::value>(
@@ -1741,14 +1742,16 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
     if (columns) return lean ? go(width, no, as_columns, yes) : go(width, no, as_columns, no);
     return lean ? go(width, no, as_rows, yes) : go(width, no, as_rows, no);
   };
+  auto narrow = [&](auto width) { return lean ? go(width, no, as_rows, yes) : go(width, no, as_rows, no); };
+  auto gather = [&](auto width) { return lean ? go(width, yes, as_rows, yes) : go(width, yes, as_rows, no); };
 #define HELIX_BN(V) std::integral_constant<int, V>{}
   switch (bn) {
-    case 256: e = conv ? go(HELIX_BN(256), yes, as_rows, no) : wide(HELIX_BN(256)); break;
+    case 256: e = conv ? gather(HELIX_BN(256)) : wide(HELIX_BN(256)); break;
     case 192: e = wide(HELIX_BN(192)); break;
-    case 128: e = conv ? go(HELIX_BN(128), yes, as_rows, no) : wide(HELIX_BN(128)); break;
-    case 64: e = conv ? go(HELIX_BN(64), yes, as_rows, no) : wide(HELIX_BN(64)); break;
-    case 32: e = conv ? go(HELIX_BN(32), yes, as_rows, no) : go(HELIX_BN(32), no, as_rows, no); break;
-    case 16: e = conv ? go(HELIX_BN(16), yes, as_rows, no) : go(HELIX_BN(16), no, as_rows, no); break;
+    case 128: e = conv ? gather(HELIX_BN(128)) : wide(HELIX_BN(128)); break;
+    case 64: e = conv ? gather(HELIX_BN(64)) : wide(HELIX_BN(64)); break;
+    case 32: e = conv ? gather(HELIX_BN(32)) : narrow(HELIX_BN(32)); break;
+    case 16: e = conv ? gather(HELIX_BN(16)) : narrow(HELIX_BN(16)); break;
     default: return HELIX_ERR_UNSUPPORTED;
   }
 #undef HELIX_BN
