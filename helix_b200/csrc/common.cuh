@@ -222,6 +222,20 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   return d;
 }
 
+// The same for rows of 64 bytes (a box of 32 halves with SWIZZLE_64B: groups of 8 rows are 512 bytes apart, layout = 4) or of
+// 32 bytes (16 halves with SWIZZLE_32B: 256 bytes, layout = 6).
+template <int ROW_BYTES>
+__device__ __forceinline__ uint64_t umma_desc_narrow(uint32_t smem_addr) {
+  static_assert(ROW_BYTES == 64 || ROW_BYTES == 32, "swizzled rows");
+  uint64_t d = 0;
+  d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);
+  d |= static_cast<uint64_t>(1) << 16;
+  d |= static_cast<uint64_t>(8 * ROW_BYTES >> 4) << 32;
+  d |= static_cast<uint64_t>(1) << 46;
+  d |= static_cast<uint64_t>(ROW_BYTES == 64 ? 4 : 6) << 61;
+  return d;
+}
+
 // Instruction descriptor of tcgen05.mma.kind::f16 with fp16 A/B (both K-major) and fp32 D.
 // Bits: [4,6) D format (1 = f32), [7,10) A format (0 = f16), [10,13) B format, 15/16 majors
 // (0 = K), [17,23) N>>3, [24,29) M>>4.

@@ -98,6 +98,7 @@ struct GemmParams {
   const __half* x;
   ConvGeom g;
   int im2col;      // A tiles come from an im2col tensor map over x: no gather warps
+  int blocks;      // blocks of 32 or 16 channels of the K axis where pixels arrive by those (BLK), else 0
   int wtaps;       // the weights' map is (channel, tap, output channel): the last channel block of a tap is filled
   // optional per-CTA timeline (null = off): kTraceWords 64-bit words per CTA, see trace_mark
   unsigned long long* trace;
@@ -210,12 +211,16 @@ struct SmemLayout {
   }
 };
 
+// BLK: the pixels of a convolution arrive in blocks of 32 or 16 channels of a tap, on the 128-row axis (32, 16) or on the other
+// (-32, -16), so that a channel count which is no multiple of 64 needs no filling; 0: slabs of 64.
+__host__ __device__ constexpr int blk_bytes(int blk) { return blk == 0 ? 64 : 2 * (blk < 0 ? -blk : blk); }
+
 // The MMA-issuing role of the one-CTA kernel, walked convergently by a whole warp (all loop state is warp-uniform, waits
 // end in a vote) with one elected lane issuing the tcgen05 instructions: descriptors and barrier addresses then live in
 // uniform registers instead of being moved there per operand from one lane's registers.  DUAL: two warps run this loop
 // and issue alternate slabs (ME = 0 / 1).  Both are compile-time constants of each copy of the loop so that
 // everything it computes stays warp-uniform for the compiler.
-template <int BN, bool CONV, bool DUAL, int ME, bool LEAN>
+template <int BN, bool CONV, bool DUAL, int ME, bool LEAN, int BLK>
 __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int cta, const int grid, const int lane,
                                                const int stages, uint8_t* sA, uint8_t* sB, uint64_t* full_bar,
                                                uint64_t* empty_bar, uint64_t* tmem_full, uint64_t* tmem_empty,
@@ -274,18 +279,27 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
           long long t2 = 0, t3 = 0;
           if (mine) {
           if (lane == 0) trace_slab<LEAN>(p, 1, n);
-          const uint64_t da = umma_desc_sw128(smem_u32(sA + (size_t)stage * kATileBytes));
-          const uint64_t db = umma_desc_sw128(smem_u32(sB + (size_t)stage * SmemLayout<BN>::kBTileBytes));
+          const uint32_t ta = smem_u32(sA + (size_t)stage * kATileBytes), tb = smem_u32(sB + (size_t)stage * SmemLayout<BN>::kBTileBytes);
+          const uint64_t da = BLK > 0 ? umma_desc_narrow<blk_bytes(BLK)>(ta) : umma_desc_sw128(ta);
+          const uint64_t db = BLK < 0 ? umma_desc_narrow<blk_bytes(BLK)>(tb) : umma_desc_sw128(tb);
+          // of a last slab only the blocks that exist are multiplied
+          const int steps = BLK == 0 ? kBK / 16 : (p.blocks - kb * (kBK * 2 / blk_bytes(BLK))) * (blk_bytes(BLK) / 32);
           if (DUAL && n > 0) {   // everything but the MMAs themselves is done before the token is awaited
             named_bar_sync(kTokBarrier + ((n - 1) & 1), 64);
             tc_fence_after_sync();
           }
           t2 = tr ? clock64() : 0;
+          const bool partial = BLK != 0 && steps < kBK / 16;
           if (ok && (LEAN || !(p.probe & 1))) {
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k) {
+              if (k > 0 && partial && k >= steps) break;
               // advancing 16 halves = 32 bytes along K inside the swizzle atom: +2 in the address field
-              umma_f16_ss_elect(d_tmem, da + 2 * k, db + 2 * k, kIdesc, (kb > w.kb0) || (k > 0));
+              // (BLK: tiles of 64- or 32-byte rows, one after the other)
+              constexpr int kPer = blk_bytes(BLK) / 32;
+              const uint32_t ka = BLK > 0 ? (k % kPer) * 2 + (k / kPer) * (kBM * blk_bytes(BLK) / 16) : 2 * k;
+              const uint32_t kn = BLK < 0 ? (k % kPer) * 2 + (k / kPer) * (BN * blk_bytes(BLK) / 16) : 2 * k;
+              umma_f16_ss_elect(d_tmem, da + ka, db + kn, kIdesc, (kb > w.kb0) || (k > 0));
             }
           }
           t3 = tr ? clock64() : 0;
@@ -327,7 +341,7 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
 // LEAN: whole tiles only, one issuing warp, no probes and no timeline -- what most launches are.  The code that is left out
 // is not run by them, but a launch of a few us starts with a cold instruction cache and pays for what lies in between.
 enum TileOut { kOutRows = 0, kOutAny = 1, kOutColumns = 2 };
-template <int BN, bool CONV, int OUT, bool LEAN>
+template <int BN, bool CONV, int OUT, bool LEAN, int BLK>
 __global__ void __launch_bounds__(CONV ? kConvThreads : kGemmThreads, 1)
 gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
@@ -415,13 +429,13 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const bool second_issuer = dual && warp == 3;
   if (warp == kMmaWarp) {
     if (dual)
-      mma_issue_loop<BN, CONV, !LEAN, 0, LEAN>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+      mma_issue_loop<BN, CONV, !LEAN, 0, LEAN, BLK>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                         abort_flag, tmem_base);
     else
-      mma_issue_loop<BN, CONV, false, 0, LEAN>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+      mma_issue_loop<BN, CONV, false, 0, LEAN, BLK>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                          abort_flag, tmem_base);
   } else if (second_issuer) {
-    mma_issue_loop<BN, CONV, !CONV && !LEAN, 1, LEAN>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
+    mma_issue_loop<BN, CONV, !CONV && !LEAN, 1, LEAN, BLK>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
                                        abort_flag, tmem_base);
   } else if (warp < kProducerWarps) {
     // ------------------------------------------------------------------ producers
@@ -487,6 +501,27 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             trace_slab<LEAN>(p, 0, my_n);
             uint64_t* const fb = &full_bar[fast_div(stage, p.fd_grp)];
             const bool load_a = LEAN || !(p.probe & 2), load_b = LEAN || !(p.probe & 4);
+            if constexpr (BLK != 0) {
+              // K is ordered (r, s, c): block q is filter tap q / cblocks, channels from BLK * (q % cblocks)
+              constexpr int kBlockBytes = (BLK > 0 ? kBM : BN) * blk_bytes(BLK), kPerSlab = kBK * 2 / blk_bytes(BLK);
+              uint8_t* const px = BLK > 0 ? sA + (size_t)stage * kATileBytes : sB + (size_t)stage * L::kBTileBytes;
+              const int n_blk = min(kPerSlab, p.blocks - kPerSlab * kb);
+              mbar_arrive_expect_tx(fb, (BLK > 0 ? L::kBTileBytes : kATileBytes) + n_blk * kBlockBytes);
+              if constexpr (BLK > 0) tma_load_3d(sB + (size_t)stage * L::kBTileBytes, &tmap_b, fb, kb * kBK, w.n_blk * BN, 0);
+              else tma_load_3d(sA + (size_t)stage * kATileBytes, &tmap_a, fb, kb * kBK, w.m_blk * kBM, 0);
+#pragma unroll
+              for (int h = 0; h < kPerSlab; ++h) {
+                if (h >= n_blk) break;
+                int tap, cb, fr, fs;
+                fast_divmod(kPerSlab * kb + h, p.fd_cblocks, tap, cb);
+                fast_divmod(tap, p.fd_s, fr, fs);
+                tma_load_im2col_4d(px + h * kBlockBytes, BLK > 0 ? &tmap_a : &tmap_b, fb, cb * (blk_bytes(BLK) / 2), pix_w, pix_h,
+                                   pix_n, (uint16_t)fs, (uint16_t)fr);
+              }
+              stage += p.load_warps;
+              if (stage >= stages) { stage -= stages; phase ^= 1; }
+              continue;
+            }
             if (load_a || load_b)
               mbar_arrive_expect_tx(fb, (load_a ? kATileBytes : 0) + (load_b ? L::kBTileBytes : 0));
             else
@@ -1147,6 +1182,14 @@ static EncodeIm2colFn get_encode_im2col_fn() {
   return fn;
 }
 
+// Window parameters inside the fields of an im2col tensor map, pixels on 16 bytes, and an input that is worth the map's set-up.
+static bool conv_map_possible(const ConvGeom& g) {
+  const int64_t bytes = (int64_t)g.NB * g.H * g.W * g.C * 2;
+  return (g.C % 8) == 0 && g.stride >= 1 && g.stride <= 8 && g.pad <= 127 && g.R <= 128 && g.S <= 128 &&
+         g.pad - (g.R - 1) >= -128 && g.pad - (g.S - 1) >= -128 && bytes >= 131072 && g.C <= 65535 &&
+         get_encode_im2col_fn() != nullptr;
+}
+
 // The im2col path reads 64-channel blocks of one filter tap (one 128-byte swizzled row per pixel; the last block of a
 // C that is no multiple of 64 is filled with zeros, on the weights' side too), and needs window parameters inside the
 // tensor map's field widths and an activation tensor of at least 128 KiB (smaller ones stay on the gathering kernel, as
@@ -1160,41 +1203,49 @@ static EncodeIm2colFn get_encode_im2col_fn() {
 // [22] 73 / 67), and to 30 G with a tenth filled at most (C = 408 [7] 32 / 36, 472 [16] 79 / 92, 680 [22] 79 / 89, 312 [19] 71 / 71; but 232 [16]
 // 71 / 64, 728 [43] 124 / 105, 440 [215] 600 / 557); C = 8 k with even k keeps its gain at any size (176, 304, 336, 432, 496, 560, 688: 0.57 ... 0.89).
 static bool conv_im2col_eligible(const ConvGeom& g) {
-  const int64_t bytes = (int64_t)g.NB * g.H * g.W * g.C * 2;
   const int filled = (g.C + kBK - 1) / kBK * kBK;
   bool worth = g.C % 32 == 0 ? filled * 3 <= g.C * 4 : filled * 5 <= g.C * 6 && g.C >= 96;
   if (g.C % 16 != 0) {
     const double macs = (double)g.NB * g.Ho * g.Wo * g.KO * g.R * g.S * g.C;
     worth = worth && (macs <= 4e9 || (filled * 10 <= g.C * 11 && macs <= 3e10));
   }
-  return (g.C % 8) == 0 && worth && g.stride >= 1 && g.stride <= 8 && g.pad <= 127 && g.R <= 128 && g.S <= 128 &&
-         g.pad - (g.R - 1) >= -128 && g.pad - (g.S - 1) >= -128 && bytes >= 131072 && g.C <= 65535 &&
-         get_encode_im2col_fn() != nullptr;
+  return worth && conv_map_possible(g);
+}
+
+// Blocks of 32 or 16 channels instead of slabs of 64 (0: none).  A row of a box costs the tensor copy as much at 32 or 64 bytes as at 128, so
+// blocks are for channel counts that slabs would fill up by a fifth or more.  Gathering / blocks, us: 3 x 3, C = 32, 56 x 56 x 32 -> 64: 21.2 / 14.4;
+// 14 x 14 x 64 -> 256: 8.1 / 5.6; C = 16, 56 x 56 x 32: 16.3 / 12.7; C = 80, 28 x 28 x 32 -> 160: 19.2 / 16.2; C = 144, 26 x 26 x 20: 16.1 / 14.0; C = 208, 20 x 20 x
+// 20: 19.4 / 16.5; 5 x 5, C = 80, 50 x 50 x 4 -> 256: 22.0 / 22.5.  Slabs / blocks: 5 x 5, C = 96, 26 x 26 x 20 -> 256: 21.6 / 18.1; 3 x 3, C = 96, 56 x 56 x 32 -> 64: 29.7 /
+// 24.7; 5 x 5, C = 160, 40 x 40 x 4 -> 320: 27.4 / 23.8; but 64-wide tiles of C = 160, 14 x 14 x 32: 9.7 / 10.2, C = 112 (16s): 9.6 / 11.0, C = 288: 15.2 / 15.9.
+static int conv_block_channels(const ConvGeom& g) {
+  if (g.R * g.S == 1 || g.KO <= 32 || (g.KO & 7) || g.C % 16 != 0 || !conv_map_possible(g)) return 0;
+  if (g.C % 32 == 0) return g.C % kBK == 32 && g.C < 256 ? 32 : 0;
+  return conv_im2col_eligible(g) || g.C > 256 ? 0 : 16;
 }
 
 // Activations x[N][H][W][C] as a 4-D im2col map (dimensions C, W, H, N): one load brings 128
 // consecutive output pixels x 64 channels for one filter tap, 128-byte swizzled like a GEMM A tile.
 // The bounding box [-pad, extent - 1 + pad - (filter - 1)] holds the window origins; stepping it
 // with the convolution stride visits exactly Wo x Ho origins per image.
-static int make_tmap_im2col(CUtensorMap* map, const void* x, const ConvGeom& g, int pixels) {
+static int make_tmap_im2col(CUtensorMap* map, const void* x, const ConvGeom& g, int pixels, int channels = kBK) {
   EncodeIm2colFn fn = get_encode_im2col_fn();
   if (!fn) return HELIX_ERR_CUDA;
   if (reinterpret_cast<uintptr_t>(x) & 15) return HELIX_ERR_ALIGN;
   struct Key {
     const void* x;
-    int v[9];
+    int v[10];
     bool operator==(const Key& o) const { return x == o.x && std::memcmp(v, o.v, sizeof(v)) == 0; }
   };
   struct KeyHash {
     size_t operator()(const Key& k) const {
       size_t h = reinterpret_cast<size_t>(k.x);
-      for (int i = 0; i < 9; ++i) h ^= (size_t)k.v[i] + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
+      for (int i = 0; i < 10; ++i) h ^= (size_t)k.v[i] + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
       return h;
     }
   };
   static std::mutex mu;
   static std::unordered_map<Key, CUtensorMap, KeyHash> cache;
-  const Key key{x, {g.NB, g.H, g.W, g.C, g.R, g.S, g.stride, g.pad, pixels}};
+  const Key key{x, {g.NB, g.H, g.W, g.C, g.R, g.S, g.stride, g.pad, pixels, channels}};
   {
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
@@ -1209,7 +1260,10 @@ static int make_tmap_im2col(CUtensorMap* map, const void* x, const ConvGeom& g, 
   int upper[2] = {g.pad - (g.S - 1), g.pad - (g.R - 1)};
   cuuint32_t estr[4] = {1, (cuuint32_t)g.stride, (cuuint32_t)g.stride, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(x), dims, strides, lower, upper,
-                  (cuuint32_t)kBK, (cuuint32_t)pixels, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  (cuuint32_t)channels, (cuuint32_t)pixels, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  channels == 16   ? CU_TENSOR_MAP_SWIZZLE_32B
+                  : channels == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                   : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return HELIX_ERR_CUDA;
   std::lock_guard<std::mutex> lock(mu);
@@ -1469,46 +1523,55 @@ void gemm_f16_default_config(int M, int N, int K, int batch, int sm_count, bool 
   default_config_impl(M, N, K, batch, sm_count, conv, true, out);
 }
 
+// Pixels through the im2col map (plain or swapped tiles) over a reduction of length k.
+static void map_config(const ConvGeom& g, int M, int k, int sm_count, helix_cfg_t* out) {
+  default_config_impl(M, g.KO, k, 1, sm_count, false, false, out);
+  // Few pixels: a GEMM would put them on the tile's wide axis and cut K, but a swapped tile reads its pixels in whole
+  // boxes of 32 and more and is not built for a cut K.  The plain tiles cut K as well.
+  if (out->swap_ab && (out->stream_k || out->split_k > 1 || out->tile_n < 32))
+    default_config_impl(M, g.KO, k, 1, sm_count, true, false, out);
+  // A 128 x N x 16 step costs max(N / 2 cycles of pipe time, (128 + N) / 4 cycles of operand fetch from shared
+  // memory): the wide tile does twice the work of a 128-wide one in 1.5x the fetch time, so 65..128 output channels
+  // are better spent as the 128 rows with 256 pixels per step: measured 17.1 -> 13.9 us on 3x3, 128 -> 128
+  // channels, 28 x 28 x 32.
+  // With more channels the pixel tiles become too few for the machine, with 64 or fewer half of
+  // every step is padding.
+  if (g.KO > 64 && g.KO <= kBM && M >= 64 * 256) {
+    out->swap_ab = 1;
+    out->stream_k = 0;
+    out->split_k = 1;
+    out->tile_n = 256;
+  }
+  // 192 pixels per step where that takes fewer or shorter rounds of a machine the launch has to itself (us: 3x3,
+  // 240 -> 240, 20 x 20 x 32: 21.2 -> 19.3; 5x5, 96 -> 256, 26 x 26 x 20: 26.1 -> 22.9), if the slabs of K are many enough:
+  // 128 -> 128, 28 x 28 x 32, gains 1.3 us in a chain of cold launches but loses 1 us between a stage's 1x1 layers
+  if (sm_count >= kWholeMachineSms && g.KO > 64 && out->split_k <= 1 && !out->stream_k) {
+    const int64_t now = plain_rounds(out->swap_ab ? g.KO : M, out->swap_ab ? M : g.KO, out->tile_n, 1, sm_count);
+    const int64_t then = plain_rounds(g.KO, M, 192, 1, sm_count);
+    const int num_kb = (k + kBK - 1) / kBK;
+    if (then * num_kb * slab_us(192) + 1.4 < now * num_kb * slab_us(out->tile_n)) {
+      out->swap_ab = 1;
+      out->tile_n = 192;
+    }
+  }
+  out->stages = max_stages(out->tile_n, false);
+}
+
 // Convolution: a 1x1, stride-1, unpadded one is a plain GEMM over the pixel list; geometries the
 // im2col tensor map covers run the GEMM kernel's schedule (one-CTA tiles); the rest gather.
-void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) {
+static void conv_default_config(const ConvGeom& g, int sm_count, bool block_map, helix_cfg_t* out) {
   const int M = (int)std::min<int64_t>((int64_t)g.NB * g.Ho * g.Wo, 0x7fffffff);
   const int K = (int)std::min<int64_t>((int64_t)g.R * g.S * g.C, 0x7fffffff);
   if (g.R == 1 && g.S == 1 && g.stride == 1 && g.pad == 0)
     default_config_impl(M, g.KO, K, 1, sm_count, false, true, out);
-  else if (conv_im2col_eligible(g)) {
-    default_config_impl(M, g.KO, im2col_k(g), 1, sm_count, false, false, out);
-    // Few pixels: a GEMM would put them on the tile's wide axis and cut K, but a swapped tile reads its pixels in whole
-    // boxes of 32 and more and is not built for a cut K.  The plain tiles cut K as well.
-    if (out->swap_ab && (out->stream_k || out->split_k > 1 || out->tile_n < 32))
-      default_config_impl(M, g.KO, im2col_k(g), 1, sm_count, true, false, out);
-    // A 128 x N x 16 step costs max(N / 2 cycles of pipe time, (128 + N) / 4 cycles of operand fetch from shared
-    // memory): the wide tile does twice the work of a 128-wide one in 1.5x the fetch time, so 65..128 output channels
-    // are better spent as the 128 rows with 256 pixels per step: measured 17.1 -> 13.9 us on 3x3, 128 -> 128
-    // channels, 28 x 28 x 32.
-    // With more channels the pixel tiles become too few for the machine, with 64 or fewer half of
-    // every step is padding.
-    if (g.KO > 64 && g.KO <= kBM && M >= 64 * 256) {
-      out->swap_ab = 1;
-      out->stream_k = 0;
-      out->split_k = 1;
-      out->tile_n = 256;
-    }
-    // 192 pixels per step where that takes fewer or shorter rounds of a machine the launch has to itself (us: 3x3,
-    // 240 -> 240, 20 x 20 x 32: 21.2 -> 19.3; 5x5, 96 -> 256, 26 x 26 x 20: 26.1 -> 22.9), if the slabs of K are many enough:
-    // 128 -> 128, 28 x 28 x 32, gains 1.3 us in a chain of cold launches but loses 1 us between a stage's 1x1 layers
-    if (sm_count >= kWholeMachineSms && g.KO > 64 && out->split_k <= 1 && !out->stream_k) {
-      const int64_t now = plain_rounds(out->swap_ab ? g.KO : M, out->swap_ab ? M : g.KO, out->tile_n, 1, sm_count);
-      const int64_t then = plain_rounds(g.KO, M, 192, 1, sm_count);
-      const int num_kb = im2col_k(g) / kBK;
-      if (then * num_kb * slab_us(192) + 1.4 < now * num_kb * slab_us(out->tile_n)) {
-        out->swap_ab = 1;
-        out->tile_n = 192;
-      }
-    }
-    out->stages = max_stages(out->tile_n, false);
-  } else
-    default_config_impl(M, g.KO, K, 1, sm_count, true, false, out);
+  else if (conv_im2col_eligible(g))
+    map_config(g, M, im2col_k(g), sm_count, out);
+  else {
+    // blocks of channels where whole tiles are the choice, gathering otherwise
+    if (block_map && conv_block_channels(g)) map_config(g, M, K, sm_count, out);
+    if (!block_map || !conv_block_channels(g) || out->stream_k || out->split_k > 1 || out->tile_n < 64)
+      default_config_impl(M, g.KO, K, 1, sm_count, true, false, out);
+  }
   // 64 -> 64 channels, 3 x 3 where the row-pair kernel's tile fits: that kernel (no tile to choose)
   if (conv_f16_rows_eligible(g, sm_count, true)) {
     out->tile_m = kBM;
@@ -1522,6 +1585,8 @@ void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) 
   }
   out->op = HELIX_OP_CONV_F16;
 }
+
+void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) { conv_default_config(g, sm_count, true, out); }
 
 // The reduction length of the implicit GEMM as the kernel walks it (whole 64-channel blocks on the im2col path).
 int64_t conv_f16_gemm_k(const ConvGeom& g) {
@@ -1580,11 +1645,11 @@ unsigned long long* gemm_f16_trace_for_grid(int grid) {
   return (g_trace_buf && g_trace_bytes >= (size_t)grid * kTraceWords * 8) ? g_trace_buf : nullptr;
 }
 
-template <int BN, bool CONV, int OUT, bool LEAN>
+template <int BN, bool CONV, int OUT, bool LEAN, int BLK>
 static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
                                   const GemmParams& p, int grid, size_t smem, cudaStream_t stream) {
   constexpr int threads = CONV ? kConvThreads : kGemmThreads;
-  auto kern = gemm_f16_tc_kernel<BN, CONV, OUT, LEAN>;
+  auto kern = gemm_f16_tc_kernel<BN, CONV, OUT, LEAN, BLK>;
   // the opt-in shared-memory size is sticky per function and device: raise it only when needed
   static std::mutex mu;
   static size_t granted[64] = {0};
@@ -1720,17 +1785,25 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   p.fd_num_kb = make_fastdiv(p.num_kb);
   p.fd_howo = make_fastdiv((conv || p.im2col) ? p.g.Ho * p.g.Wo : 1);
   p.fd_wo = make_fastdiv((conv || p.im2col) ? p.g.Wo : 1);
-  p.fd_cblocks = make_fastdiv(p.im2col ? (p.g.C + kBK - 1) / kBK : 1);
+  p.fd_cblocks = make_fastdiv(p.blocks ? p.blocks / (p.g.R * p.g.S) : p.im2col ? (p.g.C + kBK - 1) / kBK : 1);
   p.fd_s = make_fastdiv(p.im2col ? p.g.S : 1);
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
   const bool any = !p.swap && !p.tma_store, columns = p.swap && p.tma_store;
   // (narrow tiles are stored directly, and swapped ones among them keep the general variant)
   const bool lean = (bn >= 64 ? p.tma_store : !p.swap) && !p.stream_k && p.split_k <= 1 && !p.dual && p.probe == 0 && !p.trace;
+  if (p.blocks && !lean) return HELIX_ERR_UNSUPPORTED;   // conv_block() asks for nothing that needs another variant
   cudaError_t e = cudaErrorInvalidValue;
   auto go = [&](auto width, auto gather, auto out, auto slim) {
-    return launch_variant<decltype(width)::value, decltype(gather)::value, decltype(out)::value, decltype(slim)::value>(
-        ta, tb, tc, p, grid, smem, stream);
+    constexpr int kBN = decltype(width)::value, kOut = decltype(out)::value;
+    constexpr bool kConv = decltype(gather)::value, kSlim = decltype(slim)::value;
+    if constexpr (!kConv && kSlim && kBN >= 64)
+      if (p.blocks) {
+        constexpr int kSide = kOut == kOutColumns ? -1 : 1;
+        return p.g.C % 32 == 0 ? launch_variant<kBN, kConv, kOut, kSlim, 32 * kSide>(ta, tb, tc, p, grid, smem, stream)
+                               : launch_variant<kBN, kConv, kOut, kSlim, 16 * kSide>(ta, tb, tc, p, grid, smem, stream);
+      }
+    return launch_variant<kBN, kConv, kOut, kSlim, 0>(ta, tb, tc, p, grid, smem, stream);
   };
   const std::true_type yes{};
   const std::false_type no{};
@@ -1823,6 +1896,21 @@ int gemm_f16_launch(const helix_cfg_t* cfg_in, const void* A, int64_t lda, const
   return launch_common(cfg, false, ta, tb, p, C, ldc, sc, ws, ws_bytes, sm_count, independent, stream, launches);
 }
 
+// Channels of the blocks that pixels arrive by instead of slabs of 64 or gathering, 0: no blocks.  Only where the launch runs a lean variant
+// (whole tiles, no probes, no timeline, an output that TMA can store); geometries that slabs serve as well, for 128-wide and wider tiles, or C =
+// 96 in 64-wide ones on half the SMs and more (2 x 22 x 19, -> 208, 8 tiles: 6.25 / 6.5; 7 x 37 x 38 -> 64, 75 tiles: 7.1 / 6.9).
+static int conv_block(const helix_cfg_t& cfg, const ConvGeom& g, const void* y, int sm_count) {
+  const bool lean = cfg.tile_n >= 64 && !cfg.stream_k && cfg.split_k <= 1 && !(cfg.probe & 0x8f) && cfg.conv_gather != 1 &&
+                    (reinterpret_cast<uintptr_t>(y) & 15) == 0 && !(cfg.swap_ab && g.KO <= 64 && !(cfg.probe & 0x100)) &&
+                    gemm_f16_trace_for_grid(1) == nullptr;
+  if (!lean) return 0;
+  if (cfg.tile_n == 64 && conv_im2col_eligible(g)) {
+    const int64_t M = (int64_t)g.NB * g.Ho * g.Wo, rows = cfg.swap_ab ? g.KO : M, cols = cfg.swap_ab ? M : g.KO;
+    if (g.C > 96 || ((rows + kBM - 1) / kBM) * ((cols + 63) / 64) * 2 < sm_count) return 0;
+  }
+  return conv_block_channels(g);
+}
+
 int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, void* y, const ConvGeom& g, void* ws,
                     size_t ws_bytes, int* status_dev, int sm_count, bool independent, cudaStream_t stream,
                     int64_t* launches) {
@@ -1866,18 +1954,19 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
       return conv_f16_rows_launch(x, w, y, g, 0, status_dev, sm_count, independent, stream, launches);
   }
   const bool gather_forced = cfg_in && cfg_in->tile_m != 0 && cfg_in->conv_gather == 1;
-  const bool im2col = !gather_forced && conv_im2col_eligible(g);
   helix_cfg_t cfg;
   if (cfg_in && cfg_in->tile_m != 0) {
     cfg = *cfg_in;
   } else {
     conv_f16_default_config(g, sm_count, &cfg);
+    if (!conv_im2col_eligible(g) && !conv_block(cfg, g, y, sm_count)) conv_default_config(g, sm_count, false, &cfg);
     if (!ws || ws_bytes < gemm_f16_workspace_bytes(&cfg, M, N, (int)conv_f16_gemm_k(g), 1, sm_count)) {
       cfg.stream_k = 0;
       cfg.split_k = 1;
     }
   }
   if (cfg.tile_m != kBM || cfg.cta_group > 1) return HELIX_ERR_UNSUPPORTED;
+  const bool im2col = !gather_forced && (conv_im2col_eligible(g) || conv_block(cfg, g, y, sm_count) != 0);
   if (cfg.swap_ab) {
     // Output channels on the 128-row axis, pixels on the tile's wide axis: the tensor core takes
     // about the same time for a 128 x N x 16 step whatever N <= 256, so few output channels are
@@ -1894,8 +1983,15 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     ps.wtaps = g.C % kBK != 0;
     CUtensorMap tw, tx;
     int rcs;
-    if ((rcs = make_tmap_filter(&tw, w, g, kBM)) != HELIX_OK) return rcs;
-    if ((rcs = make_tmap_im2col(&tx, x, g, cfg.tile_n)) != HELIX_OK) return rcs;
+    if (const int blk = conv_block(cfg, g, y, sm_count)) {
+      ps.blocks = K / blk;
+      ps.K = K;
+      ps.wtaps = 0;
+      if ((rcs = make_tmap(&tw, w, K, g.KO, 1, K, 0, kBM)) != HELIX_OK) return rcs;
+    } else if ((rcs = make_tmap_filter(&tw, w, g, kBM)) != HELIX_OK) {
+      return rcs;
+    }
+    if ((rcs = make_tmap_im2col(&tx, x, g, cfg.tile_n, ps.blocks ? K / ps.blocks : kBK)) != HELIX_OK) return rcs;
     return launch_common(cfg, false, tw, tx, ps, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
   }
   GemmParams p{};
@@ -1911,11 +2007,18 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
   if (im2col) {
     // Same kernel as a GEMM: the one producer thread asks the im2col map for 128 pixels x 64
     // channels of one filter tap per K slab.
-    if ((rc = make_tmap_im2col(&ta, x, g, kBM)) != HELIX_OK) return rc;
-    if ((rc = make_tmap_filter(&tb, w, g, cfg.tile_n)) != HELIX_OK) return rc;
     p.K = im2col_k(g);
     p.im2col = 1;
     p.wtaps = g.C % kBK != 0;
+    if (const int blk = conv_block(cfg, g, y, sm_count)) {
+      p.blocks = K / blk;
+      p.K = K;
+      p.wtaps = 0;
+      if ((rc = make_tmap(&tb, w, K, g.KO, 1, K, 0, cfg.tile_n)) != HELIX_OK) return rc;
+    } else if ((rc = make_tmap_filter(&tb, w, g, cfg.tile_n)) != HELIX_OK) {
+      return rc;
+    }
+    if ((rc = make_tmap_im2col(&ta, x, g, kBM, p.blocks ? K / p.blocks : kBK)) != HELIX_OK) return rc;
     return launch_common(cfg, false, ta, tb, p, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
   }
   if ((rc = make_tmap(&tb, w, K, N, 1, K, 0, cfg.tile_n)) != HELIX_OK) return rc;

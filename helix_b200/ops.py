@@ -143,7 +143,11 @@ def kernel_name(launch):
             return "conv_f16_rows_kernel"
         as_gemm = r == 1 and s == 1 and stride == 1 and pad == 0
         im2col = conv_reads_tensor_map(n, h, w, ch, stride, ko, r, s, pad) and not c.conv_gather
-        gathers = not as_gemm and not im2col
+        # blocks of 32 or 16 channels (conv_block in csrc/gemm_f16_tc.cu)
+        blocks = (not c.conv_gather and c.tile_n >= 64 and not c.stream_k and c.split_k <= 1 and r * s > 1 and ko > 32 and
+                  ko % 8 == 0 and n * h * w * ch * 2 >= 131072 and stride <= 8 and
+                  (ch % 64 == 32 and ch < 256 if ch % 32 == 0 else ch % 16 == 0 and ch <= 256))
+        gathers = not as_gemm and not im2col and not blocks
     return "gemm_f16_tc_kernel<%d,%d>" % (c.tile_n, 1 if gathers else 0)
 
 
