@@ -438,6 +438,15 @@ __device__ __forceinline__ void touch_params(const P& p) {
   for (unsigned i = 0; i < sizeof(P) / 4; i += 8) asm volatile("" ::"r"(w[i]));
 }
 
+// Asks the L2 for a line before griddep_wait().  Nothing is read: should the predecessor still write there, the load after the wait
+// sees what it wrote (the L2 is where both meet).
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void tma_prefetch_3d(const void* desc, int x, int y, int z) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(desc)), "r"(x),
+               "r"(y), "r"(z)
+               : "memory");
+}
+
 // ---------------------------------------------------------------- misc loads
 __device__ __forceinline__ uint4 ldg_stream_16(const void* p) {
   uint4 v;

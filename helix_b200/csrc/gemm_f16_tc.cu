@@ -98,6 +98,7 @@ struct GemmParams {
   const __half* x;
   ConvGeom g;
   int im2col;      // A tiles come from an im2col tensor map over x: no gather warps
+  int prefetch;    // operand A of the first slabs is asked for ahead of the wait
   int blocks;      // blocks of 32 or 16 channels of the K axis where pixels arrive by those (BLK), else 0
   int wtaps;       // the weights' map is (channel, tap, output channel): the last channel block of a tap is filled
   // optional per-CTA timeline (null = off): kTraceWords 64-bit words per CTA, see trace_mark
@@ -494,6 +495,8 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
           }
           const int nkb = w.kb1 - w.kb0;
           if (idx == 0 && !p.independent) {
+            for (int n = my_n; p.prefetch && n < min(nkb, stages); n += p.load_warps)
+              tma_prefetch_3d(&tmap_a, (w.kb0 + n) * kBK, w.m_blk * kBM, w.b);
             griddep_wait();
             if (pwarp == 0) griddep_launch_dependents();
           }
@@ -1792,6 +1795,11 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   p.fd_wo = make_fastdiv((conv || p.im2col) ? p.g.Wo : 1);
   p.fd_cblocks = make_fastdiv(p.blocks ? p.blocks / (p.g.R * p.g.S) : p.im2col ? (p.g.C + kBK - 1) / kBK : 1);
   p.fd_s = make_fastdiv(p.im2col ? p.g.S : 1);
+  // Weights against up to 32 vectors are a stream that their way from HBM bounds.  Asking ahead gains where a share is long (decode
+  // steps, us without / with: 24 tokens, 2048 wide 201 / 189, 3072 wide 256 / 243, 4096 wide 359 / 357.5; 32 tokens, 2560 wide 266 / 259),
+  // not where CTAs go through many row blocks or K is short (18744 x 1224, m = 24, 17.1 / 18.5; 14904 x 4056, m = 20, 31.2 / 32.3;
+  // 952 x 600, m = 32, 5.6 / 5.8), nor for wider tiles (a decode step of 64 tokens, 4096 wide: 358 / 364).
+  p.prefetch = p.swap && p.PN <= 32 && !p.im2col && p.num_kb >= 24 && 3 * p.tiles_m <= 2 * sm_count;
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
   const bool any = !p.swap && !p.tma_store, columns = p.swap && p.tma_store;

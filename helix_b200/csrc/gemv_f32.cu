@@ -115,8 +115,6 @@ gemv_f32_stream_kernel(const float* __restrict__ W, int64_t ldw, const float* X,
   constexpr int kStep = U * 128;                    // elements of K per group
   extern __shared__ __align__(16) unsigned char stream_smem[];
   __shared__ float part[kWarps][RB * MRHS];
-  griddep_wait();
-  griddep_launch_dependents();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r_begin = static_cast<int>(static_cast<int64_t>(rows) * blockIdx.x / gridDim.x);
   const int r_end = static_cast<int>(static_cast<int64_t>(rows) * (blockIdx.x + 1) / gridDim.x);
@@ -126,6 +124,15 @@ gemv_f32_stream_kernel(const float* __restrict__ W, int64_t ldw, const float* X,
   // kw warps share a row block, taking its groups of K in turn (kw = 1: the order stated at the top of this file)
   const int rw = kWarps / kw, kwi = warp % kw, rwi = warp / kw;
   int pb = rwi, pk = kwi * kStep, pslot = 0;        // next group to issue: row block, first element
+  // one group per warp to the L2 ahead of the wait, as in the fp16 kernel
+#pragma unroll
+  for (int r = 0; r < RB; ++r)
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (pk + u * 128 + lane * 4 < K && r_begin + pb * RB + r < r_end)
+        prefetch_l2(W + static_cast<int64_t>(r_begin + pb * RB + r) * ldw + pk + u * 128 + lane * 4);
+  griddep_wait();
+  griddep_launch_dependents();
   auto issue = [&]() {
     if (pb < blocks && pk < K) {
       const int row = r_begin + pb * RB;
