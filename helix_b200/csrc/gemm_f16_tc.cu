@@ -18,11 +18,13 @@
 //     "stream-K": whole waves of tiles round-robin and the K slabs of the remaining tiles dealt
 //     evenly to all CTAs, so that every SM stays busy whatever the tile count (one SM cannot
 //     pull more than about 1/148 of the HBM bandwidth, so memory-bound shapes need all of them);
-//   * epilogue warps read TMEM with tcgen05.ld, round once to fp16 and store to global memory;
+//   * epilogue warps read TMEM with tcgen05.ld, round once to fp16 and store through shared memory and TMA (swapped tiles
+//     transposed on the way), or directly where a TMA store cannot write;
 //     partial K ranges are stored as fp32 slots; split-K slices are summed in slice order by the CTA that
 //     completes a tile last, stream-K ranges by a small second kernel (both deterministic);
 //   * swap_ab puts the large N extent on the 128-row UMMA axis when M is skinny.
-// For convolution the A-side tile is gathered by 8 producer warps with 16-byte zero-filling
+// For convolution the activations arrive through an im2col tensor map, in blocks of 64, 32 or 16 channels; where none fits
+// (conv_im2col_eligible, conv_block_channels) the A-side tile is gathered by 8 producer warps with 16-byte zero-filling
 // cp.async (8 lanes per output pixel, K axis ordered (r, s, c)), written in the same swizzled
 // layout the TMA would produce; each thread's arrival on the stage barrier fires when its copies
 // land, and the MMA thread issues fence.proxy.async before the tensor core reads the tile.
@@ -355,8 +357,8 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   constexpr int kTmemCols = L::tmem_cols();
   constexpr uint32_t kIdesc = umma_idesc_f16(kBM, BN);
 
-  // The next kernel on the stream may be scheduled once every CTA of this one has got here (an ordered launch: past
-  // its wait): its CTAs then fill SMs as ours retire instead of waiting for the whole grid to drain.
+  // The next kernel on the stream may be scheduled once every CTA of this one has got here: its CTAs then fill SMs as ours
+  // retire instead of waiting for the whole grid to drain.  (An ordered launch says so behind its wait, below.)
   if (p.independent) griddep_launch_dependents();
 
   extern __shared__ uint8_t smem_raw[];

@@ -1,5 +1,6 @@
 // Memory-bound fp16 GEMV for 1..8 right-hand sides, and products of up to 16 rows: a plain kernel (explicit configurations, split
-// K, small problems), and streaming kernels, with scalar multiply-adds up to two right-hand sides and mma.sync beyond.
+// K, small problems), and streaming kernels, with scalar multiply-adds up to two right-hand sides and mma.sync beyond (one kernel for
+// short streams, with X in shared memory, a deeper one for long ones).
 //
 //   Y[i, r] = sum_k W[r, k] * X[i, k]        W: rows x K (row-major, the HBM stream)
 //                                              X: m x K, m <= 8 (stays in L1/L2)

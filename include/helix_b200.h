@@ -91,8 +91,8 @@ typedef struct helix_cfg {
                     remaining tiles dealt evenly to all CTAs or CTA pairs (needs a workspace);
                     overrides split_k                                                    */
   int conv_gather; /* CONV_F16: 0 = activations arrive through an im2col tensor map wherever the
-                      geometry allows it (C a multiple of 64 or not far below one, tensor of 128 KiB or more), else
-                      through gathering producer warps; 1 = always gather (cp.async);
+                      geometry allows it (C a multiple of 64 or not far below one, or in blocks of 32 or 16
+                      channels; tensor of 128 KiB or more), else through gathering producer warps; 1 = always gather (cp.async);
                       3 = window-resident kernel (stride 1, C a multiple of 64, W + 2*pad <= 256);
                       4 = row-pair kernel (3 x 3, stride 1, pad 1, 64 -> 64 channels, W <= 62: pixels on
                       the accumulator rows, window and all weights resident; the library's own choice
