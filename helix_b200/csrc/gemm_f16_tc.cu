@@ -252,6 +252,7 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
         tc_fence_after_sync();
         if (lane == 0 && ME == 0) trace_mark<LEAN>(p, idx, 2);
         const uint32_t d_tmem = tmem_base + acc * BN;
+        if (idx == 0 && !p.independent) griddep_wait();
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
           // One wait per group of stages: reading shared memory (the barrier) costs the issuing warp some 200
           // cycles on top of the 45 it needs to hand one MMA to the tensor core, more than a 64-deep slab
@@ -425,8 +426,10 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   const uint32_t tmem_base = *tmem_ptr_smem;
 
   // Everything above touched only this CTA's shared memory and TMEM, so it may overlap the tail of the preceding kernel.
-  // Unless the caller declared the launch independent of its predecessor, the roles that read or write global memory wait
-  // for that kernel to complete: the producers when their first load is ready to be issued, the epilogue warps first thing.
+  // Unless the caller declared the launch independent of its predecessor, every role waits for that kernel to complete: the
+  // producers when their first load is ready to be issued, the epilogue warps first thing, the issuing and watching warps ahead of
+  // their first bounded wait -- they touch no global memory, but its clock must not run while the predecessor does, which may
+  // take any time.
 
   // the MMA-issuing role: warp kMmaWarp, and with dual issue also warp 3, which then issues no loads
   const bool second_issuer = dual && warp == 3;
@@ -466,6 +469,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         uint32_t phase = 0;
         WorkItem w;
         for (int idx = 0; get_item<LEAN>(p, cta, grid, idx, w); ++idx) {
+          if (idx == 0 && !p.independent) griddep_wait();
           for (int kb = w.kb0; kb < w.kb1; ++kb) {
             if (gpos == 0) {
               if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[gidx], phase, abort_flag, p.status));

@@ -245,6 +245,7 @@ __device__ __forceinline__ void pair_dual_issue_loop(const Gemm2Params& p, const
     tc_fence_after_sync();
     if (lane == 0 && ME == 0) trace2_tile<LEAN>(p, idx, 2);
     const uint32_t d_tmem = tmem_base + acc * BN;
+    if (idx == 0 && !p.independent) griddep_wait();
     for (int kb = it.kb0; kb < it.kb1; ++kb) {
       const int n = nslab++;
       if ((n & 1) == ME) {
@@ -336,8 +337,9 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_ptr_smem;
 
-  // Nothing so far has touched global memory: the roles that do wait for the predecessor, when their first load is ready to
-  // be issued, or first thing (epilogue).
+  // Nothing so far has touched global memory.  Every role waits for the predecessor: the loading ones when their first load is
+  // ready to be issued, the epilogue warps first thing, the issuing and watching warps ahead of their first bounded wait, whose
+  // clock must not run while the predecessor does.
 
   if (warp == 0 || warp >= 6) {
     // ------------------------------------------------------------------ TMA producers (each CTA)
@@ -359,6 +361,7 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       uint32_t phase = 0;
       Item2 it;
       for (int idx = 0; get_item2<LEAN>(p, pair, num_pairs, idx, it); ++idx) {
+        if (idx == 0 && !p.independent) griddep_wait();
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
           if (gpos == 0) {
             if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&full_bar[gidx], phase, abort_flag, p.status));
@@ -445,6 +448,7 @@ gemm_f16_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_after_sync();
         if (lane == 0) trace2_tile<LEAN>(p, idx, 2);
         const uint32_t d_tmem = tmem_base + acc * BN;
+        if (idx == 0 && !p.independent) griddep_wait();
         for (int kb = it.kb0; kb < it.kb1; ++kb) {
           // one rendezvous (or wait) per group of stages; the stages are still released one by one
           if (gpos == 0) {
