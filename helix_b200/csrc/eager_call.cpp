@@ -38,14 +38,16 @@ bool modes_active() {
   return at::impl::torch_function_mode_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set();
 }
 
-// The tensor behind `o` if it is a plain one on a CUDA device, of this type and rank, with memory of its own.
+// The tensor behind `o` if it is a plain one on the current CUDA device, of this type and rank, with memory of its own and no
+// expanded dimension (a stride of 0 stands for "contiguous" in helix_launch_t).
 const at::Tensor* plain(PyObject* o, at::ScalarType type, int64_t dim) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  if (!t.defined() || !t.is_cuda() || t.scalar_type() != type || t.dim() != dim || t.layout() != at::kStrided || !t.has_storage())
+  if (!t.defined() || !t.is_cuda() || t.scalar_type() != type || t.dim() != dim || t.layout() != at::kStrided || !t.has_storage() ||
+      t.get_device() != c10::cuda::current_device())
     return nullptr;
   for (int64_t i = 0; i < dim; ++i)
-    if (t.size(i) > INT_MAX) return nullptr;
+    if (t.size(i) > INT_MAX || (t.size(i) > 1 && t.stride(i) == 0)) return nullptr;
   return &t;
 }
 

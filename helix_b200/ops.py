@@ -37,9 +37,15 @@ def _native():
 
 
 def _require_cuda(*tensors):
+    """Operands of one launch: CUDA tensors of one device whose elements all have a place of their own (in the C ABI a leading
+    dimension or batch stride of 0 stands for a contiguous operand, so an expanded one would be read past its end)."""
     for t in tensors:
         if not t.is_cuda:
             raise ValueError("helix_b200 operators take CUDA tensors only (there is no CPU path)")
+        if t.device != tensors[0].device:
+            raise ValueError(f"operands on different devices: {tensors[0].device} and {t.device}")
+        if any(n > 1 and st == 0 for n, st in zip(t.shape, t.stride())):
+            raise ValueError("expanded operands (a stride of 0) are not supported: make them contiguous")
 
 
 def _stream(dev=None):
@@ -183,7 +189,7 @@ def _finish(launch, cfg, ws):
         launch.cfg = cfg
     need = lib.helix_workspace_bytes(ctypes.byref(launch))
     if need:
-        buf = ws if ws is not None else workspace(need)
+        buf = ws if ws is not None else workspace(need, launch._refs[0].device)
         if buf.numel() * buf.element_size() < need:
             raise ValueError(f"workspace too small: need {need} bytes")
         launch.ws = buf.data_ptr()
@@ -202,6 +208,7 @@ def launch_gemm_f16(a, b_nk, out, cfg=None, ws=None):
         assert a.stride(2) == 1 and b_nk.stride(2) == 1 and out.stride(2) == 1
         l.batch, l.M, l.K = a.shape
         l.N = b_nk.shape[1]
+        assert b_nk.shape[0] == out.shape[0] == l.batch
         l.lda, l.ldb, l.ldc = a.stride(1), b_nk.stride(1), out.stride(1)
         l.stride_a, l.stride_b, l.stride_c = a.stride(0), b_nk.stride(0), out.stride(0)
     else:
@@ -265,7 +272,7 @@ def gemv_f32(w, x, out=None, cfg=None):
         return y
     if out is None:
         out = w.new_empty((x.shape[0], w.shape[0]))
-    run(launch_gemv_f32(w, x, out, cfg))
+    _run_eager(launch_gemv_f32(w, x, out, cfg))
     return out
 
 
@@ -345,7 +352,7 @@ def conv2d_f32_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
     Ho, Wo = conv_out_hw(H, W, R, S, stride, pad)
     if out is None:
         out = x.new_empty((N, Ho, Wo, KO))
-    run(launch_conv2d_f32(x, w, out, stride, pad, cfg))
+    _run_eager(launch_conv2d_f32(x, w, out, stride, pad, cfg))
     return out
 
 
@@ -371,8 +378,15 @@ def launch_gemm_f32(a, b, out, trans_a=False, cfg=None):
 
 
 def run(launch):
-    """Queue a prepared launch on torch's current stream."""
+    """Queue a prepared launch on torch's current stream; its operands live on the current device."""
     _native().run(launch)
+
+
+def _run_eager(launch):
+    dev = launch._refs[0].device
+    if dev.index != torch.cuda.current_device():
+        raise ValueError(f"operands on {dev} while device {torch.cuda.current_device()} is current")
+    run(launch)
 
 
 # ----------------------------------------------------------------------------- eager operators
@@ -382,7 +396,7 @@ def gemm_f16(a, b_nk, out=None, cfg=None):
     shape = (*a.shape[:-1], b_nk.shape[-2])
     if out is None:
         out = a.new_empty(shape)
-    run(launch_gemm_f16(a, b_nk, out, cfg))
+    _run_eager(launch_gemm_f16(a, b_nk, out, cfg))
     return out
 
 
@@ -391,7 +405,7 @@ def gemv_f16(w, x, out=None, cfg=None):
         return y
     if out is None:
         out = w.new_empty((x.shape[0], w.shape[0]))
-    run(launch_gemv_f16(w, x, out, cfg))
+    _run_eager(launch_gemv_f16(w, x, out, cfg))
     return out
 
 
@@ -401,7 +415,7 @@ def conv2d_f16_nhwc(x, w, stride=1, pad=0, out=None, cfg=None):
     if out is None:
         Ho, Wo = conv_out_hw(x.shape[1], x.shape[2], w.shape[1], w.shape[2], stride, pad)
         out = x.new_empty((x.shape[0], Ho, Wo, w.shape[0]))
-    run(launch_conv2d_f16(x, w, out, stride, pad, cfg))
+    _run_eager(launch_conv2d_f16(x, w, out, stride, pad, cfg))
     return out
 
 
@@ -411,7 +425,7 @@ def gemm_f32(a, b, trans_a=False, out=None, cfg=None):
     M = a.shape[1] if trans_a else a.shape[0]
     if out is None:
         out = a.new_empty((M, b.shape[1]))
-    run(launch_gemm_f32(a, b, out, trans_a, cfg))
+    _run_eager(launch_gemm_f32(a, b, out, trans_a, cfg))
     return out
 
 

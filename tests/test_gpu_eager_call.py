@@ -46,6 +46,15 @@ CALLS = {
     "gemv nine vectors": lambda: ops.gemv_f16(_w["w"], _w["x"].repeat(3, 1)),
     "gemv on the CPU": lambda: ops.gemv_f16(_w["w"].cpu(), _w["x"].cpu()),
     "gemv parameter": lambda: ops.gemv_f16(torch.nn.Parameter(_w["w"]), _w["x"]),
+    "gemv one vector for all": lambda: ops.gemv_f16(_w["w"], _w["x"][:1].expand(3, -1)),
+    "gemv one row for all": lambda: ops.gemv_f16(_w["w"][:1].expand(300, -1), _w["x"]),
+    "gemv expanded output": lambda: ops.gemv_f16(_w["w"], _w["x"], out=torch.zeros(300, device="cuda", dtype=torch.float16).expand(3, 300)),
+    "gemv one expanded vector": lambda: ops.gemv_f16(_w["w"], _w["x"][:1].expand(1, -1)),
+    "gemv_f32 one vector for all": lambda: ops.gemv_f32(_w["w"].float(), _w["x"][:1].float().expand(3, -1)),
+    "gemm weights for all batches": lambda: ops.gemm_f16(_w["a3"], _w["b3"][0].expand(2, -1, -1)),
+    "gemm one batch, expanded": lambda: ops.gemm_f16(_w["a3"][:1], _w["b3"][0].expand(1, -1, -1)),
+    "gemm one row for all": lambda: ops.gemm_f16(_w["a"][:1].expand(70, -1), _w["w"]),
+    "gemm_f32 one row for all": lambda: ops.gemm_f32(_w["a"][:1].float().expand(70, -1), _w["w"].float().t().contiguous()),
     "gemv_f32": lambda: ops.gemv_f32(_w["w"].float(), _w["x"].float()),
     "gemm": lambda: ops.gemm_f16(_w["a"], _w["w"]),
     "gemm batched": lambda: ops.gemm_f16(_w["a3"], _w["b3"]),
@@ -84,6 +93,14 @@ def test_native_call_and_python_agree(monkeypatch, name):
     else:
         assert type(native) is type(python) and native.stride() == python.stride() and not native.requires_grad
         assert torch.equal(native, python)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", [n for n in CALLS if "for all" in n or "expanded output" in n])
+def test_expanded_operands_are_refused(name):
+    _w.update(w=_rand(300, 136), x=_rand(3, 136), a=_rand(70, 136), a3=_rand(2, 70, 136), b3=_rand(2, 72, 136))
+    with pytest.raises(ValueError, match="expanded"):
+        CALLS[name]()
 
 
 @pytest.mark.gpu
