@@ -423,7 +423,8 @@ __device__ __forceinline__ bool named_bar_and(int id, int nthreads, bool pred) {
 // A kernel of an ordered launch calls launch_dependents after its wait: its successor may be flagged not to wait itself,
 // and then starts -- and reads -- with nothing behind it but this call, while the caller only vouches for THIS launch
 // not writing its operands.  Whatever was queued earlier must be complete by then.  (Nothing is lost by it: until the
-// predecessor is complete the successor's CTAs could only sit beside ours.)  Flagged launches call it at entry, so that
+// predecessor is complete the successor's CTAs could only sit beside ours.)  One exception: a GEMM whose next kernel is its own stream-K
+// fix-up, which is never flagged, calls it ahead of its wait (gemm_f16_tc.cu, fixup_next).  Flagged launches call it at entry, so that
 // a run of them overlaps as a whole.  A step of sixteen one-token GEMVs with static weights takes 236.8 us that way and
 // 244.1 when every one of them holds its successor back: the launch after the next fills its FIFOs while this one's last rows drain.
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

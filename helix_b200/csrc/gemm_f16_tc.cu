@@ -83,6 +83,7 @@ struct GemmParams {
   int total_items;
   // stream-K schedule: dp_rounds whole tiles per CTA, then sk_tiles tiles cut into K-slab ranges
   int stream_k;
+  int fixup_next;  // the next kernel on the stream is this launch's fix-up, which overlaps it
   int dp_rounds;   // whole tiles each CTA computes on its own
   int sk_tiles;    // tiles whose K slabs are dealt out
   int sk_upc;      // K slabs per CTA in the dealt part (<= num_kb, so a range touches <= 2 tiles)
@@ -433,10 +434,14 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 
   // the MMA-issuing role: warp kMmaWarp, and with dual issue also warp 3, which then issues no loads
   const bool second_issuer = dual && warp == 3;
-  // The next kernel is let in when every warp has said so or has left.  With the whole tiles in shared memory a GEMM has no room
-  // beside this one anyway, and comes in as CTAs leave; the stream-K fix-up has, and all warps call for it (its launch then costs
-  // nothing: 2560 x 10240, 32 vectors, 19.6 -> 16.0 us; let in as early, a GEMM costs the loads of this one 1 %).
-  if (!LEAN && p.stream_k && warp <= kMmaWarp) griddep_launch_dependents();
+  // With the whole tiles in shared memory a GEMM has no room beside this one anyway, and comes in as CTAs leave (let in at once it
+  // costs the loads of this one 1 %).  The stream-K fix-up has room, and is called for ahead of the wait: it waits for this kernel
+  // itself, so nothing can start past it -- which is why only a launch that queues its fix-up right behind itself may do this.  All
+  // warps call, because with one calling the fix-up came late (an observation that only the time rests on: a decode step of 20 tokens, 1536
+  // wide, 177 us with one, 159 with all).  us, called for after the wait / here, decode steps of four blocks: 20 tokens, 1536 wide 165 / 151;
+  // 24 tokens, 2048 wide 205 / 187; 32 tokens, 2560 wide 254 / 226, 4096 wide 373 / 361.  A tiny kernel between such products loses
+  // (1024 x 4096 by 32 and a 256 x 256 GEMV: 11.9 / 15.8).
+  if (!LEAN && p.fixup_next && warp <= kMmaWarp) griddep_launch_dependents();
   if (warp == kMmaWarp) {
     if (dual)
       mma_issue_loop<BN, CONV, !LEAN, 0, LEAN, BLK>(p, cta, grid, lane, stages, sA, sB, full_bar, empty_bar, tmem_full, tmem_empty,
@@ -686,7 +691,7 @@ gemm_f16_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     // ------------------------------------------------------------------ epilogue
     const int quarter = warp & 3;  // TMEM lanes [32*quarter, 32*quarter + 32)
     if (!p.independent) griddep_wait();
-    if (!LEAN && p.stream_k) griddep_launch_dependents();
+    if (!LEAN && p.fixup_next) griddep_launch_dependents();
     if (!LEAN && quarter == 0 && lane == 0 && p.trace != nullptr) p.trace[(size_t)cta * kTraceWords + 2] = (unsigned long long)clock64();
     bool ok = true;
     const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
@@ -1806,6 +1811,8 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   // not where CTAs go through many row blocks or K is short (18744 x 1224, m = 24, 17.1 / 18.5; 14904 x 4056, m = 20, 31.2 / 32.3;
   // 952 x 600, m = 32, 5.6 / 5.8), nor for wider tiles (a decode step of 64 tokens, 4096 wide: 358 / 364).
   p.prefetch = p.swap && p.PN <= 32 && !p.im2col && p.num_kb >= 24 && 3 * p.tiles_m <= 2 * sm_count;
+  const dim3 fgrid((kBM * (bn >> 2) + 255) / 256, std::max(p.sk_tiles, 1));
+  p.fixup_next = fixup && bn <= 32 && (int64_t)fgrid.x * fgrid.y <= 2 * sm_count;
   p.trace = gemm_f16_trace_for_grid(grid);
   p.probe = conv ? 0 : (cfg.probe & 7);
   const bool any = !p.swap && !p.tma_store, columns = p.swap && p.tma_store;
@@ -1850,8 +1857,7 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   if (e != cudaSuccess) return HELIX_ERR_CUDA;
   ++*launches;
   if (fixup) {
-    const dim3 fgrid((kBM * (bn >> 2) + 255) / 256, p.sk_tiles);
-    if (bn <= 32 && (int64_t)fgrid.x * fgrid.y <= 2 * sm_count) {
+    if (p.fixup_next) {
       if (launch_overlapped(gemm_streamk_fixup_kernel, fgrid, dim3(256), 0, stream, p, bn, grid, true) != cudaSuccess)
         return HELIX_ERR_CUDA;
     } else {

@@ -207,7 +207,7 @@ gemv_f16_stream_kernel(const __half* __restrict__ W, int64_t ldw, const __half* 
       if (pk < K && r_begin + pb * kBlockRows + u < r_end)
         prefetch_l2(W + static_cast<int64_t>(r_begin + pb * kBlockRows + u) * ldw + pk);
     griddep_wait();
-    if (!(order_mode & kHoldNext)) griddep_launch_dependents();
+    griddep_launch_dependents();
   }
   auto issue = [&]() {
     if (pb < blocks && pk < k_limit) {
@@ -558,7 +558,7 @@ gemv_f16_deep_kernel(const __half* __restrict__ W, int64_t ldw, const __half* X,
           for (int j = 0; j < J; ++j) prefetch_l2(src[u] + i * k_step + j * 32);
         }
     griddep_wait();
-    if (!(order_mode & kHoldNext)) griddep_launch_dependents();
+    griddep_launch_dependents();
   }
   auto issue_w = [&]() {
     if (pb < blocks && pk < K) {
