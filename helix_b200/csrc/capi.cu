@@ -90,6 +90,12 @@ helix::ConvGeom conv_geom(const int* c) {
   return g;
 }
 
+// The GEMM's choice depends on whether TMA stores can write its C: planning asks with the launch's own.
+void gemm_default(const helix_launch_t* l, int sms, helix_cfg_t* out) {
+  helix::gemm_f16_default_config(l->M, l->N, l->K, l->batch > 0 ? l->batch : 1, sms,
+                                 helix::gemm_f16_tma_writes(l->c, l->ldc, l->stride_c, l->M, l->N), out);
+}
+
 int dispatch(const helix_launch_t* l, void* status_dev, cudaStream_t stream) {
   if (!l) return HELIX_ERR_INVALID;
   helix_devinfo_t info;
@@ -237,13 +243,13 @@ int helix_default_config(const helix_launch_t* l, helix_cfg_t* out) {
   std::memset(out, 0, sizeof(*out));
   switch (l->op) {
     case HELIX_OP_GEMM_F16:
-      helix::gemm_f16_default_config(l->M, l->N, l->K, l->batch > 0 ? l->batch : 1, sms, false, out);
+      gemm_default(l, sms, out);
       return HELIX_OK;
     case HELIX_OP_CONV_F16: {
       const helix::ConvGeom g = conv_geom(l->conv);
       const int64_t M = (int64_t)g.NB * g.Ho * g.Wo, K = (int64_t)g.R * g.S * g.C;
       if (M <= 0 || M > 0x7fffffff || K <= 0 || K > 0x7fffffff) return HELIX_ERR_INVALID;
-      helix::conv_f16_default_config(g, sms, out);
+      helix::conv_f16_default_config(g, l->c, sms, out);
       return HELIX_OK;
     }
     case HELIX_OP_GEMV_F16:
@@ -283,7 +289,7 @@ size_t helix_workspace_bytes(const helix_launch_t* l) {
   switch (l->op) {
     case HELIX_OP_GEMM_F16: {
       helix_cfg_t cfg = l->cfg;
-      if (!have_cfg) helix::gemm_f16_default_config(l->M, l->N, l->K, l->batch > 0 ? l->batch : 1, sms, false, &cfg);
+      if (!have_cfg) gemm_default(l, sms, &cfg);
       return helix::gemm_f16_workspace_bytes(&cfg, l->M, l->N, l->K, l->batch > 0 ? l->batch : 1, sms);
     }
     case HELIX_OP_CONV_F16: {
@@ -292,7 +298,7 @@ size_t helix_workspace_bytes(const helix_launch_t* l) {
       if (M <= 0 || M > 0x7fffffff || K > 0x7fffffff / 2) return 0;
       if (g.C == 4) return 0;   // the four-channel first-layer kernel keeps everything on chip
       helix_cfg_t cfg = l->cfg;
-      if (!have_cfg) helix::conv_f16_default_config(g, sms, &cfg);
+      if (!have_cfg) helix::conv_f16_default_config(g, l->c, sms, &cfg);
       return helix::gemm_f16_workspace_bytes(&cfg, (int)M, g.KO, (int)helix::conv_f16_gemm_k(g), 1, sms);
     }
     case HELIX_OP_GEMV_F16: {

@@ -1360,9 +1360,9 @@ static int64_t plain_rounds(int pm, int pn, int bn, int batch, int sm_count) {
 // Built-in choice when the caller brings no profiled dictionary (the profiled cost model of
 // the scripts layer supersedes it).  Skinny M goes on the UMMA N axis (swap_ab); otherwise the
 // tile width minimising waves x slabs x slab time wins; stream-K is used when whole-tile
-// scheduling would leave a large part of the machine idle.
+// scheduling would leave a large part of the machine idle.  `tma_c`: TMA stores can write C (gemm_f16_tma_writes).
 static void default_config_impl(int M, int N, int K, int batch, int sm_count, bool conv, bool allow_pair,
-                                helix_cfg_t* out, bool tma_c = true) {
+                                bool tma_c, helix_cfg_t* out) {
   *out = helix_cfg_t{};
   out->op = conv ? HELIX_OP_CONV_F16 : HELIX_OP_GEMM_F16;
   out->tile_m = kBM;
@@ -1538,17 +1538,23 @@ static void default_config_impl(int M, int N, int K, int batch, int sm_count, bo
   }
 }
 
-void gemm_f16_default_config(int M, int N, int K, int batch, int sm_count, bool conv, helix_cfg_t* out) {
-  default_config_impl(M, N, K, batch, sm_count, conv, true, out);
+bool gemm_f16_tma_writes(const void* C, int64_t ldc, int64_t sc, int M, int N) {
+  if (ldc == 0) ldc = N;
+  if (sc == 0) sc = (int64_t)M * ldc;
+  return (ldc & 7) == 0 && (sc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+}
+
+void gemm_f16_default_config(int M, int N, int K, int batch, int sm_count, bool tma_c, helix_cfg_t* out) {
+  default_config_impl(M, N, K, batch, sm_count, false, true, tma_c, out);
 }
 
 // Pixels through the im2col map (plain or swapped tiles) over a reduction of length k.
-static void map_config(const ConvGeom& g, int M, int k, int sm_count, helix_cfg_t* out) {
-  default_config_impl(M, g.KO, k, 1, sm_count, false, false, out);
+static void map_config(const ConvGeom& g, int M, int k, int sm_count, bool tma_c, helix_cfg_t* out) {
+  default_config_impl(M, g.KO, k, 1, sm_count, false, false, tma_c, out);
   // Few pixels: a GEMM would put them on the tile's wide axis and cut K, but a swapped tile reads its pixels in whole
   // boxes of 32 and more and is not built for a cut K.  The plain tiles cut K as well.
   if (out->swap_ab && (out->stream_k || out->split_k > 1 || out->tile_n < 32))
-    default_config_impl(M, g.KO, k, 1, sm_count, true, false, out);
+    default_config_impl(M, g.KO, k, 1, sm_count, true, false, tma_c, out);
   // A 128 x N x 16 step costs max(N / 2 cycles of pipe time, (128 + N) / 4 cycles of operand fetch from shared
   // memory): the wide tile does twice the work of a 128-wide one in 1.5x the fetch time, so 65..128 output channels
   // are better spent as the 128 rows with 256 pixels per step: measured 17.1 -> 13.9 us on 3x3, 128 -> 128
@@ -1578,18 +1584,18 @@ static void map_config(const ConvGeom& g, int M, int k, int sm_count, helix_cfg_
 
 // Convolution: a 1x1, stride-1, unpadded one is a plain GEMM over the pixel list; geometries the
 // im2col tensor map covers run the GEMM kernel's schedule (one-CTA tiles); the rest gather.
-static void conv_default_config(const ConvGeom& g, int sm_count, bool block_map, helix_cfg_t* out) {
+static void conv_default_config(const ConvGeom& g, int sm_count, bool tma_c, bool block_map, helix_cfg_t* out) {
   const int M = (int)std::min<int64_t>((int64_t)g.NB * g.Ho * g.Wo, 0x7fffffff);
   const int K = (int)std::min<int64_t>((int64_t)g.R * g.S * g.C, 0x7fffffff);
   if (g.R == 1 && g.S == 1 && g.stride == 1 && g.pad == 0)
-    default_config_impl(M, g.KO, K, 1, sm_count, false, true, out);
+    default_config_impl(M, g.KO, K, 1, sm_count, false, true, tma_c, out);
   else if (conv_im2col_eligible(g))
-    map_config(g, M, im2col_k(g), sm_count, out);
+    map_config(g, M, im2col_k(g), sm_count, tma_c, out);
   else {
     // blocks of channels where whole tiles are the choice, gathering otherwise
-    if (block_map && conv_block_channels(g)) map_config(g, M, K, sm_count, out);
+    if (block_map && conv_block_channels(g)) map_config(g, M, K, sm_count, tma_c, out);
     if (!block_map || !conv_block_channels(g) || out->stream_k || out->split_k > 1 || out->tile_n < 64)
-      default_config_impl(M, g.KO, K, 1, sm_count, true, false, out);
+      default_config_impl(M, g.KO, K, 1, sm_count, true, false, tma_c, out);
   }
   // 64 -> 64 channels, 3 x 3 where the row-pair kernel's tile fits: that kernel (no tile to choose)
   if (conv_f16_rows_eligible(g, sm_count, true)) {
@@ -1604,8 +1610,6 @@ static void conv_default_config(const ConvGeom& g, int sm_count, bool block_map,
   }
   out->op = HELIX_OP_CONV_F16;
 }
-
-void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out) { conv_default_config(g, sm_count, true, out); }
 
 // The reduction length of the implicit GEMM as the kernel walks it (whole 64-channel blocks on the im2col path).
 int64_t conv_f16_gemm_k(const ConvGeom& g) {
@@ -1791,8 +1795,7 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   // whole tiles of a row-major, 16-byte-aligned C leave through a TMA store, swapped ones transposed (not the M = 64 ones)
   CUtensorMap tc = tb;
   p.tma_store = 0;
-  if (bn >= 64 && (ldc & 7) == 0 && (sc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 &&
-      !(p.swap && (p.m64 || p.split_k > 1)) &&
+  if (bn >= 64 && gemm_f16_tma_writes(C, ldc, sc, p.swap ? p.PN : p.PM, p.swap ? p.PM : p.PN) && !(p.swap && (p.m64 || p.split_k > 1)) &&
       (p.swap ? make_tmap(&tc, C, p.PM, p.PN, p.batch, ldc, sc, 64) : make_tmap(&tc, C, p.PN, p.PM, p.batch, ldc, sc, 32)) == HELIX_OK)
     p.tma_store = 1;
   // a launch that shares its workspace with its neighbours on the stream is never independent of them
@@ -1885,8 +1888,7 @@ int gemm_f16_launch(const helix_cfg_t* cfg_in, const void* A, int64_t lda, const
   if (cfg_in && cfg_in->tile_m != 0) {
     cfg = *cfg_in;
   } else {
-    const bool tma_c = (ldc & 7) == 0 && (sc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
-    default_config_impl(M, N, K, batch, sm_count, false, true, &cfg, tma_c);
+    gemm_f16_default_config(M, N, K, batch, sm_count, gemm_f16_tma_writes(C, ldc, sc, M, N), &cfg);
     const size_t need = gemm_f16_workspace_bytes(&cfg, M, N, K, batch, sm_count);
     const bool scratch = need > 0 && ws && ws_bytes >= need;
     if (batch == 1 && gemv_f16_stream_covers(B, ldb, A, lda, N, K, M, sm_count, scratch))
@@ -1936,6 +1938,13 @@ static int conv_block(const helix_cfg_t& cfg, const ConvGeom& g, const void* y, 
   return conv_block_channels(g);
 }
 
+// The library's choice for an output at y: what a launch without a configuration runs, and what planning reports and sizes.
+void conv_f16_default_config(const ConvGeom& g, const void* y, int sm_count, helix_cfg_t* out) {
+  const bool tma_c = gemm_f16_tma_writes(y, g.KO, 0, 1, g.KO);
+  conv_default_config(g, sm_count, tma_c, true, out);
+  if (!conv_im2col_eligible(g) && !conv_block(*out, g, y, sm_count)) conv_default_config(g, sm_count, tma_c, false, out);
+}
+
 int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, void* y, const ConvGeom& g, void* ws,
                     size_t ws_bytes, int* status_dev, int sm_count, bool independent, cudaStream_t stream,
                     int64_t* launches) {
@@ -1974,7 +1983,7 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
   // 32 x 56 x 56: 11.9 us against 19.8 us for the 64-wide implicit GEMM, bit-identical results)
   if (!(cfg_in && cfg_in->tile_m != 0)) {
     helix_cfg_t own;
-    conv_f16_default_config(g, sm_count, &own);
+    conv_f16_default_config(g, y, sm_count, &own);
     if (own.conv_gather == 4)
       return conv_f16_rows_launch(x, w, y, g, 0, status_dev, sm_count, independent, stream, launches);
   }
@@ -1983,8 +1992,7 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
   if (cfg_in && cfg_in->tile_m != 0) {
     cfg = *cfg_in;
   } else {
-    conv_f16_default_config(g, sm_count, &cfg);
-    if (!conv_im2col_eligible(g) && !conv_block(cfg, g, y, sm_count)) conv_default_config(g, sm_count, false, &cfg);
+    conv_f16_default_config(g, y, sm_count, &cfg);
     if (!ws || ws_bytes < gemm_f16_workspace_bytes(&cfg, M, N, (int)conv_f16_gemm_k(g), 1, sm_count)) {
       cfg.stream_k = 0;
       cfg.split_k = 1;

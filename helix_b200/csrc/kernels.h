@@ -69,9 +69,10 @@ struct ConvGeom {
 };
 int gemm_f16_num_configs();
 void gemm_f16_get_config(int idx, helix_cfg_t* out);
-// Fills *out with the library's default choice for the problem.
-void gemm_f16_default_config(int M, int N, int K, int batch, int sm_count, bool conv, helix_cfg_t* out);
-void conv_f16_default_config(const ConvGeom& g, int sm_count, helix_cfg_t* out);
+// Fill *out with the library's default choice for the problem and its output (tma_c: TMA stores can write it).
+bool gemm_f16_tma_writes(const void* C, int64_t ldc, int64_t sc, int M, int N);
+void gemm_f16_default_config(int M, int N, int K, int batch, int sm_count, bool tma_c, helix_cfg_t* out);
+void conv_f16_default_config(const ConvGeom& g, const void* y, int sm_count, helix_cfg_t* out);
 int64_t conv_f16_gemm_k(const ConvGeom& g);
 // ---- conv_f32.cu (FFMA GEMM over the windows, gathered by its loader or through a column matrix)
 size_t conv_f32_workspace_bytes(const ConvGeom& g);

@@ -168,7 +168,8 @@ int helix_get_config(int op, int idx, helix_cfg_t* out);
 /* The configuration the library would pick for `launch` when launch->cfg is zeroed: the built-in
  * analytic stand-in for cost_model() (scripts/Ampere_FP16/Ampere_FP16_gemm.py:420-430), used when
  * no profiled dictionary is at hand.  For GEMVs and fp16 products of up to 16 rows it is that of the kernels which
- * configurations select; a zeroed cfg may also run one of the streaming kernels, which none names. */
+ * configurations select; a zeroed cfg may also run one of the streaming kernels, which none names.  The choice of a GEMM or
+ * convolution in fp16 depends on where its output lies (c, ldc, stride_c): fill these in first, here and below. */
 int helix_default_config(const helix_launch_t* launch, helix_cfg_t* out);
 
 /* Bytes of workspace a launch needs (0 when none).  Decided by sizes: a kernel that the pointers' alignment

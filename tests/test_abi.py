@@ -101,3 +101,24 @@ def test_conv_f32_workspace_is_column_matrix_plus_transposed_weights(lib):
     assert lib.helix_workspace_bytes(ctypes.byref(l)) == 256
     c = Cfg()
     assert lib.helix_default_config(ctypes.byref(l), ctypes.byref(c)) == 0 and c.op == _lib.OP_CONV_F32 and c.tile_m > 0
+
+
+def test_planning_sees_the_output_that_the_launch_writes(lib):
+    """Tall tiles of M by 128 columns leave through transposed TMA stores; a C that those cannot write (odd leading dimension or
+    address) runs another choice, and that is the one reported and given its workspace."""
+    def plan(c, ldc, stride=0, batch=1):
+        l = Launch()
+        l.op, l.M, l.N, l.K, l.batch, l.ldc, l.c, l.stride_c = _lib.OP_GEMM_F16, 21020, 128, 4560, batch, ldc, c, stride
+        cfg = Cfg()
+        assert lib.helix_default_config(ctypes.byref(l), ctypes.byref(cfg)) == 0
+        need = lib.helix_workspace_bytes(ctypes.byref(l))
+        l.cfg = cfg
+        assert need == lib.helix_workspace_bytes(ctypes.byref(l))      # what the reported configuration asks for
+        return cfg, need
+
+    for c, ldc in ((0, 0), (4096, 128), (4096, 136)):
+        cfg, need = plan(c, ldc)
+        assert cfg.swap_ab == 1 and cfg.stream_k == 0 and need == 0
+    for c, ldc, stride in ((4096, 129, 0), (4098, 128, 0), (4096, 128, 21020 * 128 + 4)):
+        cfg, need = plan(c, ldc, stride)
+        assert cfg.swap_ab == 0 and cfg.stream_k == 1 and need > 0

@@ -457,3 +457,24 @@ def test_conv_on_both_sides_of_its_operand_choice(oracle, geom):
     util.assert_f16_close(got[:1], y32, f"conv {geom}")
     gather = _run(x, w, stride, pad, ops.make_cfg(OP_CONV_F16, tile_m=128, tile_n=128, tile_k=64, conv_gather=1))
     util.assert_f16_close(got, gather.astype(np.float32), f"conv {geom} against gathering")
+
+
+@pytest.mark.parametrize("geom", [(3, 96, 26, 26, 256, 5, 5, 1, 2), (4, 80, 30, 30, 128, 5, 5, 1, 2), (32, 128, 28, 28, 128, 3, 3, 1, 1)])
+def test_an_output_off_16_bytes_is_planned_as_it_runs(geom):
+    """Such an output cannot be stored by TMA: no channel blocks, no transposed tiles, and the workspace is that of what runs."""
+    nb, c, h, w, ko, r, _, stride, pad = geom
+    x = torch.randn((nb, h, w, c), device="cuda", dtype=torch.float16)
+    f = torch.randn((ko, r, r, c), device="cuda", dtype=torch.float16) * 0.05
+    flat = torch.full((nb * h * w * ko + 8,), 7.0, device="cuda", dtype=torch.float16)
+    y = flat[1:1 + nb * h * w * ko].view(nb, h, w, ko)
+    l = ops.launch_conv2d_f16(x, f, y, stride, pad)
+    ops.run(l)
+    l.cfg = ops.default_config(l)
+    own = torch.zeros_like(flat)
+    l.c = own[1:].data_ptr()
+    ops.run(l)                                       # the reported configuration, with the workspace that was planned
+    torch.cuda.synchronize()
+    ops.check_status()
+    assert torch.equal(own[1:1 + y.numel()], y.view(-1)) and bool((flat[1 + y.numel():] == 7.0).all()) and float(flat[0]) == 7.0
+    ref = torch.nn.functional.conv2d(x.double().permute(0, 3, 1, 2), f.double().permute(0, 3, 1, 2), stride=stride, padding=pad)
+    assert float((y.double().permute(0, 3, 1, 2) - ref).norm() / ref.norm()) < 2.0 ** -11     # one rounding to half on fp32 sums
