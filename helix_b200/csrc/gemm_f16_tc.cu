@@ -343,7 +343,8 @@ __device__ __forceinline__ void mma_issue_loop(const GemmParams& p, const int ct
 // How whole tiles leave: by TMA stores of 32 rows (or directly, where neither that nor the others apply), rows of C that a TMA
 // store cannot write, swapped tiles by transposed TMA stores.  Variants of their own: as branches beside the TMA store
 // the others made chains of short launches 2 % slower.
-// LEAN: whole tiles only, one issuing warp, no probes and no timeline -- what most launches are.  The code that is left out
+// LEAN: whole tiles only, one issuing warp, no probes and no timeline -- what most launches are (a timeline is taken of the
+// general variant).  The code that is left out
 // is not run by them, but a launch of a few us starts with a cold instruction cache and pays for what lies in between.
 enum TileOut { kOutRows = 0, kOutAny = 1, kOutColumns = 2 };
 template <int BN, bool CONV, int OUT, bool LEAN, int BLK>
@@ -1821,12 +1822,13 @@ static int launch_common(const helix_cfg_t& cfg, bool conv, const CUtensorMap& t
   const bool any = !p.swap && !p.tma_store, columns = p.swap && p.tma_store;
   // (narrow tiles are stored directly, and swapped ones among them keep the general variant)
   const bool lean = (bn >= 64 ? p.tma_store : !p.swap) && !p.stream_k && p.split_k <= 1 && !p.dual && p.probe == 0 && !p.trace;
-  if (p.blocks && !lean) return HELIX_ERR_UNSUPPORTED;   // conv_block() asks for nothing that needs another variant
+  // conv_block() asks for whole tiles without probes only
+  if (p.blocks && !lean && !(p.trace && p.tma_store)) return HELIX_ERR_UNSUPPORTED;
   cudaError_t e = cudaErrorInvalidValue;
   auto go = [&](auto width, auto gather, auto out, auto slim) {
     constexpr int kBN = decltype(width)::value, kOut = decltype(out)::value;
     constexpr bool kConv = decltype(gather)::value, kSlim = decltype(slim)::value;
-    if constexpr (!kConv && kSlim && kBN >= 64)
+    if constexpr (!kConv && kOut != kOutAny && kBN >= 64)
       if (p.blocks) {
         constexpr int kSide = kOut == kOutColumns ? -1 : 1;
         return p.g.C % 32 == 0 ? launch_variant<kBN, kConv, kOut, kSlim, 32 * kSide>(ta, tb, tc, p, grid, smem, stream)
@@ -1923,14 +1925,13 @@ int gemm_f16_launch(const helix_cfg_t* cfg_in, const void* A, int64_t lda, const
   return launch_common(cfg, false, ta, tb, p, C, ldc, sc, ws, ws_bytes, sm_count, independent, stream, launches);
 }
 
-// Channels of the blocks that pixels arrive by instead of slabs of 64 or gathering, 0: no blocks.  Only where the launch runs a lean variant
-// (whole tiles, no probes, no timeline, an output that TMA can store); geometries that slabs serve as well, for 128-wide and wider tiles, or C =
+// Channels of the blocks that pixels arrive by instead of slabs of 64 or gathering, 0: no blocks.  Only for whole tiles without probes and an
+// output that TMA can store, i.e. where the launch runs a lean variant (or its timeline is taken); geometries that slabs serve as well, for 128-wide and wider tiles, or C =
 // 96 in 64-wide ones on half the SMs and more (2 x 22 x 19, -> 208, 8 tiles: 6.25 / 6.5; 7 x 37 x 38 -> 64, 75 tiles: 7.1 / 6.9).
 static int conv_block(const helix_cfg_t& cfg, const ConvGeom& g, const void* y, int sm_count) {
-  const bool lean = cfg.tile_n >= 64 && !cfg.stream_k && cfg.split_k <= 1 && !(cfg.probe & 0x8f) && cfg.conv_gather != 1 &&
-                    (reinterpret_cast<uintptr_t>(y) & 15) == 0 && !(cfg.swap_ab && g.KO <= 64 && !(cfg.probe & 0x100)) &&
-                    gemm_f16_trace_for_grid(1) == nullptr;
-  if (!lean) return 0;
+  const bool whole = cfg.tile_n >= 64 && !cfg.stream_k && cfg.split_k <= 1 && !(cfg.probe & 0x8f) && cfg.conv_gather != 1 &&
+                     (reinterpret_cast<uintptr_t>(y) & 15) == 0 && !(cfg.swap_ab && g.KO <= 64 && !(cfg.probe & 0x100));
+  if (!whole) return 0;
   if (cfg.tile_n == 64 && conv_im2col_eligible(g)) {
     const int64_t M = (int64_t)g.NB * g.Ho * g.Wo, rows = cfg.swap_ab ? g.KO : M, cols = cfg.swap_ab ? M : g.KO;
     if (g.C > 96 || ((rows + kBM - 1) / kBM) * ((cols + 63) / 64) * 2 < sm_count) return 0;

@@ -450,7 +450,7 @@ def time_launches(launches, warmup=3, iters=20, use_graph=False):
 def capture_timeline(launch, warm=2):
     """Run `launch` (a one-CTA fp16 GEMM / convolution) with timeline capture on and return an int64
     array [CTAs, words] of the stamps described at helix_trace_buffer; rows of CTAs that did not run
-    stay zero."""
+    stay zero.  The stamps are those of the kernel's general variant: `launch` without capture may run a leaner one."""
     lib = _lib.load()
     words = lib.helix_trace_words_per_cta()
     ctas = device_info().sm_count

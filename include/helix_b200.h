@@ -282,7 +282,8 @@ int helix_gemv_f16_static(const void* W, int64_t ldw, const void* X, int64_t ldx
  * 20 work items of the CTA, six clock64 stamps: first / last load request, MMA issue start / end,
  * epilogue start / end; then, for the CTA's first 32 K slabs, the clock64 at which each was
  * requested (32 words) and at which the MMA issuer found it loaded (32 words).  Later launches
- * overwrite earlier ones.  Pass NULL to switch capture off (the default). */
+ * overwrite earlier ones.  Captured launches run the general variant of their kernel (the same operands, schedule and
+ * bits); without a buffer, whole tiles run one that leaves out this and other code, and is faster where launches are short.  Pass NULL to switch capture off (the default). */
 int helix_trace_buffer(void* device_buf, size_t bytes);
 int helix_trace_words_per_cta(void);
 
