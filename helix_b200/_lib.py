@@ -76,6 +76,7 @@ SIGNATURES = {
     "helix_get_config": (_I, [_I, _I, ctypes.POINTER(Cfg)]),
     "helix_default_config": (_I, [ctypes.POINTER(Launch), ctypes.POINTER(Cfg)]),
     "helix_workspace_bytes": (_Z, [ctypes.POINTER(Launch)]),
+    "helix_conv_pixel_channels": (_I, [ctypes.POINTER(Launch)]),
     "helix_launch": (_I, [ctypes.POINTER(Launch), _P, _P]),
     "helix_gemm_f16": (_I, [ctypes.POINTER(Cfg), _P, _L, _P, _L, _P, _L, _I, _I, _I, _I, _L, _L, _L, _P, _Z, _P, _P]),
     "helix_gemv_f16": (_I, [ctypes.POINTER(Cfg), _P, _L, _P, _L, _P, _L, _L, _I, _I, _I, _P, _Z, _P, _P]),

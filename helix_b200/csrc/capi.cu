@@ -316,6 +316,22 @@ size_t helix_workspace_bytes(const helix_launch_t* l) {
   }
 }
 
+int helix_conv_pixel_channels(const helix_launch_t* l) {
+  if (!l || l->op != HELIX_OP_CONV_F16) return HELIX_ERR_INVALID;
+  const helix::ConvGeom g = conv_geom(l->conv);
+  helix_cfg_t cfg = l->cfg;
+  if (cfg.tile_m == 0) {
+    const int rc = helix_default_config(l, &cfg);
+    if (rc != HELIX_OK) return rc;
+  }
+  const bool own_kernel = g.C == 4 || cfg.conv_gather >= 3 || (g.R == 1 && g.S == 1 && g.stride == 1 && g.pad == 0);
+  if (own_kernel || g.Ho <= 0 || g.Wo <= 0) return HELIX_ERR_INVALID;
+  helix_devinfo_t info;
+  int sms = (query_device(-1, &info) == HELIX_OK) ? info.sm_count : 148;
+  if (l->cfg.max_ctas > 0) sms = std::max(2, std::min(sms, l->cfg.max_ctas));
+  return helix::conv_f16_pixel_channels(cfg, g, l->c, sms);
+}
+
 int helix_launch(const helix_launch_t* launch, void* status_dev, void* stream) {
   return dispatch(launch, status_dev, static_cast<cudaStream_t>(stream));
 }

@@ -1189,25 +1189,30 @@ typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-static EncodeIm2colFn get_encode_im2col_fn() {
+// `lacking`: there is a driver and it has no such function (planning without a driver plans for one that has it)
+static EncodeIm2colFn get_encode_im2col_fn(bool* lacking = nullptr) {
   static EncodeIm2colFn fn = nullptr;
+  static bool none = false;
   static std::once_flag once;
   std::call_once(once, [] {
     void* sym = nullptr;
     cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &sym, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeIm2colFn>(sym);
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &sym, cudaEnableDefault, &qres) == cudaSuccess) {
+      none = qres != cudaDriverEntryPointSuccess;
+      if (!none) fn = reinterpret_cast<EncodeIm2colFn>(sym);
+    }
   });
+  if (lacking) *lacking = none;
   return fn;
 }
 
 // Window parameters inside the fields of an im2col tensor map, pixels on 16 bytes, and an input that is worth the map's set-up.
 static bool conv_map_possible(const ConvGeom& g) {
   const int64_t bytes = (int64_t)g.NB * g.H * g.W * g.C * 2;
+  bool lacking;
+  (void)get_encode_im2col_fn(&lacking);
   return (g.C % 8) == 0 && g.stride >= 1 && g.stride <= 8 && g.pad <= 127 && g.R <= 128 && g.S <= 128 &&
-         g.pad - (g.R - 1) >= -128 && g.pad - (g.S - 1) >= -128 && bytes >= 131072 && g.C <= 65535 &&
-         get_encode_im2col_fn() != nullptr;
+         g.pad - (g.R - 1) >= -128 && g.pad - (g.S - 1) >= -128 && bytes >= 131072 && g.C <= 65535 && !lacking;
 }
 
 // The im2col path reads 64-channel blocks of one filter tap (one 128-byte swizzled row per pixel; the last block of a
@@ -1939,6 +1944,13 @@ static int conv_block(const helix_cfg_t& cfg, const ConvGeom& g, const void* y, 
   return conv_block_channels(g);
 }
 
+// Channels of a tap that one box of the im2col map brings per pixel: 64 (slabs), 32 or 16 (blocks); 0 where warps gather.
+int conv_f16_pixel_channels(const helix_cfg_t& cfg, const ConvGeom& g, const void* y, int sm_count) {
+  if (cfg.conv_gather == 1) return 0;
+  const int block = conv_block(cfg, g, y, sm_count);
+  return block ? block : conv_im2col_eligible(g) ? kBK : 0;
+}
+
 // The library's choice for an output at y: what a launch without a configuration runs, and what planning reports and sizes.
 void conv_f16_default_config(const ConvGeom& g, const void* y, int sm_count, helix_cfg_t* out) {
   const bool tma_c = gemm_f16_tma_writes(y, g.KO, 0, 1, g.KO);
@@ -1988,7 +2000,6 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     if (own.conv_gather == 4)
       return conv_f16_rows_launch(x, w, y, g, 0, status_dev, sm_count, independent, stream, launches);
   }
-  const bool gather_forced = cfg_in && cfg_in->tile_m != 0 && cfg_in->conv_gather == 1;
   helix_cfg_t cfg;
   if (cfg_in && cfg_in->tile_m != 0) {
     cfg = *cfg_in;
@@ -2000,7 +2011,8 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     }
   }
   if (cfg.tile_m != kBM || cfg.cta_group > 1) return HELIX_ERR_UNSUPPORTED;
-  const bool im2col = !gather_forced && (conv_im2col_eligible(g) || conv_block(cfg, g, y, sm_count) != 0);
+  const int channels = conv_f16_pixel_channels(cfg, g, y, sm_count);
+  const bool im2col = channels != 0, blocks = im2col && channels < kBK;
   if (cfg.swap_ab) {
     // Output channels on the 128-row axis, pixels on the tile's wide axis: the tensor core takes
     // about the same time for a 128 x N x 16 step whatever N <= 256, so few output channels are
@@ -2017,15 +2029,15 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     ps.wtaps = g.C % kBK != 0;
     CUtensorMap tw, tx;
     int rcs;
-    if (const int blk = conv_block(cfg, g, y, sm_count)) {
-      ps.blocks = K / blk;
+    if (blocks) {
+      ps.blocks = K / channels;
       ps.K = K;
       ps.wtaps = 0;
       if ((rcs = make_tmap(&tw, w, K, g.KO, 1, K, 0, kBM)) != HELIX_OK) return rcs;
     } else if ((rcs = make_tmap_filter(&tw, w, g, kBM)) != HELIX_OK) {
       return rcs;
     }
-    if ((rcs = make_tmap_im2col(&tx, x, g, cfg.tile_n, ps.blocks ? K / ps.blocks : kBK)) != HELIX_OK) return rcs;
+    if ((rcs = make_tmap_im2col(&tx, x, g, cfg.tile_n, channels)) != HELIX_OK) return rcs;
     return launch_common(cfg, false, tw, tx, ps, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
   }
   GemmParams p{};
@@ -2044,15 +2056,15 @@ int conv_f16_launch(const helix_cfg_t* cfg_in, const void* x, const void* w, voi
     p.K = im2col_k(g);
     p.im2col = 1;
     p.wtaps = g.C % kBK != 0;
-    if (const int blk = conv_block(cfg, g, y, sm_count)) {
-      p.blocks = K / blk;
+    if (blocks) {
+      p.blocks = K / channels;
       p.K = K;
       p.wtaps = 0;
       if ((rc = make_tmap(&tb, w, K, g.KO, 1, K, 0, cfg.tile_n)) != HELIX_OK) return rc;
     } else if ((rc = make_tmap_filter(&tb, w, g, cfg.tile_n)) != HELIX_OK) {
       return rc;
     }
-    if ((rc = make_tmap_im2col(&ta, x, g, kBM, p.blocks ? K / p.blocks : kBK)) != HELIX_OK) return rc;
+    if ((rc = make_tmap_im2col(&ta, x, g, kBM, channels)) != HELIX_OK) return rc;
     return launch_common(cfg, false, ta, tb, p, y, N, 0, ws, ws_bytes, sm_count, independent, stream, launches);
   }
   if ((rc = make_tmap(&tb, w, K, N, 1, K, 0, cfg.tile_n)) != HELIX_OK) return rc;

@@ -74,6 +74,7 @@ bool gemm_f16_tma_writes(const void* C, int64_t ldc, int64_t sc, int M, int N);
 void gemm_f16_default_config(int M, int N, int K, int batch, int sm_count, bool tma_c, helix_cfg_t* out);
 void conv_f16_default_config(const ConvGeom& g, const void* y, int sm_count, helix_cfg_t* out);
 int64_t conv_f16_gemm_k(const ConvGeom& g);
+int conv_f16_pixel_channels(const helix_cfg_t& cfg, const ConvGeom& g, const void* y, int sm_count);
 // ---- conv_f32.cu (FFMA GEMM over the windows, gathered by its loader or through a column matrix)
 size_t conv_f32_workspace_bytes(const ConvGeom& g);
 int conv_f32_launch(const helix_cfg_t* cfg, const float* x, const float* w, float* y, const ConvGeom& g, void* ws,

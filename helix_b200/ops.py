@@ -148,18 +148,24 @@ def kernel_name(launch):
         if rows_geom and c.conv_gather == 4:    # explicit, or the library's default for this geometry
             return "conv_f16_rows_kernel"
         as_gemm = r == 1 and s == 1 and stride == 1 and pad == 0
-        im2col = conv_reads_tensor_map(n, h, w, ch, stride, ko, r, s, pad) and not c.conv_gather
-        # blocks of 32 or 16 channels (conv_block in csrc/gemm_f16_tc.cu)
-        blocks = (not c.conv_gather and c.tile_n >= 64 and not c.stream_k and c.split_k <= 1 and r * s > 1 and ko > 32 and
-                  ko % 8 == 0 and n * h * w * ch * 2 >= 131072 and stride <= 8 and
-                  (ch % 64 == 32 and ch < 256 if ch % 32 == 0 else ch % 16 == 0 and ch <= 256))
-        gathers = not as_gemm and not im2col and not blocks
+        if c.conv_gather >= 3 and not as_gemm:
+            return "conv_f16_win_kernel" if c.conv_gather == 3 else "conv_f16_rows_kernel"
+        gathers = not as_gemm and conv_pixel_channels(launch) == 0
     return "gemm_f16_tc_kernel<%d,%d>" % (c.tile_n, 1 if gathers else 0)
 
 
+def conv_pixel_channels(launch):
+    """Channels of a filter tap that an fp16 convolution's kernel fetches per pixel through the im2col tensor map (64, 32 or 16), or
+    0 where warps gather its pixels (helix_conv_pixel_channels)."""
+    n = _lib.load().helix_conv_pixel_channels(ctypes.byref(launch))
+    if n < 0:
+        check(n, "helix_conv_pixel_channels")
+    return n
+
+
 def conv_reads_tensor_map(n, h, w, ch, stride, ko=0, r=1, s=1, pad=0):
-    """True where the implicit GEMM fetches its input through the im2col tensor map (conv_im2col_eligible in
-    csrc/gemm_f16_tc.cu): the channels a 64-channel block is filled up with must be few and, where ch is no multiple of 16,
+    """True where the implicit GEMM may fetch its input through the im2col tensor map in slabs of 64 channels (conv_im2col_eligible in
+    csrc/gemm_f16_tc.cu; conv_pixel_channels says what a launch does): the channels a 64-channel block is filled up with must be few and, where ch is no multiple of 16,
     the layer small (`ko` output channels of an r x s filter)."""
     filled = (ch + 63) // 64 * 64
     few = filled * 3 <= ch * 4 if ch % 32 == 0 else filled * 5 <= ch * 6 and ch >= 96

@@ -97,8 +97,8 @@ typedef struct helix_cfg {
                       4 = row-pair kernel (3 x 3, stride 1, pad 1, 64 -> 64 channels, W <= 62: pixels on
                       the accumulator rows, window and all weights resident; the library's own choice
                       for that geometry when W >= 46 and there are at least three row pairs per SM).
-                      With swap_ab = 1 (im2col geometries only) the output channels take the
-                      128-row axis and tile_n pixels the other one                          */
+                      With swap_ab = 1 (geometries of the tensor map only, in slabs of 64 channels or in blocks) the
+                      output channels take the 128-row axis and tile_n pixels the other one  */
   int max_ctas;  /* > 0: the launch spreads over at most this many SMs (also honoured when the rest of
                     the struct is zero, i.e. with the library's own choice): lets two independent
                     launches on two streams share the machine, each with longer-lived CTAs      */
@@ -176,6 +176,11 @@ int helix_default_config(const helix_launch_t* launch, helix_cfg_t* out);
  * or the geometry then selects may leave it unread (streaming GEMVs and skinny products, fp32
  * convolutions without a column matrix). */
 size_t helix_workspace_bytes(const helix_launch_t* launch);
+
+/* How an fp16 convolution's pixels reach shared memory under launch->cfg (or the library's choice, when zeroed): 64, 32
+ * or 16 = through the im2col tensor map, so many channels of a filter tap at a time; 0 = gathered by warps.
+ * HELIX_ERR_INVALID for other operators and for convolutions that run as a GEMM (1 x 1) or have a kernel of their own. */
+int helix_conv_pixel_channels(const helix_launch_t* launch);
 
 /* Queue one launch.  Generic form of the four typed entry points below. */
 int helix_launch(const helix_launch_t* launch, void* status_dev, void* stream);
