@@ -146,11 +146,12 @@ def gemm_time(prof_dict, key, M, N, K, batch=1, conv=False, overlapped=False, op
     sms = _param(prof_dict, "sm_count", DEFAULT_SMS)
     pm, pn = (N, M) if swap else (M, N)
     # the library's own rules, which the slab figures cannot express: a tile twice as wide as the problem does the
-    # narrower tile's work at a wider tile's price, and swapping operands only pays when the row count is the skinny
-    # dimension (a convolution's swapped tile is covered above)
+    # narrower tile's work at a wider tile's price, and swapping operands pays when the row count is the skinny
+    # dimension or, in whole tiles of 128 and more rows per tile, where N fills its 128-row blocks and C can be stored
+    # transposed (default_config_impl in csrc/gemm_f16_tc.cu; a convolution's swapped tile is covered above)
     if bn > 16 and bn // 2 >= pn:
         return float("inf")
-    if swap and not conv and M > 64:
+    if swap and not conv and M > 64 and not (mode == 0 and bn >= 128 and M > TILE_M and N > TILE_M // 2 and N % 8 == 0):
         return float("inf")
     if group == 2:
         if conv or swap or mode or pm <= tm or K < 8 * TILE_K:   # short K is epilogue bound: pairs gain nothing
@@ -235,11 +236,12 @@ def gemv_time(prof_dict, key, rows, K, m):
     return t_fixed + bytes_ * s_per_byte * growth
 
 
-def cost_model(prof_dict, M, N, K, batch=1, conv=False, overlapped=False, operand_bytes=None):
+def cost_model(prof_dict, M, N, K, batch=1, conv=False, overlapped=False, operand_bytes=None, walks=None):
     """Best configuration key for C[M,N] = A[M,K] * B[N,K]^T; first element 0 means GEMV.
 
     Same call shape as the reference's cost_model(prof_dict, M, N, K)
-    (Ampere_FP16_gemm.py:420-430), but K and the batch count enter the estimate.
+    (Ampere_FP16_gemm.py:420-430), but K and the batch count enter the estimate.  `walks`: the configurations of a
+    convolution that read its pixels through the tensor map in blocks of less than 64 channels, with the K they walk.
     """
     best_key, best = None, float("inf")
     for key in prof_dict:
@@ -251,7 +253,9 @@ def cost_model(prof_dict, M, N, K, batch=1, conv=False, overlapped=False, operan
             rows, m = (N, M) if M <= N else (M, N)
             t = gemv_time(prof_dict, key, rows, K, m)
         else:
-            t = gemm_time(prof_dict, key, M, N, K, batch, conv, overlapped, operand_bytes)
+            in_blocks = bool(walks) and key in walks
+            t = gemm_time(prof_dict, key, M, N, walks[key] if in_blocks else K, batch, "im2col" if in_blocks else conv, overlapped,
+                          operand_bytes)
         if t < best:
             best, best_key = t, key
     return best_key

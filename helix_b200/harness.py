@@ -367,6 +367,22 @@ def gemv_passes_time(M, N, K, cfg=None):
     return avg * (-(-M // 8))
 
 
+def conv_block_walks(prof_dict, batch, C, H, W, OC, kH, kW, stride, pad):
+    """{key: reduction length} of the configurations that bring this convolution's pixels in blocks of 32 or 16 channels, which
+    need no filling up to 64 and serve swapped tiles too.  The library says which they are."""
+    walks = {}
+    l = ops.Launch()
+    l.op = OP_CONV_F16
+    for i, v in enumerate((batch, H, W, C, OC, kH, kW, stride, pad)):
+        l.conv[i] = v
+    for key in prof_dict:
+        if len(key) == 6 and key[0] != 0 and key[3] == 1:
+            l.cfg = key_to_cfg(key, conv=True)
+            if ops.conv_pixel_channels(l) in (16, 32):
+                walks[key] = kH * kW * C
+    return walks
+
+
 def conv_f16_result(prof_dict, batch, IC, H, W, OC, kH, kW, stride, pad):
     """(cost_ms, tflops) of one NHWC convolution as a single implicit GEMM
     (get_Ampere_FP16_conv_Helix_result, Ampere_FP16_conv.py:431-446: im2col time + GEMM time)."""
@@ -381,10 +397,11 @@ def conv_f16_result(prof_dict, batch, IC, H, W, OC, kH, kW, stride, pad):
     im2col = ops.conv_reads_tensor_map(batch, H, W, C, stride, OC, kH, kW, pad)
     # the convolution harness times one buffer set with ordered launches: a lone launch
     real_bytes = 2.0 * (batch * H * W * C + OC * kH * kW * C + M * N)        # x, w and y once each
-    # through the map the kernel walks whole 64-channel blocks of every tap
+    # through the map in slabs the kernel walks whole 64-channel blocks of every tap
     Kw = kH * kW * (-(-C // 64) * 64) if im2col and not as_gemm else (K + 7) // 8 * 8
-    key = costmodel.cost_model(prof_dict, M, N, Kw, 1,
-                               conv=False if as_gemm else ("im2col" if im2col else True), operand_bytes=real_bytes)
+    walks = {} if as_gemm else conv_block_walks(prof_dict, batch, C, H, W, OC, kH, kW, stride, pad)
+    key = costmodel.cost_model(prof_dict, M, N, Kw, 1, conv=False if as_gemm else ("im2col" if im2col else True),
+                               operand_bytes=real_bytes, walks=walks)
     if key is None or key[0] == 0:
         key = (costmodel.max_stages(128), 128, 128, 1, 0, 0)
     t = time_conv_f16(batch, IC, H, W, OC, kH, kW, stride, pad, key_to_cfg(key, conv=True, prof_dict=prof_dict))
