@@ -19,7 +19,8 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(CSRC, "_obj")
 LIB_PATH = os.path.join(PKG_DIR, "libhelix_b200.so")
 SOURCES = ["capi.cu", "gemv_f16.cu", "sgemm_f32.cu", "gemm_f16_tc.cu", "gemm_f16_tc2.cu", "conv_f16_halo.cu", "conv_f16_stem.cu", "conv_f16_rows.cu", "conv_f32.cu", "gemv_f32.cu"]
-HEADERS = ["common.cuh", "conv_common.cuh", "sgemm_f32_ring.cuh", "kernels.h", os.path.join("..", "..", "include", "helix_b200.h")]
+ABI_HEADER = os.path.join("..", "..", "include", "helix_b200.h")
+HEADERS = ["common.cuh", "conv_common.cuh", "sgemm_f32_ring.cuh", "kernels.h", ABI_HEADER]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 
@@ -33,17 +34,20 @@ def _build_eager():
     import torch
     home = os.path.dirname(torch.__file__)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"] +
+    tmp = EAGER_PATH + ".tmp"
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+            f'-DHELIX_TORCH_VERSION="{torch.__version__}"'] +
            ["-I" + d for d in (os.path.join(home, "include"), os.path.join(home, "include", "torch", "csrc", "api", "include"),
                                os.path.join(cuda, "include"), sysconfig.get_paths()["include"])] +
-           [EAGER_SRC, "-o", EAGER_PATH, "-L" + os.path.join(home, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+           [EAGER_SRC, "-o", tmp, "-L" + os.path.join(home, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
     stamp = os.path.join(OBJ_DIR, "eager_call.sha")
-    dig = _digest([EAGER_SRC, os.path.join(CSRC, HEADERS[-1])], " ".join(cmd) + torch.__version__)
+    dig = _digest([EAGER_SRC, os.path.join(CSRC, ABI_HEADER)], " ".join(cmd))
     if os.path.exists(EAGER_PATH) and os.path.exists(stamp) and open(stamp).read() == dig:
         return
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed for eager_call.cpp:\n{res.stdout}\n{res.stderr}")
+    os.replace(tmp, EAGER_PATH)         # a process that has the old one mapped keeps it
     with open(stamp, "w") as f:
         f.write(dig)
 

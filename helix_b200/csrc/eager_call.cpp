@@ -267,4 +267,17 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_eager_call", nullptr, -1, methods
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__eager_call(void) { return PyModule_Create(&module); }
+// Tensors are read through the C++ headers of one torch: under another version the module refuses to be imported.
+PyMODINIT_FUNC PyInit__eager_call(void) {
+  Ref torch, version;
+  torch.p = PyImport_ImportModule("torch");
+  version.p = torch.p ? PyObject_GetAttrString(torch.p, "__version__") : nullptr;
+  const char* now = version.p && PyUnicode_Check(version.p) ? PyUnicode_AsUTF8(version.p) : nullptr;
+  if (!now) {
+    if (!PyErr_Occurred()) PyErr_SetString(PyExc_ImportError, "torch has no version");
+    return nullptr;
+  }
+  if (std::strcmp(now, HELIX_TORCH_VERSION) != 0)
+    return PyErr_Format(PyExc_ImportError, "built for torch %s, not %s", HELIX_TORCH_VERSION, now);
+  return PyModule_Create(&module);
+}

@@ -8,6 +8,7 @@ kernels: fp16 GEMM takes A[M,K] and B stored [N,K]; fp32 GEMM takes A[M,K] (or
 K x M with ``trans_a``) and B[K,N].
 """
 import ctypes
+import warnings
 
 import torch
 
@@ -19,16 +20,32 @@ _workspaces = {}
 _eager = None
 
 
+class _PythonCalls:
+    """In the place of the native module where that cannot be imported: it covers nothing, and launches through ctypes."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+    @staticmethod
+    def run(launch):
+        dev = torch.cuda.current_device()
+        check(_lib.load().helix_launch(ctypes.byref(launch), status_word(dev).data_ptr(), _stream(dev)), "helix_launch")
+
+
 def _native():
     """The native form of the eager operators (csrc/eager_call.cpp): a call it does not cover returns None and goes through
-    the Python implementation below."""
+    the Python implementation below.  Without it (not built, or built for another torch, which it checks itself) every call does:
+    the same launches, some 8 us of host time more for each."""
     global _eager
     if _eager is None:
         lib = _lib.load()
         try:
             from . import _eager_call
         except ImportError as e:
-            raise ImportError("helix_b200/_eager_call is missing: build it with `python -m helix_b200.build`.") from e
+            warnings.warn(f"helix_b200/_eager_call is not used ({e}): eager operators go through ctypes, which is slower.  Build it "
+                          "with `python -m helix_b200.build`.", RuntimeWarning, stacklevel=3)
+            _eager = _PythonCalls()
+            return _eager
         _eager_call.connect(ctypes.cast(lib.helix_launch, ctypes.c_void_p).value,
                             ctypes.cast(lib.helix_workspace_bytes, ctypes.c_void_p).value,
                             _status_words, status_word, workspace, check)
