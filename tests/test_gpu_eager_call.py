@@ -1,6 +1,9 @@
 """Eager operators: the native call against the Python implementation it stands for, over the forms both accept and refuse."""
+import threading
+
 import pytest
 import torch
+from torch.overrides import TorchFunctionMode
 
 from helix_b200 import _lib, ops
 
@@ -93,6 +96,89 @@ def test_native_call_and_python_agree(monkeypatch, name):
     else:
         assert type(native) is type(python) and native.stride() == python.stride() and not native.requires_grad
         assert torch.equal(native, python)
+
+
+# what the native module must serve itself (or refuse, where the launch does); everything else it leaves to Python
+SERVES = {"gemv", "gemv rows apart", "gemv own output", "gemv transposed output", "gemv few rows, cut K", "gemv parameter",
+          "gemv one expanded vector", "gemv_f32", "gemm", "gemm batched", "gemm rows apart", "gemm workspace", "gemm one batch, expanded",
+          "gemm_f32", "gemm_f32 transposed", "conv", "conv strided own output", "conv_f32"}
+REFUSES = {"gemv unaligned", "gemv nine vectors"}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", list(CALLS))
+def test_native_call_serves_what_it_should(monkeypatch, name):
+    torch.manual_seed(3)
+    _w.update(w=_rand(300, 136), x=_rand(3, 136), long=_rand(64, 16384), longx=_rand(2, 16384), a=_rand(70, 136),
+              a3=_rand(2, 70, 136), b3=_rand(2, 72, 136), img=_rand(2, 9, 11, 8), flt=_rand(16, 3, 3, 8))
+    native, seen = ops._native(), []
+
+    class Watch:
+        def __getattr__(self, op):
+            def call(*args):
+                seen.append("refused")
+                got = getattr(native, op)(*args)
+                seen[-1] = "left" if got is None else "served"
+                return got
+            return native.run if op == "run" else call
+
+    monkeypatch.setattr(ops, "_native", Watch)
+    try:
+        CALLS[name]()
+    except Exception:
+        pass
+    torch.cuda.synchronize()
+    assert seen == ["served" if name in SERVES else "refused" if name in REFUSES else "left"]
+
+
+@pytest.mark.gpu
+def test_native_call_leaves_function_modes_to_python():
+    a, b = _rand(70, 136), _rand(300, 136)
+    plain, calls = ops.gemm_f16(a, b), []
+
+    class Mode(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            calls.append(func)
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        assert ops._native().gemm_f16(a, b, None) is None
+        got = ops.gemm_f16(a, b)
+    assert torch.equal(got, plain) and calls
+
+
+@pytest.mark.gpu
+def test_native_calls_follow_streams_and_threads():
+    a, b, w, x = _rand(70, 136), _rand(300, 136), _rand(300, 136), _rand(3, 136)
+    assert not ops.launch_gemm_f16(a, b, torch.empty(70, 300, device="cuda", dtype=torch.float16)).ws    # no scratch is shared
+    want = ops.gemm_f16(a, b), ops.gemv_f16(w, x)
+    zeros = torch.zeros_like(a)
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work():
+        try:
+            torch.cuda.set_device(0)
+            side = torch.cuda.Stream()
+            with torch.cuda.stream(side):
+                mine = torch.empty_like(a)
+                for _ in range(50):
+                    mine.copy_(zeros)                       # the product must come after these on this thread's stream
+                    torch.cuda._sleep(20000)
+                    mine.copy_(a)
+                    got = ops.gemm_f16(mine, b), ops.gemv_f16(w, x)
+                    side.synchronize()
+                    if not all(torch.equal(g, r) for g, r in zip(got, want)):
+                        wrong.append("differs")
+        except Exception as e:
+            wrong.append(repr(e))
+
+    threads = [threading.Thread(target=work) for _ in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
 
 
 @pytest.mark.gpu

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from helix_b200 import ops
+from helix_b200._lib import LAUNCH_INDEPENDENT
 
 pytestmark = pytest.mark.gpu
 
@@ -40,4 +41,31 @@ def test_deep_streams(rows, K, m):
         assert bool((out[:, m:] == 7.0).all()) if transposed else bool((out[:, rows:] == 7.0).all())
         if not ctas or m <= 8:     # a product of more rows may go to the tiles on a share of the machine
             results.append(y.clone())
+    assert all(torch.equal(results[0], r) for r in results[1:])
+
+
+# flagged products of nine and more rows, with the workspace (the library then holds the next launch back) and without it, which is
+# the only way to two CTAs on an SM; few rows (J = 4) and more, one block and several per CTA
+@pytest.mark.parametrize("rows,K,m", [(2400, 4608, 16), (1024, 8192, 11), (4884, 4112, 9), (14300, 1040, 16), (2400, 4368, 9)])
+def test_deep_streams_of_flagged_products(rows, K, m):
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(rows + m)
+    w = torch.empty((rows, K), dtype=torch.float16, device="cuda").normal_(0, 0.05, generator=gen)
+    x = torch.empty((m, K), dtype=torch.float16, device="cuda").normal_(0, 1, generator=gen)
+    ref = torch.matmul(x.double(), w.double().t())
+    results = []
+    for flag, scratch in ((0, True), (0, False), (LAUNCH_INDEPENDENT, True), (LAUNCH_INDEPENDENT, False)):
+        out = torch.full((m, rows + 3), 7.0, dtype=torch.float16, device="cuda")
+        l = ops.launch_gemm_f16(x, w, out[:, :rows])
+        assert l.ws and l.ws_bytes
+        if not scratch:
+            l.ws, l.ws_bytes = None, 0
+        l.flags = flag
+        torch.cuda.synchronize()
+        ops.run(l)
+        torch.cuda.synchronize()
+        # one rounding to half (2^-11) on top of fp32 sums
+        assert float((out[:, :rows].double() - ref).norm() / ref.norm()) < 2.0 ** -11
+        assert bool((out[:, rows:] == 7.0).all())
+        results.append(out)
     assert all(torch.equal(results[0], r) for r in results[1:])
