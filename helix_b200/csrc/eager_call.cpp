@@ -38,22 +38,21 @@ bool modes_active() {
   return at::impl::torch_function_mode_enabled() || c10::impl::TorchDispatchModeTLS::any_modes_set();
 }
 
-// The tensor behind `o` if it is a plain one on the current CUDA device, of this type and rank, with memory of its own and no
-// expanded dimension (a stride of 0 stands for "contiguous" in helix_launch_t).
+// The tensor behind `o` if it is a plain one on a CUDA device, of this type and rank, with memory of its own and no expanded
+// dimension (a stride of 0 stands for "contiguous" in helix_launch_t).
 const at::Tensor* plain(PyObject* o, at::ScalarType type, int64_t dim) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  if (!t.defined() || !t.is_cuda() || t.scalar_type() != type || t.dim() != dim || t.layout() != at::kStrided || !t.has_storage() ||
-      t.get_device() != c10::cuda::current_device())
+  if (!t.defined() || !t.is_cuda() || t.scalar_type() != type || t.dim() != dim || t.layout() != at::kStrided || !t.has_storage())
     return nullptr;
+  const at::IntArrayRef sizes = t.sizes(), strides = t.strides();
   for (int64_t i = 0; i < dim; ++i)
-    if (t.size(i) > INT_MAX || (t.size(i) > 1 && t.stride(i) == 0)) return nullptr;
+    if (sizes[i] > INT_MAX || (sizes[i] > 1 && strides[i] == 0)) return nullptr;
   return &t;
 }
 
-// Queues `l` on the current stream; false with a Python exception set.
-bool queue(helix_launch_t& l, bool own_workspace) {
-  const int dev = c10::cuda::current_device();
+// Queues `l` on the current stream of `dev`, the current device; false with a Python exception set.
+bool queue(helix_launch_t& l, bool own_workspace, int dev) {
   Ref key, made, ws;
   if (own_workspace) {
     const size_t need = g_workspace_bytes(&l);
@@ -91,9 +90,11 @@ bool queue(helix_launch_t& l, bool own_workspace) {
 
 PyObject* none() { Py_RETURN_NONE; }
 
-// `made` is the output when the caller brought none.
-PyObject* finish(helix_launch_t& l, PyObject* out, at::Tensor&& made) {
-  if (!queue(l, true)) return nullptr;
+// `made` is the output when the caller brought none; a, b and c are all on the current device or the call is not covered.
+PyObject* finish(helix_launch_t& l, PyObject* out, at::Tensor&& made, const at::Tensor* a, const at::Tensor* b, const at::Tensor* c) {
+  const int dev = c10::cuda::current_device();
+  if (a->get_device() != dev || b->get_device() != dev || c->get_device() != dev) return none();
+  if (!queue(l, true, dev)) return nullptr;
   if (out != Py_None) {
     Py_INCREF(out);
     return out;
@@ -123,7 +124,7 @@ PyObject* gemv(PyObject* const* args, Py_ssize_t nargs, int op, at::ScalarType t
   l.M = static_cast<int>(m); l.N = static_cast<int>(rows); l.K = static_cast<int>(w->size(1));
   l.lda = w->stride(0); l.ldb = x->stride(0);
   l.ldc = y->stride(0); l.ldc_inner = y->stride(1);
-  return finish(l, args[2], std::move(made));
+  return finish(l, args[2], std::move(made), w, x, y);
   END_HANDLE_TH_ERRORS
 }
 PyObject* gemv_f16(PyObject*, PyObject* const* args, Py_ssize_t nargs) { return gemv(args, nargs, HELIX_OP_GEMV_F16, at::kHalf); }
@@ -158,7 +159,7 @@ PyObject* gemm_f16(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   l.M = static_cast<int>(M); l.N = static_cast<int>(N); l.K = static_cast<int>(a->size(dim - 1));
   l.lda = a->stride(dim - 2); l.ldb = b->stride(dim - 2); l.ldc = c->stride(dim - 2);
   if (dim == 3) { l.stride_a = a->stride(0); l.stride_b = b->stride(0); l.stride_c = c->stride(0); }
-  return finish(l, args[2], std::move(made));
+  return finish(l, args[2], std::move(made), a, b, c);
   END_HANDLE_TH_ERRORS
 }
 
@@ -188,7 +189,7 @@ PyObject* gemm_f32(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   l.M = static_cast<int>(M); l.N = static_cast<int>(N); l.K = static_cast<int>(K);
   l.lda = a->stride(0); l.ldb = b->stride(0); l.ldc = c->stride(0);
   l.trans_a = ta ? 1 : 0;
-  return finish(l, args[3], std::move(made));
+  return finish(l, args[3], std::move(made), a, b, c);
   END_HANDLE_TH_ERRORS
 }
 
@@ -220,7 +221,7 @@ PyObject* conv2d(PyObject* const* args, Py_ssize_t nargs, int op, at::ScalarType
   l.a = x->data_ptr(); l.b = w->data_ptr(); l.c = y->data_ptr();
   const int64_t geom[9] = {x->size(0), H, W, x->size(3), w->size(0), R, S, stride, pad};
   for (int i = 0; i < 9; ++i) l.conv[i] = static_cast<int>(geom[i]);
-  return finish(l, args[4], std::move(made));
+  return finish(l, args[4], std::move(made), x, w, y);
   END_HANDLE_TH_ERRORS
 }
 PyObject* conv2d_f16(PyObject*, PyObject* const* args, Py_ssize_t nargs) { return conv2d(args, nargs, HELIX_OP_CONV_F16, at::kHalf); }
@@ -239,7 +240,7 @@ PyObject* run(PyObject*, PyObject* launch) {
   helix_launch_t l;
   std::memcpy(&l, view.buf, sizeof(l));
   PyBuffer_Release(&view);
-  if (!queue(l, false)) return nullptr;
+  if (!queue(l, false, c10::cuda::current_device())) return nullptr;
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }

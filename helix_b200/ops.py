@@ -59,9 +59,9 @@ def _require_cuda(*tensors):
     for t in tensors:
         if not t.is_cuda:
             raise ValueError("helix_b200 operators take CUDA tensors only (there is no CPU path)")
-        if t.device != tensors[0].device:
+        if t.get_device() != tensors[0].get_device():
             raise ValueError(f"operands on different devices: {tensors[0].device} and {t.device}")
-        if any(n > 1 and st == 0 for n, st in zip(t.shape, t.stride())):
+        if 0 in t.stride() and any(n > 1 and st == 0 for n, st in zip(t.shape, t.stride())):
             raise ValueError("expanded operands (a stride of 0) are not supported: make them contiguous")
 
 

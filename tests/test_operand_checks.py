@@ -35,6 +35,7 @@ def test_expanded_operands_are_refused(name):
 def _on(index, *shape):
     """What the checks read of a tensor on device `index`, which this machine may not have."""
     return types.SimpleNamespace(is_cuda=True, device=torch.device("cuda", index), shape=shape, dtype=H, dim=lambda: len(shape),
+                                 get_device=lambda: index,
                                  stride=lambda: (shape[-1], 1))
 
 
