@@ -374,14 +374,13 @@ def extras(peaks):
 
 
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum, averaged over the launches of one
-# pass over one copy of the sweep) for each kernel, from single-pass ncu captures; the capture commands are
-# in profiles/bench_sweep_launch_list.md.  Kernels that capture did not list report null.
+# pass over one copy of the sweep) for each kernel, from an ncu capture of each distinct unit by itself, with the
+# tile the sweep gives it; how it was taken stands in profiles/bench_sweep_launch_list.md.  Kernels that the
+# capture did not list report null.
 SWEEP_DRAM_BYTES_PER_LAUNCH = {
-    "gemm_f16_tc2_kernel<256>": 15810162, "gemm_f16_tc2_kernel<192>": 34526677,
-    "gemm_f16_tc_kernel<256,0>": 30764491, "gemm_f16_tc_kernel<64,0>": 68126530,
-    "gemm_f16_tc_kernel<128,0>": 14688633, "gemm_f16_tc_kernel<64,1>": 26433792,
-    "conv_f16_stem_kernel<4>": 13823700,   # profiles/conv_f16_stem_kernel_7x7_c3_224x224.md
-    "conv_f16_rows_kernel": 12970000,      # profiles/conv_f16_rows_kernel_3x3_c64_56x56.md
+    "gemm_f16_tc2_kernel<256>": 23538101, "gemm_f16_tc_kernel<256,0>": 22677876,
+    "gemm_f16_tc_kernel<64,0>": 100804898, "gemm_f16_tc_kernel<128,0>": 32304064,
+    "conv_f16_stem_kernel<4>": 12918528, "conv_f16_rows_kernel": 12960597,
 }
 
 
@@ -619,7 +618,7 @@ def bench_helix(args, rank, world, local_rank):
         "roofline": {"bound": "tensor", "achieved": tg["TFLOP/s"], "peak": peaks["tflops"], "unit": "TFLOP/s",
                      "frac": tg["TFLOP/s"] / peaks["tflops"],
                      "traffic": SWEEP_DRAM_BYTES_PER_LAUNCH.get(top),
-                     "traffic_source": "constant from a single-pass ncu capture of one sweep pass (profiles/bench_sweep_launch_list.md), not measured by this run",
+                     "traffic_source": "constant from an ncu capture of the sweep's distinct units (profiles/bench_sweep_launch_list.md), not measured by this run",
                      "kernel": top, "launches_per_copy": tg["launches"], "share_of_copy": tg["share"],
                      "us_per_launch": tg["us"] / tg["launches"],
                      "algorithmic_flop_per_launch": tg["flop"] / tg["launches"],
